@@ -9,6 +9,7 @@ import ctypes as C
 from pathlib import Path
 
 LIB_PATH = Path(__file__).resolve().parent / "_lib" / "libd2dmoe_b200.so"
+HOST_PATH = LIB_PATH.with_name("_d2d_torch.so")
 
 F32, BF16 = 0, 1
 ACT = {"relu": 0, "gelu": 1, "tanh": 2, "leaky_relu": 3, "gelu_tanh": 4}
@@ -72,6 +73,23 @@ def _load() -> C.CDLL:
 lib = _load()
 if lib.d2d_abi_version() != 2:
     raise ImportError("libd2dmoe_b200.so: ABI version mismatch")
+
+
+def _load_host():
+    """The native host path of the module forwards (csrc/d2d_torch.cpp)."""
+    import importlib.machinery
+    import importlib.util
+
+    import torch  # noqa: F401  (its libraries have to be loaded first)
+    if not HOST_PATH.exists():
+        raise ImportError(f"{HOST_PATH} not found: build it with `python d2dmoe_b200/build.py`")
+    loader = importlib.machinery.ExtensionFileLoader("_d2d_torch", str(HOST_PATH))
+    mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("_d2d_torch", loader))
+    loader.exec_module(mod)
+    return mod
+
+
+host = _load_host()
 
 
 def check(code: int, where: str) -> None:

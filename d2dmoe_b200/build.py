@@ -20,6 +20,8 @@ PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 LIBDIR = PKG / "_lib"
 LIB = LIBDIR / "libd2dmoe_b200.so"
+HOST_SRC = CSRC / "d2d_torch.cpp"        # native host path of the module forwards
+HOST_LIB = LIBDIR / "_d2d_torch.so"
 STAMP = LIBDIR / "build.stamp"
 
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -39,7 +41,7 @@ def sources() -> list[Path]:
 
 def _digest() -> str:
     h = hashlib.sha256()
-    for p in sorted(list(CSRC.glob("*.cu")) + list(CSRC.glob("*.cuh")) +
+    for p in sorted(list(CSRC.glob("*.cu")) + list(CSRC.glob("*.cuh")) + [HOST_SRC] +
                     [PKG.parent / "include" / "d2dmoe.h"]):
         h.update(p.name.encode())
         h.update(p.read_bytes())
@@ -48,7 +50,22 @@ def _digest() -> str:
 
 
 def is_current() -> bool:
-    return LIB.exists() and STAMP.exists() and STAMP.read_text().strip() == _digest()
+    return LIB.exists() and HOST_LIB.exists() and STAMP.exists() and STAMP.read_text().strip() == _digest()
+
+
+def _host_command(out: Path) -> list[str]:
+    """g++ command of the torch-facing host module, which calls the CUDA library's C ABI."""
+    import sysconfig
+
+    import torch
+    from torch.utils.cpp_extension import include_paths
+    torch_lib = Path(torch.__file__).parent / "lib"
+    inc = [f"-I{d}" for d in include_paths("cuda") + [sysconfig.get_paths()["include"]]]
+    return (["g++", "-O2", "-std=c++17", "-fPIC", "-shared",
+             f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"] + inc +
+            [str(HOST_SRC), "-o", str(out), f"-L{torch_lib}", "-ltorch_python", "-ltorch_cuda",
+             "-ltorch_cpu", "-lc10_cuda", "-lc10", f"-L{LIBDIR}", "-ld2dmoe_b200",
+             "-Wl,-rpath,$ORIGIN"])
 
 
 def build(force: bool = False, verbose: bool = False) -> Path:
@@ -77,6 +94,7 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     link = [_nvcc(), "-gencode", "arch=compute_100a,code=sm_100a", "-shared",
             "-Xcompiler", "-fPIC", "-o", str(LIB)] + [str(o) for o in objs]
     subprocess.run(link, check=True)
+    subprocess.run(_host_command(HOST_LIB), check=True)
     STAMP.write_text(_digest())
     return LIB
 

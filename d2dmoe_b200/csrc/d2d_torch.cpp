@@ -1,0 +1,284 @@
+// Native host path of the module forwards: one call from Python per layer call.
+//
+// A layer call launches three or four kernels that take 20 to 100 us together; preparing it in
+// Python (attribute walks, argument checks, thirty ctypes conversions) took 55 to 60 us, so every
+// call below about 10k tokens was bound by the host.  Here the facts that do not change between
+// calls (weight addresses, shapes, packed copies) are kept in a plan, and a call only checks that
+// the plan still describes the module, allocates the outputs and enters the C ABI.
+//
+// The plan never serves stale weights: each of its links names the dictionary slot a parameter or
+// sub-module sits in, and a call compares what is in the slot now (object, storage address, version
+// counter) with what the plan was made from.  A mismatch returns None and the caller makes a
+// new plan.
+#define PY_SSIZE_T_CLEAN
+#include <Python.h>
+
+#include <ATen/ATen.h>
+#include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <vector>
+
+#include "../../include/d2dmoe.h"
+
+namespace {
+
+struct Link {
+  PyObject* dict;      // slot holder; null: roots[root]
+  int root;
+  PyObject* key;
+  PyObject* obj;       // what the slot held when the plan was made
+  const void* data;    // tensors: storage address and version counter
+  int64_t version;
+  bool tensor;
+};
+
+struct Plan {
+  std::vector<Link> links;
+  at::Tensor hold[2];                  // packed router / experts images
+  const void *wa = nullptr, *wb = nullptr, *rp = nullptr;
+  const void *w1 = nullptr, *b1 = nullptr, *wup = nullptr, *w2 = nullptr, *ep = nullptr;
+  const void* last_bias = nullptr;
+  int64_t d = 0, R = 0, E = 0, H = 0, act = 0;
+  at::ScalarType dtype = at::kFloat;
+  c10::Device device = c10::Device(c10::kCUDA, 0);
+  ~Plan() {
+    for (Link& l : links) {
+      Py_XDECREF(l.dict);
+      Py_XDECREF(l.key);
+      Py_XDECREF(l.obj);
+    }
+  }
+};
+
+constexpr const char* kPlan = "d2dmoe_b200.plan";
+
+void plan_free(PyObject* cap) { delete static_cast<Plan*>(PyCapsule_GetPointer(cap, kPlan)); }
+
+const at::Tensor* tensor_of(PyObject* o) {
+  return o != nullptr && THPVariable_Check(o) ? &THPVariable_Unpack(o) : nullptr;
+}
+
+const void* ptr_of(PyObject* o) {
+  const at::Tensor* t = tensor_of(o);
+  return t ? t->data_ptr() : nullptr;
+}
+
+bool still_valid(const Plan& p, PyObject* const* roots) {
+  for (const Link& l : p.links) {
+    PyObject* now = PyDict_GetItemWithError(l.dict ? l.dict : roots[l.root], l.key);   // borrowed
+    if (now != l.obj) return false;
+    if (l.tensor) {
+      const at::Tensor& t = THPVariable_Unpack(now);
+      if (t.data_ptr() != l.data || t._version() != l.version) return false;
+    }
+  }
+  return !PyErr_Occurred();
+}
+
+// make_plan(links, (wa, wb, router_packed), (w1, b1, w_up, w2, experts_packed), last_bias, act)
+//   links: sequence of (holder, key); holder = a dict, or 0 / 1 for the module's own _modules /
+//   _parameters, which run_layer receives with every call (the plan does not refer to its module)
+PyObject* make_plan(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  if (n != 7) {
+    PyErr_SetString(PyExc_TypeError, "make_plan takes 7 arguments");
+    return nullptr;
+  }
+  auto p = std::make_unique<Plan>();
+  PyObject* const roots[2] = {a[5], a[6]};
+  PyObject* seq = PySequence_Fast(a[0], "links");
+  if (!seq) return nullptr;
+  for (Py_ssize_t i = 0; i < PySequence_Fast_GET_SIZE(seq); ++i) {
+    PyObject* it = PySequence_Fast_GET_ITEM(seq, i);
+    PyObject* holder = PyTuple_GetItem(it, 0);
+    PyObject* key = PyTuple_GetItem(it, 1);
+    if (!holder || !key) {
+      Py_DECREF(seq);
+      return nullptr;
+    }
+    Link l = {};
+    if (PyLong_Check(holder)) {
+      l.root = PyLong_AsLong(holder) == 1 ? 1 : 0;
+    } else {
+      Py_INCREF(holder);
+      l.dict = holder;
+    }
+    Py_INCREF(key);
+    l.key = key;
+    PyObject* now = PyDict_GetItemWithError(l.dict ? l.dict : roots[l.root], key);
+    Py_XINCREF(now);
+    l.obj = now;
+    if (const at::Tensor* t = tensor_of(now)) {
+      l.tensor = true;
+      l.data = t->data_ptr();
+      l.version = t->_version();
+    }
+    p->links.push_back(l);
+  }
+  Py_DECREF(seq);
+  PyObject *r = a[1], *e = a[2];
+  if (r != Py_None) {
+    const at::Tensor* wa = tensor_of(PyTuple_GetItem(r, 0));
+    TORCH_CHECK(wa, "router weight");
+    p->wa = wa->data_ptr();
+    p->wb = ptr_of(PyTuple_GetItem(r, 1));
+    p->R = wa->size(0);
+    if (const at::Tensor* t = tensor_of(PyTuple_GetItem(r, 2))) {
+      p->hold[0] = *t;
+      p->rp = t->data_ptr();
+    }
+  }
+  const at::Tensor* w1 = tensor_of(PyTuple_GetItem(e, 0));
+  TORCH_CHECK(w1 && w1->dim() == 3 && w1->is_cuda(), "expert weights");
+  p->w1 = w1->data_ptr();
+  p->b1 = ptr_of(PyTuple_GetItem(e, 1));
+  p->wup = ptr_of(PyTuple_GetItem(e, 2));
+  p->w2 = ptr_of(PyTuple_GetItem(e, 3));
+  if (const at::Tensor* t = tensor_of(PyTuple_GetItem(e, 4))) {
+    p->hold[1] = *t;
+    p->ep = t->data_ptr();
+  }
+  p->E = w1->size(0);
+  p->d = w1->size(1);
+  p->H = w1->size(2);
+  p->dtype = w1->scalar_type();
+  p->device = w1->device();
+  p->last_bias = ptr_of(a[3]);
+  p->act = PyLong_AsLong(a[4]);
+  if (PyErr_Occurred()) return nullptr;
+  return PyCapsule_New(p.release(), kPlan, plan_free);
+  END_HANDLE_TH_ERRORS
+}
+
+// buffers of one call: ops.Workspace of (tokens, experts, device), from the module's cache
+struct Buffers {
+  void *mask, *idx, *off, *ws, *status;
+  size_t ws_bytes;
+};
+
+PyObject* s_get;      // "raw"
+
+bool buffers_of(PyObject* cache, const Plan& p, int64_t N, Buffers* b) {
+  // the cache is a dictionary (tokens, experts, device index) -> Workspace with a miss handler
+  PyObject* key = Py_BuildValue("(LLi)", (long long)N, (long long)p.E, (int)p.device.index());
+  if (!key) return false;
+  PyObject* w = PyDict_GetItemWithError(cache, key);       // borrowed
+  PyObject* made = nullptr;
+  if (!w && !PyErr_Occurred()) w = made = PyObject_GetItem(cache, key);   // __missing__ allocates
+  Py_DECREF(key);
+  if (!w) return false;
+  PyObject* raw = PyObject_GetAttr(w, s_get);               // bytes: five addresses and a size
+  Py_XDECREF(made);                                         // the cache keeps it
+  if (!raw) return false;
+  const bool ok = PyBytes_Check(raw) && PyBytes_GET_SIZE(raw) == 48;
+  if (ok) {
+    uint64_t v[6];
+    memcpy(v, PyBytes_AS_STRING(raw), 48);
+    *b = {(void*)v[0], (void*)v[1], (void*)v[2], (void*)v[3], (void*)v[4], (size_t)v[5]};
+  } else {
+    PyErr_SetString(PyExc_TypeError, "workspace addresses");
+  }
+  Py_DECREF(raw);
+  return ok;
+}
+
+// run_layer(plan, modules, parameters, workspaces, x, tau, residual, scores, norm)
+//   -> (out, routing) | status code (int) | None: the plan does not fit this call
+// scores: None or [.., E] of x's dtype.  norm: None or (kind, gamma, beta|None, eps, gamma_offset):
+// x + layer(norm(x)).
+PyObject* run_layer(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  if (n != 9) {
+    PyErr_SetString(PyExc_TypeError, "run_layer takes 9 arguments");
+    return nullptr;
+  }
+  Plan* p = static_cast<Plan*>(PyCapsule_GetPointer(a[0], kPlan));
+  if (!p) return nullptr;
+  const at::Tensor* xp = tensor_of(a[4]);
+  if (!xp || !xp->is_cuda() || xp->scalar_type() != p->dtype || xp->device() != p->device ||
+      xp->dim() < 1 || xp->size(-1) != p->d || xp->numel() == 0 || !still_valid(*p, a + 1)) {
+    if (PyErr_Occurred()) return nullptr;
+    Py_RETURN_NONE;
+  }
+  const at::Tensor x = xp->contiguous();
+  const int64_t N = x.numel() / p->d;
+  const double tau = PyFloat_AsDouble(a[5]);
+  const int residual = PyObject_IsTrue(a[6]);
+  if (PyErr_Occurred()) return nullptr;
+  const float mult = (float)(1.0 - tau);
+  at::Tensor scores;
+  const bool given = a[7] != Py_None;
+  if (given) {
+    const at::Tensor* sp = tensor_of(a[7]);
+    if (!sp || !sp->is_cuda() || sp->scalar_type() != p->dtype || sp->device() != p->device ||
+        sp->numel() != N * p->E)
+      Py_RETURN_NONE;
+    scores = sp->contiguous();
+  } else if (!p->wa) {
+    Py_RETURN_NONE;
+  }
+  c10::cuda::CUDAGuard guard(p->device);
+  Buffers b;
+  if (!buffers_of(a[3], *p, N, &b)) return nullptr;
+  const auto stream = (d2d_stream_t)c10::cuda::getCurrentCUDAStream(p->device.index()).stream();
+  const int dt = p->dtype == at::kBFloat16 ? D2D_BF16 : D2D_F32;
+  const auto opts = x.options();
+  at::Tensor out = at::detail::empty_cuda(x.sizes(), opts);
+  c10::SmallVector<int64_t, 5> rs(x.sizes().begin(), x.sizes().end());
+  rs.back() = p->E;
+  at::Tensor rt = at::detail::empty_cuda(rs, opts);
+  const void* xin = x.data_ptr();
+  const void* lb = p->last_bias;
+  int res = residual ? 1 : 0, rc = D2D_OK;
+  at::Tensor xn;
+  if (a[8] != Py_None) {
+    PyObject* nm = a[8];
+    xn = at::detail::empty_cuda(x.sizes(), opts);
+    const long kind = PyLong_AsLong(PyTuple_GetItem(nm, 0));
+    const double eps = PyFloat_AsDouble(PyTuple_GetItem(nm, 3));
+    const double goff = PyFloat_AsDouble(PyTuple_GetItem(nm, 4));
+    if (PyErr_Occurred()) return nullptr;
+    const at::Tensor* gt = tensor_of(PyTuple_GetItem(nm, 1));
+    const at::Tensor* bt = tensor_of(PyTuple_GetItem(nm, 2));
+    TORCH_CHECK(gt && gt->numel() == p->d && (!bt || bt->numel() == p->d), "norm parameters");
+    const at::Tensor g = gt->contiguous(), bb = bt ? bt->contiguous() : at::Tensor();
+    rc = d2d_prenorm_init(xin, g.data_ptr(), bt ? bb.data_ptr() : nullptr, (float)eps, (int)kind,
+                          (float)goff, lb, xn.data_ptr(), out.data_ptr(), N, (int)p->d, dt, stream);
+    xin = xn.data_ptr();
+    lb = nullptr;
+    res = D2D_OUT_PREINITIALISED;
+  }
+  if (rc == D2D_OK)
+    rc = d2d_moe_forward(xin, given ? nullptr : p->wa, given ? nullptr : p->wb,
+                         given ? nullptr : p->rp, given ? scores.data_ptr() : nullptr, mult, p->w1,
+                         p->b1, p->wup, p->w2, p->ep, lb, res, out.data_ptr(), (uint32_t*)b.mask,
+                         (int32_t*)b.idx, (int32_t*)b.off, N, (int)p->d, (int)p->R, (int)p->E,
+                         (int)p->H, (int)p->act, dt, b.ws, b.ws_bytes, (int*)b.status,
+                         rt.data_ptr(), stream);
+  if (rc != D2D_OK) return PyLong_FromLong(rc);
+  PyObject* res_t = PyTuple_New(2);
+  if (!res_t) return nullptr;
+  PyTuple_SET_ITEM(res_t, 0, THPVariable_Wrap(std::move(out)));
+  PyTuple_SET_ITEM(res_t, 1, THPVariable_Wrap(std::move(rt)));
+  return res_t;
+  END_HANDLE_TH_ERRORS
+}
+
+PyMethodDef kMethods[] = {
+    {"make_plan", (PyCFunction)(void (*)(void))make_plan, METH_FASTCALL, nullptr},
+    {"run_layer", (PyCFunction)(void (*)(void))run_layer, METH_FASTCALL, nullptr},
+    {nullptr, nullptr, 0, nullptr}};
+
+PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_d2d_torch", nullptr, -1, kMethods,
+                       nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__d2d_torch(void) {
+  s_get = PyUnicode_InternFromString("raw");
+  return PyModule_Create(&kModule);
+}

@@ -26,6 +26,7 @@ import torch
 from torch import nn
 
 from . import ops
+from ._capi import ACT, D2DError, host
 
 ACTIVATION_TO_NAME = {nn.GELU: "gelu", nn.Tanh: "tanh", nn.ReLU: "relu", nn.LeakyReLU: "leaky_relu"}
 
@@ -56,21 +57,41 @@ def _uniform_init(p: torch.Tensor) -> torch.Tensor:
     return p
 
 
-class _WorkspaceCache:
-    """Per-module cache of caller-owned buffers, keyed by (tokens, device)."""
-
-    def __init__(self):
-        self._w = {}
+class _WorkspaceCache(dict):
+    """Per-module cache of caller-owned buffers: (tokens, experts, device index) -> Workspace."""
 
     def get(self, n: int, E: int, device) -> ops.Workspace:
-        key = (n, E, str(device))
-        w = self._w.get(key)
-        if w is None:
-            if len(self._w) > 8:
-                self._w.clear()
-            w = ops.Workspace.allocate(n, E, device)
-            self._w[key] = w
+        device = torch.device(device)
+        i = device.index
+        return self[(n, E, torch.cuda.current_device() if i is None else i)]
+
+    def __missing__(self, key):
+        n, E, index = key
+        if len(self) > 8:
+            self.clear()
+        w = self[key] = ops.Workspace.allocate(n, E, torch.device("cuda", index))
         return w
+
+    def __deepcopy__(self, memo):
+        return _WorkspaceCache()
+
+    def __reduce__(self):
+        return _WorkspaceCache, ()
+
+
+class _Plan:
+    """Holder of a layer's native call plan (csrc/d2d_torch.cpp); copies start without one."""
+
+    __slots__ = ("handle",)
+
+    def __init__(self):
+        self.handle = None
+
+    def __deepcopy__(self, memo):
+        return _Plan()
+
+    def __reduce__(self):
+        return _Plan, ()
 
 
 class _PackedCache:
@@ -392,6 +413,7 @@ class MoeficationMoE(MoELayer):
         self.tau = None
         self.add_residual_connection = add_residual_connection
         self._wsp = _WorkspaceCache()
+        self._plan = _Plan()
 
     # -- routing for the modes that are not fused ---------------------------------
     def gate(self, x):
@@ -419,8 +441,84 @@ class MoeficationMoE(MoELayer):
         else:
             ops.mask_from_scores(s2, self.tau, wsp)
 
-    @torch.no_grad()
+    # -- native call path -----------------------------------------------------------
+    def _make_plan(self):
+        """Plan of the one-call layer for the parameters as they are now, or None when the
+        modules are not the plain ones of this file or not on a GPU."""
+        ex, router = self.experts, self.router
+        if type(ex) not in (B200KernelExperts, B200GluExperts) or router is None:
+            return None
+        p = ex.kernel_params()
+        if not p["w1"].is_cuda:
+            return None
+        links = [(0, "experts"), (0, "router"), (1, "last_bias")]
+        if type(ex) is B200GluExperts:
+            links.append((ex._modules, "layers"))
+            for i in ("0", "1", "2"):
+                links += [(ex.layers._modules, i), (ex.layers._modules[i]._parameters, "w")]
+        else:
+            links += [(ex._parameters, k) for k in ("w1", "b1", "w2")]
+        r = None
+        if type(router) is MoeficationRouter and router.fusable():
+            wa, wb = router.layers[0].weight, router.layers[2].weight
+            if wa.dtype != p["w1"].dtype or wa.device != p["w1"].device:
+                return None
+            links.append((router._modules, "layers"))
+            for i in ("0", "2"):
+                links += [(router.layers._modules, i),
+                          (router.layers._modules[i]._parameters, "weight")]
+            r = (wa, wb, router.packed())
+        tensors = [t for t in (p["w1"], p["b1"], p["w_up"], p["w2"]) if t is not None]
+        if self.bias:
+            tensors.append(self.last_bias)
+        if any(t.dtype != p["w1"].dtype or t.device != p["w1"].device or not t.is_contiguous()
+               for t in tensors + list(r[:2] if r else ())):
+            return None
+        return host.make_plan(links, r, (p["w1"], p["b1"], p["w_up"], p["w2"], ex.packed()),
+                              self.last_bias if self.bias else None, ACT[p["act"]],
+                              self._modules, self._parameters)
+
+    def _run_native(self, x, residual, scores=None, norm=None):
+        """The layer as one native call -> (out, routing tensor), or None when it has to take
+        the general path."""
+        for _ in range(2):
+            h = self._plan.handle
+            if h is not None:
+                r = host.run_layer(h, self._modules, self._parameters, self._wsp, x, self.tau,
+                                   residual, scores, norm)
+                if type(r) is tuple:
+                    return r
+                if r is not None:
+                    raise D2DError(r, "d2d_moe_forward")
+            with torch.no_grad():
+                self._plan.handle = self._make_plan()
+            if self._plan.handle is None:
+                return None
+        return None
+
     def forward(self, x):
+        ex = self._modules["experts"]
+        if (self.forward_mode == "dynk_max" and x.is_cuda and ex._capture is None
+                and ex._forward_mode in _KERNEL_MODES):
+            router = self._modules.get("router")
+            r = None
+            if router is not None:
+                if type(router) is MoeficationRouter and router._fusable:
+                    r = self._run_native(x, self.add_residual_connection)
+                else:
+                    with torch.no_grad():
+                        s = router(x)
+                    r = self._run_native(x, self.add_residual_connection, s)
+                    if r is None:
+                        return self._forward_general(x, s)
+            if r is not None:
+                return r[0], {self.name: (r[1],)}
+        return self._forward_general(x)
+
+    @torch.no_grad()
+    def _forward_general(self, x, s=None):
+        """The layer through the stage-level entry points; ``s``: the router's output on ``x``
+        where it has been computed already."""
         if not x.is_cuda:
             raise RuntimeError("d2dmoe_b200 runs on CUDA tensors only (there is no CPU path)")
         self.experts._check_mode()
@@ -450,7 +548,7 @@ class MoeficationMoE(MoELayer):
         elif self.forward_mode == "dynk_max" and not capture:
             # any other router: its scores come from device tensor ops, the rule and the
             # rest of the layer from the library
-            s = self.router(x)
+            s = self.router(x) if s is None else s
             s2 = s.reshape(N, E).contiguous()
             rt = torch.empty(N, E, dtype=s.dtype, device=x.device)
             ops.moe_forward(x2d, None, None, self.tau, p["w1"], p["b1"], p["w2"], p["act"], out,
@@ -488,9 +586,10 @@ class MoeficationMoE(MoELayer):
         parameters, torch's RMSNorm, and Gemma-style RMSNorm modules (weight applied as
         1 + weight, transformers GemmaRMSNorm)."""
         if isinstance(norm, nn.LayerNorm):
-            if norm.weight is None or len(norm.normalized_shape) != 1:
+            w = norm.weight
+            if w is None or len(norm.normalized_shape) != 1:
                 return None
-            return ops.NORM_LAYER, norm.weight, norm.bias, float(norm.eps), 0.0
+            return ops.NORM_LAYER, w, norm.bias, float(norm.eps), 0.0
         name = type(norm).__name__
         if "RMSNorm" in name and getattr(norm, "weight", None) is not None:
             eps = getattr(norm, "eps", None)
@@ -501,7 +600,6 @@ class MoeficationMoE(MoELayer):
             return ops.NORM_RMS, norm.weight, None, float(eps), 1.0 if "Gemma" in name else 0.0
         return None
 
-    @torch.no_grad()
     def forward_block(self, x, norm):
         """``x + self(norm(x))``: the second half of an upstream transformer block
         (architectures/moe/moe_models.py:69-76 ViT, :91-100 GPT, :148-156 Gemma:
@@ -511,39 +609,25 @@ class MoeficationMoE(MoELayer):
         outputs to that.  Returns ``(x + out, {name: (routing_tensor,)})``.  Falls back to the
         three separate steps when the layer is not in its fused form."""
         na = self._norm_args(norm)
+        ex, router = self._modules["experts"], self._modules.get("router")
         # (affine parameters in another dtype than x -- mixed-precision norms -- keep the
         # framework's own normalisation: the fused pass computes in the dtype of x)
         fused = (na is not None and x.is_cuda and self.forward_mode == "dynk_max"
                  and na[1].dtype == x.dtype and (na[2] is None or na[2].dtype == x.dtype)
                  and na[1].device == x.device
-                 and getattr(self.experts, "_capture", None) is None
-                 and isinstance(self.router, MoeficationRouter) and self.router.fusable()
+                 and getattr(ex, "_capture", None) is None
+                 and isinstance(router, MoeficationRouter) and router.fusable()
                  and not self.add_residual_connection
                  and (x.size(-1) * x.element_size()) % 16 == 0
                  and x.size(-1) * x.element_size() <= 8192 and x.numel() > 0)
-        if not fused:
+        if fused:
+            ex._check_mode()
+            r = self._run_native(x, False, None, na)
+            if r is not None:
+                return r[0], {self.name: (r[1],)}
+        with torch.no_grad():
             y, gd = self.forward(norm(x))
             return x + y, gd
-        self.experts._check_mode()
-        kind, gamma, beta, eps, goff = na
-        orig_size = x.size()
-        E = self.num_experts
-        x2d = x.reshape(-1, x.size(-1)).contiguous()
-        N = x2d.size(0)
-        p = self.experts.kernel_params()
-        xn = torch.empty_like(x2d)
-        out = torch.empty_like(x2d)
-        rt = torch.empty(N, E, dtype=x.dtype, device=x.device)
-        wsp = self._wsp.get(N, E, x.device)
-        ops.prenorm_init(x2d, gamma.detach().contiguous(),
-                         None if beta is None else beta.detach().contiguous(), eps, kind, xn, out,
-                         last_bias=self.last_bias.view(-1) if self.bias else None,
-                         gamma_offset=goff)
-        ops.moe_forward(xn, self.router.layers[0].weight, self.router.layers[2].weight, self.tau,
-                        p["w1"], p["b1"], p["w2"], p["act"], out, wsp, w_up=p["w_up"],
-                        add_residual=ops.OUT_PREINITIALISED, router_packed=self.router.packed(),
-                        experts_packed=self.experts.packed(), routing_out=rt)
-        return out.view(orig_size), {self.name: (rt.view(*orig_size[:-1], E),)}
 
     @torch.no_grad()
     def forward_host(self, x_host: torch.Tensor, out_host: torch.Tensor | None = None,

@@ -7,6 +7,7 @@ the library.  CUDA tensors only: a CPU tensor raises.
 from __future__ import annotations
 
 import ctypes as C
+import struct
 from dataclasses import dataclass
 
 import numpy as np
@@ -87,6 +88,12 @@ class Workspace:
     offsets: torch.Tensor        # [E+1] int32
     ws: torch.Tensor             # bytes
     status: torch.Tensor         # [1] int32 device status word
+
+    def __post_init__(self):
+        # the addresses as the native host path reads them
+        self.raw = struct.pack("6Q", self.mask_bits.data_ptr(), self.token_idx.data_ptr(),
+                               self.offsets.data_ptr(), self.ws.data_ptr(), self.status.data_ptr(),
+                               self.ws.numel())
 
     @staticmethod
     def allocate(n: int, E: int, device) -> "Workspace":
