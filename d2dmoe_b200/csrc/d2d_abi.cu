@@ -58,8 +58,8 @@ int d2d_router_mask(const void* x, const void* wa, const void* wb, const void* r
   if (router_packed_opt && umma_router_supported(d, R, E, dtype) && aligned(x, 16) &&
       aligned(last_bias_opt, 16) && aligned(out_init_opt, 16) && aligned(router_packed_opt, 1024))
     return launch_router_mask_umma(x, router_packed_opt, thresh_mult, mask_bits, scores_opt,
-                                   nullptr, last_bias_opt, add_residual, out_init_opt, nullptr, N, d, R, E,
-                                   dev_status, s);
+                                   nullptr, last_bias_opt, add_residual ? x : nullptr, out_init_opt,
+                                   true, nullptr, N, d, R, E, dev_status, s);
   return launch_router_mask_simt(x, wa, wb, thresh_mult, mask_bits, scores_opt, last_bias_opt,
                                  add_residual, out_init_opt, N, d, R, E, dtype, dev_status, s);
 }
@@ -198,6 +198,7 @@ int d2d_moe_forward(const void* x, const void* wa, const void* wb, const void* r
                     d2d_stream_t stream) {
   int rc, nl = 0;
   bool counts_ready = false, rt_done = routing_tensor_opt == nullptr;
+  DirectRows dr;
   g_last_forward_launches = 0;
   if (!wa && !scores_in_opt) return D2D_ERR_BAD_ARG;
   if (!mask_bits || !token_idx || !offsets || !ws || !aligned(ws, 16)) return D2D_ERR_BAD_ARG;
@@ -217,6 +218,8 @@ int d2d_moe_forward(const void* x, const void* wa, const void* wb, const void* r
     add_residual = 0;
     last_bias_opt = nullptr;
   }
+  const bool umma_experts = experts_packed_opt && aligned(experts_packed_opt, 1024) &&
+                            umma_experts_supported(d, E, H, w_up_opt != nullptr, dtype);
   if (scores_in_opt) {
     // rule + counts table + output init in one launch when the shape allows it
     rc = launch_gate_scores_fused(scores_in_opt, thresh_mult, mask_bits, routing_tensor_opt,
@@ -238,10 +241,17 @@ int d2d_moe_forward(const void* x, const void* wa, const void* wb, const void* r
     }
   } else if (router_packed_opt && wb && R >= 1 && umma_router_supported(d, R, E, dtype) &&
              aligned(last_bias_opt, 16) && aligned(router_packed_opt, 1024)) {
-    // the tensor-core router also fills the compaction's counts table
+    // the tensor-core router also fills the compaction's counts table; where the tensor-core
+    // expert kernel follows it leaves the rows of tokens with one expert to that kernel
+    const void* resid = add_residual ? x : nullptr;
+    if (!pre && !resid && umma_experts) {
+      dr.mask_bits = mask_bits;
+      dr.last_bias = last_bias_opt;
+    }
     rc = launch_router_mask_umma(x, router_packed_opt, thresh_mult, mask_bits, nullptr,
-                                 routing_tensor_opt, last_bias_opt, add_residual, out_init,
-                                 (int32_t*)ws, N, d, R, E, dev_status, (cudaStream_t)stream);
+                                 routing_tensor_opt, last_bias_opt, resid, out_init,
+                                 dr.mask_bits == nullptr, (int32_t*)ws, N, d, R, E, dev_status,
+                                 (cudaStream_t)stream);
     counts_ready = true;
     rt_done = true;
     nl += 1;
@@ -265,9 +275,12 @@ int d2d_moe_forward(const void* x, const void* wa, const void* wb, const void* r
     nl += 1;
   }
   g_last_forward_launches = nl + 1;
-  return d2d_experts_ffn(x, token_idx, offsets, w1, b1_opt, w_up_opt, w2, experts_packed_opt,
-                         nullptr, 0, /*accumulate=*/1, out, N, d, E, H, act, dtype, dev_status,
-                         stream);
+  if (umma_experts)
+    return launch_experts_umma(x, token_idx, offsets, experts_packed_opt, out, N, d, E, H,
+                               w_up_opt != nullptr, act, dev_status, (cudaStream_t)stream,
+                               NormCapture(), dr);
+  return launch_experts_simt(x, token_idx, offsets, w1, b1_opt, w_up_opt, w2, out, N, d, E, H, act,
+                             dtype, dev_status, (cudaStream_t)stream);
 }
 
 int d2d_last_forward_launches(void) { return g_last_forward_launches; }

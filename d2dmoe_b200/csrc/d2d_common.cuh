@@ -111,8 +111,31 @@ __device__ __forceinline__ void red_add_bf16x8(bf16* p, uint32_t a, uint32_t b, 
                "r"(c), "r"(d)
                : "memory");
 }
+// eight bf16 pairs-wise sums, each rounded once
+__device__ __forceinline__ uint4 add_bf16x8(uint4 a, uint4 b) {
+  uint4 r;
+  const __nv_bfloat162* x = reinterpret_cast<const __nv_bfloat162*>(&a);
+  const __nv_bfloat162* y = reinterpret_cast<const __nv_bfloat162*>(&b);
+  __nv_bfloat162* z = reinterpret_cast<__nv_bfloat162*>(&r);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) z[i] = __hadd2_rn(x[i], y[i]);
+  return r;
+}
 __device__ __forceinline__ void red_add_1(float* p, float a) { atomicAdd(p, a); }
 __device__ __forceinline__ void red_add_1(bf16* p, float a) { atomicAdd(p, __float2bfloat16_rn(a)); }
+
+// 32 x 32 bit matrix, one row per lane, turned over: bit i of lane b's result = bit b of lane i's
+// word (block swaps of size 16, 8, 4, 2, 1)
+__device__ __forceinline__ uint32_t transpose32(uint32_t x, int lane) {
+  uint32_t m = 0x0000ffffu;
+#pragma unroll
+  for (int j = 16; j > 0; j >>= 1) {
+    const uint32_t y = __shfl_xor_sync(0xffffffffu, x, j);
+    x = (lane & j) == 0 ? (x & m) | ((y & m) << j) : (x & ~m) | ((y >> j) & m);
+    m ^= m << (j >> 1);
+  }
+  return x;
+}
 
 __host__ __device__ __forceinline__ int ceil_div(int a, int b) { return (a + b - 1) / b; }
 __host__ __device__ __forceinline__ int64_t ceil_div64(int64_t a, int64_t b) { return (a + b - 1) / b; }
@@ -152,6 +175,9 @@ int launch_expand_mask(const uint32_t* mask_bits, void* rt, int64_t N, int E, in
                        cudaStream_t s);
 int launch_pack_mask(const void* rt, uint32_t* mask_bits, int64_t N, int E, int dtype,
                      cudaStream_t s);
+// SM count of the current device, and the dynamic shared memory opt-in of `kernel` on it (both
+// hold per device and are looked up once; safe from several host threads)
+int device_launch_facts(const void* kernel, size_t smem, int* sms);
 size_t compact_workspace_bytes(int64_t n_max, int E);
 int compact_row_cells(int E);      // cells (bytes) per row of the compaction's counts table
 // counts_ready: the byte table counts_ws[tile of 128 tokens][compact_row_cells(E)] is already

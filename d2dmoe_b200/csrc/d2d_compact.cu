@@ -45,13 +45,9 @@ compact_count_kernel(const uint32_t* __restrict__ mask_bits, uint8_t* __restrict
       w[r] = (t < N && j < nw) ? mask_bits[t * nw + j] : 0u;
     }
     int mine = 0;
-    const int nb = max(0, min(32, E - 32 * j));
-    for (int b = 0; b < nb; ++b) {
-      int cb = 0;
 #pragma unroll
-      for (int r = 0; r < 4; ++r) cb += __popc(__ballot_sync(0xffffffffu, (w[r] >> b) & 1u));
-      if (lane == b) mine = cb;
-    }
+    for (int r = 0; r < 4; ++r) mine += __popc(transpose32(w[r], lane));
+    if (32 * j + lane >= E) mine = 0;
     if (32 * j + lane < EP) counts[tile * EP + 32 * j + lane] = (uint8_t)mine;   // pads are 0
   }
 }
@@ -70,74 +66,80 @@ compact_scatter_kernel(const uint32_t* __restrict__ mask_bits, const uint8_t* __
   const int64_t t = (int64_t)chunk * CHUNK + w * 32 + lane;
 
   grid_launch_dependents();
-  for (int i = tid; i < ROWS * E; i += NTS) cnt[i] = 0;
   for (int e = tid; e < 2 * EP; e += NTS) tot[e] = 0;      // tot and pre are adjacent
   __syncthreads();
   grid_dependency_wait();      // mask and counts table come from the previous kernel
-  // this thread's mask words (warps 0..ROWS-1: one row of 32 tokens each); the loads are in
-  // flight during the table sweep and the words stay in registers for both passes
+  // this thread's mask words (one row of 32 tokens per warp); the loads are in flight during
+  // the table sweep and the words stay in registers for both passes
   uint32_t word[MAX_E / 32];
 #pragma unroll
   for (int j = 0; j < MAX_E / 32; ++j)
-    word[j] = (w < ROWS && j < nw && t < N) ? mask_bits[t * nw + j] : 0u;
+    word[j] = (j < nw && t < N) ? mask_bits[t * nw + j] : 0u;
   // sweep of the byte table: thread (tsub, g) adds up the 16 cells of group g over the tiles
-  // tsub, tsub + stride, ...; sums over all tiles and over the tiles before this chunk
+  // tsub, tsub + stride, ..., the ones before this chunk and the rest apart.  Cells are added as
+  // pairs of 16-bit halves (two instructions per four cells); a segment is short enough that
+  // neither a thread's sums nor the sums over a warp's lanes pass 65535.
   {
     const int G = EP >> 4;                      // 16-cell groups per table row (power of two)
     const int g = tid & (G - 1), tsub = tid / G, stride = NTS / G;
     const int first_tile = chunk * TILES_PER_CHUNK;
-    int a[16], b[16];
+    const int seg = (65535 / CTILE) * min(G, 32) / 32 / 4 * 4 * stride;
+    for (int s0 = 0; s0 < ntiles; s0 += seg) {
+      const int s1 = min(ntiles, s0 + seg);
+      uint32_t acc[2][8];                       // [earlier chunks, the rest][pairs]
 #pragma unroll
-    for (int q = 0; q < 16; ++q) a[q] = b[q] = 0;
-    for (int t0 = tsub; t0 < ntiles; t0 += 4 * stride) {
-      uint4 v[4];
+      for (int q = 0; q < 8; ++q) acc[0][q] = acc[1][q] = 0u;
+      for (int t0 = s0 + tsub; t0 < s1; t0 += 4 * stride) {
+        uint4 v[4];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {      // four independent loads in flight
-        const int tt = t0 + u * stride;
-        v[u] = tt < ntiles ? __ldg(reinterpret_cast<const uint4*>(counts + (int64_t)tt * EP) + g)
-                           : make_uint4(0u, 0u, 0u, 0u);
-      }
+        for (int u = 0; u < 4; ++u) {      // four independent loads in flight
+          const int tt = t0 + u * stride;
+          v[u] = tt < s1 ? __ldg(reinterpret_cast<const uint4*>(counts + (int64_t)tt * EP) + g)
+                         : make_uint4(0u, 0u, 0u, 0u);
+        }
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const uint32_t ww[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
-        const bool before = t0 + u * stride < first_tile;
+        for (int u = 0; u < 4; ++u) {
+          const uint32_t ww[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+          const uint32_t early = t0 + u * stride < first_tile ? 0xffffffffu : 0u;
 #pragma unroll
-        for (int q = 0; q < 16; ++q) {
-          const int c = (ww[q >> 2] >> (8 * (q & 3))) & 0xff;
-          a[q] += c;
-          if (before) b[q] += c;
+          for (int k = 0; k < 4; ++k) {
+            const uint32_t lo = ww[k] & 0x00ff00ffu, hi = (ww[k] >> 8) & 0x00ff00ffu;
+            acc[0][2 * k] += lo & early;
+            acc[0][2 * k + 1] += hi & early;
+            acc[1][2 * k] += lo & ~early;
+            acc[1][2 * k + 1] += hi & ~early;
+          }
         }
       }
-    }
-    // lanes that hold the same group (lane mod G equal) are added up by shuffles, then one
-    // lane per group and warp adds into shared memory
-    for (int o = 16; o >= G; o >>= 1) {
+      // lanes that hold the same group (lane mod G equal) are added up by shuffles, then one
+      // lane per group and warp adds into shared memory
+      for (int o = 16; o >= G; o >>= 1) {
 #pragma unroll
-      for (int q = 0; q < 16; ++q) {
-        a[q] += __shfl_xor_sync(0xffffffffu, a[q], o);
-        b[q] += __shfl_xor_sync(0xffffffffu, b[q], o);
+        for (int q = 0; q < 8; ++q) {
+          acc[0][q] += __shfl_xor_sync(0xffffffffu, acc[0][q], o);
+          acc[1][q] += __shfl_xor_sync(0xffffffffu, acc[1][q], o);
+        }
       }
-    }
-    if (lane < G && lane < 32) {
+      if (lane < G) {
 #pragma unroll
-      for (int q = 0; q < 16; ++q) {
-        if (a[q]) atomicAdd(&tot[16 * g + q], a[q]);
-        if (b[q]) atomicAdd(&pre[16 * g + q], b[q]);
+        for (int q = 0; q < 8; ++q)
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {         // cell of (pair q, half h)
+            const int c = 16 * g + 4 * (q >> 1) + (q & 1) + 2 * h;
+            const int b = (acc[0][q] >> (16 * h)) & 0xffff, r = (acc[1][q] >> (16 * h)) & 0xffff;
+            if (b) atomicAdd(&pre[c], b);
+            if (b + r) atomicAdd(&tot[c], b + r);
+          }
       }
     }
   }
-  // per-row popcounts of this chunk
+  // each warp turns its 32 tokens x 32 experts bit blocks over: lane b then holds the tokens of
+  // expert 32j + b as one word (5 shuffles instead of one ballot per expert and pass)
 #pragma unroll
   for (int j = 0; j < MAX_E / 32; ++j) {
-    if (j >= nw || w >= ROWS) break;
-    if (__ballot_sync(0xffffffffu, word[j] != 0u) == 0u) continue;
-    const int nb = min(32, E - 32 * j);
-    int mine = 0;
-    for (int b = 0; b < nb; ++b) {
-      const int cb = __popc(__ballot_sync(0xffffffffu, (word[j] >> b) & 1u));
-      if (lane == b) mine = cb;
-    }
-    if (lane < nb) cnt[w * E + 32 * j + lane] = mine;
+    if (j >= nw) break;
+    word[j] = transpose32(word[j], lane);
+    if (32 * j + lane < E) cnt[w * E + 32 * j + lane] = __popc(word[j]);
   }
   __syncthreads();
   // exclusive scan of the expert totals (E <= 256: one warp, 8 values per lane)
@@ -175,19 +177,13 @@ compact_scatter_kernel(const uint32_t* __restrict__ mask_bits, const uint8_t* __
     }
   }
   __syncthreads();
+  const int32_t row0 = (int32_t)(t - lane);
 #pragma unroll
   for (int j = 0; j < MAX_E / 32; ++j) {
-    if (j >= nw || w >= ROWS) break;
-    if (__ballot_sync(0xffffffffu, word[j] != 0u) == 0u) continue;
-    const int nb = min(32, E - 32 * j);
-    for (int b = 0; b < nb; ++b) {
-      const uint32_t bit = (word[j] >> b) & 1u;
-      const uint32_t v = __ballot_sync(0xffffffffu, bit);
-      if (bit) {
-        const int rank = __popc(v & ((1u << lane) - 1u));
-        token_idx[cnt[w * E + 32 * j + b] + rank] = (int32_t)t;
-      }
-    }
+    if (j >= nw) break;
+    if (32 * j + lane >= E) continue;
+    int32_t* dst = token_idx + cnt[w * E + 32 * j + lane];
+    for (uint32_t m = word[j]; m != 0u; m &= m - 1) *dst++ = row0 + __ffs(m) - 1;
   }
 }
 

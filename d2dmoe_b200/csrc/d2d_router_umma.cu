@@ -1,0 +1,538 @@
+// Router of the layer on the tensor cores (bf16): per 128 consecutive tokens
+//     s = |bf16(relu(bf16(x Wa^T)) Wb^T)|,  keep e iff s_e >= bf16(max s * mult)
+// (architectures/moe/moefication.py:328-330 and :80-85), written as mask bits, the 0/1 routing
+// tensor and the compaction's counts table; the same CTA writes the initial rows of the layer
+// output that the expert kernel will add to.
+//
+// One persistent CTA per SM, 16 warps, one 128-token tile after another:
+//   warp 10     one thread loads stages (a 128-row x 64-column TMA box of x and the matching 64-deep
+//               slice of Wa, one barrier for both) and, once, the whole of Wb
+//   warp  8     one thread issues x Wa^T (tcgen05, N = R in one instruction) into accumulator 1
+//   warps 0-3   accumulator 1 -> relu, bf16 -> hidden tile in TENSOR memory
+//   warp  9     one thread issues hidden Wb^T, its A operand read from tensor memory
+//   warps 4-7   scores -> row maximum, threshold, mask words, routing rows, counts
+//   warps 12-15 the tile's initial output rows
+//
+// Bound: HBM.  A layer reads x once; the initial rows are written only for tokens whose row
+// the expert kernel has to ADD to (more than one expert, or none): a token kept by exactly
+// one expert gets its row from that expert's store.  Compared with the form that shared its
+// tile loop with the expert kernel (hidden tile in shared memory, separate rings for x and Wa,
+// Wb streamed per tile, eight warps each doing both epilogues, every initial row written by the
+// TMA unit in front of the loads) the second epilogue no longer sits between two tiles.
+#include "d2d_tmap.cuh"
+#include "d2d_umma_api.cuh"
+#include "d2d_umma_ptx.cuh"
+
+namespace d2d {
+using namespace umma;
+namespace {
+
+constexpr int NTHREADS = 512;
+constexpr int WARP_MMA1 = 8, WARP_MMA2 = 9, WARP_LOAD = 10, WARP_INIT0 = 12;
+constexpr int NS_MAX = 8;                    // stages (upper bound)
+constexpr int MAX_E = 128;
+constexpr size_t SMEM_TILES = 220 * 1024;    // stages + Wb
+constexpr uint32_t TM_HID = 256, TM_ACC2 = 384;   // tensor-memory columns (accumulator 1 at 0)
+
+struct Geo {
+  int kc1;                  // d / 64
+  int nsub, nsubw;          // Wa packed as nsub blocks of nsubw rows per 64-deep slice
+  int kc2;                  // ceil(R / 64): 64-deep slices of Wb
+  int nd;                   // E rounded up to 16
+  int ns;                   // stages
+  int wa_bytes;             // Wa bytes per stage
+  long long w1_bytes, stride;
+};
+
+Geo router_geo(int d, int R, int E) {
+  Geo g;
+  g.kc1 = d / 64;
+  g.nsub = R > 128 ? 2 : 1;
+  g.nsubw = R / g.nsub;
+  g.kc2 = (R + 63) / 64;
+  g.nd = (E + 15) / 16 * 16;
+  g.wa_bytes = R * 128;
+  g.w1_bytes = (long long)g.kc1 * g.wa_bytes;
+  const long long wb = (long long)g.kc2 * g.nd * 128;
+  g.stride = (g.w1_bytes + wb + 512 + 1023) / 1024 * 1024;
+  const int ns = (int)((SMEM_TILES - wb) / (SLOT + (g.wa_bytes + 1023) / 1024 * 1024));
+  g.ns = ns < NS_MAX ? ns : NS_MAX;
+  return g;
+}
+
+struct Params {
+  long long N;
+  int d, R, E;
+  const uint8_t* packed;
+  Geo g;
+  float mult;
+  uint32_t* mask_bits;
+  bf16* scores;             // optional [N, E]
+  bf16* rt_out;             // optional: 0/1 routing tensor [N, E]
+  uint8_t* tile_counts;     // optional: bytes [tiles][EP], kept tokens per expert
+  int EP;
+  bf16* out_init;           // optional: initial output rows last_bias (+ resid)
+  const bf16* last_bias;
+  const bf16* resid;
+  int init_all;             // every row; 0: rows not kept by exactly one expert
+  int* dev_status;
+  uint32_t wait_limit;
+  int withhold;             // test hook: CTA 0 never loads its first weight slice
+};
+
+struct Ctl {
+  unsigned long long full[NS_MAX], empty[NS_MAX];
+  unsigned long long wb_full, acc1_full[2], acc1_empty[2], hid_full, g2_done, acc2_empty;
+  unsigned long long init_full[2], init_empty[2];
+  uint32_t tmem_base;
+  int abort_flag;
+  int wait_limit;           // must follow abort_flag (mbar_wait reads abort_flag[1])
+  int cnt[2][4][MAX_E];     // kept tokens per expert of a 32-token row group
+  uint32_t init_rows[2][4];
+};
+
+// bits i (even experts) and 16 + i (odd experts) -> bits 2i and 2i + 1
+__device__ __forceinline__ uint32_t interleave16(uint32_t v) {
+  uint32_t t = (v ^ (v >> 8)) & 0x0000ff00u;
+  v ^= t ^ (t << 8);
+  t = (v ^ (v >> 4)) & 0x00f000f0u;
+  v ^= t ^ (t << 4);
+  t = (v ^ (v >> 2)) & 0x0c0c0c0cu;
+  v ^= t ^ (t << 2);
+  t = (v ^ (v >> 1)) & 0x22222222u;
+  return v ^ t ^ (t << 1);
+}
+
+__device__ void role_load(const Params& p, Ctl* c, const CUtensorMap* tmx, uint32_t ring,
+                          uint32_t wb, uint32_t stage_bytes) {
+  volatile int* af = &c->abort_flag;
+  const Geo& g = p.g;
+  const int tiles = (int)((p.N + TILE_M - 1) / TILE_M);
+  const uint32_t wb_bytes = (uint32_t)(g.kc2 * g.nd * 128);
+  bool withheld = (p.withhold & 1) != 0 && blockIdx.x == 0;
+  RingPos r = {0, 0};
+  bool first = true;
+  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    for (int kc = 0; kc < g.kc1; ++kc) {
+      if (!mbar_wait_fast(smem_u32(&c->empty[r.s]), r.ph ^ 1, af, p.dev_status)) return;
+      const uint32_t bar = smem_u32(&c->full[r.s]), dst = ring + r.s * stage_bytes;
+      mbar_arrive_expect_tx(bar, SLOT + g.wa_bytes);
+      tma_load_2d(dst, tmx, kc * 64, tile * TILE_M, bar);
+      if (withheld) withheld = false;
+      else bulk_g2s(dst + SLOT, p.packed + (long long)kc * g.wa_bytes, g.wa_bytes, bar);
+      r.next(g.ns);
+    }
+    if (first) {           // after the first tile's stages: Wb is needed only behind its hidden tile
+      first = false;
+      const uint32_t bar = smem_u32(&c->wb_full);
+      mbar_arrive_expect_tx(bar, wb_bytes);
+      bulk_g2s(wb, p.packed + g.w1_bytes, wb_bytes, bar);
+    }
+  }
+}
+
+__device__ void role_mma1(const Params& p, Ctl* c, uint32_t ring, uint32_t stage_bytes,
+                          uint32_t tmem) {
+  volatile int* af = &c->abort_flag;
+  const Geo& g = p.g;
+  const int tiles = (int)((p.N + TILE_M - 1) / TILE_M);
+  const uint32_t idesc = instr_desc(TILE_M, p.R);
+  const uint64_t d0 = smem_desc(ring);
+  const uint32_t hi = (uint32_t)(d0 >> 32), lo0 = (uint32_t)d0;
+  const int nacc = p.R <= 128 ? 2 : 1;
+  RingPos r = {0, 0}, a = {0, 0};
+  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    if (!mbar_wait_fast(smem_u32(&c->acc1_empty[a.s]), a.ph ^ 1, af, p.dev_status)) return;
+    tc_fence_after();
+    const uint32_t acc = tmem + a.s * 128;
+    for (int kc = 0; kc < g.kc1; ++kc) {
+      if (!mbar_wait_fast(smem_u32(&c->full[r.s]), r.ph, af, p.dev_status)) return;
+      tc_fence_after();
+      const uint32_t alo = lo0 + r.s * (stage_bytes >> 4), blo = alo + (SLOT >> 4);
+#pragma unroll
+      for (uint32_t k = 0; k < 4; ++k)
+        umma_bf16(acc, ((uint64_t)hi << 32) | (alo + 2 * k), ((uint64_t)hi << 32) | (blo + 2 * k),
+                  idesc, (kc | k) != 0);
+      umma_commit(smem_u32(&c->empty[r.s]));
+      r.next(g.ns);
+    }
+    umma_commit(smem_u32(&c->acc1_full[a.s]));
+    a.next(nacc);
+  }
+}
+
+__device__ void role_mma2(const Params& p, Ctl* c, uint32_t wb, uint32_t tmem) {
+  volatile int* af = &c->abort_flag;
+  const Geo& g = p.g;
+  const int tiles = (int)((p.N + TILE_M - 1) / TILE_M);
+  const uint32_t idesc = instr_desc(TILE_M, g.nd);
+  const uint64_t d0 = smem_desc(wb);
+  const uint32_t hi = (uint32_t)(d0 >> 32), lo0 = (uint32_t)d0;
+  const int ksteps = p.R >> 4;
+  uint32_t ph = 0;
+  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ph ^= 1) {
+    if (tile == (int)blockIdx.x &&
+        !mbar_wait_fast(smem_u32(&c->wb_full), 0, af, p.dev_status))
+      return;
+    if (!mbar_wait_fast(smem_u32(&c->acc2_empty), ph ^ 1, af, p.dev_status)) return;
+    if (!mbar_wait_fast(smem_u32(&c->hid_full), ph, af, p.dev_status)) return;
+    tc_fence_after();
+    for (int k = 0; k < ksteps; ++k)
+      umma_bf16_ta(tmem + TM_ACC2, tmem + TM_HID + 8 * k,
+                   ((uint64_t)hi << 32) | (lo0 + (uint32_t)(k >> 2) * (g.nd * 8) + 2 * (k & 3)),
+                   idesc, k != 0);
+    umma_commit(smem_u32(&c->g2_done));
+  }
+}
+
+// warps 0-3, thread = tile row = TMEM lane: hidden tile = bf16 relu of accumulator 1
+__device__ void role_hidden(const Params& p, Ctl* c, uint32_t tmem, int et) {
+  volatile int* af = &c->abort_flag;
+  const int tiles = (int)((p.N + TILE_M - 1) / TILE_M);
+  const uint32_t lane_base = (uint32_t)(et & ~31) << 16;
+  const int nacc = p.R <= 128 ? 2 : 1;
+  RingPos a = {0, 0};
+  uint32_t ph = 0;
+  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ph ^= 1) {
+    if (!mbar_wait_fast(smem_u32(&c->acc1_full[a.s]), a.ph, af, p.dev_status)) return;
+    // the previous tile's second product has read the hidden tile
+    if (!mbar_wait_fast(smem_u32(&c->g2_done), ph ^ 1, af, p.dev_status)) return;
+    tc_fence_after();
+    const uint32_t src = tmem + lane_base + a.s * 128, dst = tmem + lane_base + TM_HID;
+    for (int c0 = 0; c0 < p.R; c0 += 16) {
+      uint32_t v[16], w[8];
+      tmem_ld16(src + c0, v);
+      tmem_wait_ld();
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        __nv_bfloat162 h =
+            __floats2bfloat162_rn(__uint_as_float(v[2 * q]), __uint_as_float(v[2 * q + 1]));
+        h = __hmax2(h, __float2bfloat162_rn(0.f));
+        w[q] = *reinterpret_cast<uint32_t*>(&h);
+      }
+      tmem_st8(dst + (c0 >> 1), w);
+    }
+    tmem_wait_st();
+    tc_fence_before();
+    mbar_arrive(smem_u32(&c->acc1_empty[a.s]));
+    mbar_arrive(smem_u32(&c->hid_full));
+    a.next(nacc);
+  }
+}
+
+// warps 4-7, thread = tile row: the row's scores stay in registers as packed bf16 pairs
+// (NB blocks of 16 experts), so tensor memory is read once and handed back at once
+template <int NB>
+__device__ void role_gate(const Params& p, Ctl* c, uint32_t tmem, int et) {
+  volatile int* af = &c->abort_flag;
+  const int tiles = (int)((p.N + TILE_M - 1) / TILE_M);
+  const int lane = et & 31, q4 = et >> 5, E = p.E;
+  constexpr int NW = (NB + 1) / 2;                    // mask words that can be non-zero
+  const int nw = (E + 31) >> 5;                       // == NW
+  const uint32_t lane_base = (uint32_t)(et & ~31) << 16;
+  uint32_t ph = 0, buf = 0, ibuf_ph = 0;
+  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ph ^= 1, buf ^= 1) {
+    const long long trow = (long long)tile * TILE_M + et;
+    const bool live = trow < p.N;
+    if (!mbar_wait_fast(smem_u32(&c->g2_done), ph, af, p.dev_status)) return;
+    tc_fence_after();
+    uint32_t s[NB * 8];
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+      uint32_t v[16];
+      tmem_ld16(tmem + lane_base + TM_ACC2 + 16 * b, v);
+      tmem_wait_ld();
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const __nv_bfloat162 h = __habs2(
+            __floats2bfloat162_rn(__uint_as_float(v[2 * q]), __uint_as_float(v[2 * q + 1])));
+        s[8 * b + q] = *reinterpret_cast<const uint32_t*>(&h);
+      }
+    }
+    tc_fence_before();
+    mbar_arrive(smem_u32(&c->acc2_empty));
+    // columns past E have zero weights, hence score 0: no effect on a maximum of magnitudes
+    __nv_bfloat162 m2 = *reinterpret_cast<const __nv_bfloat162*>(&s[0]);
+#pragma unroll
+    for (int q = 1; q < NB * 8; ++q)
+      m2 = __hmax2_nan(m2, *reinterpret_cast<const __nv_bfloat162*>(&s[q]));
+    const float m = nanmax(__low2float(m2), __high2float(m2));
+    const __nv_bfloat162 thr = __float2bfloat162_rn(__fmul_rn(m, p.mult));
+    uint32_t word[NW];
+#pragma unroll
+    for (int j = 0; j < NW; ++j) word[j] = 0u;
+#pragma unroll
+    for (int q = 0; q < NB * 8; ++q) {
+      const uint32_t k = __hge2_mask(*reinterpret_cast<const __nv_bfloat162*>(&s[q]), thr);
+      word[q >> 4] |= k & (0x00010001u << (q & 15));
+      if (p.scores && live) {
+        if (2 * q < E)
+          p.scores[trow * E + 2 * q] = __ushort_as_bfloat16((unsigned short)(s[q] & 0xffff));
+        if (2 * q + 1 < E)
+          p.scores[trow * E + 2 * q + 1] = __ushort_as_bfloat16((unsigned short)(s[q] >> 16));
+      }
+      s[q] = k & 0x3f803f80u;                         // the routing entries: bf16 1.0 or 0
+    }
+    int kept = 0;
+#pragma unroll
+    for (int j = 0; j < NW; ++j) {
+      word[j] = interleave16(word[j]);
+      if (32 * j + 32 > E) word[j] &= (1u << (E - 32 * j)) - 1u;      // E > 32 j
+      if (!live) word[j] = 0u;
+      kept += __popc(word[j]);
+      if (live) p.mask_bits[trow * nw + j] = word[j];
+    }
+    if (p.out_init) {
+      const bool todo = live && (p.init_all || kept != 1);
+      const uint32_t rows = __ballot_sync(0xffffffffu, todo);
+      if (!mbar_wait_fast(smem_u32(&c->init_empty[buf]), ibuf_ph ^ 1, af, p.dev_status)) return;
+      if (lane == 0) {
+        c->init_rows[buf][q4] = rows;
+        mbar_arrive(smem_u32(&c->init_full[buf]));
+      }
+      __syncwarp();
+      ibuf_ph ^= buf;
+    }
+    if (p.tile_counts) {
+#pragma unroll
+      for (int j = 0; j < NW; ++j)
+        c->cnt[buf][q4][32 * j + lane] = __popc(transpose32(word[j], lane));
+      // one barrier per tile: the other half of cnt is written before anybody passes it again
+      asm volatile("bar.sync 1, 128;" ::: "memory");
+      if (et < p.EP) {
+        int n = 0;
+        if (et < E)
+          n = c->cnt[buf][0][et] + c->cnt[buf][1][et] + c->cnt[buf][2][et] + c->cnt[buf][3][et];
+        p.tile_counts[(long long)tile * p.EP + et] = (uint8_t)n;
+      }
+    }
+    if (p.rt_out && live) {
+      bf16* dst = p.rt_out + trow * E;
+      if ((E & 7) == 0) {
+#pragma unroll
+        for (int h = 0; h < NB * 2; ++h)
+          if (8 * h < E)
+            *reinterpret_cast<uint4*>(dst + 8 * h) =
+                make_uint4(s[4 * h], s[4 * h + 1], s[4 * h + 2], s[4 * h + 3]);
+      } else {
+#pragma unroll
+        for (int q = 0; q < NB * 8; ++q) {
+          if (2 * q < E) dst[2 * q] = __ushort_as_bfloat16((unsigned short)(s[q] & 0xffff));
+          if (2 * q + 1 < E) dst[2 * q + 1] = __ushort_as_bfloat16((unsigned short)(s[q] >> 16));
+        }
+      }
+    }
+  }
+}
+
+// warps 12-15: warp q writes the initial rows of the tile's tokens 32q .. 32q+31 that ask for one
+__device__ void role_init(const Params& p, Ctl* c, int q4, int lane) {
+  volatile int* af = &c->abort_flag;
+  const int tiles = (int)((p.N + TILE_M - 1) / TILE_M);
+  const int v8 = p.d >> 3;
+  uint32_t ph = 0, buf = 0;
+  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ph ^= buf, buf ^= 1) {
+    if (!mbar_wait_fast(smem_u32(&c->init_full[buf]), ph, af, p.dev_status)) return;
+    const uint32_t rows = c->init_rows[buf][q4];
+    __syncwarp();
+    if (lane == 0) mbar_arrive(smem_u32(&c->init_empty[buf]));
+    if (rows == 0u) continue;
+    const long long row0 = (long long)tile * TILE_M + 32 * q4;
+    for (int c8 = lane; c8 < v8; c8 += 32) {
+      uint4 bz = make_uint4(0u, 0u, 0u, 0u);
+      if (p.last_bias) bz = __ldg(reinterpret_cast<const uint4*>(p.last_bias) + c8);
+      if (!p.resid) {
+        for (uint32_t m = rows; m != 0u; m &= m - 1)
+          *(reinterpret_cast<uint4*>(p.out_init + (row0 + __ffs(m) - 1) * p.d) + c8) = bz;
+        continue;
+      }
+      for (uint32_t m = rows; m != 0u;) {
+        uint4 xv[4];
+        int rr[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {        // four rows in flight
+          rr[u] = m != 0u ? __ffs(m) - 1 : -1;
+          m &= m - 1;
+          if (rr[u] >= 0)
+            xv[u] = __ldg(reinterpret_cast<const uint4*>(p.resid + (row0 + rr[u]) * p.d) + c8);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (rr[u] >= 0)
+            *(reinterpret_cast<uint4*>(p.out_init + (row0 + rr[u]) * p.d) + c8) =
+                add_bf16x8(bz, xv[u]);
+      }
+    }
+  }
+}
+
+__global__ void __launch_bounds__(NTHREADS, 1)
+router_tiles_kernel(const Params p, const __grid_constant__ CUtensorMap tmx) {
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t raw = smem_u32(smem_raw);
+  const uint32_t base = (raw + 1023u) & ~1023u;
+  const uint32_t stage_bytes = SLOT + (uint32_t)(p.g.wa_bytes + 1023) / 1024 * 1024;
+  const uint32_t wb = base + p.g.ns * stage_bytes;
+  const uint32_t wb_bytes = (uint32_t)(p.g.kc2 * p.g.nd * 128);
+  Ctl* c = reinterpret_cast<Ctl*>(smem_raw + (wb - raw) + (wb_bytes + 1023) / 1024 * 1024);
+  const int tid = threadIdx.x, warp = tid >> 5;
+  // Programmatic dependent launch: the next kernel of the stream may be scheduled while this one
+  // runs (it waits for this grid before it reads anything); this CTA initialises its barriers
+  // while the previous kernel drains and reads global memory only after the wait below.
+  grid_launch_dependents();
+  if (tid == 0) {
+    for (int i = 0; i < NS_MAX; ++i) {
+      mbar_init(smem_u32(&c->full[i]), 1);
+      mbar_init(smem_u32(&c->empty[i]), 1);
+    }
+    mbar_init(smem_u32(&c->wb_full), 1);
+    mbar_init(smem_u32(&c->hid_full), 128);
+    mbar_init(smem_u32(&c->g2_done), 1);
+    mbar_init(smem_u32(&c->acc2_empty), 128);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(smem_u32(&c->acc1_full[i]), 1);
+      mbar_init(smem_u32(&c->acc1_empty[i]), 128);
+      mbar_init(smem_u32(&c->init_full[i]), 4);
+      mbar_init(smem_u32(&c->init_empty[i]), 4);
+    }
+    c->abort_flag = 0;
+    c->wait_limit = (int)p.wait_limit;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    fence_proxy_async();
+  }
+  if (warp == WARP_MMA1) tmem_alloc(smem_u32(&c->tmem_base), 512);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  grid_dependency_wait();
+  const uint32_t tmem = c->tmem_base;
+
+  if (warp < 4) {
+    role_hidden(p, c, tmem, tid);
+  } else if (warp < 8) {
+    switch (p.g.nd >> 4) {
+      case 1: role_gate<1>(p, c, tmem, tid - 128); break;
+      case 2: role_gate<2>(p, c, tmem, tid - 128); break;
+      case 3: role_gate<3>(p, c, tmem, tid - 128); break;
+      case 4: role_gate<4>(p, c, tmem, tid - 128); break;
+      case 5: role_gate<5>(p, c, tmem, tid - 128); break;
+      case 6: role_gate<6>(p, c, tmem, tid - 128); break;
+      case 7: role_gate<7>(p, c, tmem, tid - 128); break;
+      default: role_gate<8>(p, c, tmem, tid - 128); break;
+    }
+  } else if (warp == WARP_MMA1) {
+    if (elect_one()) role_mma1(p, c, base, stage_bytes, tmem);
+    __syncwarp();
+  } else if (warp == WARP_MMA2) {
+    if (elect_one()) role_mma2(p, c, wb, tmem);
+    __syncwarp();
+  } else if (warp == WARP_LOAD) {
+    if (elect_one()) role_load(p, c, &tmx, base, wb, stage_bytes);
+    __syncwarp();
+  } else if (warp >= WARP_INIT0 && p.out_init) {
+    role_init(p, c, warp - WARP_INIT0, tid & 31);
+  }
+
+  // A launch that gave up may still have copies and MMAs in flight that use this CTA's
+  // shared and tensor memory: give them time to land before both are released.
+  if (*reinterpret_cast<volatile int*>(&c->abort_flag) != 0)
+    for (int i = 0; i < 64; ++i) __nanosleep(1000);
+  tc_fence_before();
+  __syncthreads();
+  if (warp == WARP_MMA1) {
+    __syncwarp();
+    tc_fence_after();
+    tmem_dealloc(tmem, 512);
+  }
+}
+
+__global__ void prepack_router_kernel(const bf16* __restrict__ wa, const bf16* __restrict__ wb,
+                                      uint8_t* __restrict__ packed, Geo g, int d, int R, int E) {
+  const long long n1 = (long long)g.kc1 * g.nsub * g.nsubw * 64;
+  const long long n2 = (long long)g.kc2 * g.nd * 64;
+  const bf16 zero = __float2bfloat16_rn(0.f);
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n1 + n2;
+       i += (long long)gridDim.x * blockDim.x) {
+    if (i < n1) {
+      const int k = (int)(i % 64);
+      const int n = (int)((i / 64) % g.nsubw);
+      const int sub = (int)((i / (64LL * g.nsubw)) % g.nsub);
+      const int kc = (int)(i / (64LL * g.nsubw * g.nsub));
+      const bf16 v = wa[(long long)(sub * g.nsubw + n) * d + kc * 64 + k];
+      *reinterpret_cast<bf16*>(packed + (long long)(kc * g.nsub + sub) * g.nsubw * 128 +
+                               swz(n, k)) = v;
+    } else {
+      const long long q = i - n1;
+      const int k = (int)(q % 64);
+      const int n = (int)((q / 64) % g.nd);
+      const int k2 = (int)(q / (64LL * g.nd));
+      const int kk = k2 * 64 + k;
+      const bf16 v = (n < E && kk < R) ? wb[(long long)n * R + kk] : zero;
+      *reinterpret_cast<bf16*>(packed + g.w1_bytes + (long long)k2 * g.nd * 128 + swz(n, k)) = v;
+    }
+  }
+}
+
+size_t smem_bytes(const Geo& g) {
+  const size_t stage = SLOT + (size_t)(g.wa_bytes + 1023) / 1024 * 1024;
+  const size_t wb = (size_t)(g.kc2 * g.nd * 128 + 1023) / 1024 * 1024;
+  return 1024 + g.ns * stage + wb + sizeof(Ctl) + 64;
+}
+
+static_assert(1024 + SMEM_TILES + 1024 + sizeof(Ctl) + 64 <= 232448,
+              "shared-memory plan exceeds the 227 KB a CTA may use");
+
+}  // namespace
+
+bool umma_router_supported(int d, int R, int E, int dtype) {
+  return dtype == D2D_BF16 && d >= 64 && d % 64 == 0 && R >= 16 && R % 16 == 0 &&
+         (R <= 128 || R == 256) && E >= 1 && E <= MAX_E;
+}
+
+size_t umma_router_packed_bytes(int d, int R, int E) { return (size_t)router_geo(d, R, E).stride; }
+
+int launch_prepack_router(const void* wa, const void* wb, void* packed, int d, int R, int E,
+                          cudaStream_t s) {
+  const Geo g = router_geo(d, R, E);
+  prepack_router_kernel<<<64, 256, 0, s>>>((const bf16*)wa, (const bf16*)wb, (uint8_t*)packed, g, d,
+                                           R, E);
+  return cudaGetLastError() == cudaSuccess ? D2D_OK : D2D_ERR_LAUNCH;
+}
+
+int launch_router_mask_umma(const void* x, const void* packed, float mult, uint32_t* mask_bits,
+                            void* scores, void* rt_out, const void* last_bias, const void* resid,
+                            void* out_init, bool init_all, int32_t* tile_counts, int64_t N, int d,
+                            int R, int E, int* dev_status, cudaStream_t s) {
+  Params p = {};
+  p.N = N;
+  p.d = d;
+  p.R = R;
+  p.E = E;
+  p.packed = (const uint8_t*)packed;
+  p.g = router_geo(d, R, E);
+  p.mult = mult;
+  p.mask_bits = mask_bits;
+  p.scores = (bf16*)scores;
+  p.rt_out = (bf16*)rt_out;
+  p.tile_counts = reinterpret_cast<uint8_t*>(tile_counts);
+  p.EP = compact_row_cells(E);
+  p.out_init = (bf16*)out_init;
+  p.last_bias = (const bf16*)last_bias;
+  p.resid = (const bf16*)resid;
+  p.init_all = init_all ? 1 : 0;
+  p.dev_status = dev_status;
+  umma_debug_read(&p.wait_limit, &p.withhold);
+  const size_t smem = smem_bytes(p.g);
+  int sms = 0;
+  int rc = device_launch_facts((const void*)router_tiles_kernel, smem, &sms);
+  if (rc != D2D_OK) return rc;
+  // x as boxes of 64 columns x 128 consecutive rows; rows past the last token arrive as zeros
+  alignas(64) CUtensorMap tmx;
+  rc = encode_tmap_2d_b16(&tmx, x, (uint64_t)d, (uint64_t)N, (uint64_t)d * 2, 64, TILE_M, true);
+  if (rc != D2D_OK) return rc == D2D_ERR_BAD_ARG ? D2D_ERR_LAUNCH : rc;
+  const int64_t tiles = (N + TILE_M - 1) / TILE_M;
+  const int64_t grid = tiles < sms ? tiles : sms;
+  return launch_pdl(router_tiles_kernel, dim3((unsigned)grid), dim3(NTHREADS), smem, s, p, tmx);
+}
+
+}  // namespace d2d
