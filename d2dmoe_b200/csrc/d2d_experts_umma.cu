@@ -15,21 +15,27 @@
 //     from tensor memory, and no shared memory is spent on it (rings of 128 + 48 KB);
 //   * two tiles are in work at once: the first product of one runs while the second product of
 //     the other runs and is written out;
-//   * accumulator 2 has four 64-column buffers (gated form: two per tile), so that the
-//     commit -> drain -> release -> issue loop of a buffer passes while the others are in use;
-//   * eight warps drain accumulator 2, each on its own (convert, transpose through its own 4 KB,
-//     add or store), in straight-line code: with twenty warps in eight different loops,
-//     instruction fetch is what a branch costs;
+//   * the second product works in steps of 128 output columns (64 where d or the tensor memory
+//     does not allow it) over two or more accumulator-2 buffers: a step costs its issuing thread
+//     some 300 cycles besides the products, so few and large ones;
+//   * eight warps drain accumulator 2, each 64 columns of its 32 rows and on its own (convert,
+//     transpose through its own 4 KB, add or store whole 128-byte lines), in straight-line
+//     code: with twenty warps in eight different loops instruction fetch is what a branch costs;
+//     (sixteen warps with 32 columns each: 59.6 instead of 56.5 us on the 50432-token layer);
 //   * the lists are cut into equal tiles of a size that fills the last round of the persistent
-//     grid; where there are fewer tiles than SMs the output columns are split as well.
+//     grid; where there are fewer tiles than SMs the output columns are split as well;
+//   * where the weights of all experts stay in L2, the tiles are taken window by window of the
+//     token range, all experts of a window next to each other, so that a row of x is read and
+//     a row of out is added to in L2 by every expert but the first; last window first, because
+//     its rows are what the router has left in L2.
 //
 // Tensor memory (512 columns).  Two-layer form: accumulator 1 / hidden of tile t at 128 (t & 1),
-// accumulator-2 buffers at 256 + 64 b.  Gated form: a tile has a half (256 columns): gate at 0,
-// up at H, hidden in place at 0, and once epilogue 1 is done two accumulator-2 buffers at 64
-// and 192.
+// accumulator-2 buffers from 256 on (two of 128 or four of 64 columns).  Gated form: a tile has a
+// half (256 columns): gate at 0, up at H, hidden in place at 0, and once epilogue 1 is done
+// three 64-column accumulator-2 buffers from 64 on.
 //
-// Warps: 0-3 epilogue 1; 4-7 and 8-11 drain groups 0 and 1 (even and odd steps); 12-15 row gather
-// (cp.async); 16 first product; 17 second product; 18 W1 tiles, 19 W2 tiles (bulk copies).
+// Warps: 0-3 epilogue 1; 4-11 drain; 12-15 row gather (cp.async); 16 first product; 17 second
+// product; 18 weights (bulk copies); 19 the tiles and their row lists.
 //
 // Every wait is bounded: when one runs out the kernel records D2D_ERR_TIMEOUT in the status word,
 // all roles leave their loops, TMEM is freed and the kernel returns.
@@ -43,22 +49,23 @@ using namespace umma;
 namespace {
 
 constexpr int NTHREADS = 640;
-constexpr int WARP_DRAIN0 = 4, WARP_GATHER0 = 12, WARP_MMA1 = 16, WARP_MMA2 = 17, WARP_W1 = 18,
-              WARP_W2 = 19;
+constexpr int WARP_DRAIN0 = 4, WARP_GATHER0 = 12, WARP_MMA1 = 16, WARP_MMA2 = 17, WARP_W = 18;
+constexpr int TILE_RING = 4;                  // tiles known ahead of the slowest role
+constexpr int TILE_READERS = 4 + 8 + 4 + 1 + 1 + 2;   // warps 0-15, both products, both weight streams
 constexpr int MAX_E = 128;
 constexpr int NS_MAX = 8, NS2_MAX = 8;        // stages of the two rings (upper bounds)
-constexpr int ND = 64;                        // output columns per step of the second product
 constexpr int STG = 8 * 4096;                 // transposition blocks of the drain warps
 constexpr int SMEM_TILES = 220 * 1024;        // both rings + STG
+constexpr long long L2_WEIGHTS = 32 << 20;    // weights up to this size are taken to stay in L2
 
 struct Geo {
   int kc1;         // d / 64
   int w1_stage;    // W1 (and W_up) bytes per 64-deep slice
   int kc2;         // ceil(H / 64)
-  int nc;          // d / 64: steps of the second product
+  int nd, nc;      // output columns per step of the second product, steps
   int ns, ns2;     // ring stages
   int stage;       // bytes of a stage of the first ring: rows of x (16 KB), then w1_stage
-  int w2_stage;    // W2 bytes per step: 64 output columns x kc2 slices
+  int w2_piece;    // W2 bytes of a step's 64-deep slice (one stage of the second ring)
   long long w1_bytes, bias_off, stride;   // packed layout per expert
 };
 
@@ -67,16 +74,17 @@ Geo experts_geo(int d, int H, bool glu) {
   g.kc1 = d / 64;
   g.w1_stage = (glu ? 2 : 1) * H * 128;
   g.kc2 = (H + 63) / 64;
-  g.nc = d / ND;
+  g.nd = !glu && d % 128 == 0 ? 128 : 64;
+  g.nc = d / g.nd;
   g.stage = SLOT + g.w1_stage;
-  g.w2_stage = g.kc2 * ND * 128;
-  // at least three steps of W2, then as many stages of the first ring as fit, the rest for W2
-  const int ns = (SMEM_TILES - STG - 3 * g.w2_stage) / g.stage;
+  g.w2_piece = g.nd * 128;
+  // at least three W2 pieces, then as many stages of the first ring as fit, the rest for W2
+  const int ns = (SMEM_TILES - STG - 3 * g.w2_piece) / g.stage;
   g.ns = ns < NS_MAX ? ns : NS_MAX;
-  const int ns2 = (SMEM_TILES - STG - g.ns * g.stage) / g.w2_stage;
+  const int ns2 = (SMEM_TILES - STG - g.ns * g.stage) / g.w2_piece;
   g.ns2 = ns2 < NS2_MAX ? ns2 : NS2_MAX;
   g.w1_bytes = (long long)g.kc1 * g.w1_stage;
-  g.bias_off = g.w1_bytes + (long long)g.nc * g.w2_stage;
+  g.bias_off = g.w1_bytes + (long long)g.nc * g.kc2 * g.w2_piece;
   g.stride = (g.bias_off + 512 + 1023) / 1024 * 1024;
   return g;
 }
@@ -99,180 +107,316 @@ struct Params {
   int norm_layer, norm_ord;    // D2D_NORM_OF_INTERMEDIATE / D2D_NORM_OF_OUTPUT (0: none); 1 or 2
 };
 
+struct Tile {
+  int e;                           // expert; -1: no more tiles
+  int n0, n1;                      // steps of the second product
+  int pad;
+  uint32_t direct[4];              // rows that are stored instead of added to
+  int list[TILE_M];                // tokens, -1: no row
+  uint32_t bias[64];               // b1 of the expert as bf16 pairs
+};
+
 struct Ctl {
   unsigned long long full[NS_MAX], empty[NS_MAX], full2[NS2_MAX], empty2[NS2_MAX];
-  unsigned long long acc1_full[2], ctx_free[2], hid_full[2], acc2_full[4], acc2_empty[4];
-  unsigned long long list_full[2], list_empty[2];
+  unsigned long long acc1_full[2], ctx_free[2], hid_full[2], acc2_full[6], acc2_empty[6];
+  unsigned long long tile_full[TILE_RING], direct_full[TILE_RING], tile_empty[TILE_RING];
+  unsigned long long np_full[4], np_empty[4];
   uint32_t tmem_base;
   int abort_flag;
   int wait_limit;                  // must follow abort_flag (mbar_wait reads abort_flag[1])
-  int total_tiles;                 // tiles x column parts
-  int parts;                       // column parts per tile
-  int dense_e;                     // > 0: every expert lists all N tokens (number of experts)
-  alignas(16) uint32_t bias_s[2][64];   // b1 of the tile's expert as bf16 pairs
-  int list[2][128];                // the tile's tokens; sign bit: row is stored; -1: no row
-  float npart[128];                // row norm terms of drain group 1
-  int off[MAX_E + 1];              // list offsets
-  int tstart[MAX_E + 1];           // first tile of each expert
-  int rows[MAX_E];                 // rows per tile of each expert
+  float npart[TILE_M];             // norm terms that the other drain group saw
+  alignas(16) Tile tile[TILE_RING];
 };
 
-// columns of tile t's tensor memory, and of its accumulator-2 buffer b
+// columns of a tile's tensor memory
 template <bool GLU>
 __device__ __forceinline__ uint32_t tm_tile(uint32_t tmem, uint32_t ctx) {
   return tmem + ctx * (GLU ? 256 : 128);
 }
+
+// Accumulator-2 buffers in rotation: one ring for all tiles, gated form one per context.
 template <bool GLU>
-__device__ __forceinline__ uint32_t tm_acc2(uint32_t tmem, uint32_t b) {
-  return GLU ? tmem + (b >> 1) * 256 + (b & 1) * 128 + 64 : tmem + 256 + b * 64;
-}
-
-struct Tile {
-  int e, r0, nrows, n0, n1;        // rows of the token list, steps of the second product
-};
-
-__device__ __forceinline__ Tile tile_info(const Params& p, const Ctl* c, int tile) {
-  Tile t;
-  int part = 0;
-  const int parts = c->parts;
-  if (parts > 1) {
-    part = tile % parts;
-    tile /= parts;
+struct Acc2Ring {
+  RingPos r0 = {0, 0}, r1 = {0, 0};
+  __device__ __forceinline__ RingPos at(uint32_t ctx) const { return GLU && ctx ? r1 : r0; }
+  __device__ __forceinline__ uint32_t slot(uint32_t ctx) const {       // barrier index
+    return GLU ? 3 * ctx + at(ctx).s : r0.s;
   }
-  t.n0 = part * p.g.nc / parts;
-  t.n1 = (part + 1) * p.g.nc / parts;
-  int k;
-  if (c->dense_e > 0) {
-    // Every expert runs on every token (mode 'all' upstream: router training, label capture):
-    // window-major order, the E tiles of one window of tokens next to each other, so that the
-    // window's rows of x and out stay in L2.
-    k = tile / p.E;
-    t.e = tile - k * p.E;
-  } else {
-    int lo = 0, hi = p.E;
-    while (hi - lo > 1) {
-      const int mid = (lo + hi) >> 1;
-      if (c->tstart[mid] <= tile) lo = mid; else hi = mid;
+  __device__ __forceinline__ uint32_t column(uint32_t tmem, uint32_t ctx, int nd) const {
+    return GLU ? tmem + 256 * ctx + 64 + 64 * at(ctx).s : tmem + 256 + nd * r0.s;
+  }
+  __device__ __forceinline__ void next(uint32_t ctx, int nd) {
+    if (GLU) {
+      if (ctx) r1.next(3); else r0.next(3);
+    } else {
+      r0.next(nd == 128 ? 2 : 4);
     }
-    t.e = lo;
-    k = tile - c->tstart[lo];
   }
-  t.r0 = c->off[t.e] + k * c->rows[t.e];
-  t.nrows = min(c->rows[t.e], c->off[t.e + 1] - t.r0);
-  return t;
-}
+};
 
 // ---------------------------------------------------------------------------
 // roles
 // ---------------------------------------------------------------------------
+// Warp 19: cuts the lists into tiles, finds the ones of this CTA and hands them to the other roles
+// with their row lists, then the expert's bias and which rows are stored (tokens that one expert
+// keeps): those loads depend on the list's, and only the epilogue warps wait for them.
+//
+// Tiles have S rows at most, S as small as the number of rounds of the grid allows:
+// T = sum ceil(n_e / S) <= rows / S + E, so R rounds of G CTAs are enough for S = rows / (R G - E),
+// and R is the least with S <= 128.  (524 rows per SM: five tiles of about 109 rows per CTA
+// instead of four of 128 and one of 12.)  An expert's tiles are equal.
+// The first pass over the set-up runs on no rows, while the previous kernel drains: instructions
+// executed for the first time cost some 20 cycles each, and everything waits for the first tile.
+__device__ void role_list(const Params& p, Ctl* c, int lane, bool one_window) {
+  volatile int* af = &c->abort_flag;
+  const int nw = (p.E + 31) >> 5;
+  int off[5], n[4], nt[4], total = 0, rounds = 1;
+#pragma unroll 1
+  for (int pass = 0; pass < 2; ++pass) {
+    if (pass) grid_dependency_wait();
+    const int E = pass ? p.E : 0;
+    int rows = 0, used = 0;
+    bool all_n = true;                   // every expert of this lane lists exactly N tokens
+#pragma unroll
+    for (int q = 0; q < 5; ++q) {
+      const int e = 4 * lane + q;
+      off[q] = e <= E && E > 0 ? p.offsets[e] : 0;
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int e = 4 * lane + q;
+      const bool bad = off[q + 1] < off[q] || off[q] < 0 || off[q + 1] > p.N * (long long)p.E;
+      n[q] = e < E && !bad ? off[q + 1] - off[q] : 0;
+      if (e < E && bad) report(p.dev_status, D2D_ERR_INDEX_RANGE);
+      all_n = all_n && (e >= E || n[q] == p.N);
+      rows += n[q];
+      used += n[q] > 0 ? 1 : 0;
+    }
+    rows = __reduce_add_sync(0xffffffffu, rows);
+    used = __reduce_add_sync(0xffffffffu, used);
+    const float G = (float)gridDim.x;
+    const float R = ceilf(((float)rows * (1.0f / TILE_M) + (float)used) / G);
+    const int S =
+        max(32, min(TILE_M, (int)ceilf((float)rows / fmaxf(R * G - (float)used, 1.0f))));
+    const float inv = 1.0f / (float)S;
+    int sum = 0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {        // ceil(n / S): float quotient, exact correction
+      nt[q] = (int)((float)n[q] * inv);
+      while ((long long)nt[q] * S < n[q]) ++nt[q];
+      while (nt[q] > 0 && (long long)(nt[q] - 1) * S >= n[q]) --nt[q];
+      sum += nt[q];
+    }
+    total = __reduce_add_sync(0xffffffffu, sum);
+    // windows: one per round of the grid, or a single one (expert by expert) where each window
+    // would stream all the weights again; with every expert on every token they pay all the same
+    rounds = one_window && !__all_sync(0xffffffffu, all_n) ? 1 : max(1, (int)R);
+  }
+  // fewer than half as many tiles as CTAs: split the output columns (the first product is
+  // repeated, the second product, W2 and the output are shared out)
+  int parts = 1;
+  if (total > 0 && 2 * total <= (int)gridDim.x && p.norm_layer == 0)
+    parts = min((int)gridDim.x / total, p.g.nc);
+  const float inv_rounds = 1.0f / (float)rounds;
+
+  // the current window's tiles of my experts: lo .. hi - 1
+  int lo[4], hi[4], w = rounds, start = 0, count = 0, incl = 0;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) lo[q] = nt[q];
+  RingPos r = {0, 0};
+#pragma unroll 1
+  for (int u = blockIdx.x;; u += gridDim.x, r.next(TILE_RING)) {
+    const int tile = u / parts, part = u - tile * parts;
+    Tile* t = &c->tile[r.s];
+    if (tile >= total) {
+      if (!mbar_wait_fast(smem_u32(&c->tile_empty[r.s]), r.ph ^ 1, af, p.dev_status)) return;
+      if (lane == 0) t->e = -1;
+      __syncwarp();
+      mbar_arrive(smem_u32(&c->tile_full[r.s]));
+      return;
+    }
+    while (tile >= start + count) {
+      start += count;
+      --w;
+      int mine = 0;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        hi[q] = lo[q];
+        lo[q] = w == 0 ? 0 : min(hi[q], (int)((float)nt[q] * ((float)w * inv_rounds)));
+        mine += hi[q] - lo[q];
+      }
+      incl = mine;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+      }
+      count = __shfl_sync(0xffffffffu, incl, 31);
+    }
+    const int owner = __ffs(__ballot_sync(0xffffffffu, incl > tile - start)) - 1;
+    int e = 0, r0 = 0, nrows = 0;
+    if (lane == owner) {
+      int k = tile - start - (incl - (hi[0] + hi[1] + hi[2] + hi[3] - lo[0] - lo[1] - lo[2] - lo[3]));
+      bool found = false;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int m = hi[q] - lo[q];
+        if (!found && k < m) {
+          found = true;
+          e = 4 * lane + q;
+          const int size = (n[q] + nt[q] - 1) / nt[q];
+          const int first = (lo[q] + k) * size;
+          r0 = off[q] + first;
+          nrows = min(size, n[q] - first);      // (may be negative where the last tiles are empty)
+        }
+        if (!found) k -= m;
+      }
+    }
+    e = __shfl_sync(0xffffffffu, e, owner);
+    r0 = __shfl_sync(0xffffffffu, r0, owner);
+    nrows = __shfl_sync(0xffffffffu, nrows, owner);
+    int tok[4];
+#pragma unroll
+    for (int g = 0; g < 4; ++g)          // a lane has rows lane + 32 g
+      tok[g] = 32 * g + lane < nrows ? p.token_idx[r0 + 32 * g + lane] : 0;
+    if (!mbar_wait_fast(smem_u32(&c->tile_empty[r.s]), r.ph ^ 1, af, p.dev_status)) return;
+    if (lane == 0) {
+      t->e = e;
+      t->n0 = part * p.g.nc / parts;
+      t->n1 = (part + 1) * p.g.nc / parts;
+    }
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+      if (tok[g] < 0 || tok[g] >= p.N) {
+        report(p.dev_status, D2D_ERR_INDEX_RANGE);
+        tok[g] = -1;
+      }
+      if (32 * g + lane >= nrows) tok[g] = -1;
+      t->list[32 * g + lane] = tok[g];
+    }
+    __syncwarp();
+    mbar_arrive(smem_u32(&c->tile_full[r.s]));
+    const float4 b1 = 4 * lane < p.H
+                          ? __ldg(reinterpret_cast<const float4*>(
+                                p.packed + (long long)e * p.g.stride + p.g.bias_off) + lane)
+                          : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+      int kept = 0;
+      if (p.mask_bits && tok[g] >= 0)
+        for (int q = 0; q < nw; ++q) kept += __popc(p.mask_bits[(long long)tok[g] * nw + q]);
+      const uint32_t d = __ballot_sync(0xffffffffu, kept == 1);
+      if (lane == 0) t->direct[g] = d;
+    }
+    t->bias[2 * lane] = pack_bf16x2(b1.x, b1.y);
+    t->bias[2 * lane + 1] = pack_bf16x2(b1.z, b1.w);
+    __syncwarp();
+    mbar_arrive(smem_u32(&c->direct_full[r.s]));
+  }
+}
+
 // Warps 12-15: rows of x by 16-byte cp.async (4 rows x 128 bytes per warp instruction, software
-// swizzle; a TMA gather spends a request per 128-byte row and was 1.6 times slower).  Inside
-// a warp's 32 rows those that are stored come first, so that an output instruction (4 rows)
-// mostly does one thing.  Rows past the list's end are not loaded: whatever their slots hold
-// reaches only accumulator rows nobody reads.
+// swizzle; a TMA gather spends a request per 128-byte row and was 1.6 times slower).  Rows past
+// the list's end repeat the 32-row group's first one, a group without rows loads nothing: what
+// their slots hold reaches only accumulator rows nobody reads.
 __device__ void role_gather(const Params& p, Ctl* c, uint32_t ring, int w, int lane) {
   volatile int* af = &c->abort_flag;
-  const int j = lane & 7, nw = (p.E + 31) >> 5, total = c->total_tiles;
+  const int j = lane & 7;
   uint32_t dstoff[8];
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     const int row = w * 32 + i * 4 + (lane >> 3);
     dstoff[i] = (row >> 3) * 1024 + (row & 7) * 128 + ((j ^ (row & 7)) << 4);
   }
-  int tok = -1, kept = 0;
-  bool mine = false;
-  auto fetch = [&](int tile) {           // token of my row, -1: none
-    tok = -1;
-    mine = false;
-    if (tile >= total) return;
-    const Tile t = tile_info(p, c, tile);
-    mine = w * 32 + lane < t.nrows;
-    if (mine) tok = p.token_idx[t.r0 + w * 32 + lane];
-  };
-  auto fetch_kept = [&]() {              // how many experts keep it
-    kept = 0;
-    if (mine && (tok < 0 || tok >= p.N)) {
-      report(p.dev_status, D2D_ERR_INDEX_RANGE);
-      tok = -1;
-    }
-    if (p.mask_bits && tok >= 0)
-      for (int q = 0; q < nw; ++q) kept += __popc(p.mask_bits[(long long)tok * nw + q]);
-  };
-  fetch(blockIdx.x);
-  fetch_kept();
-  RingPos r = {0, 0};
-  uint32_t b = 0, ph = 0;
-  for (int tile = blockIdx.x; tile < total; tile += gridDim.x) {
-    if (!mbar_wait_fast(smem_u32(&c->list_empty[b]), ph ^ 1, af, p.dev_status)) return;
-    int* list = c->list[b] + w * 32;
-    {
-      const bool direct = kept == 1;
-      const uint32_t dm = __ballot_sync(0xffffffffu, direct), lt = (1u << lane) - 1u;
-      const uint32_t live = __ballot_sync(0xffffffffu, tok >= 0) & ~dm;
-      const uint32_t none = ~(dm | live);
-      const int slot = direct     ? __popc(dm & lt)
-                       : tok >= 0 ? __popc(dm) + __popc(live & lt)
-                                  : __popc(dm | live) + __popc(none & lt);
-      list[slot] = tok < 0 ? -1 : direct ? (int)((uint32_t)tok | 0x80000000u) : tok;
-      __syncwarp();
-    }
+  RingPos r = {0, 0}, q = {0, 0};
+  for (;; q.next(TILE_RING)) {
+    if (!mbar_wait_fast(smem_u32(&c->tile_full[q.s]), q.ph, af, p.dev_status)) return;
+    if (c->tile[q.s].e < 0) return;
+    const int* list = c->tile[q.s].list + w * 32;
+    const int v0 = list[0];
     const bf16* src[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       const int v = list[i * 4 + (lane >> 3)];
-      src[i] = v == -1 ? nullptr : p.x + (size_t)(v & 0x7fffffff) * p.d + j * 8;
+      src[i] = p.x + (size_t)max(v < 0 ? v0 : v, 0) * p.d + j * 8;
     }
-    mbar_arrive(smem_u32(&c->list_full[b]));
-    ph ^= b;
-    b ^= 1;
-    fetch(tile + gridDim.x);             // in flight while this tile's rows are gathered
-    const int kmask = p.g.kc1 > 2 ? 2 : p.g.kc1 - 1;
+    __syncwarp();
+    if (lane == 0) mbar_arrive(smem_u32(&c->tile_empty[q.s]));
+    const bool rows = v0 >= 0;           // warp-uniform
     for (int kc = 0; kc < p.g.kc1; ++kc) {
       if (!mbar_wait_fast(smem_u32(&c->empty[r.s]), r.ph ^ 1, af, p.dev_status)) return;
-      const uint32_t base = ring + r.s * p.g.stage;
+      if (rows) {
+        const uint32_t base = ring + r.s * p.g.stage;
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
-        if (src[i]) cp_async16(base + dstoff[i], src[i] + kc * 64);
+        for (int i = 0; i < 8; ++i) cp_async16(base + dstoff[i], src[i] + kc * 64);
+      }
       cp_async_arrive_noinc(smem_u32(&c->full[r.s]));
       r.next(p.g.ns);
-      if (kc == kmask) fetch_kept();
     }
   }
 }
 
-// The four roles below each run in ONE thread of their warp for the whole launch: their loops are
+// The three roles below each run in ONE thread of their warp for the whole launch: their loops are
 // chains of dependent instructions, votes and re-convergence would only lengthen the chain.
-__device__ void role_w1(const Params& p, Ctl* c, uint32_t ring) {
+
+// Weights of both rings.  The two streams (W1 slices, W2 steps) advance independently: whichever
+// ring has a free stage gets its next piece.
+__device__ void role_weights(const Params& p, Ctl* c, uint32_t ring, uint32_t ring2) {
   volatile int* af = &c->abort_flag;
   const Geo& g = p.g;
   bool withheld = (p.withhold & 1) != 0 && blockIdx.x == 0;
-  RingPos r = {0, 0};
-  for (int tile = blockIdx.x; tile < c->total_tiles; tile += gridDim.x) {
-    const uint8_t* src = p.packed + (long long)tile_info(p, c, tile).e * g.stride;
-    for (int kc = 0; kc < g.kc1; ++kc, src += g.w1_stage) {
-      if (!mbar_wait_fast(smem_u32(&c->empty[r.s]), r.ph ^ 1, af, p.dev_status)) return;
-      const uint32_t bar = smem_u32(&c->full[r.s]);
+  RingPos r1 = {0, 0}, r2 = {0, 0}, q1 = {0, 0}, q2 = {0, 0};
+  int j1 = 0, j2 = 0;                    // pieces left of the current tile; -1: no more tiles
+  const uint8_t *s1 = nullptr, *s2 = nullptr;
+  uint32_t idle = 0;
+  while (j1 >= 0 || j2 >= 0) {
+    bool progress = false;
+    if (j1 == 0 && mbar_test_wait(smem_u32(&c->tile_full[q1.s]), q1.ph)) {
+      const int e = c->tile[q1.s].e;
+      j1 = e < 0 ? -1 : g.kc1;
+      s1 = p.packed + (long long)e * g.stride;
+      mbar_arrive(smem_u32(&c->tile_empty[q1.s]));
+      q1.next(TILE_RING);
+      progress = true;
+    }
+    if (j1 > 0 && mbar_test_wait(smem_u32(&c->empty[r1.s]), r1.ph ^ 1)) {
+      const uint32_t bar = smem_u32(&c->full[r1.s]);
       mbar_arrive_expect_tx(bar, g.w1_stage);
       if (withheld) withheld = false;    // test hook: this stage never fills, its wait runs out
-      else bulk_g2s(ring + r.s * g.stage + SLOT, src, g.w1_stage, bar);
-      r.next(g.ns);
+      else bulk_g2s(ring + r1.s * g.stage + SLOT, s1, g.w1_stage, bar);
+      s1 += g.w1_stage;
+      r1.next(g.ns);
+      --j1;
+      progress = true;
     }
-  }
-}
-
-__device__ void role_w2(const Params& p, Ctl* c, uint32_t ring2) {
-  volatile int* af = &c->abort_flag;
-  const Geo& g = p.g;
-  RingPos r = {0, 0};
-  for (int tile = blockIdx.x; tile < c->total_tiles; tile += gridDim.x) {
-    const Tile t = tile_info(p, c, tile);
-    const uint8_t* src = p.packed + (long long)t.e * g.stride + g.w1_bytes;
-    for (int n = t.n0; n < t.n1; ++n) {
-      if (!mbar_wait_fast(smem_u32(&c->empty2[r.s]), r.ph ^ 1, af, p.dev_status)) return;
-      const uint32_t bar = smem_u32(&c->full2[r.s]);
-      mbar_arrive_expect_tx(bar, g.w2_stage);
-      bulk_g2s(ring2 + r.s * g.w2_stage, src + (long long)n * g.w2_stage, g.w2_stage, bar);
-      r.next(g.ns2);
+    if (j2 == 0 && mbar_test_wait(smem_u32(&c->tile_full[q2.s]), q2.ph)) {
+      const Tile* t = &c->tile[q2.s];
+      const int e = t->e;
+      j2 = e < 0 ? -1 : (t->n1 - t->n0) * g.kc2;
+      s2 = p.packed + (long long)e * g.stride + g.w1_bytes + (long long)t->n0 * g.kc2 * g.w2_piece;
+      mbar_arrive(smem_u32(&c->tile_empty[q2.s]));
+      q2.next(TILE_RING);
+      progress = true;
+    }
+    if (j2 > 0 && mbar_test_wait(smem_u32(&c->empty2[r2.s]), r2.ph ^ 1)) {
+      const uint32_t bar = smem_u32(&c->full2[r2.s]);
+      mbar_arrive_expect_tx(bar, g.w2_piece);
+      bulk_g2s(ring2 + r2.s * g.w2_piece, s2, g.w2_piece, bar);
+      s2 += g.w2_piece;
+      r2.next(g.ns2);
+      --j2;
+      progress = true;
+    }
+    if (progress) {
+      idle = 0;
+    } else {
+      if (++idle > 64) __nanosleep(idle > 4096 ? 256 : 32);
+      if ((idle & 63) == 0 && *af != 0) return;
+      if (idle >= p.wait_limit) {
+        *af = 1;
+        report(p.dev_status, D2D_ERR_TIMEOUT);
+        return;
+      }
     }
   }
 }
@@ -287,9 +431,12 @@ __device__ void role_mma1(const Params& p, Ctl* c, uint32_t ring, uint32_t tmem)
   const uint64_t d0 = smem_desc(ring);
   const uint64_t hi = (d0 >> 32) << 32;
   const uint32_t lo0 = (uint32_t)d0;
-  RingPos r = {0, 0};
+  RingPos r = {0, 0}, q = {0, 0};
   uint32_t ctx = 0, ph = 0;
-  for (int tile = blockIdx.x; tile < c->total_tiles; tile += gridDim.x) {
+  for (;; q.next(TILE_RING)) {
+    if (!mbar_wait_fast(smem_u32(&c->tile_full[q.s]), q.ph, af, p.dev_status)) return;
+    if (c->tile[q.s].e < 0) return;
+    mbar_arrive(smem_u32(&c->tile_empty[q.s]));
     const uint32_t acc = tm_tile<GLU>(tmem, ctx);
     if (!mbar_wait_fast(smem_u32(&c->ctx_free[ctx]), ph ^ 1, af, p.dev_status)) return;
     tc_fence_after();
@@ -309,39 +456,42 @@ __device__ void role_mma1(const Params& p, Ctl* c, uint32_t ring, uint32_t tmem)
   }
 }
 
-// second product: one 64-column step after another, each into the next accumulator-2 buffer
+// second product: one step after another, each into the next accumulator-2 buffer
 template <bool GLU>
 __device__ void role_mma2(const Params& p, Ctl* c, uint32_t ring2, uint32_t tmem) {
   volatile int* af = &c->abort_flag;
   const Geo& g = p.g;
-  const uint32_t idesc = instr_desc(TILE_M, ND);
+  const uint32_t idesc = instr_desc(TILE_M, g.nd);
   const uint64_t d0 = smem_desc(ring2);
   const uint64_t hi = (d0 >> 32) << 32;
   const uint32_t lo0 = (uint32_t)d0;
-  const int ks = p.H >> 4;
-  RingPos r = {0, 0};
-  uint32_t ctx = 0, ph = 0, step = 0, uses = 0;   // uses: bit b = parity of buffer b's uses so far
-  for (int tile = blockIdx.x; tile < c->total_tiles; tile += gridDim.x) {
-    const Tile t = tile_info(p, c, tile);
+  RingPos r = {0, 0}, q = {0, 0};
+  Acc2Ring<GLU> ar;
+  uint32_t ctx = 0, ph = 0;
+  for (;; q.next(TILE_RING)) {
+    if (!mbar_wait_fast(smem_u32(&c->tile_full[q.s]), q.ph, af, p.dev_status)) return;
+    if (c->tile[q.s].e < 0) return;
+    const int n0 = c->tile[q.s].n0, n1 = c->tile[q.s].n1;
+    mbar_arrive(smem_u32(&c->tile_empty[q.s]));
     const uint32_t hid = tm_tile<GLU>(tmem, ctx);
-    if (GLU) step = 0;
     if (!mbar_wait_fast(smem_u32(&c->hid_full[ctx]), ph, af, p.dev_status)) return;
-    for (int n = t.n0; n < t.n1; ++n, ++step) {
-      const uint32_t b = GLU ? 2 * ctx + (step & 1) : step & 3;
-      if (!mbar_wait_fast(smem_u32(&c->full2[r.s]), r.ph, af, p.dev_status)) return;
-      if (!mbar_wait_fast(smem_u32(&c->acc2_empty[b]), ((uses >> b) & 1) ^ 1, af, p.dev_status))
-        return;
-      uses ^= 1u << b;
-      tc_fence_after();
-      const uint32_t acc = tm_acc2<GLU>(tmem, b), blo = lo0 + r.s * ((uint32_t)g.w2_stage >> 4);
-      umma_bf16_ta(acc, hid, hi | blo, idesc, 0);
-#pragma unroll
-      for (int k = 1; k < 8; ++k)
-        if (k < ks)
-          umma_bf16_ta(acc, hid + 8 * k, hi | (blo + (k >> 2) * (ND * 8) + 2 * (k & 3)), idesc, 1);
+    for (int n = n0; n < n1; ++n) {
+      const uint32_t b = ar.slot(ctx), acc = ar.column(tmem, ctx, g.nd);
+      if (!mbar_wait_fast(smem_u32(&c->acc2_empty[b]), ar.at(ctx).ph ^ 1, af, p.dev_status)) return;
+      for (int k2 = 0; k2 < g.kc2; ++k2) {
+        if (!mbar_wait_fast(smem_u32(&c->full2[r.s]), r.ph, af, p.dev_status)) return;
+        tc_fence_after();
+        const uint32_t blo = lo0 + r.s * ((uint32_t)g.w2_piece >> 4), ha = hid + 32 * k2;
+        const int ks = (p.H >> 4) - 4 * k2;
+        umma_bf16_ta(acc, ha, hi | blo, idesc, k2);
+        if (ks > 1) umma_bf16_ta(acc, ha + 8, hi | (blo + 2), idesc, 1);
+        if (ks > 2) umma_bf16_ta(acc, ha + 16, hi | (blo + 4), idesc, 1);
+        if (ks > 3) umma_bf16_ta(acc, ha + 24, hi | (blo + 6), idesc, 1);
+        umma_commit(smem_u32(&c->empty2[r.s]));
+        r.next(g.ns2);
+      }
       umma_commit(smem_u32(&c->acc2_full[b]));
-      umma_commit(smem_u32(&c->empty2[r.s]));
-      r.next(g.ns2);
+      ar.next(ctx, g.nd);
     }
     // the hidden tile has been read (gated form: the drain warps free the tile's columns)
     if (!GLU) umma_commit(smem_u32(&c->ctx_free[ctx]));
@@ -389,25 +539,18 @@ __device__ void role_ep1(const Params& p, Ctl* c, uint32_t tmem, int et) {
   volatile int* af = &c->abort_flag;
   const uint32_t lane_base = (uint32_t)(et & ~31) << 16;
   const int nord = p.norm_ord;
+  RingPos q = {0, 0};
   uint32_t ctx = 0, ph = 0;
-  for (int tile = blockIdx.x; tile < c->total_tiles; tile += gridDim.x) {
-    const Tile t = tile_info(p, c, tile);
-    // two copies of the bias alternate: a warp already on the next tile never overwrites pairs
-    // another warp still reads
-    uint32_t* bp = c->bias_s[ctx];
-    if (et < (p.H >> 1)) {
-      const float2 b = __ldg(reinterpret_cast<const float2*>(p.packed + (long long)t.e * p.g.stride +
-                                                             p.g.bias_off) + et);
-      bp[et] = pack_bf16x2(b.x, b.y);
-    }
-    asm volatile("bar.sync 2, 128;" ::: "memory");
-    // labels by-product (intermediate layer): this thread's row, its token loaded up front
+  for (;; q.next(TILE_RING)) {
+    if (!mbar_wait_fast(smem_u32(&c->tile_full[q.s]), q.ph, af, p.dev_status)) return;
+    const Tile* t = &c->tile[q.s];
+    const int e = t->e;
+    if (e < 0) return;
+    if (!mbar_wait_fast(smem_u32(&c->direct_full[q.s]), q.ph, af, p.dev_status)) return;
+    const uint32_t* bp = t->bias;
+    // labels by-product (intermediate layer): this thread's row
     float nacc = 0.f;
-    int ntok = -1;
-    if (NORM) {
-      if (!mbar_wait_fast(smem_u32(&c->list_full[ctx]), ph, af, p.dev_status)) return;
-      ntok = c->list[ctx][et];
-    }
+    const int ntok = NORM ? t->list[et] : -1;
     if (!mbar_wait_fast(smem_u32(&c->acc1_full[ctx]), ph, af, p.dev_status)) return;
     tc_fence_after();
     const uint32_t acc = tm_tile<GLU>(tmem, ctx) + lane_base;
@@ -425,9 +568,11 @@ __device__ void role_ep1(const Params& p, Ctl* c, uint32_t tmem, int et) {
     }
     tmem_wait_st();
     tc_fence_before();
+    __syncwarp();
+    if ((et & 31) == 0) mbar_arrive(smem_u32(&c->tile_empty[q.s]));
     mbar_arrive(smem_u32(&c->hid_full[ctx]));
     if (NORM && ntok != -1)
-      p.norms[(long long)t.e * p.N + (ntok & 0x7fffffff)] =
+      p.norms[(long long)e * p.N + ntok] =
           __float2bfloat16_rn(nord == 1 ? nacc : sqrtf(nacc));
     ph ^= ctx;
     ctx ^= 1;
@@ -458,56 +603,67 @@ __device__ __forceinline__ void role_ep1_act(const Params& p, Ctl* c, uint32_t t
   }
 }
 
-// Warps 4-11: drain group j takes every other step; warp q4 of it rows 32 q4 .. +31.
+// Warps 4-11: warp q4 of group j has rows 32 q4 .. +31 and 64 columns: with 128-column steps the two
+// groups share each one, with 64-column steps they take every other one.
 // Thread = row out of tensor memory; through the warp's own 4 KB the 64 columns are turned into
 // 8 lanes per row, so that one instruction covers 4 whole 128-byte lines of the output.
-// The loop is straight-line code: with the norm terms and the store / add choice as branches inside
-// it, a step of some 150 instructions took 2900 cycles, most of them waiting for instructions
-// (twenty warps in eight different loops share the instruction caches).
 template <bool GLU, bool NORM>
 __device__ void role_drain(const Params& p, Ctl* c, uint32_t stg, uint32_t tmem, int j, int q4,
                            int lane) {
   volatile int* af = &c->abort_flag;
-  const uint32_t lane_base = (uint32_t)(q4 * 32) << 16;
+  const Geo& g = p.g;
   const uint32_t blk = stg + (j * 4 + q4) * 4096;
   const uint32_t wr = blk + lane * 128, x7 = lane & 7;
   const int rl = lane >> 3, pl = lane & 7;
   const int nord = p.norm_ord;
-  uint32_t ctx = 0, ph = 0, step = 0, uses = 0;    // uses: bit b = parity of buffer b's uses so far
-  for (int tile = blockIdx.x; tile < c->total_tiles; tile += gridDim.x) {
-    const Tile t = tile_info(p, c, tile);
-    if (!mbar_wait_fast(smem_u32(&c->list_full[ctx]), ph, af, p.dev_status)) return;
-    const int* list = c->list[ctx] + q4 * 32;
+  const bool wide = g.nd == 128;
+  const int col0 = wide ? 64 * j : 0;                // my columns of a step
+  const uint32_t src0 = ((uint32_t)(q4 * 32) << 16) + col0;
+  Acc2Ring<GLU> ar;
+  RingPos q = {0, 0};
+  uint32_t ctx = 0;
+  int turn = wide ? j : 0;                           // group whose step is next
+  uint32_t nph = 0;
+  for (;; q.next(TILE_RING)) {
+    if (!mbar_wait_fast(smem_u32(&c->tile_full[q.s]), q.ph, af, p.dev_status)) return;
+    const Tile* t = &c->tile[q.s];
+    const int e = t->e, n0 = t->n0, n1 = t->n1;
+    if (e < 0) return;
+    if (!mbar_wait_fast(smem_u32(&c->direct_full[q.s]), q.ph, af, p.dev_status)) return;
+    const uint32_t direct = t->direct[q4];
     int rt[8];
 #pragma unroll
-    for (int it = 0; it < 8; ++it) rt[it] = list[it * 4 + rl];
-    const int mine = list[lane];
-    const bool any_direct = __any_sync(0xffffffffu, mine < -1);
-    // (epilogue 1 reads the list as well where it collects norms: keep it until the tile is done)
+    for (int it = 0; it < 8; ++it) {     // sign bit: the row is stored
+      const uint32_t v = (uint32_t)t->list[q4 * 32 + it * 4 + rl];
+      rt[it] = (int)(v | (((direct >> (it * 4 + rl)) & 1u) << 31));
+    }
+    const int mine = NORM ? t->list[q4 * 32 + lane] : -1;
     __syncwarp();
-    if (lane == 0 && p.norm_layer == 0) mbar_arrive(smem_u32(&c->list_empty[ctx]));
+    if (lane == 0) mbar_arrive(smem_u32(&c->tile_empty[q.s]));
     float nacc = 0.f;
-    if (GLU) step = 0;
-    const int first = t.n0 + ((step + j) & 1);       // my first step of this tile
-    const uint32_t step0 = step;
-    step += t.n1 - t.n0;
-    for (int n = first; n < t.n1; n += 2) {
-      const uint32_t q = step0 + (n - t.n0), b = GLU ? 2 * ctx + (q & 1) : q & 3;
-      bf16* o = p.out + n * ND + pl * 8;
+    for (int n = n0; n < n1; ++n) {
+      const bool skip = turn != j;
+      if (!wide) turn ^= 1;
+      if (skip) {
+        ar.next(ctx, g.nd);
+        continue;
+      }
+      const int col = n * g.nd + col0 + pl * 8;
       uint4 bz = make_uint4(0u, 0u, 0u, 0u);
-      if (any_direct && p.last_bias)
-        bz = __ldg(reinterpret_cast<const uint4*>(p.last_bias + n * ND + pl * 8));
-      if (!mbar_wait_fast(smem_u32(&c->acc2_full[b]), (uses >> b) & 1, af, p.dev_status)) return;
-      uses ^= 1u << b;
+      if (direct != 0u && p.last_bias)
+        bz = __ldg(reinterpret_cast<const uint4*>(p.last_bias + col));
+      const uint32_t b = ar.slot(ctx);
+      if (!mbar_wait_fast(smem_u32(&c->acc2_full[b]), ar.at(ctx).ph, af, p.dev_status)) return;
       tc_fence_after();
       uint32_t v[64];
-      const uint32_t acc = tm_acc2<GLU>(tmem, b) + lane_base;
+      const uint32_t acc = ar.column(tmem, ctx, g.nd) + src0;
       tmem_ld32(acc, v);
       tmem_ld32(acc + 32, v + 32);
       tmem_wait_ld();
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&c->acc2_empty[b]));
+      ar.next(ctx, g.nd);
 #pragma unroll
       for (int pc = 0; pc < 8; ++pc) {      // piece XOR row: conflict-free 16-byte stores
         uint32_t ww[4];
@@ -532,7 +688,8 @@ __device__ void role_drain(const Params& p, Ctl* c, uint32_t stg, uint32_t tmem,
         val[it] = ld_shared_v4(blk + rr * 128 + ((pl ^ (rr & 7)) << 4));
       }
       __syncwarp();
-      if (any_direct) {
+      bf16* o = p.out + col;
+      if (direct != 0u) {
 #pragma unroll
         for (int it = 0; it < 8; ++it)
           put_row(o + (size_t)(rt[it] & 0x7fffffff) * p.d, rt[it], val[it],
@@ -543,23 +700,28 @@ __device__ void role_drain(const Params& p, Ctl* c, uint32_t stg, uint32_t tmem,
           put_row(o + (size_t)(rt[it] & 0x7fffffff) * p.d, rt[it], val[it], val[it]);
       }
     }
-    // every read of this context's tensor memory by this warp is done
-    __syncwarp();
-    if (lane == 0) {
-      if (GLU) mbar_arrive(smem_u32(&c->ctx_free[ctx]));
-      if (p.norm_layer != 0) mbar_arrive(smem_u32(&c->list_empty[ctx]));
+    // every read of this tile's tensor memory by this warp is done
+    if (GLU) {
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&c->ctx_free[ctx]));
     }
     if (NORM) {
-      // the other group saw the other steps of the same rows
-      if (j == 1) c->npart[q4 * 32 + lane] = nacc;
-      asm volatile("bar.sync 3, 256;" ::: "memory");
-      if (j == 0) nacc += c->npart[q4 * 32 + lane];
-      asm volatile("bar.sync 3, 256;" ::: "memory");
-      if (mine != -1 && j == 0)
-        p.norms[(long long)t.e * p.N + (mine & 0x7fffffff)] =
-            __float2bfloat16_rn(nord == 1 ? nacc : sqrtf(nacc));
+      // the other group saw the other columns of the same rows
+      const uint32_t nf = smem_u32(&c->np_full[q4]), ne = smem_u32(&c->np_empty[q4]);
+      if (j == 1) {
+        if (!mbar_wait_fast(ne, nph ^ 1, af, p.dev_status)) return;
+        c->npart[q4 * 32 + lane] = nacc;
+        mbar_arrive(nf);
+      } else {
+        if (!mbar_wait_fast(nf, nph, af, p.dev_status)) return;
+        nacc += c->npart[q4 * 32 + lane];
+        mbar_arrive(ne);
+        if (mine != -1)
+          p.norms[(long long)e * p.N + mine] =
+              __float2bfloat16_rn(nord == 1 ? nacc : sqrtf(nacc));
+      }
+      nph ^= 1;
     }
-    ph ^= ctx;
     ctx ^= 1;
   }
 }
@@ -567,82 +729,6 @@ __device__ void role_drain(const Params& p, Ctl* c, uint32_t stg, uint32_t tmem,
 // ---------------------------------------------------------------------------
 // kernel
 // ---------------------------------------------------------------------------
-// One warp cuts the lists into tiles.  Candidate sizes are eighths of the largest tile; a tile
-// costs its weights plus its rows' bytes, and the launch as many tiles as the fullest CTA
-// gets, so the size that fills the last round of the grid wins (524 rows per SM: five tiles of
-// 105 rows instead of four of 128 and one of 12).  Rates: 64 bytes per clock and SM for loads, 24 for the
-// output, measured on an SM's memory interface alone.
-__device__ void cut_tiles(const Params& p, Ctl* c, int lane) {
-  const int E = p.E, unit = TILE_M / 8;
-  int off[5], n[4];
-  bool all_n = true;                     // every expert of this lane lists exactly N tokens
-#pragma unroll
-  for (int q = 0; q < 5; ++q) {
-    const int e = 4 * lane + q;
-    off[q] = e <= E ? p.offsets[e] : 0;
-    if (e <= E) c->off[e] = off[q];
-  }
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const int e = 4 * lane + q;
-    n[q] = e < E ? off[q + 1] - off[q] : 0;
-    if (e < E && n[q] != p.N) all_n = false;
-    if (e < E && (n[q] < 0 || off[q] < 0 || off[q + 1] > p.N * (long long)E)) {
-      report(p.dev_status, D2D_ERR_INDEX_RANGE);
-      n[q] = 0;
-    }
-    n[q] = max(n[q], 0);
-  }
-  const unsigned grid = gridDim.x;
-  const unsigned fixed = (unsigned)(p.g.bias_off >> 6) + 2000, per_row = (unsigned)p.d / 8;
-  unsigned best_cost = 0xffffffffu, tiles = 0;
-  int best = 8;
-  for (int k = 8; k >= 1; --k) {
-    unsigned mine = 0;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) mine += (unsigned)(n[q] + k * unit - 1) / (unsigned)(k * unit);
-    const unsigned T = __reduce_add_sync(0xffffffffu, mine);
-    const unsigned cost = ((T + grid - 1) / grid) * (fixed + k * unit * per_row);
-    if (cost < best_cost) {
-      best_cost = cost;
-      best = k;
-      tiles = T;
-    }
-  }
-  const int size = best * unit;
-  int sum = 0, nt[4];
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const int e = 4 * lane + q;
-    nt[q] = (n[q] + size - 1) / size;
-    if (e < E) c->rows[e] = nt[q] > 0 ? (n[q] + nt[q] - 1) / nt[q] : 1;   // equal tiles
-    sum += nt[q];
-  }
-  int incl = sum;
-  for (int o = 1; o < 32; o <<= 1) {
-    const int v = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += v;
-  }
-  int run = incl - sum;
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const int e = 4 * lane + q;
-    if (e <= E) c->tstart[e] = run;
-    run += nt[q];
-  }
-  const bool dense = __all_sync(0xffffffffu, all_n) && E > 1;
-  if (lane == 0) {
-    // fewer than half as many tiles as CTAs: split the output columns (the first product is
-    // repeated, the second product, W2 and the output are shared out)
-    int parts = tiles > 0 ? (int)(grid / tiles) : 1;
-    parts = max(1, min(parts, p.g.nc));
-    if (p.norm_layer != 0) parts = 1;
-    c->parts = parts;
-    c->total_tiles = (int)tiles * parts;
-    c->dense_e = dense ? E : 0;
-  }
-}
-
 // NORM: 0 none, D2D_NORM_OF_INTERMEDIATE, D2D_NORM_OF_OUTPUT
 template <bool GLU, int NORM>
 __global__ void __launch_bounds__(NTHREADS, 1) experts_tiles_kernel(const Params p) {
@@ -650,7 +736,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) experts_tiles_kernel(const Params
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t ring = (raw + 1023u) & ~1023u;
   const uint32_t ring2 = ring + p.g.ns * p.g.stage;
-  const uint32_t stg = ring2 + p.g.ns2 * p.g.w2_stage;
+  const uint32_t stg = ring2 + p.g.ns2 * p.g.w2_piece;
   Ctl* c = reinterpret_cast<Ctl*>(smem_raw + (stg - raw) + STG);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // Programmatic dependent launch: see router_tiles_kernel.
@@ -669,12 +755,18 @@ __global__ void __launch_bounds__(NTHREADS, 1) experts_tiles_kernel(const Params
       mbar_init(smem_u32(&c->acc1_full[i]), 1);
       mbar_init(smem_u32(&c->ctx_free[i]), GLU ? 8 : 1);
       mbar_init(smem_u32(&c->hid_full[i]), 128);
-      mbar_init(smem_u32(&c->list_full[i]), 128);
-      mbar_init(smem_u32(&c->list_empty[i]), 8);
     }
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < TILE_RING; ++i) {
+      mbar_init(smem_u32(&c->tile_full[i]), 32);
+      mbar_init(smem_u32(&c->direct_full[i]), 32);
+      mbar_init(smem_u32(&c->tile_empty[i]), TILE_READERS);
+      mbar_init(smem_u32(&c->np_full[i]), 32);
+      mbar_init(smem_u32(&c->np_empty[i]), 32);
+    }
+    static_assert(TILE_RING == 4, "np barriers: one per row quarter");
+    for (int i = 0; i < 6; ++i) {
       mbar_init(smem_u32(&c->acc2_full[i]), 1);
-      mbar_init(smem_u32(&c->acc2_empty[i]), 4);
+      mbar_init(smem_u32(&c->acc2_empty[i]), p.g.nd >> 4);    // four warps per 64 columns
     }
     c->abort_flag = 0;
     c->wait_limit = (int)p.wait_limit;
@@ -682,12 +774,11 @@ __global__ void __launch_bounds__(NTHREADS, 1) experts_tiles_kernel(const Params
     fence_proxy_async();
   }
   if (warp == WARP_MMA1) tmem_alloc(smem_u32(&c->tmem_base), 512);
-  grid_dependency_wait();
-  if (warp == 1) cut_tiles(p, c, lane);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = c->tmem_base;
+  if (warp <= WARP_W) grid_dependency_wait();
 
   if (warp < WARP_DRAIN0) {
     role_ep1_act<GLU, NORM == D2D_NORM_OF_INTERMEDIATE>(p, c, tmem, tid);
@@ -703,12 +794,11 @@ __global__ void __launch_bounds__(NTHREADS, 1) experts_tiles_kernel(const Params
   } else if (warp == WARP_MMA2) {
     if (elect_one()) role_mma2<GLU>(p, c, ring2, tmem);
     __syncwarp();
-  } else if (warp == WARP_W1) {
-    if (elect_one()) role_w1(p, c, ring);
+  } else if (warp == WARP_W) {
+    if (elect_one()) role_weights(p, c, ring, ring2);
     __syncwarp();
   } else {
-    if (elect_one()) role_w2(p, c, ring2);
-    __syncwarp();
+    role_list(p, c, lane, (long long)p.E * p.g.stride > L2_WEIGHTS);
   }
 
   // A launch that gave up may still have copies and MMAs in flight that use this CTA's
@@ -726,7 +816,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) experts_tiles_kernel(const Params
 
 // Weights packed once into exactly the shared-memory images the MMA reads (K-major, 128-byte
 // swizzle), so that a stage's weights are one contiguous bulk copy: per expert the 64-deep slices
-// of W1 (gated form: H gate rows, then H up rows), the 64-column x 64-deep pieces of W2, b1 in fp32.
+// of W1 (gated form: H gate rows, then H up rows), the nd-column x 64-deep pieces of W2, b1 in fp32.
 __global__ void prepack_experts_kernel(const bf16* __restrict__ w1, const bf16* __restrict__ b1,
                                        const bf16* __restrict__ w_up, const bf16* __restrict__ w2,
                                        uint8_t* __restrict__ packed, Geo g, int d, int E, int H) {
@@ -734,7 +824,7 @@ __global__ void prepack_experts_kernel(const bf16* __restrict__ w1, const bf16* 
   uint8_t* pe = packed + (long long)e * g.stride;
   const int rows1 = g.w1_stage >> 7;
   const long long n1 = (long long)g.kc1 * rows1 * 64;
-  const long long n2 = (long long)g.nc * g.kc2 * ND * 64;
+  const long long n2 = (long long)g.nc * g.kc2 * g.nd * 64;
   const bf16 zero = __float2bfloat16_rn(0.f);
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n1 + n2 + H;
        i += (long long)gridDim.x * blockDim.x) {
@@ -748,13 +838,13 @@ __global__ void prepack_experts_kernel(const bf16* __restrict__ w1, const bf16* 
       *reinterpret_cast<bf16*>(pe + (long long)kc * g.w1_stage + swz(n, k)) = v;
     } else if (i < n1 + n2) {
       const long long q = i - n1;
-      const int n = (int)(q % ND);
-      const int k = (int)((q / ND) % 64);
-      const int k2 = (int)((q / (64LL * ND)) % g.kc2);
-      const int nci = (int)(q / (64LL * ND * g.kc2));
+      const int n = (int)(q % g.nd);
+      const int k = (int)((q / g.nd) % 64);
+      const int k2 = (int)((q / (64LL * g.nd)) % g.kc2);
+      const int nci = (int)(q / (64LL * g.nd * g.kc2));
       const int kk = k2 * 64 + k;
-      const bf16 v = kk < H ? w2[((long long)e * H + kk) * d + nci * ND + n] : zero;
-      *reinterpret_cast<bf16*>(pe + g.w1_bytes + (long long)(nci * g.kc2 + k2) * (ND * 128) +
+      const bf16 v = kk < H ? w2[((long long)e * H + kk) * d + nci * g.nd + n] : zero;
+      *reinterpret_cast<bf16*>(pe + g.w1_bytes + (long long)(nci * g.kc2 + k2) * g.w2_piece +
                                swz(n, k)) = v;
     } else {
       const int h = (int)(i - n1 - n2);
@@ -818,7 +908,7 @@ int launch_experts_umma(const void* x, const int32_t* token_idx, const int32_t* 
   p.norm_ord = nc.ord;
   umma_debug_read(&p.wait_limit, &p.withhold);
   const size_t smem =
-      1024 + (size_t)p.g.ns * p.g.stage + (size_t)p.g.ns2 * p.g.w2_stage + STG + sizeof(Ctl) + 64;
+      1024 + (size_t)p.g.ns * p.g.stage + (size_t)p.g.ns2 * p.g.w2_piece + STG + sizeof(Ctl) + 64;
   auto kernel = glu ? (p.norm_layer == 0                          ? experts_tiles_kernel<true, 0>
                        : p.norm_layer == D2D_NORM_OF_INTERMEDIATE ? experts_tiles_kernel<true, 1>
                                                                   : experts_tiles_kernel<true, 2>)
