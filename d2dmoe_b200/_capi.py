@@ -43,6 +43,9 @@ SIGNATURES = {
                                    _i64, _i, _i, _i, _i, _i, _p, _p]),
     "d2d_moe_forward": (_i, [_p, _p, _p, _p, _p, _f, _p, _p, _p, _p, _p, _p, _i, _p,
                              _p, _p, _p, _i64, _i, _i, _i, _i, _i, _i, _p, _sz, _p, _p, _p]),
+    "d2d_moe_forward_rule": (_i, [_p, _p, _p, _p, _p, _p, _i, _i, _f, _f, _p, _p, _p, _p, _p, _p, _i,
+                                  _p, _p, _p, _p, _i64, _i, _i, _i, _i, _i, _i, _p, _sz, _p, _p,
+                                  _p, _i, _i, _p]),
     "d2d_prepack_experts_bytes": (_i, [_i, _i, _i, _i, _i, C.POINTER(_sz)]),
     "d2d_prepack_experts": (_i, [_p, _p, _p, _p, _p, _i, _i, _i, _i, _p]),
     "d2d_prepack_router_bytes": (_i, [_i, _i, _i, _i, C.POINTER(_sz)]),

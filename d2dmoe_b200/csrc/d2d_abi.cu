@@ -188,19 +188,21 @@ int d2d_experts_ffn_norms(const void* x, const int32_t* token_idx, const int32_t
                           dev_status, stream);
 }
 
-int d2d_moe_forward(const void* x, const void* wa, const void* wb, const void* router_packed_opt,
-                    const void* scores_in_opt, float thresh_mult, const void* w1,
-                    const void* b1_opt, const void* w_up_opt, const void* w2,
-                    const void* experts_packed_opt, const void* last_bias_opt, int add_residual,
-                    void* out, uint32_t* mask_bits, int32_t* token_idx, int32_t* offsets,
-                    int64_t N, int d, int R, int E, int H, int act, int dtype, void* ws,
-                    size_t ws_bytes, int* dev_status, void* routing_tensor_opt,
-                    d2d_stream_t stream) {
-  int rc, nl = 0;
-  bool counts_ready = false, rt_done = routing_tensor_opt == nullptr;
-  DirectRows dr;
+int d2d_moe_forward_rule(const void* x, const void* wa, const void* wb,
+                         const void* router_packed_opt, const void* scores_in_opt,
+                         void* scores_scratch, int rule, int k, float tau, float thresh_mult,
+                         const void* w1, const void* b1_opt, const void* w_up_opt, const void* w2,
+                         const void* experts_packed_opt, const void* last_bias_opt,
+                         int add_residual, void* out, uint32_t* mask_bits, int32_t* token_idx,
+                         int32_t* offsets, int64_t N, int d, int R, int E, int H, int act,
+                         int dtype, void* ws, size_t ws_bytes, int* dev_status,
+                         void* routing_tensor_opt, void* norms_opt, int norm_layer, int norm_ord,
+                         d2d_stream_t stream) {
+  int rc = D2D_OK, nl = 0;
+  cudaStream_t s = (cudaStream_t)stream;
   g_last_forward_launches = 0;
-  if (!wa && !scores_in_opt) return D2D_ERR_BAD_ARG;
+  if (rule < D2D_RULE_MAX || rule > D2D_RULE_ALL) return D2D_ERR_BAD_ARG;
+  if (rule != D2D_RULE_ALL && !wa && !scores_in_opt) return D2D_ERR_BAD_ARG;
   if (!mask_bits || !token_idx || !offsets || !ws || !aligned(ws, 16)) return D2D_ERR_BAD_ARG;
   // every argument check of the later stages comes before the first launch
   if (!x || !w1 || !w2 || !out || N < 0 || d < 1 || E < 1 || H < 1) return D2D_ERR_BAD_ARG;
@@ -210,6 +212,19 @@ int d2d_moe_forward(const void* x, const void* wa, const void* wb, const void* r
   if (!dtype_ok(dtype) || act < D2D_RELU || act > D2D_GELU_TANH) return D2D_ERR_UNSUPPORTED;
   if (ws_bytes < compact_workspace_bytes(N, E)) return D2D_ERR_WORKSPACE;
   if (add_residual < 0 || add_residual > D2D_OUT_PREINITIALISED) return D2D_ERR_BAD_ARG;
+  if (rule == D2D_RULE_TOPK && (k < 1 || k > E)) return D2D_ERR_BAD_ARG;
+  const bool ranked = rule == D2D_RULE_TOPK || rule == D2D_RULE_DYNK;
+  if (ranked && !scores_in_opt && !scores_scratch) return D2D_ERR_BAD_ARG;
+  if (rule != D2D_RULE_ALL && !scores_in_opt && (!wb || R < 1)) return D2D_ERR_BAD_ARG;
+  NormCapture nc;
+  if (norms_opt) {
+    if (rule != D2D_RULE_ALL || !aligned(norms_opt, 4) || (norm_ord != 1 && norm_ord != 2) ||
+        (norm_layer != D2D_NORM_OF_INTERMEDIATE && norm_layer != D2D_NORM_OF_OUTPUT))
+      return D2D_ERR_BAD_ARG;
+    nc.norms = norms_opt;
+    nc.layer = norm_layer;
+    nc.ord = norm_ord;
+  }
   if (N == 0) return D2D_OK;
   // out already initialised by the caller (d2d_prenorm_init): the first kernel writes no rows
   const bool pre = add_residual == D2D_OUT_PREINITIALISED;
@@ -220,67 +235,112 @@ int d2d_moe_forward(const void* x, const void* wa, const void* wb, const void* r
   }
   const bool umma_experts = experts_packed_opt && aligned(experts_packed_opt, 1024) &&
                             umma_experts_supported(d, E, H, w_up_opt != nullptr, dtype);
-  if (scores_in_opt) {
+  const bool umma_router = router_packed_opt && umma_router_supported(d, R, E, dtype) &&
+                           aligned(last_bias_opt, 16) && aligned(router_packed_opt, 1024);
+  // where the tensor-core expert kernel follows, the rows of tokens with one expert are left to it
+  DirectRows dr;
+  const bool may_store = !pre && !add_residual && umma_experts && aligned(last_bias_opt, 16);
+  auto leave_rows = [&]() {
+    dr.mask_bits = mask_bits;
+    dr.last_bias = last_bias_opt;
+  };
+  bool counts_ready = false, lists_ready = false, rt_done = routing_tensor_opt == nullptr;
+  const void* scores = scores_in_opt;
+
+  if (rule == D2D_RULE_ALL) {
+    rc = launch_all_experts(mask_bits, routing_tensor_opt, token_idx, offsets, x, last_bias_opt,
+                            add_residual, out_init, N, d, E, dtype, s);
+    if (rc == D2D_ERR_UNSUPPORTED && out_init) {     // rows that need the scalar initial value
+      rc = launch_init_out(x, last_bias_opt, add_residual, out, N, d, dtype, s);
+      nl += 1;
+      if (rc == D2D_OK)
+        rc = launch_all_experts(mask_bits, routing_tensor_opt, token_idx, offsets, x, nullptr, 0,
+                                nullptr, N, d, E, dtype, s);
+    }
+    nl += 1;
+    lists_ready = rt_done = true;
+  } else if (ranked && !scores) {
+    // scores of the fused router for the rule below; its own mask is overwritten there
+    rc = umma_router
+             ? launch_router_mask_umma(x, router_packed_opt, thresh_mult, mask_bits,
+                                       scores_scratch, nullptr, nullptr, nullptr, nullptr, true,
+                                       nullptr, N, d, R, E, dev_status, s)
+             : launch_router_mask_simt(x, wa, wb, thresh_mult, mask_bits, scores_scratch, nullptr,
+                                       0, nullptr, N, d, R, E, dtype, dev_status, s);
+    nl += 1;
+    scores = scores_scratch;
+  }
+  if (rc != D2D_OK) return rc;
+
+  if (scores && rule != D2D_RULE_ALL) {
     // rule + counts table + output init in one launch when the shape allows it
-    rc = launch_gate_scores_fused(scores_in_opt, thresh_mult, mask_bits, routing_tensor_opt,
-                                  (int32_t*)ws, x, last_bias_opt, add_residual, out_init, N, d, E,
-                                  dtype, (cudaStream_t)stream);
+    rc = launch_gate_scores_fused(scores, rule, k, tau, thresh_mult, mask_bits,
+                                  routing_tensor_opt, (int32_t*)ws, x, last_bias_opt, add_residual,
+                                  out_init, may_store, N, d, E, dtype, s);
     if (rc == D2D_OK) {
-      counts_ready = true;
-      rt_done = true;
+      counts_ready = rt_done = true;
+      if (may_store) leave_rows();
       nl += 1;
     } else if (rc == D2D_ERR_UNSUPPORTED) {
-      rc = d2d_mask_from_scores(scores_in_opt, thresh_mult, mask_bits, N, E, dtype, dev_status,
-                                stream);
+      rc = ranked ? launch_gate_rule(scores, rule, k, tau, mask_bits, N, E, dtype, s)
+                  : launch_mask_from_scores(scores, thresh_mult, mask_bits, N, E, dtype,
+                                            dev_status, s);
       if (rc != D2D_OK) return rc;
       nl += 1;
       if (!pre) {
-        rc = d2d_init_out(x, last_bias_opt, add_residual, out, N, d, dtype, stream);
+        rc = launch_init_out(x, last_bias_opt, add_residual, out, N, d, dtype, s);
         nl += 1;
       }
     }
-  } else if (router_packed_opt && wb && R >= 1 && umma_router_supported(d, R, E, dtype) &&
-             aligned(last_bias_opt, 16) && aligned(router_packed_opt, 1024)) {
-    // the tensor-core router also fills the compaction's counts table; where the tensor-core
-    // expert kernel follows it leaves the rows of tokens with one expert to that kernel
-    const void* resid = add_residual ? x : nullptr;
-    if (!pre && !resid && umma_experts) {
-      dr.mask_bits = mask_bits;
-      dr.last_bias = last_bias_opt;
-    }
+  } else if (rule == D2D_RULE_MAX && umma_router) {
+    // the tensor-core router also fills the compaction's counts table
     rc = launch_router_mask_umma(x, router_packed_opt, thresh_mult, mask_bits, nullptr,
-                                 routing_tensor_opt, last_bias_opt, resid, out_init,
-                                 dr.mask_bits == nullptr, (int32_t*)ws, N, d, R, E, dev_status,
-                                 (cudaStream_t)stream);
-    counts_ready = true;
-    rt_done = true;
+                                 routing_tensor_opt, last_bias_opt, add_residual ? x : nullptr,
+                                 out_init, !may_store, (int32_t*)ws, N, d, R, E, dev_status, s);
+    if (may_store) leave_rows();
+    counts_ready = rt_done = true;
     nl += 1;
-  } else {
+  } else if (rule == D2D_RULE_MAX) {
     // general-shape router: mask bits, routing tensor and the output's initial value
-    if (!wb || R < 1) return D2D_ERR_BAD_ARG;
     rc = launch_router_mask_simt(x, wa, wb, thresh_mult, mask_bits, nullptr, last_bias_opt,
-                                 add_residual, out_init, N, d, R, E, dtype, dev_status,
-                                 (cudaStream_t)stream, routing_tensor_opt);
+                                 add_residual, out_init, N, d, R, E, dtype, dev_status, s,
+                                 routing_tensor_opt);
     rt_done = true;
     nl += 1;
   }
   if (rc != D2D_OK) return rc;
-  rc = launch_compact(mask_bits, token_idx, offsets, N, E, (int32_t*)ws, dev_status,
-                      (cudaStream_t)stream, counts_ready);
-  if (rc != D2D_OK) return rc;
-  nl += counts_ready ? 1 : 2;      // [count,] scatter
+  if (!lists_ready) {
+    rc = launch_compact(mask_bits, token_idx, offsets, N, E, (int32_t*)ws, dev_status, s,
+                        counts_ready);
+    if (rc != D2D_OK) return rc;
+    nl += counts_ready ? 1 : 2;    // [count,] scatter
+  }
   if (!rt_done) {                  // paths whose first kernel does not write the routing tensor
-    rc = launch_expand_mask(mask_bits, routing_tensor_opt, N, E, dtype, (cudaStream_t)stream);
+    rc = launch_expand_mask(mask_bits, routing_tensor_opt, N, E, dtype, s);
     if (rc != D2D_OK) return rc;
     nl += 1;
   }
   g_last_forward_launches = nl + 1;
   if (umma_experts)
     return launch_experts_umma(x, token_idx, offsets, experts_packed_opt, out, N, d, E, H,
-                               w_up_opt != nullptr, act, dev_status, (cudaStream_t)stream,
-                               NormCapture(), dr);
+                               w_up_opt != nullptr, act, dev_status, s, nc, dr);
   return launch_experts_simt(x, token_idx, offsets, w1, b1_opt, w_up_opt, w2, out, N, d, E, H, act,
-                             dtype, dev_status, (cudaStream_t)stream);
+                             dtype, dev_status, s, nc);
+}
+
+int d2d_moe_forward(const void* x, const void* wa, const void* wb, const void* router_packed_opt,
+                    const void* scores_in_opt, float thresh_mult, const void* w1,
+                    const void* b1_opt, const void* w_up_opt, const void* w2,
+                    const void* experts_packed_opt, const void* last_bias_opt, int add_residual,
+                    void* out, uint32_t* mask_bits, int32_t* token_idx, int32_t* offsets,
+                    int64_t N, int d, int R, int E, int H, int act, int dtype, void* ws,
+                    size_t ws_bytes, int* dev_status, void* routing_tensor_opt,
+                    d2d_stream_t stream) {
+  return d2d_moe_forward_rule(x, wa, wb, router_packed_opt, scores_in_opt, nullptr, D2D_RULE_MAX,
+                              0, 0.f, thresh_mult, w1, b1_opt, w_up_opt, w2, experts_packed_opt,
+                              last_bias_opt, add_residual, out, mask_bits, token_idx, offsets, N,
+                              d, R, E, H, act, dtype, ws, ws_bytes, dev_status,
+                              routing_tensor_opt, nullptr, 0, 0, stream);
 }
 
 int d2d_last_forward_launches(void) { return g_last_forward_launches; }

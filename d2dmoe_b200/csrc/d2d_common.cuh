@@ -162,10 +162,15 @@ int launch_gate_rule(const void* scores, int rule, int k, float tau, uint32_t* m
                      int64_t N, int E, int dtype, cudaStream_t s);
 int launch_mask_from_scores(const void* scores, float mult, uint32_t* mask_bits, int64_t N, int E,
                             int dtype, int* dev_status, cudaStream_t s);
-int launch_gate_scores_fused(const void* scores, float mult, uint32_t* mask_bits, void* rt,
-                             int32_t* tile_counts, const void* x, const void* last_bias,
-                             int add_residual, void* out, int64_t N, int d, int E, int dtype,
-                             cudaStream_t s);
+// rule 0: dynk_max with threshold multiplier mult; D2D_RULE_TOPK (k), D2D_RULE_DYNK (tau).
+// direct: initial rows only of tokens not kept by exactly one expert
+int launch_gate_scores_fused(const void* scores, int rule, int k, float tau, float mult,
+                             uint32_t* mask_bits, void* rt, int32_t* tile_counts, const void* x,
+                             const void* last_bias, int add_residual, void* out, bool direct,
+                             int64_t N, int d, int E, int dtype, cudaStream_t s);
+int launch_all_experts(uint32_t* mask_bits, void* rt, int32_t* token_idx, int32_t* offsets,
+                       const void* x, const void* last_bias, int add_residual, void* out,
+                       int64_t N, int d, int E, int dtype, cudaStream_t s);
 int launch_init_out(const void* x, const void* last_bias, int add_residual, void* out, int64_t N,
                     int d, int dtype, cudaStream_t s);
 int launch_prenorm_init(const void* x, const void* gamma, const void* beta, float eps, int kind,

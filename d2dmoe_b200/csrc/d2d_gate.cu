@@ -316,53 +316,66 @@ gate_rule_kernel(const T* __restrict__ scores, int rule, int k, float tau,
   }
 }
 
-// The rule on given scores, fused with what the layer needs next: the compaction's counts
-// table (per 128-token tile) and the output's initial value.  One CTA = one 128-token
-// tile; warp w handles tokens 16w..16w+15 (lane = expert), then all threads write the
-// tile's initial output rows with 16-byte stores.  Needs d % (16/sizeof(T)) == 0.
+// The initial rows of a 128-token tile's output, T(last_bias + x): warp w of eight writes rows w,
+// w + 8, ... of those whose bit in `rows` is set (null: all); a lane keeps its 16-byte column
+// pieces of last_bias in registers.
+template <typename T>
+__device__ __forceinline__ void init_tile_rows(const T* x, const T* last_bias, int add_residual,
+                                               T* out, int64_t t0, int n, int d,
+                                               const uint32_t* rows, int w, int lane) {
+  constexpr int V = 16 / sizeof(T);
+  for (int cv = lane; cv < d / V; cv += 32) {
+    uint4 bz = make_uint4(0u, 0u, 0u, 0u);
+    if (last_bias) bz = __ldg(reinterpret_cast<const uint4*>(last_bias) + cv);
+#pragma unroll 4
+    for (int r = w; r < n; r += NT / 32) {
+      if (rows && !((rows[r >> 5] >> (r & 31)) & 1u)) continue;
+      uint4 o = bz;
+      if (add_residual) {
+        const uint4 xv = __ldg(reinterpret_cast<const uint4*>(x + (t0 + r) * d) + cv);
+        const T* a = reinterpret_cast<const T*>(&bz);
+        const T* b = reinterpret_cast<const T*>(&xv);
+        T rr[V];
+#pragma unroll
+        for (int q = 0; q < V; ++q)
+          rr[q] = DT<T>::from_f(DT<T>::to_f(a[q]) + DT<T>::to_f(b[q]));
+        o = *reinterpret_cast<const uint4*>(rr);
+      }
+      *(reinterpret_cast<uint4*>(out + (t0 + r) * d) + cv) = o;
+    }
+  }
+}
+
+// The dynk_max rule on given scores, fused with what the layer needs next: the compaction's counts
+// table (per 128-token tile) and the output's initial rows, all of them or (`direct`) those
+// of tokens not kept by exactly one expert (the expert kernel stores the others).  One CTA = one
+// 128-token tile; warp w handles tokens 16w..16w+15 (lane = expert).  Needs
+// d % (16/sizeof(T)) == 0.
 template <typename T>
 __global__ void __launch_bounds__(NT)
 gate_scores_fused_kernel(const T* __restrict__ scores, float mult,
                          uint32_t* __restrict__ mask_bits, T* __restrict__ rt,
                          uint8_t* __restrict__ tile_counts, int EP,
                          const T* __restrict__ x, const T* __restrict__ last_bias,
-                         int add_residual, T* __restrict__ out, int64_t N, int d, int E) {
+                         int add_residual, T* __restrict__ out, int direct, int64_t N, int d,
+                         int E) {
   __shared__ int cnt[256];
-  constexpr int V = 16 / sizeof(T);
+  __shared__ uint32_t rows[4];
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const int nw = (E + 31) / 32;
   const int64_t t0 = (int64_t)blockIdx.x * 128;
+  const int ntok = (int)min((int64_t)128, N - t0);
+  grid_launch_dependents();
   for (int e = tid; e < E; e += NT) cnt[e] = 0;
-  // the tile's initial output rows first: these stores depend on nothing the rule computes
-  // and drain while it runs.  Warp w writes rows w, w+8, ...; a lane keeps its 16-byte
-  // column pieces of last_bias in registers.
-  if (out) {
-    const int dv = d / V;
-    const int rows = (int)min((int64_t)128, N - t0);
-    for (int cv = lane; cv < dv; cv += 32) {
-      uint4 bz = make_uint4(0u, 0u, 0u, 0u);
-      if (last_bias) bz = __ldg(reinterpret_cast<const uint4*>(last_bias) + cv);
-#pragma unroll 4
-      for (int r = w; r < rows; r += NT / 32) {
-        uint4 o = bz;
-        if (add_residual) {
-          const uint4 xv = __ldg(reinterpret_cast<const uint4*>(x + (t0 + r) * d) + cv);
-          const T* a = reinterpret_cast<const T*>(&bz);
-          const T* b = reinterpret_cast<const T*>(&xv);
-          T rr[V];
-#pragma unroll
-          for (int q = 0; q < V; ++q)
-            rr[q] = DT<T>::from_f(DT<T>::to_f(a[q]) + DT<T>::to_f(b[q]));
-          o = *reinterpret_cast<const uint4*>(rr);
-        }
-        *(reinterpret_cast<uint4*>(out + (t0 + r) * d) + cv) = o;
-      }
-    }
-  }
+  if (tid < 4) rows[tid] = 0u;
+  grid_dependency_wait();
+  // all rows: first, their stores depend on nothing the rule computes and drain while it runs
+  if (out && !direct)
+    init_tile_rows(x, last_bias, add_residual, out, t0, ntok, d, nullptr, w, lane);
   __syncthreads();
   int mine[8] = {0, 0, 0, 0, 0, 0, 0, 0};       // kept-count of expert lane+32j over my tokens
-  // warp w applies the rule to tokens 16w..16w+15 (lane = expert); the scores of four tokens
-  // are loaded before the first of them is reduced, so the loads overlap
+  uint32_t init = 0u;                           // bit i: token 16 w + i wants its row initialised
+  // the scores of four tokens are loaded before the first of them is reduced, so the loads overlap
   for (int i0 = 0; i0 < 16; i0 += 4) {
     float s[4][8];
 #pragma unroll
@@ -385,6 +398,7 @@ gate_scores_fused_kernel(const T* __restrict__ scores, float mult,
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) m = nanmax(m, __shfl_xor_sync(0xffffffffu, m, o));
       const float thr = DT<T>::round(__fmul_rn(m, mult));
+      int kept = 0;
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         if (j >= nw) break;
@@ -393,38 +407,51 @@ gate_scores_fused_kernel(const T* __restrict__ scores, float mult,
         if (lane == 0) mask_bits[t * nw + j] = word;
         if (rt && lane + 32 * j < E) rt[t * E + lane + 32 * j] = DT<T>::from_f(keep ? 1.0f : 0.0f);
         mine[j] += keep ? 1 : 0;
+        kept += __popc(word);
       }
+      if (kept != 1) init |= 1u << (i0 + u);
     }
   }
 #pragma unroll
   for (int j = 0; j < 8; ++j)
     if (j < nw && lane + 32 * j < E && mine[j]) atomicAdd(&cnt[lane + 32 * j], mine[j]);
+  if (lane == 0) atomicOr(&rows[w >> 1], init << (16 * (w & 1)));
   __syncthreads();
   for (int e = tid; e < EP; e += NT)
     tile_counts[(int64_t)blockIdx.x * EP + e] = (uint8_t)(e < E ? cnt[e] : 0);
+  if (out && direct) init_tile_rows(x, last_bias, add_residual, out, t0, ntok, d, rows, w, lane);
 }
 
-// The same kernel for rows of at most 8 sixteen-byte vectors (E <= 64 in bf16, E <= 32 in
-// fp32, E * sizeof(T) a multiple of 16): one LANE per token.  A lane loads its token's
-// whole score row with vector loads and finds the row maximum, the threshold and the mask
-// word(s) in its own registers, with no cross-lane traffic, so a warp settles 32 tokens in
-// the time the warp-per-token form needs for one; warps 0-3 take the tile's 128 tokens.
-// The per-expert counts of the tile come from one ballot per expert and warp.
-template <typename T, int NV>
+// The rules on score rows of at most 8 sixteen-byte vectors (E <= 64 in bf16, E <= 32 in fp32,
+// E * sizeof(T) a multiple of 16): one LANE per token.  A lane loads its token's whole score row
+// with vector loads and settles it in its own registers, with no cross-lane traffic; warps 0-3
+// take the tile's 128 tokens.  Outputs as above, for all three rules:
+//   RULE 0             dynk_max: maximum, threshold
+//   D2D_RULE_TOPK      k times the first largest of the scores not yet taken
+//   D2D_RULE_DYNK      the same on the shares, until their running sum reaches tau
+// (order of equal values, NaN, summation and rounding as in gate_rule_kernel, which ranks every
+// expert against every other with one warp per token: 15 us for 12608 tokens x 24, before counts,
+// routing tensor and initial rows.)
+template <typename T, int NV, int RULE>
 __global__ void __launch_bounds__(NT)
-gate_scores_fused_rows_kernel(const T* __restrict__ scores, float mult,
+gate_scores_fused_rows_kernel(const T* __restrict__ scores, float mult, int k, float tau,
                               uint32_t* __restrict__ mask_bits, T* __restrict__ rt,
                               uint8_t* __restrict__ tile_counts, int EP,
                               const T* __restrict__ x, const T* __restrict__ last_bias,
-                              int add_residual, T* __restrict__ out, int64_t N, int d, int E) {
-  __shared__ int cnt[64];
+                              int add_residual, T* __restrict__ out, int direct, int64_t N, int d,
+                              int E) {
+  __shared__ int cnt[4][64];
+  __shared__ uint32_t rows[4];
   constexpr int V = 16 / sizeof(T);
   constexpr int EMAX = NV * V;
+  constexpr int NW = (EMAX + 31) / 32;
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const int nw = (E + 31) / 32;
   const int64_t t0 = (int64_t)blockIdx.x * 128;
-  if (tid < 64) cnt[tid] = 0;
-  // this lane's score row first: the loads fly while the initial output rows are issued
+  const int ntok = (int)min((int64_t)128, N - t0);
+  grid_launch_dependents();
+  grid_dependency_wait();
+  // this lane's score row first: the loads fly while initial output rows are issued
   const int64_t t = t0 + w * 32 + lane;
   uint4 raw[NV];
   if (w < 4) {
@@ -433,61 +460,143 @@ gate_scores_fused_rows_kernel(const T* __restrict__ scores, float mult,
       raw[v] = t < N ? __ldg(reinterpret_cast<const uint4*>(scores + t * E) + v)
                      : make_uint4(0u, 0u, 0u, 0u);
   }
-  if (out) {
-    const int dv = d / V;
-    const int rows = (int)min((int64_t)128, N - t0);
-    for (int cv = lane; cv < dv; cv += 32) {
-      uint4 bz = make_uint4(0u, 0u, 0u, 0u);
-      if (last_bias) bz = __ldg(reinterpret_cast<const uint4*>(last_bias) + cv);
-#pragma unroll 4
-      for (int r = w; r < rows; r += NT / 32) {
-        uint4 o = bz;
-        if (add_residual) {
-          const uint4 xv = __ldg(reinterpret_cast<const uint4*>(x + (t0 + r) * d) + cv);
-          const T* a = reinterpret_cast<const T*>(&bz);
-          const T* b = reinterpret_cast<const T*>(&xv);
-          T rr[V];
-#pragma unroll
-          for (int q = 0; q < V; ++q)
-            rr[q] = DT<T>::from_f(DT<T>::to_f(a[q]) + DT<T>::to_f(b[q]));
-          o = *reinterpret_cast<const uint4*>(rr);
-        }
-        *(reinterpret_cast<uint4*>(out + (t0 + r) * d) + cv) = o;
-      }
-    }
-  }
-  __syncthreads();
+  if (out && !direct)
+    init_tile_rows(x, last_bias, add_residual, out, t0, ntok, d, nullptr, w, lane);
   if (w < 4) {
     const T* sv = reinterpret_cast<const T*>(raw);
-    float m = -INFINITY;
-#pragma unroll
-    for (int e = 0; e < EMAX; ++e)
-      if (e < E) m = nanmax(m, DT<T>::to_f(sv[e]));
-    const float thr = DT<T>::round(__fmul_rn(m, mult));
     uint32_t word[2] = {0u, 0u};
-    uint4 one[NV];
-    T* ov = reinterpret_cast<T*>(one);
+    if (RULE == 0) {
+      float m = -INFINITY;
 #pragma unroll
-    for (int e = 0; e < EMAX; ++e) {
-      const bool keep = e < E && DT<T>::to_f(sv[e]) >= thr;
-      if (keep) word[e >> 5] |= 1u << (e & 31);
-      ov[e] = DT<T>::from_f(keep ? 1.0f : 0.0f);
-    }
-    if (t < N) {
-      for (int j = 0; j < nw; ++j) mask_bits[t * nw + j] = word[j];
-      if (rt) {
+      for (int e = 0; e < EMAX; ++e)
+        if (e < E) m = nanmax(m, DT<T>::to_f(sv[e]));
+      const float thr = DT<T>::round(__fmul_rn(m, mult));
 #pragma unroll
-        for (int v = 0; v < NV; ++v) *(reinterpret_cast<uint4*>(rt + t * E) + v) = one[v];
+      for (int e = 0; e < EMAX; ++e)
+        if (e < E && DT<T>::to_f(sv[e]) >= thr) word[e >> 5] |= 1u << (e & 31);
+    } else {
+      float v[EMAX];
+#pragma unroll
+      for (int e = 0; e < EMAX; ++e) v[e] = DT<T>::to_f(sv[e]);
+      bool negative = false;
+      if (RULE == D2D_RULE_DYNK) {
+        float s[32];                     // the balanced sum a warp's butterfly makes of 32 lanes
+#pragma unroll
+        for (int l = 0; l < 32; ++l) {
+          s[l] = 0.f;
+#pragma unroll
+          for (int e = l; e < EMAX; e += 32)
+            if (e < E) s[l] += v[e];
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+          for (int l = 0; l < o; ++l) s[l] += s[l + o];
+        const float tot = DT<T>::round(s[0]);
+#pragma unroll
+        for (int e = 0; e < EMAX; ++e) {
+          v[e] = DT<T>::round(v[e] / tot);
+          negative |= e < E && v[e] < 0.f;
+        }
+      }
+      const float tau_t = DT<T>::round(tau);
+      const int most = RULE == D2D_RULE_TOPK ? k : E;
+      uint32_t taken[2] = {0u, 0u};
+      typename Acc<T>::type acc = 0;
+      bool more = true;                  // the expert of the next rank is kept
+      for (int r = 0; r < most; ++r) {
+        float m = 0.f;
+        int best = -1;
+#pragma unroll
+        for (int e = 0; e < EMAX; ++e) {
+          const bool free = e < E && !((taken[e >> 5] >> (e & 31)) & 1u);
+          if (free && (best < 0 || v[e] > m || (v[e] != v[e] && m == m))) {
+            m = v[e];
+            best = e;
+          }
+        }
+        const uint32_t b0 = best < 32 ? 1u << (best & 31) : 0u;
+        const uint32_t b1 = best >= 32 ? 1u << (best & 31) : 0u;
+        taken[0] |= b0;
+        taken[1] |= b1;
+        if (more) {
+          word[0] |= b0;
+          word[1] |= b1;
+        }
+        if (RULE == D2D_RULE_DYNK) {
+          acc += m;
+          more = DT<T>::round((float)acc) < tau_t;
+          // without negative shares the running sum only grows
+          if (!__any_sync(0xffffffffu, more || negative)) break;
+        }
       }
     }
-    for (int e = 0; e < E; ++e) {
-      const int c = __popc(__ballot_sync(0xffffffffu, t < N && ((word[e >> 5] >> (e & 31)) & 1u)));
-      if (lane == 0 && c) atomicAdd(&cnt[e], c);
+    const bool live = t < N;
+    if (!live) word[0] = word[1] = 0u;
+    const uint32_t todo =
+        __ballot_sync(0xffffffffu, live && __popc(word[0]) + __popc(word[1]) != 1);
+    if (lane == 0) rows[w] = todo;
+    if (live) {
+      for (int j = 0; j < nw; ++j) mask_bits[t * nw + j] = word[j];
+      if (rt) {
+        uint4 one[NV];
+        T* ov = reinterpret_cast<T*>(one);
+#pragma unroll
+        for (int e = 0; e < EMAX; ++e)
+          ov[e] = DT<T>::from_f((word[e >> 5] >> (e & 31)) & 1u ? 1.0f : 0.0f);
+#pragma unroll
+        for (int q = 0; q < NV; ++q) *(reinterpret_cast<uint4*>(rt + t * E) + q) = one[q];
+      }
     }
+#pragma unroll
+    for (int j = 0; j < NW; ++j)         // lane b: how many of the warp's tokens keep expert 32j + b
+      cnt[w][32 * j + lane] = __popc(transpose32(word[j], lane));
   }
   __syncthreads();
   for (int e = tid; e < EP; e += NT)
-    tile_counts[(int64_t)blockIdx.x * EP + e] = (uint8_t)(e < E ? cnt[e] : 0);
+    tile_counts[(int64_t)blockIdx.x * EP + e] =
+        (uint8_t)(e < E ? cnt[0][e] + cnt[1][e] + cnt[2][e] + cnt[3][e] : 0);
+  if (out && direct) init_tile_rows(x, last_bias, add_residual, out, t0, ntok, d, rows, w, lane);
+}
+
+// Mode 'all' (every expert on every token): mask, routing tensor, lists and offsets, and the
+// output's initial value, in one launch instead of a fill, pack, count, scatter and init.
+template <typename T>
+__global__ void __launch_bounds__(NT)
+all_experts_kernel(uint32_t* __restrict__ mask_bits, T* __restrict__ rt,
+                   int32_t* __restrict__ token_idx, int32_t* __restrict__ offsets,
+                   const T* __restrict__ x, const T* __restrict__ last_bias, int add_residual,
+                   T* __restrict__ out, int64_t N, int d, int E) {
+  constexpr int V = 16 / sizeof(T);
+  const int64_t step = (int64_t)gridDim.x * NT, i0 = (int64_t)blockIdx.x * NT + threadIdx.x;
+  const int nw = (E + 31) / 32;
+  grid_launch_dependents();
+  grid_dependency_wait();
+  for (int e = 0; e < E; ++e)
+    for (int64_t t = i0; t < N; t += step) {
+      token_idx[e * N + t] = (int32_t)t;
+      if (rt) rt[e * N + t] = DT<T>::from_f(1.f);
+    }
+  for (int64_t i = i0; i < N * nw; i += step) {
+    const int j = (int)(i % nw);
+    mask_bits[i] = 32 * j + 32 <= E ? 0xffffffffu : (1u << (E - 32 * j)) - 1u;
+  }
+  for (int64_t e = i0; e <= E; e += step) offsets[e] = (int32_t)(e * N);
+  if (out)
+    for (int64_t i = i0; i < N * (d / V); i += step) {
+      uint4 o = make_uint4(0u, 0u, 0u, 0u);
+      if (last_bias) o = __ldg(reinterpret_cast<const uint4*>(last_bias) + (int)(i % (d / V)));
+      if (add_residual) {
+        const uint4 xv = __ldg(reinterpret_cast<const uint4*>(x) + i);
+        const T* a = reinterpret_cast<const T*>(&o);
+        const T* b = reinterpret_cast<const T*>(&xv);
+        T r[V];
+#pragma unroll
+        for (int q = 0; q < V; ++q) r[q] = DT<T>::from_f(DT<T>::to_f(a[q]) + DT<T>::to_f(b[q]));
+        o = *reinterpret_cast<const uint4*>(r);
+      }
+      *(reinterpret_cast<uint4*>(out) + i) = o;
+    }
 }
 
 template <typename T>
@@ -623,27 +732,31 @@ int launch_gate_rule(const void* scores, int rule, int k, float tau, uint32_t* m
 
 // returns D2D_ERR_UNSUPPORTED when the shape does not allow the fused form (caller then uses
 // the separate kernels)
-int launch_gate_scores_fused(const void* scores, float mult, uint32_t* mask_bits, void* rt,
-                             int32_t* tile_counts, const void* x, const void* last_bias,
-                             int add_residual, void* out, int64_t N, int d, int E, int dtype,
-                             cudaStream_t s) {
+int launch_gate_scores_fused(const void* scores, int rule, int k, float tau, float mult,
+                             uint32_t* mask_bits, void* rt, int32_t* tile_counts, const void* x,
+                             const void* last_bias, int add_residual, void* out, bool direct,
+                             int64_t N, int d, int E, int dtype, cudaStream_t s) {
   const int V = dtype == D2D_F32 ? 4 : 8;
   auto al16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
   if (E > 256 || d % V != 0 || !al16(out) || !al16(x) || !al16(last_bias))
     return D2D_ERR_UNSUPPORTED;
   const int64_t grid = ceil_div64(N, 128);
   if (grid > 0x7fffffffLL) return D2D_ERR_UNSUPPORTED;
+  const int EP = compact_row_cells(E);
+  uint8_t* counts = reinterpret_cast<uint8_t*>(tile_counts);
   // score rows of whole 16-byte vectors, at most 8 of them: one lane per token
   const int row_bytes = E * (dtype == D2D_F32 ? 4 : 2);
   const bool rows_form = row_bytes % 16 == 0 && row_bytes <= 128 && al16(scores) &&
                          (rt == nullptr || al16(rt));
 #define D2D_ROWS_CASE(T, NVV)                                                                 \
-  case NVV:                                                                                   \
-    gate_scores_fused_rows_kernel<T, NVV><<<(unsigned)grid, NT, 0, s>>>(                      \
-        (const T*)scores, mult, mask_bits, (T*)rt, reinterpret_cast<uint8_t*>(tile_counts),   \
-        compact_row_cells(E), (const T*)x, (const T*)last_bias, add_residual, (T*)out, N, d,  \
-        E);                                                                                   \
-    break;
+  case NVV: {                                                                                 \
+    auto kn = rule == 0               ? gate_scores_fused_rows_kernel<T, NVV, 0>              \
+              : rule == D2D_RULE_TOPK ? gate_scores_fused_rows_kernel<T, NVV, D2D_RULE_TOPK>  \
+                                      : gate_scores_fused_rows_kernel<T, NVV, D2D_RULE_DYNK>; \
+    return launch_pdl(kn, dim3((unsigned)grid), dim3(NT), 0, s, (const T*)scores, mult, k,    \
+                      tau, mask_bits, (T*)rt, counts, EP, (const T*)x, (const T*)last_bias,   \
+                      add_residual, (T*)out, direct ? 1 : 0, N, d, E);                        \
+  }
   if (rows_form) {
     if (dtype == D2D_F32) {
       switch (row_bytes / 16) {
@@ -658,20 +771,38 @@ int launch_gate_scores_fused(const void* scores, float mult, uint32_t* mask_bits
         D2D_ROWS_CASE(bf16, 7) D2D_ROWS_CASE(bf16, 8)
       }
     }
-    return cudaGetLastError() == cudaSuccess ? D2D_OK : D2D_ERR_LAUNCH;
   }
 #undef D2D_ROWS_CASE
+  if (rule != 0) return D2D_ERR_UNSUPPORTED;
   if (dtype == D2D_F32)
-    gate_scores_fused_kernel<float><<<(unsigned)grid, NT, 0, s>>>(
-        (const float*)scores, mult, mask_bits, (float*)rt, reinterpret_cast<uint8_t*>(tile_counts),
-        compact_row_cells(E), (const float*)x,
-        (const float*)last_bias, add_residual, (float*)out, N, d, E);
-  else
-    gate_scores_fused_kernel<bf16><<<(unsigned)grid, NT, 0, s>>>(
-        (const bf16*)scores, mult, mask_bits, (bf16*)rt, reinterpret_cast<uint8_t*>(tile_counts),
-        compact_row_cells(E), (const bf16*)x,
-        (const bf16*)last_bias, add_residual, (bf16*)out, N, d, E);
-  return cudaGetLastError() == cudaSuccess ? D2D_OK : D2D_ERR_LAUNCH;
+    return launch_pdl(gate_scores_fused_kernel<float>, dim3((unsigned)grid), dim3(NT), 0, s,
+                      (const float*)scores, mult, mask_bits, (float*)rt, counts, EP,
+                      (const float*)x, (const float*)last_bias, add_residual, (float*)out,
+                      direct ? 1 : 0, N, d, E);
+  return launch_pdl(gate_scores_fused_kernel<bf16>, dim3((unsigned)grid), dim3(NT), 0, s,
+                    (const bf16*)scores, mult, mask_bits, (bf16*)rt, counts, EP, (const bf16*)x,
+                    (const bf16*)last_bias, add_residual, (bf16*)out, direct ? 1 : 0, N, d, E);
+}
+
+// mask, routing tensor, lists, offsets and initial output of mode 'all' (out null: not written;
+// d a multiple of 16 bytes and aligned buffers, else D2D_ERR_UNSUPPORTED)
+int launch_all_experts(uint32_t* mask_bits, void* rt, int32_t* token_idx, int32_t* offsets,
+                       const void* x, const void* last_bias, int add_residual, void* out,
+                       int64_t N, int d, int E, int dtype, cudaStream_t s) {
+  const int V = dtype == D2D_F32 ? 4 : 8;
+  auto al16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
+  if (E > 256 || N * (int64_t)E > 0x7fffffffLL) return D2D_ERR_UNSUPPORTED;
+  if (out && (d % V != 0 || !al16(out) || !al16(x) || !al16(last_bias)))
+    return D2D_ERR_UNSUPPORTED;
+  const int64_t work = out ? (N * (d / V) > N ? N * (d / V) : N) : N;
+  const int grid = grid_for(work, NT, 148 * 8);
+  if (dtype == D2D_F32)
+    return launch_pdl(all_experts_kernel<float>, dim3((unsigned)grid), dim3(NT), 0, s, mask_bits,
+                      (float*)rt, token_idx, offsets, (const float*)x, (const float*)last_bias,
+                      add_residual, (float*)out, N, d, E);
+  return launch_pdl(all_experts_kernel<bf16>, dim3((unsigned)grid), dim3(NT), 0, s, mask_bits,
+                    (bf16*)rt, token_idx, offsets, (const bf16*)x, (const bf16*)last_bias,
+                    add_residual, (bf16*)out, N, d, E);
 }
 
 int launch_init_out(const void* x, const void* last_bias, int add_residual, void* out, int64_t N,

@@ -220,6 +220,24 @@ __device__ void role_hidden(const Params& p, Ctl* c, uint32_t tmem, int et) {
   }
 }
 
+// one row of E bf16 values held as packed pairs
+template <int NB>
+__device__ __forceinline__ void store_row(bf16* dst, const uint32_t* s, int E) {
+  if ((E & 7) == 0 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
+#pragma unroll
+    for (int h = 0; h < NB * 2; ++h)
+      if (8 * h < E)
+        *reinterpret_cast<uint4*>(dst + 8 * h) =
+            make_uint4(s[4 * h], s[4 * h + 1], s[4 * h + 2], s[4 * h + 3]);
+  } else {
+#pragma unroll
+    for (int q = 0; q < NB * 8; ++q) {
+      if (2 * q < E) dst[2 * q] = __ushort_as_bfloat16((unsigned short)(s[q] & 0xffff));
+      if (2 * q + 1 < E) dst[2 * q + 1] = __ushort_as_bfloat16((unsigned short)(s[q] >> 16));
+    }
+  }
+}
+
 // warps 4-7, thread = tile row: the row's scores stay in registers as packed bf16 pairs
 // (NB blocks of 16 experts), so tensor memory is read once and handed back at once
 template <int NB>
@@ -258,6 +276,7 @@ __device__ void role_gate(const Params& p, Ctl* c, uint32_t tmem, int et) {
       m2 = __hmax2_nan(m2, *reinterpret_cast<const __nv_bfloat162*>(&s[q]));
     const float m = nanmax(__low2float(m2), __high2float(m2));
     const __nv_bfloat162 thr = __float2bfloat162_rn(__fmul_rn(m, p.mult));
+    if (p.scores && live) store_row<NB>(p.scores + trow * E, s, E);
     uint32_t word[NW];
 #pragma unroll
     for (int j = 0; j < NW; ++j) word[j] = 0u;
@@ -265,12 +284,6 @@ __device__ void role_gate(const Params& p, Ctl* c, uint32_t tmem, int et) {
     for (int q = 0; q < NB * 8; ++q) {
       const uint32_t k = __hge2_mask(*reinterpret_cast<const __nv_bfloat162*>(&s[q]), thr);
       word[q >> 4] |= k & (0x00010001u << (q & 15));
-      if (p.scores && live) {
-        if (2 * q < E)
-          p.scores[trow * E + 2 * q] = __ushort_as_bfloat16((unsigned short)(s[q] & 0xffff));
-        if (2 * q + 1 < E)
-          p.scores[trow * E + 2 * q + 1] = __ushort_as_bfloat16((unsigned short)(s[q] >> 16));
-      }
       s[q] = k & 0x3f803f80u;                         // the routing entries: bf16 1.0 or 0
     }
     int kept = 0;
@@ -306,22 +319,7 @@ __device__ void role_gate(const Params& p, Ctl* c, uint32_t tmem, int et) {
         p.tile_counts[(long long)tile * p.EP + et] = (uint8_t)n;
       }
     }
-    if (p.rt_out && live) {
-      bf16* dst = p.rt_out + trow * E;
-      if ((E & 7) == 0) {
-#pragma unroll
-        for (int h = 0; h < NB * 2; ++h)
-          if (8 * h < E)
-            *reinterpret_cast<uint4*>(dst + 8 * h) =
-                make_uint4(s[4 * h], s[4 * h + 1], s[4 * h + 2], s[4 * h + 3]);
-      } else {
-#pragma unroll
-        for (int q = 0; q < NB * 8; ++q) {
-          if (2 * q < E) dst[2 * q] = __ushort_as_bfloat16((unsigned short)(s[q] & 0xffff));
-          if (2 * q + 1 < E) dst[2 * q + 1] = __ushort_as_bfloat16((unsigned short)(s[q] >> 16));
-        }
-      }
-    }
+    if (p.rt_out && live) store_row<NB>(p.rt_out + trow * E, s, E);
   }
 }
 

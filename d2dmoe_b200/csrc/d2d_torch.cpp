@@ -186,14 +186,15 @@ bool buffers_of(PyObject* cache, const Plan& p, int64_t N, Buffers* b) {
   return ok;
 }
 
-// run_layer(plan, modules, parameters, workspaces, x, tau, residual, scores, norm)
-//   -> (out, routing) | status code (int) | None: the plan does not fit this call
+// run_layer(plan, modules, parameters, workspaces, x, rule, k, tau, residual, scores, norm, capture)
+//   -> (out, routing[, norms]) | status code (int) | None: the plan does not fit this call
+// rule: D2D_RULE_*; k / tau as that rule reads them (MAX: threshold 1 - tau).
 // scores: None or [.., E] of x's dtype.  norm: None or (kind, gamma, beta|None, eps, gamma_offset):
-// x + layer(norm(x)).
+// x + layer(norm(x)).  capture: None or (norm layer, ord), with D2D_RULE_ALL.
 PyObject* run_layer(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
-  if (n != 9) {
-    PyErr_SetString(PyExc_TypeError, "run_layer takes 9 arguments");
+  if (n != 12) {
+    PyErr_SetString(PyExc_TypeError, "run_layer takes 12 arguments");
     return nullptr;
   }
   Plan* p = static_cast<Plan*>(PyCapsule_GetPointer(a[0], kPlan));
@@ -206,19 +207,23 @@ PyObject* run_layer(PyObject*, PyObject* const* a, Py_ssize_t n) {
   }
   const at::Tensor x = xp->contiguous();
   const int64_t N = x.numel() / p->d;
-  const double tau = PyFloat_AsDouble(a[5]);
-  const int residual = PyObject_IsTrue(a[6]);
+  const int rule = (int)PyLong_AsLong(a[5]);
+  const int k = (int)PyLong_AsLong(a[6]);
+  const bool reads_tau = rule == D2D_RULE_MAX || rule == D2D_RULE_DYNK;
+  const double tau = reads_tau ? PyFloat_AsDouble(a[7]) : 0.0;
+  const int residual = PyObject_IsTrue(a[8]);
   if (PyErr_Occurred()) return nullptr;
   const float mult = (float)(1.0 - tau);
-  at::Tensor scores;
-  const bool given = a[7] != Py_None;
+  const bool ranked = rule == D2D_RULE_TOPK || rule == D2D_RULE_DYNK;
+  at::Tensor scores, scratch;
+  const bool given = a[9] != Py_None;
   if (given) {
-    const at::Tensor* sp = tensor_of(a[7]);
+    const at::Tensor* sp = tensor_of(a[9]);
     if (!sp || !sp->is_cuda() || sp->scalar_type() != p->dtype || sp->device() != p->device ||
         sp->numel() != N * p->E)
       Py_RETURN_NONE;
     scores = sp->contiguous();
-  } else if (!p->wa) {
+  } else if (!p->wa && rule != D2D_RULE_ALL) {
     Py_RETURN_NONE;
   }
   c10::cuda::CUDAGuard guard(p->device);
@@ -231,12 +236,20 @@ PyObject* run_layer(PyObject*, PyObject* const* a, Py_ssize_t n) {
   c10::SmallVector<int64_t, 5> rs(x.sizes().begin(), x.sizes().end());
   rs.back() = p->E;
   at::Tensor rt = at::detail::empty_cuda(rs, opts);
+  if (ranked && !given) scratch = at::detail::empty_cuda({N, p->E}, opts);
   const void* xin = x.data_ptr();
   const void* lb = p->last_bias;
   int res = residual ? 1 : 0, rc = D2D_OK;
-  at::Tensor xn;
-  if (a[8] != Py_None) {
-    PyObject* nm = a[8];
+  at::Tensor xn, norms;
+  int norm_layer = 0, norm_ord = 0;
+  if (a[11] != Py_None) {
+    norm_layer = (int)PyLong_AsLong(PyTuple_GetItem(a[11], 0));
+    norm_ord = (int)PyLong_AsLong(PyTuple_GetItem(a[11], 1));
+    if (PyErr_Occurred()) return nullptr;
+    norms = at::detail::empty_cuda({p->E, N}, opts);
+  }
+  if (a[10] != Py_None) {
+    PyObject* nm = a[10];
     xn = at::detail::empty_cuda(x.sizes(), opts);
     const long kind = PyLong_AsLong(PyTuple_GetItem(nm, 0));
     const double eps = PyFloat_AsDouble(PyTuple_GetItem(nm, 3));
@@ -253,17 +266,20 @@ PyObject* run_layer(PyObject*, PyObject* const* a, Py_ssize_t n) {
     res = D2D_OUT_PREINITIALISED;
   }
   if (rc == D2D_OK)
-    rc = d2d_moe_forward(xin, given ? nullptr : p->wa, given ? nullptr : p->wb,
-                         given ? nullptr : p->rp, given ? scores.data_ptr() : nullptr, mult, p->w1,
-                         p->b1, p->wup, p->w2, p->ep, lb, res, out.data_ptr(), (uint32_t*)b.mask,
-                         (int32_t*)b.idx, (int32_t*)b.off, N, (int)p->d, (int)p->R, (int)p->E,
-                         (int)p->H, (int)p->act, dt, b.ws, b.ws_bytes, (int*)b.status,
-                         rt.data_ptr(), stream);
+    rc = d2d_moe_forward_rule(
+        xin, given ? nullptr : p->wa, given ? nullptr : p->wb, given ? nullptr : p->rp,
+        given ? scores.data_ptr() : nullptr, scratch.defined() ? scratch.data_ptr() : nullptr, rule,
+        k, (float)tau, mult, p->w1, p->b1, p->wup, p->w2, p->ep, lb, res, out.data_ptr(),
+        (uint32_t*)b.mask, (int32_t*)b.idx, (int32_t*)b.off, N, (int)p->d, (int)p->R, (int)p->E,
+        (int)p->H, (int)p->act, dt, b.ws, b.ws_bytes, (int*)b.status, rt.data_ptr(),
+        norms.defined() ? norms.data_ptr() : nullptr, norm_layer, norm_ord, stream);
   if (rc != D2D_OK) return PyLong_FromLong(rc);
-  PyObject* res_t = PyTuple_New(2);
+  const bool has_norms = norms.defined();
+  PyObject* res_t = PyTuple_New(has_norms ? 3 : 2);
   if (!res_t) return nullptr;
   PyTuple_SET_ITEM(res_t, 0, THPVariable_Wrap(std::move(out)));
   PyTuple_SET_ITEM(res_t, 1, THPVariable_Wrap(std::move(rt)));
+  if (has_norms) PyTuple_SET_ITEM(res_t, 2, THPVariable_Wrap(std::move(norms)));
   return res_t;
   END_HANDLE_TH_ERRORS
 }

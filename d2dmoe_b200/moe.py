@@ -48,6 +48,10 @@ ACTIVATION_NAME_MAP = {
 # forward_mode strings of the upstream experts class that mean "the fast GPU path"
 _KERNEL_MODES = ("b200", "triton_atomic", "triton")
 
+# routing modes of a layer that run as one library call
+_RULES = {"dynk_max": ops.RULE_MAX, "topk": ops.RULE_TOPK, "dynk": ops.RULE_DYNK,
+          "all": ops.RULE_ALL}
+
 
 def _uniform_init(p: torch.Tensor) -> torch.Tensor:
     """uniform(-1/sqrt(last dim), +1/sqrt(last dim)) (architectures/moe/moe_layers.py:19-24)."""
@@ -314,6 +318,16 @@ MOE_IMPL_MAP = {
 _HOST_STREAMS: dict = {}
 
 
+def _hooked(router) -> bool:
+    """True when a forward hook waits for a call of the router or of one of its layers."""
+    g = nn.modules.module
+    if g._global_forward_hooks or g._global_forward_pre_hooks:
+        return True
+    layers = router._modules["layers"]
+    return any(m._forward_hooks or m._forward_pre_hooks
+               for m in (router, layers, *layers._modules.values()))
+
+
 class MoELayer(nn.Module):
     def __init__(self, name, num_experts):
         nn.Module.__init__(self)      # not super(): bind_upstream() may re-base this class
@@ -446,12 +460,12 @@ class MoeficationMoE(MoELayer):
         """Plan of the one-call layer for the parameters as they are now, or None when the
         modules are not the plain ones of this file or not on a GPU."""
         ex, router = self.experts, self.router
-        if type(ex) not in (B200KernelExperts, B200GluExperts) or router is None:
+        if type(ex) not in (B200KernelExperts, B200GluExperts):
             return None
         p = ex.kernel_params()
         if not p["w1"].is_cuda:
             return None
-        links = [(0, "experts"), (0, "router"), (1, "last_bias")]
+        links = [(0, "experts"), (0, "router"), (1, "last_bias")]     # (an empty slot is a fact too)
         if type(ex) is B200GluExperts:
             links.append((ex._modules, "layers"))
             for i in ("0", "1", "2"):
@@ -478,14 +492,15 @@ class MoeficationMoE(MoELayer):
                               self.last_bias if self.bias else None, ACT[p["act"]],
                               self._modules, self._parameters)
 
-    def _run_native(self, x, residual, scores=None, norm=None):
-        """The layer as one native call -> (out, routing tensor), or None when it has to take
-        the general path."""
+    def _run_native(self, x, rule, residual, scores=None, norm=None, capture=None):
+        """The layer as one native call -> (out, routing tensor[, norms]), or None when it has
+        to take the general path."""
+        k = int(self.k) if rule == ops.RULE_TOPK else 0
         for _ in range(2):
             h = self._plan.handle
             if h is not None:
-                r = host.run_layer(h, self._modules, self._parameters, self._wsp, x, self.tau,
-                                   residual, scores, norm)
+                r = host.run_layer(h, self._modules, self._parameters, self._wsp, x, rule, k,
+                                   self.tau, residual, scores, norm, capture)
                 if type(r) is tuple:
                     return r
                 if r is not None:
@@ -498,22 +513,31 @@ class MoeficationMoE(MoELayer):
 
     def forward(self, x):
         ex = self._modules["experts"]
-        if (self.forward_mode == "dynk_max" and x.is_cuda and ex._capture is None
-                and ex._forward_mode in _KERNEL_MODES):
-            router = self._modules.get("router")
-            r = None
-            if router is not None:
-                if type(router) is MoeficationRouter and router._fusable:
-                    r = self._run_native(x, self.add_residual_connection)
-                else:
-                    with torch.no_grad():
-                        s = router(x)
-                    r = self._run_native(x, self.add_residual_connection, s)
-                    if r is None:
-                        return self._forward_general(x, s)
-            if r is not None:
-                return r[0], {self.name: (r[1],)}
-        return self._forward_general(x)
+        rule = _RULES.get(self.forward_mode)
+        capture = getattr(ex, "_capture", None)
+        if (rule is None or not x.is_cuda or ex._forward_mode not in _KERNEL_MODES
+                or (capture is not None and rule != ops.RULE_ALL)):
+            return self._forward_general(x)
+        router = self._modules.get("router")
+        scores = None
+        if rule == ops.RULE_ALL:
+            if capture is not None:
+                capture = (ops.NORM_OF[capture[0]], capture[1])
+        elif router is None or x.numel() == 0:
+            return self._forward_general(x)
+        elif (type(router) is not MoeficationRouter or not router._fusable
+              or (rule != ops.RULE_MAX and _hooked(router))):
+            # (only 'dynk_max' has always skipped the router module's call)
+            with torch.no_grad():
+                scores = router(x)
+        if rule == ops.RULE_TOPK and not 1 <= int(self.k) <= self.num_experts:
+            raise RuntimeError("selected index k out of range")       # as torch.topk
+        r = self._run_native(x, rule, self.add_residual_connection, scores, None, capture)
+        if r is None:
+            return self._forward_general(x, scores)
+        if capture is not None:
+            ex._deliver_norms({"norms": r[2]})
+        return r[0], {self.name: (r[1],)}
 
     @torch.no_grad()
     def _forward_general(self, x, s=None):
@@ -557,7 +581,7 @@ class MoeficationMoE(MoELayer):
                             experts_packed=self.experts.packed(), routing_out=rt)
             rt = rt.view(*orig_size[:-1], E)
         elif self.forward_mode in ("topk", "dynk") and not capture:
-            s = self.router(x)
+            s = self.router(x) if s is None else s
             self._rule_mask(s.reshape(N, E).contiguous(), wsp)
             ops.compact(wsp, N, E)
             ops.experts_ffn(x2d, wsp, p["w1"], p["b1"], p["w2"], p["act"], out, w_up=p["w_up"],
@@ -622,7 +646,7 @@ class MoeficationMoE(MoELayer):
                  and x.size(-1) * x.element_size() <= 8192 and x.numel() > 0)
         if fused:
             ex._check_mode()
-            r = self._run_native(x, False, None, na)
+            r = self._run_native(x, ops.RULE_MAX, False, None, na)
             if r is not None:
                 return r[0], {self.name: (r[1],)}
         with torch.no_grad():

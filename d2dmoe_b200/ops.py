@@ -129,7 +129,7 @@ def router_mask(x2d, wa, wb, tau, wsp: Workspace, *, packed=None, scores_out=Non
               "d2d_router_mask")
 
 
-RULE_TOPK, RULE_DYNK = 1, 2
+RULE_MAX, RULE_TOPK, RULE_DYNK, RULE_ALL = 0, 1, 2, 3
 
 
 def mask_rule_from_scores(scores2d, rule: str, wsp: Workspace, k=None, tau=None):

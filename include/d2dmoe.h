@@ -241,6 +241,28 @@ int d2d_moe_forward(const void* x, const void* wa, const void* wb, const void* r
                     void* ws, size_t ws_bytes, int* dev_status,
                     void* routing_tensor_opt, d2d_stream_t stream);
 
+/* d2d_moe_forward for every routing mode of MoeficationMoE.gate
+ * (architectures/moe/moefication.py:54-88):
+ *   D2D_RULE_MAX   as d2d_moe_forward (thresh_mult)
+ *   D2D_RULE_TOPK  the k largest scores (k)
+ *   D2D_RULE_DYNK  cumulative share (tau, as in d2d_mask_rule_from_scores)
+ *   D2D_RULE_ALL   every expert on every token; no router, no scores
+ * TOPK and DYNK take scores_in_opt, or wa / wb and scores_scratch [N, E] in T, which receives the
+ * router's scores.  norms_opt [E, N] with norm_layer / norm_ord (see d2d_experts_ffn_norms) goes
+ * with D2D_RULE_ALL only; NULL and 0 otherwise. */
+#define D2D_RULE_MAX 0
+#define D2D_RULE_ALL 3
+int d2d_moe_forward_rule(const void* x, const void* wa, const void* wb,
+                         const void* router_packed_opt, const void* scores_in_opt,
+                         void* scores_scratch, int rule, int k, float tau, float thresh_mult,
+                         const void* w1, const void* b1_opt, const void* w_up_opt, const void* w2,
+                         const void* experts_packed_opt, const void* last_bias_opt,
+                         int add_residual, void* out, uint32_t* mask_bits, int32_t* token_idx,
+                         int32_t* offsets, int64_t N, int d, int R, int E, int H, int act,
+                         int dtype, void* ws, size_t ws_bytes, int* dev_status,
+                         void* routing_tensor_opt, void* norms_opt, int norm_layer, int norm_ord,
+                         d2d_stream_t stream);
+
 /* Number of kernels the calling thread's last d2d_moe_forward issued (3 on the tensor-core
  * path: router + rule, compaction scatter, expert FFN; more on the general-shape
  * paths).  Introspection for benchmarks; no upstream counterpart. */
