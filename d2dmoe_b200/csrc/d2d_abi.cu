@@ -313,7 +313,7 @@ int d2d_moe_forward_rule(const void* x, const void* wa, const void* wb,
     rc = launch_compact(mask_bits, token_idx, offsets, N, E, (int32_t*)ws, dev_status, s,
                         counts_ready);
     if (rc != D2D_OK) return rc;
-    nl += counts_ready ? 1 : 2;    // [count,] scatter
+    nl += compact_counts_itself(N, E) || counts_ready ? 1 : 2;    // [count,] scatter
   }
   if (!rt_done) {                  // paths whose first kernel does not write the routing tensor
     rc = launch_expand_mask(mask_bits, routing_tensor_opt, N, E, dtype, s);

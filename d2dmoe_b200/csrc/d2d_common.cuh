@@ -185,11 +185,20 @@ int launch_pack_mask(const void* rt, uint32_t* mask_bits, int64_t N, int E, int 
 int device_launch_facts(const void* kernel, size_t smem, int* sms);
 size_t compact_workspace_bytes(int64_t n_max, int E);
 int compact_row_cells(int E);      // cells (bytes) per row of the compaction's counts table
+bool compact_counts_itself(int64_t N, int E);   // no count kernel needed
 // counts_ready: the byte table counts_ws[tile of 128 tokens][compact_row_cells(E)] is already
 // filled (by the router kernel); otherwise a count kernel fills it first
 int launch_compact(const uint32_t* mask_bits, int32_t* token_idx, int32_t* offsets, int64_t N,
                    int E, int32_t* counts_ws, int* dev_status, cudaStream_t s,
                    bool counts_ready);
+// fp32 with 16-byte vectors everywhere, else D2D_ERR_UNSUPPORTED
+int launch_router_fp32(const void* x, const void* wa, const void* wb, float mult,
+                       uint32_t* mask_bits, void* scores, void* rt, const void* last_bias,
+                       int add_residual, void* out_init, int64_t N, int d, int R, int E,
+                       cudaStream_t s);
+int launch_experts_fp32(const void* x, const int32_t* token_idx, const int32_t* offsets,
+                        const void* w1, const void* b1, const void* w2, void* out, int64_t N, int d,
+                        int E, int H, int act, int* dev_status, cudaStream_t s);
 int launch_experts_simt(const void* x, const int32_t* token_idx, const int32_t* offsets,
                         const void* w1, const void* b1, const void* w_up, const void* w2,
                         void* out, int64_t N, int d, int E, int H, int act, int dtype,

@@ -371,6 +371,11 @@ int launch_experts_simt(const void* x, const int32_t* token_idx, const int32_t* 
                         int* dev_status, cudaStream_t s, NormCapture nc) {
   if (E > MAX_E) return D2D_ERR_UNSUPPORTED;
   if (dtype == D2D_F32) {
+    if (!w_up && !nc.norms) {
+      const int rc = launch_experts_fp32(x, token_idx, offsets, w1, b1, w2, out, N, d, E, H, act,
+                                         dev_status, s);
+      if (rc != D2D_ERR_UNSUPPORTED) return rc;
+    }
     return w_up ? launch_t<float, true>(x, token_idx, offsets, w1, b1, w_up, w2, out, N, d, E, H,
                                         act, dev_status, s, nc)
                 : launch_t<float, false>(x, token_idx, offsets, w1, b1, w_up, w2, out, N, d, E, H,

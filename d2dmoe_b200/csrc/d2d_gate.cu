@@ -697,6 +697,11 @@ int launch_router_mask_simt(const void* x, const void* wa, const void* wb, float
                             int dtype, int* dev_status, cudaStream_t s, void* rt_out) {
   (void)dev_status;
   if (E > 256 || R > 1024) return D2D_ERR_UNSUPPORTED;
+  if (dtype == D2D_F32) {
+    const int rc = launch_router_fp32(x, wa, wb, mult, mask_bits, scores, rt_out, last_bias,
+                                      add_residual, out_init, N, d, R, E, s);
+    if (rc != D2D_ERR_UNSUPPORTED) return rc;
+  }
   // 16-token tiles while 32-token tiles would not give every SM of a B200 a tile
   const bool small = ceil_div64(N, 32) < 148;
 #define D2D_ROUTER_SIMT(T_, TM_)                                                                \
