@@ -64,19 +64,25 @@ struct Geo {
   int kc2;         // ceil(H / 64)
   int nd, nc;      // output columns per step of the second product, steps
   int ns, ns2;     // ring stages
-  int stage;       // bytes of a stage of the first ring: rows of x (16 KB), then w1_stage
+  int a_slot;      // bytes of a stage's rows of x
+  int stage;       // bytes of a stage of the first ring: a_slot, then w1_stage
   int w2_piece;    // W2 bytes of a step's 64-deep slice (one stage of the second ring)
   long long w1_bytes, bias_off, stride;   // packed layout per expert
 };
 
-Geo experts_geo(int d, int H, bool glu) {
+// n: tokens of the call.  A list has at most n rows, so with n <= 32 (64) a tile needs only the first
+// quarter (half) of its 16 KB of x: the MMA still reads 128 rows, but what stands in the other
+// rows' place reaches only accumulator rows nobody reads.  A decode step of the gated form keeps
+// four stages of weights in flight instead of three.
+Geo experts_geo(int d, int H, bool glu, long long n) {
   Geo g;
   g.kc1 = d / 64;
   g.w1_stage = (glu ? 2 : 1) * H * 128;
   g.kc2 = (H + 63) / 64;
   g.nd = !glu && d % 128 == 0 ? 128 : 64;
   g.nc = d / g.nd;
-  g.stage = SLOT + g.w1_stage;
+  g.a_slot = n <= 32 ? SLOT / 4 : n <= 64 ? SLOT / 2 : SLOT;
+  g.stage = g.a_slot + g.w1_stage;
   g.w2_piece = g.nd * 128;
   // at least three W2 pieces, then as many stages of the first ring as fit, the rest for W2
   const int ns = (SMEM_TILES - STG - 3 * g.w2_piece) / g.stage;
@@ -196,8 +202,8 @@ __device__ void role_list(const Params& p, Ctl* c, int lane, bool one_window) {
     used = __reduce_add_sync(0xffffffffu, used);
     const float G = (float)gridDim.x;
     const float R = ceilf(((float)rows * (1.0f / TILE_M) + (float)used) / G);
-    const int S =
-        max(32, min(TILE_M, (int)ceilf((float)rows / fmaxf(R * G - (float)used, 1.0f))));
+    const int S =                        // (never more rows than a stage has room for)
+        max(32, min(p.g.a_slot >> 7, (int)ceilf((float)rows / fmaxf(R * G - (float)used, 1.0f))));
     const float inv = 1.0f / (float)S;
     int sum = 0;
 #pragma unroll
@@ -383,7 +389,7 @@ __device__ void role_weights(const Params& p, Ctl* c, uint32_t ring, uint32_t ri
       const uint32_t bar = smem_u32(&c->full[r1.s]);
       mbar_arrive_expect_tx(bar, g.w1_stage);
       if (withheld) withheld = false;    // test hook: this stage never fills, its wait runs out
-      else bulk_g2s(ring + r1.s * g.stage + SLOT, s1, g.w1_stage, bar);
+      else bulk_g2s(ring + r1.s * g.stage + g.a_slot, s1, g.w1_stage, bar);
       s1 += g.w1_stage;
       r1.next(g.ns);
       --j1;
@@ -443,7 +449,7 @@ __device__ void role_mma1(const Params& p, Ctl* c, uint32_t ring, uint32_t tmem)
     for (int kc = 0; kc < g.kc1; ++kc) {
       if (!mbar_wait_fast(smem_u32(&c->full[r.s]), r.ph, af, p.dev_status)) return;
       tc_fence_after();
-      const uint32_t alo = lo0 + r.s * ((uint32_t)g.stage >> 4), blo = alo + (SLOT >> 4);
+      const uint32_t alo = lo0 + r.s * ((uint32_t)g.stage >> 4), blo = alo + ((uint32_t)g.a_slot >> 4);
 #pragma unroll
       for (uint32_t k = 0; k < 4; ++k)
         umma_bf16(acc, hi | (alo + 2 * k), hi | (blo + 2 * k), idesc, (kc | k) != 0);
@@ -873,12 +879,12 @@ bool umma_experts_supported(int d, int E, int H, bool glu, int dtype) {
 }
 
 size_t umma_experts_packed_bytes(int d, int E, int H, bool glu) {
-  return (size_t)experts_geo(d, H, glu).stride * (size_t)E;
+  return (size_t)experts_geo(d, H, glu, TILE_M).stride * (size_t)E;
 }
 
 int launch_prepack_experts(const void* w1, const void* b1, const void* w_up, const void* w2,
                            void* packed, int d, int E, int H, cudaStream_t s) {
-  const Geo g = experts_geo(d, H, w_up != nullptr);
+  const Geo g = experts_geo(d, H, w_up != nullptr, TILE_M);
   dim3 grid(64, E);
   prepack_experts_kernel<<<grid, 256, 0, s>>>((const bf16*)w1, (const bf16*)b1, (const bf16*)w_up,
                                               (const bf16*)w2, (uint8_t*)packed, g, d, E, H);
@@ -896,7 +902,7 @@ int launch_experts_umma(const void* x, const int32_t* token_idx, const int32_t* 
   p.H = H;
   p.act = act;
   p.packed = (const uint8_t*)packed;
-  p.g = experts_geo(d, H, glu);
+  p.g = experts_geo(d, H, glu, N);
   p.token_idx = token_idx;
   p.offsets = offsets;
   p.out = (bf16*)out;

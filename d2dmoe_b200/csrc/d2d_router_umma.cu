@@ -323,20 +323,27 @@ __device__ void role_gate(const Params& p, Ctl* c, uint32_t tmem, int et) {
   }
 }
 
-// warps 12-15: warp q writes the initial rows of the tile's tokens 32q .. 32q+31 that ask for one
-__device__ void role_init(const Params& p, Ctl* c, int q4, int lane) {
+// warps 12-15: the initial rows of the tile's tokens that ask for one.  Warp w has rows 32 w .. + 31;
+// where only the first 32 have any (a call of few tokens) the warps share a row instead, every
+// fourth 512-byte piece each (32 tokens x 2048: 12 -> 4 us).
+__device__ void role_init(const Params& p, Ctl* c, int w, int lane) {
   volatile int* af = &c->abort_flag;
   const int tiles = (int)((p.N + TILE_M - 1) / TILE_M);
   const int v8 = p.d >> 3;
   uint32_t ph = 0, buf = 0;
   for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ph ^= buf, buf ^= 1) {
     if (!mbar_wait_fast(smem_u32(&c->init_full[buf]), ph, af, p.dev_status)) return;
-    const uint32_t rows = c->init_rows[buf][q4];
+    const uint32_t others =
+        c->init_rows[buf][1] | c->init_rows[buf][2] | c->init_rows[buf][3];
+    const bool share = others == 0u;
+    const int q = share ? 0 : w;
+    const uint32_t rows = c->init_rows[buf][q];
     __syncwarp();
     if (lane == 0) mbar_arrive(smem_u32(&c->init_empty[buf]));
     if (rows == 0u) continue;
-    const long long row0 = (long long)tile * TILE_M + 32 * q4;
-    for (int c8 = lane; c8 < v8; c8 += 32) {
+    const long long row0 = (long long)tile * TILE_M + 32 * q;
+    const int step = share ? 128 : 32;
+    for (int c8 = lane + (share ? 32 * w : 0); c8 < v8; c8 += step) {
       uint4 bz = make_uint4(0u, 0u, 0u, 0u);
       if (p.last_bias) bz = __ldg(reinterpret_cast<const uint4*>(p.last_bias) + c8);
       if (!p.resid) {
