@@ -295,8 +295,8 @@ __device__ void role_gate(const Params& p, Ctl* c, uint32_t tmem, int et) {
       kept += __popc(word[j]);
       if (live) p.mask_bits[trow * nw + j] = word[j];
     }
-    if (p.out_init) {
-      const bool todo = live && (p.init_all || kept != 1);
+    if (p.out_init && !p.init_all) {
+      const bool todo = live && kept != 1;
       const uint32_t rows = __ballot_sync(0xffffffffu, todo);
       if (!mbar_wait_fast(smem_u32(&c->init_empty[buf]), ibuf_ph ^ 1, af, p.dev_status)) return;
       if (lane == 0) {
@@ -332,14 +332,23 @@ __device__ void role_init(const Params& p, Ctl* c, int w, int lane) {
   const int v8 = p.d >> 3;
   uint32_t ph = 0, buf = 0;
   for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ph ^= buf, buf ^= 1) {
-    if (!mbar_wait_fast(smem_u32(&c->init_full[buf]), ph, af, p.dev_status)) return;
-    const uint32_t others =
-        c->init_rows[buf][1] | c->init_rows[buf][2] | c->init_rows[buf][3];
-    const bool share = others == 0u;
-    const int q = share ? 0 : w;
-    const uint32_t rows = c->init_rows[buf][q];
-    __syncwarp();
-    if (lane == 0) mbar_arrive(smem_u32(&c->init_empty[buf]));
+    bool share = false;
+    int q = w;
+    uint32_t rows;
+    if (p.init_all) {                  // no need to know what the gate says
+      const long long left = p.N - (long long)tile * TILE_M;
+      share = left <= 32;
+      q = share ? 0 : w;
+      const long long n = left - 32 * q;
+      rows = n >= 32 ? 0xffffffffu : n > 0 ? (1u << n) - 1u : 0u;
+    } else {
+      if (!mbar_wait_fast(smem_u32(&c->init_full[buf]), ph, af, p.dev_status)) return;
+      share = (c->init_rows[buf][1] | c->init_rows[buf][2] | c->init_rows[buf][3]) == 0u;
+      q = share ? 0 : w;
+      rows = c->init_rows[buf][q];
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&c->init_empty[buf]));
+    }
     if (rows == 0u) continue;
     const long long row0 = (long long)tile * TILE_M + 32 * q;
     const int step = share ? 128 : 32;
@@ -352,17 +361,17 @@ __device__ void role_init(const Params& p, Ctl* c, int w, int lane) {
         continue;
       }
       for (uint32_t m = rows; m != 0u;) {
-        uint4 xv[4];
-        int rr[4];
+        uint4 xv[8];
+        int rr[8];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {        // four rows in flight
+        for (int u = 0; u < 8; ++u) {        // eight rows in flight
           rr[u] = m != 0u ? __ffs(m) - 1 : -1;
           m &= m - 1;
           if (rr[u] >= 0)
             xv[u] = __ldg(reinterpret_cast<const uint4*>(p.resid + (row0 + rr[u]) * p.d) + c8);
         }
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
+        for (int u = 0; u < 8; ++u)
           if (rr[u] >= 0)
             *(reinterpret_cast<uint4*>(p.out_init + (row0 + rr[u]) * p.d) + c8) =
                 add_bf16x8(bz, xv[u]);
