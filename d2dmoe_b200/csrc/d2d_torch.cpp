@@ -15,11 +15,13 @@
 
 #include <ATen/ATen.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDAException.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include <memory>
 #include <vector>
 
 #include "../../include/d2dmoe.h"
@@ -284,7 +286,126 @@ PyObject* run_layer(PyObject*, PyObject* const* a, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
+// ---- host-buffer pipeline -------------------------------------------------------
+// Two staging buffers for slices of x, three for slices of the output; the events say when the
+// stream that last used one is done with it (never recorded: at once).
+constexpr int kIn = 2, kOut = 3;
+struct HostPipe {
+  int device = 0;
+  cudaEvent_t in_full[kIn] = {}, in_free[kIn] = {}, out_full[kOut] = {}, out_free[kOut] = {},
+              caller = nullptr;
+  unsigned long long n = 0;            // slices so far, over all calls
+  std::vector<cudaEvent_t*> all() {
+    std::vector<cudaEvent_t*> v = {&caller};
+    for (auto& e : in_full) v.push_back(&e);
+    for (auto& e : in_free) v.push_back(&e);
+    for (auto& e : out_full) v.push_back(&e);
+    for (auto& e : out_free) v.push_back(&e);
+    return v;
+  }
+};
+constexpr const char* kPipe = "d2dmoe_b200.host_pipe";
+void pipe_free(PyObject* cap) {
+  auto* h = static_cast<HostPipe*>(PyCapsule_GetPointer(cap, kPipe));
+  for (cudaEvent_t* e : h->all())
+    if (*e) cudaEventDestroy(*e);
+  delete h;
+}
+
+PyObject* make_pipe(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  TORCH_CHECK(n == 1, "make_pipe(device index)");
+  auto h = std::make_unique<HostPipe>();
+  h->device = (int)PyLong_AsLong(a[0]);
+  if (PyErr_Occurred()) return nullptr;
+  c10::cuda::CUDAGuard guard((c10::DeviceIndex)h->device);
+  for (cudaEvent_t* e : h->all())
+    C10_CUDA_CHECK(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
+  return PyCapsule_New(h.release(), kPipe, pipe_free);
+  END_HANDLE_TH_ERRORS
+}
+
+// run_host(plan, modules, parameters, workspaces, pipe, x_host, out_host, staging (kIn + kOut tensors),
+//          (stream in, stream run, stream out), slices, rule, k, tau, residual, sync)
+//   -> True | status code (int) | None: the plan does not fit this call
+// Slice i's copy in, the kernels of slice i - 1 and the copy out of slice i - 2 overlap.  The same
+// pipeline issued from Python took 70 us of host time per slice, more than a slice's copies.
+PyObject* run_host(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  TORCH_CHECK(n == 15, "run_host takes 15 arguments");
+  Plan* p = static_cast<Plan*>(PyCapsule_GetPointer(a[0], kPlan));
+  HostPipe* h = static_cast<HostPipe*>(PyCapsule_GetPointer(a[4], kPipe));
+  if (!p || !h) return nullptr;
+  const at::Tensor *xh = tensor_of(a[5]), *oh = tensor_of(a[6]);
+  if (!xh || !oh || xh->scalar_type() != p->dtype || oh->scalar_type() != p->dtype ||
+      !xh->is_contiguous() || !oh->is_contiguous() || !oh->is_cpu() || xh->sizes() != oh->sizes() ||
+      xh->dim() < 2 || xh->size(-1) != p->d || xh->numel() == 0 || h->device != p->device.index() ||
+      !still_valid(*p, a + 1)) {
+    if (PyErr_Occurred()) return nullptr;
+    Py_RETURN_NONE;
+  }
+  void* stage[kIn + kOut];
+  for (int i = 0; i < kIn + kOut; ++i) stage[i] = const_cast<void*>(ptr_of(PyTuple_GetItem(a[7], i)));
+  cudaStream_t st[3];
+  for (int i = 0; i < 3; ++i) st[i] = (cudaStream_t)PyLong_AsVoidPtr(PyTuple_GetItem(a[8], i));
+  const int64_t slices = PyLong_AsLongLong(a[9]);
+  const int rule = (int)PyLong_AsLong(a[10]), k = (int)PyLong_AsLong(a[11]);
+  const bool reads_tau = rule == D2D_RULE_MAX || rule == D2D_RULE_DYNK;
+  const double tau = reads_tau ? PyFloat_AsDouble(a[12]) : 0.0;
+  const int residual = PyObject_IsTrue(a[13]), sync = PyObject_IsTrue(a[14]);
+  if (PyErr_Occurred()) return nullptr;
+  if ((rule != D2D_RULE_ALL && !p->wa) || (rule != D2D_RULE_ALL && rule != D2D_RULE_MAX))
+    Py_RETURN_NONE;
+  c10::cuda::CUDAGuard guard(p->device);
+  const cudaStream_t cur = c10::cuda::getCurrentCUDAStream(p->device.index()).stream();
+  if (sync) {                          // what the caller's stream has queued comes first
+    C10_CUDA_CHECK(cudaEventRecord(h->caller, cur));
+    for (cudaStream_t s : st) C10_CUDA_CHECK(cudaStreamWaitEvent(s, h->caller, 0));
+  }
+  const int dt = p->dtype == at::kBFloat16 ? D2D_BF16 : D2D_F32;
+  const int64_t B = xh->size(0), per = xh->numel() / B;      // values of one batch entry
+  const size_t es = xh->element_size();
+  const char* src = static_cast<const char*>(xh->data_ptr());
+  char* dst = static_cast<char*>(oh->data_ptr());
+  int rc = D2D_OK;
+  for (int64_t i = 0; i < slices && rc == D2D_OK; ++i, ++h->n) {
+    const int64_t lo = B * i / slices, hi = B * (i + 1) / slices, N = (hi - lo) * per / p->d;
+    const int b = (int)(h->n % kIn), o = (int)(h->n % kOut);
+    const size_t bytes = (size_t)((hi - lo) * per) * es, at = (size_t)(lo * per) * es;
+    Buffers buf;
+    if (!buffers_of(a[3], *p, N, &buf)) return nullptr;
+    C10_CUDA_CHECK(cudaStreamWaitEvent(st[0], h->in_free[b], 0));
+    C10_CUDA_CHECK(cudaMemcpyAsync(stage[b], src + at, bytes, cudaMemcpyHostToDevice, st[0]));
+    C10_CUDA_CHECK(cudaEventRecord(h->in_full[b], st[0]));
+    C10_CUDA_CHECK(cudaStreamWaitEvent(st[1], h->in_full[b], 0));
+    C10_CUDA_CHECK(cudaStreamWaitEvent(st[1], h->out_free[o], 0));
+    rc = d2d_moe_forward_rule(stage[b], p->wa, p->wb, p->rp, nullptr, nullptr, rule, k, (float)tau,
+                              (float)(1.0 - tau), p->w1, p->b1, p->wup, p->w2, p->ep, p->last_bias,
+                              residual ? 1 : 0, stage[kIn + o], (uint32_t*)buf.mask,
+                              (int32_t*)buf.idx, (int32_t*)buf.off, N, (int)p->d, (int)p->R,
+                              (int)p->E, (int)p->H, (int)p->act, dt, buf.ws, buf.ws_bytes,
+                              (int*)buf.status, nullptr, nullptr, 0, 0, (d2d_stream_t)st[1]);
+    C10_CUDA_CHECK(cudaEventRecord(h->in_free[b], st[1]));
+    C10_CUDA_CHECK(cudaEventRecord(h->out_full[o], st[1]));
+    C10_CUDA_CHECK(cudaStreamWaitEvent(st[2], h->out_full[o], 0));
+    C10_CUDA_CHECK(cudaMemcpyAsync(dst + at, stage[kIn + o], bytes, cudaMemcpyDeviceToHost, st[2]));
+    C10_CUDA_CHECK(cudaEventRecord(h->out_free[o], st[2]));
+  }
+  if (sync) {                          // the last copy out is behind everything else
+    cudaError_t err;
+    Py_BEGIN_ALLOW_THREADS
+    err = cudaStreamSynchronize(st[2]);
+    Py_END_ALLOW_THREADS
+    C10_CUDA_CHECK(err);
+  }
+  if (rc != D2D_OK) return PyLong_FromLong(rc);
+  Py_RETURN_TRUE;
+  END_HANDLE_TH_ERRORS
+}
+
 PyMethodDef kMethods[] = {
+    {"make_pipe", (PyCFunction)(void (*)(void))make_pipe, METH_FASTCALL, nullptr},
+    {"run_host", (PyCFunction)(void (*)(void))run_host, METH_FASTCALL, nullptr},
     {"make_plan", (PyCFunction)(void (*)(void))make_plan, METH_FASTCALL, nullptr},
     {"run_layer", (PyCFunction)(void (*)(void))run_layer, METH_FASTCALL, nullptr},
     {nullptr, nullptr, 0, nullptr}};

@@ -83,6 +83,21 @@ class _WorkspaceCache(dict):
         return _WorkspaceCache, ()
 
 
+class _HostBuffers:
+    """Staging buffers and events of ``forward_host``; copies of a module start without them."""
+
+    __slots__ = ("shape", "dtype", "device", "bufs", "pipe", "streams")
+
+    def __init__(self):
+        self.shape = self.dtype = self.device = self.bufs = self.pipe = self.streams = None
+
+    def __deepcopy__(self, memo):
+        return _HostBuffers()
+
+    def __reduce__(self):
+        return _HostBuffers, ()
+
+
 class _Plan:
     """Holder of a layer's native call plan (csrc/d2d_torch.cpp); copies start without one."""
 
@@ -428,6 +443,7 @@ class MoeficationMoE(MoELayer):
         self.add_residual_connection = add_residual_connection
         self._wsp = _WorkspaceCache()
         self._plan = _Plan()
+        self._host = _HostBuffers()
 
     # -- routing for the modes that are not fused ---------------------------------
     def gate(self, x):
@@ -679,6 +695,8 @@ class MoeficationMoE(MoELayer):
             st = tuple(torch.cuda.Stream(device=dev) for _ in range(3))
             _HOST_STREAMS[dev] = st
         s_in, s_run, s_out = st
+        if self._host_native(x_host, out_host, chunks, sync, st, dev):
+            return out_host
         cur = torch.cuda.current_stream(dev)
         if sync:
             for s_ in st:
@@ -722,6 +740,54 @@ class MoeficationMoE(MoELayer):
                 cur.wait_stream(s_)
             cur.synchronize()
         return out_host
+
+    def _host_native(self, x_host, out_host, chunks, sync, st, dev) -> bool:
+        """The pipeline of forward_host issued by native code; False when this call has to take
+        the general one (a router or hooks that run in Python, other dtypes or layouts)."""
+        ex, router = self.experts, self.router
+        rule = _RULES.get(self.forward_mode)
+        if (rule not in (ops.RULE_MAX, ops.RULE_ALL) or getattr(ex, "_capture", None) is not None
+                or ex._forward_mode not in _KERNEL_MODES or x_host.dim() < 2 or x_host.numel() == 0
+                or (rule == ops.RULE_MAX and not (type(router) is MoeficationRouter
+                                                  and router._fusable))):
+            return False
+        B = x_host.shape[0]
+        rows = max(B * (i + 1) // chunks - B * i // chunks for i in range(chunks))
+        shape = (rows,) + tuple(x_host.shape[1:])
+        hp = self._host
+        if hp.shape != shape or hp.dtype != x_host.dtype or hp.device != dev:
+            # Copies and kernels of earlier sync=False calls may still use the old staging
+            # buffers: drain the streams before they go back to the allocator (a host wait, but
+            # only when the slice shape changes); the allocator is told who uses the new ones.
+            for s_ in st:
+                s_.synchronize()
+            new = dict(dtype=x_host.dtype, device=dev)
+            with torch.cuda.stream(st[0]):
+                bufs = [torch.empty(shape, **new) for _ in range(2)]
+            with torch.cuda.stream(st[1]):
+                bufs += [torch.empty(shape, **new) for _ in range(3)]
+            for b in bufs[:2]:
+                b.record_stream(st[1])
+            for b in bufs[2:]:
+                b.record_stream(st[2])
+            hp.shape, hp.dtype, hp.device, hp.bufs = shape, x_host.dtype, dev, tuple(bufs)
+            hp.pipe = host.make_pipe(torch.device(dev).index or 0)
+            hp.streams = tuple(s_.cuda_stream for s_ in st)
+        for _ in range(2):
+            h = self._plan.handle
+            if h is not None:
+                r = host.run_host(h, self._modules, self._parameters, self._wsp, hp.pipe, x_host,
+                                  out_host, hp.bufs, hp.streams, chunks, rule, 0, self.tau,
+                                  self.add_residual_connection, sync)
+                if r is True:
+                    return True
+                if r is not None:
+                    raise D2DError(r, "d2d_moe_forward")
+            with torch.no_grad():
+                self._plan.handle = self._make_plan()
+            if self._plan.handle is None:
+                return False
+        return False
 
     @staticmethod
     def host_synchronize(device=None) -> None:
