@@ -298,7 +298,8 @@ int d2d_moe_forward_rule(const void* x, const void* wa, const void* wb,
                                  routing_tensor_opt, last_bias_opt, add_residual ? x : nullptr,
                                  out_init, !may_store, (int32_t*)ws, N, d, R, E, dev_status, s);
     if (may_store) leave_rows();
-    counts_ready = rt_done = true;
+    counts_ready = !umma_router_splits(N, d, R, E);
+    rt_done = true;
     nl += 1;
   } else if (rule == D2D_RULE_MAX) {
     // general-shape router: mask bits, routing tensor and the output's initial value

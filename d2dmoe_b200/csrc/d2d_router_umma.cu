@@ -19,6 +19,8 @@
 // tile loop with the expert kernel (hidden tile in shared memory, separate rings for x and Wa,
 // Wb streamed per tile, eight warps each doing both epilogues, every initial row written by the
 // TMA unit in front of the loads) the second epilogue no longer sits between two tiles.
+#include <cooperative_groups.h>
+
 #include "d2d_tmap.cuh"
 #include "d2d_umma_api.cuh"
 #include "d2d_umma_ptx.cuh"
@@ -185,6 +187,17 @@ __device__ void role_mma2(const Params& p, Ctl* c, uint32_t wb, uint32_t tmem) {
   }
 }
 
+// 16 hidden columns as 8 packed bf16 pairs: relu(T(x Wa^T))
+__device__ __forceinline__ void relu_pairs(const uint32_t* v, uint32_t* w) {
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    __nv_bfloat162 h =
+        __floats2bfloat162_rn(__uint_as_float(v[2 * q]), __uint_as_float(v[2 * q + 1]));
+    h = __hmax2(h, __float2bfloat162_rn(0.f));
+    w[q] = *reinterpret_cast<uint32_t*>(&h);
+  }
+}
+
 // warps 0-3, thread = tile row = TMEM lane: hidden tile = bf16 relu of accumulator 1
 __device__ void role_hidden(const Params& p, Ctl* c, uint32_t tmem, int et) {
   volatile int* af = &c->abort_flag;
@@ -203,13 +216,7 @@ __device__ void role_hidden(const Params& p, Ctl* c, uint32_t tmem, int et) {
       uint32_t v[16], w[8];
       tmem_ld16(src + c0, v);
       tmem_wait_ld();
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        __nv_bfloat162 h =
-            __floats2bfloat162_rn(__uint_as_float(v[2 * q]), __uint_as_float(v[2 * q + 1]));
-        h = __hmax2(h, __float2bfloat162_rn(0.f));
-        w[q] = *reinterpret_cast<uint32_t*>(&h);
-      }
+      relu_pairs(v, w);
       tmem_st8(dst + (c0 >> 1), w);
     }
     tmem_wait_st();
@@ -460,6 +467,201 @@ router_tiles_kernel(const Params p, const __grid_constant__ CUtensorMap tmx) {
   }
 }
 
+// ---------------------------------------------------------------------------
+// few tokens, large router
+// ---------------------------------------------------------------------------
+// A call of at most a few tiles leaves the chip idle above: one CTA streams all of Wa (1 MB for
+// 2048 x 256) through its own 64 bytes per clock, 15 us for 32 tokens.  Here a cluster of eight
+// CTAs has a tile: each takes an eighth of the hidden columns (all of d, an eighth of Wa), their
+// share of the scores (K = R / 8), and after an exchange through distributed shared memory every
+// eighth row of the tile.  A row's score is the fp32 sum of eight shares, rounded once.
+// Warps 0-3: accumulators (thread = row), then all eight warps settle rows; 4: loads; 5: MMAs.
+constexpr int CL = 8, CL_THREADS = 256, CL_NS = 8;
+
+struct ClCtl {
+  unsigned long long full[CL_NS], empty[CL_NS];
+  unsigned long long wb_full, acc1_full, hid_full, acc2_full;
+  uint32_t tmem_base;
+  int abort_flag;
+  int wait_limit;           // must follow abort_flag
+};
+
+__global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CL_THREADS, 1)
+router_cluster_kernel(const Params p, const __grid_constant__ CUtensorMap tmx) {
+  extern __shared__ uint8_t smem_raw[];
+  cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  const uint32_t raw = smem_u32(smem_raw);
+  const uint32_t ring = (raw + 1023u) & ~1023u;
+  const Geo& g = p.g;
+  const int cw = p.R / CL;                              // my hidden columns
+  const uint32_t wa_bytes = cw * 128, stage_bytes = SLOT + (wa_bytes + 1023) / 1024 * 1024;
+  const uint32_t wb = ring + CL_NS * stage_bytes;       // the 64-deep slice of Wb that has my columns
+  const uint32_t wb_bytes = g.nd * 128;
+  ClCtl* c = reinterpret_cast<ClCtl*>(smem_raw + (wb - raw) + wb_bytes);
+  float* share = reinterpret_cast<float*>(smem_raw + (ring - raw));   // [128][E + 1], over the ring
+  const int EP = p.E + 1;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int rank = (int)cluster.block_rank(), tile = blockIdx.x / CL;
+  volatile int* af = &c->abort_flag;
+  grid_launch_dependents();
+  if (tid == 0) {
+    for (int i = 0; i < CL_NS; ++i) {
+      mbar_init(smem_u32(&c->full[i]), 1);
+      mbar_init(smem_u32(&c->empty[i]), 1);
+    }
+    mbar_init(smem_u32(&c->wb_full), 1);
+    mbar_init(smem_u32(&c->acc1_full), 1);
+    mbar_init(smem_u32(&c->hid_full), 128);
+    mbar_init(smem_u32(&c->acc2_full), 1);
+    c->abort_flag = 0;
+    c->wait_limit = (int)p.wait_limit;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    fence_proxy_async();
+  }
+  if (warp == 5) tmem_alloc(smem_u32(&c->tmem_base), 256);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  grid_dependency_wait();
+  const uint32_t tmem = c->tmem_base;                   // accumulator 1 / hidden at 0, 2 at 128
+
+  if (warp == 4) {
+    if (elect_one()) {
+      bool withheld = (p.withhold & 1) != 0 && blockIdx.x == 0;
+      const uint8_t* wa = p.packed + rank * wa_bytes;
+      mbar_arrive_expect_tx(smem_u32(&c->wb_full), wb_bytes);
+      bulk_g2s(wb, p.packed + g.w1_bytes + (long long)(rank * cw / 64) * wb_bytes, wb_bytes,
+               smem_u32(&c->wb_full));
+      RingPos r = {0, 0};
+      for (int kc = 0; kc < g.kc1; ++kc) {
+        if (!mbar_wait_fast(smem_u32(&c->empty[r.s]), r.ph ^ 1, af, p.dev_status)) break;
+        const uint32_t bar = smem_u32(&c->full[r.s]), dst = ring + r.s * stage_bytes;
+        mbar_arrive_expect_tx(bar, SLOT + wa_bytes);
+        tma_load_2d(dst, &tmx, kc * 64, tile * TILE_M, bar);
+        if (withheld) withheld = false;
+        else bulk_g2s(dst + SLOT, wa + (long long)kc * g.wa_bytes, wa_bytes, bar);
+        r.next(CL_NS);
+      }
+    }
+    __syncwarp();
+  } else if (warp == 5) {
+    if (elect_one()) {
+      const uint64_t d0 = smem_desc(ring), dw = smem_desc(wb);
+      const uint64_t hi = (d0 >> 32) << 32;
+      const uint32_t lo0 = (uint32_t)d0, id1 = instr_desc(TILE_M, cw), id2 = instr_desc(TILE_M, g.nd);
+      RingPos r = {0, 0};
+      bool ok = true;
+      for (int kc = 0; ok && kc < g.kc1; ++kc) {
+        ok = mbar_wait_fast(smem_u32(&c->full[r.s]), r.ph, af, p.dev_status);
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t alo = lo0 + r.s * (stage_bytes >> 4), blo = alo + (SLOT >> 4);
+#pragma unroll
+        for (uint32_t k = 0; k < 4; ++k)
+          umma_bf16(tmem, hi | (alo + 2 * k), hi | (blo + 2 * k), id1, (kc | k) != 0);
+        umma_commit(smem_u32(&c->empty[r.s]));
+        r.next(CL_NS);
+      }
+      if (ok) umma_commit(smem_u32(&c->acc1_full));
+      ok = ok && mbar_wait_fast(smem_u32(&c->wb_full), 0, af, p.dev_status) &&
+           mbar_wait_fast(smem_u32(&c->hid_full), 0, af, p.dev_status);
+      if (ok) {
+        tc_fence_after();
+        const uint32_t b0 = (uint32_t)dw + 2 * ((rank * cw & 63) >> 4);
+        for (int k = 0; k < (cw >> 4); ++k)
+          umma_bf16_ta(tmem + 128, tmem + 8 * k, hi | (b0 + 2 * k), id2, k != 0);
+        umma_commit(smem_u32(&c->acc2_full));
+      }
+    }
+    __syncwarp();
+  } else if (warp < 4) {
+    const uint32_t lb = (uint32_t)(tid & ~31) << 16;
+    bool ok = __all_sync(0xffffffffu,
+                         mbar_wait_fast(smem_u32(&c->acc1_full), 0, af, p.dev_status));
+    if (ok) {
+      tc_fence_after();
+      for (int c0 = 0; c0 < cw; c0 += 16) {
+        uint32_t v[16], w[8];
+        tmem_ld16(tmem + lb + c0, v);
+        tmem_wait_ld();
+        relu_pairs(v, w);
+        tmem_st8(tmem + lb + (c0 >> 1), w);
+      }
+      tmem_wait_st();
+      tc_fence_before();
+      mbar_arrive(smem_u32(&c->hid_full));
+      ok = __all_sync(0xffffffffu,
+                      mbar_wait_fast(smem_u32(&c->acc2_full), 0, af, p.dev_status));
+    }
+    if (ok) {                    // (both products are done: the ring is free)
+      tc_fence_after();
+      for (int c0 = 0; c0 < p.E; c0 += 16) {
+        uint32_t v[16];
+        tmem_ld16(tmem + lb + 128 + c0, v);
+        tmem_wait_ld();
+#pragma unroll
+        for (int q = 0; q < 16; ++q)
+          if (c0 + q < p.E) share[tid * EP + c0 + q] = __uint_as_float(v[q]);
+      }
+      tc_fence_before();
+    }
+  }
+  // (a CTA that gave up takes part in both cluster barriers all the same)
+  if (*af != 0)
+    for (int i = 0; i < 64; ++i) __nanosleep(1000);
+  __syncthreads();
+  tc_fence_after();
+  if (warp == 5) tmem_dealloc(tmem, 256);
+  cluster.sync();
+
+  const int nw = (p.E + 31) >> 5, v8 = p.d >> 3;
+  const int nrows = (int)min((long long)TILE_M, p.N - (long long)tile * TILE_M);
+  const float* part[CL];
+#pragma unroll
+  for (int k = 0; k < CL; ++k) part[k] = cluster.map_shared_rank(share, k);
+  for (int row = rank + CL * warp; row < nrows; row += CL * (CL_THREADS / 32)) {
+    const long long t = (long long)tile * TILE_M + row;
+    float sc[MAX_E / 32], m = -INFINITY;
+#pragma unroll
+    for (int j = 0; j < MAX_E / 32; ++j) {
+      const int e = lane + 32 * j;
+      sc[j] = 0.f;
+      if (e < p.E) {
+        float a[CL];
+#pragma unroll
+        for (int k = 0; k < CL; ++k) a[k] = part[k][row * EP + e];
+        sc[j] = fabsf(bfr(((a[0] + a[1]) + (a[2] + a[3])) + ((a[4] + a[5]) + (a[6] + a[7]))));
+        m = nanmax(m, sc[j]);
+        if (p.scores) p.scores[t * p.E + e] = __float2bfloat16_rn(sc[j]);
+      }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = nanmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+    const float thr = bfr(__fmul_rn(m, p.mult));
+    int kept = 0;
+#pragma unroll
+    for (int j = 0; j < MAX_E / 32; ++j) {
+      if (j >= nw) break;
+      const int e = lane + 32 * j;
+      const bool keep = e < p.E && sc[j] >= thr;
+      const uint32_t word = __ballot_sync(0xffffffffu, keep);
+      kept += __popc(word);
+      if (lane == 0) p.mask_bits[t * nw + j] = word;
+      if (p.rt_out && e < p.E) p.rt_out[t * p.E + e] = __float2bfloat16_rn(keep ? 1.f : 0.f);
+    }
+    if (p.out_init && (p.init_all || kept != 1)) {
+      for (int c8 = lane; c8 < v8; c8 += 32) {
+        uint4 o = make_uint4(0u, 0u, 0u, 0u);
+        if (p.last_bias) o = __ldg(reinterpret_cast<const uint4*>(p.last_bias) + c8);
+        if (p.resid)
+          o = add_bf16x8(o, __ldg(reinterpret_cast<const uint4*>(p.resid + t * p.d) + c8));
+        *(reinterpret_cast<uint4*>(p.out_init + t * p.d) + c8) = o;
+      }
+    }
+  }
+  cluster.sync();                // the others may still read this CTA's shares
+}
+
 __global__ void prepack_router_kernel(const bf16* __restrict__ wa, const bf16* __restrict__ wb,
                                       uint8_t* __restrict__ packed, Geo g, int d, int R, int E) {
   const long long n1 = (long long)g.kc1 * g.nsub * g.nsubw * 64;
@@ -513,6 +715,14 @@ int launch_prepack_router(const void* wa, const void* wb, void* packed, int d, i
   return cudaGetLastError() == cudaSuccess ? D2D_OK : D2D_ERR_LAUNCH;
 }
 
+// The cluster form: where the eight CTAs of every tile find an SM each (16 tiles) and Wa is worth
+// splitting (below 512 KB its stream is shorter than the exchange); it writes no counts table, so the
+// mask has to be short enough for the scatter kernel to count itself.
+bool umma_router_splits(int64_t N, int d, int R, int E) {
+  return N <= 16 * TILE_M && (int64_t)d * R >= 256 * 1024 && R % (16 * CL) == 0 &&
+         compact_counts_itself(N, E);
+}
+
 int launch_router_mask_umma(const void* x, const void* packed, float mult, uint32_t* mask_bits,
                             void* scores, void* rt_out, const void* last_bias, const void* resid,
                             void* out_init, bool init_all, int32_t* tile_counts, int64_t N, int d,
@@ -536,15 +746,24 @@ int launch_router_mask_umma(const void* x, const void* packed, float mult, uint3
   p.init_all = init_all ? 1 : 0;
   p.dev_status = dev_status;
   umma_debug_read(&p.wait_limit, &p.withhold);
-  const size_t smem = smem_bytes(p.g);
-  int sms = 0;
-  int rc = device_launch_facts((const void*)router_tiles_kernel, smem, &sms);
-  if (rc != D2D_OK) return rc;
+  const int64_t tiles = (N + TILE_M - 1) / TILE_M;
   // x as boxes of 64 columns x 128 consecutive rows; rows past the last token arrive as zeros
   alignas(64) CUtensorMap tmx;
-  rc = encode_tmap_2d_b16(&tmx, x, (uint64_t)d, (uint64_t)N, (uint64_t)d * 2, 64, TILE_M, true);
+  int rc = encode_tmap_2d_b16(&tmx, x, (uint64_t)d, (uint64_t)N, (uint64_t)d * 2, 64, TILE_M, true);
   if (rc != D2D_OK) return rc == D2D_ERR_BAD_ARG ? D2D_ERR_LAUNCH : rc;
-  const int64_t tiles = (N + TILE_M - 1) / TILE_M;
+  if (umma_router_splits(N, d, R, E)) {
+    const size_t wa_stage = SLOT + (size_t)(R / CL * 128 + 1023) / 1024 * 1024;
+    const size_t smem = 1024 + CL_NS * wa_stage + (size_t)p.g.nd * 128 + sizeof(ClCtl) + 64;
+    static_assert((TILE_M * (MAX_E + 1)) * 4 <= CL_NS * SLOT, "shares fit the ring");
+    rc = device_launch_facts((const void*)router_cluster_kernel, smem, nullptr);
+    if (rc != D2D_OK) return rc;
+    return launch_pdl(router_cluster_kernel, dim3((unsigned)(tiles * CL)), dim3(CL_THREADS), smem, s,
+                      p, tmx);
+  }
+  const size_t smem = smem_bytes(p.g);
+  int sms = 0;
+  rc = device_launch_facts((const void*)router_tiles_kernel, smem, &sms);
+  if (rc != D2D_OK) return rc;
   const int64_t grid = tiles < sms ? tiles : sms;
   return launch_pdl(router_tiles_kernel, dim3((unsigned)grid), dim3(NTHREADS), smem, s, p, tmx);
 }

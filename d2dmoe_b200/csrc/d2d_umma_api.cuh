@@ -23,6 +23,8 @@ bool umma_router_supported(int d, int R, int E, int dtype);
 size_t umma_router_packed_bytes(int d, int R, int E);
 int launch_prepack_router(const void* wa, const void* wb, void* packed, int d, int R, int E,
                           cudaStream_t s);
+// true: the launch below writes no tile_counts for this size
+bool umma_router_splits(int64_t N, int d, int R, int E);
 // out_init: initial output rows last_bias (+ resid), every row (init_all) or only those of tokens
 // not kept by exactly one expert (the expert kernel stores the others, see DirectRows)
 int launch_router_mask_umma(const void* x, const void* packed, float mult, uint32_t* mask_bits,

@@ -1,0 +1,210 @@
+"""Sizes at which the kernels of the layer change form or run out of tile: token counts around
+32 / 64 / 128, lists that are empty, single or everything, widths outside the multiples the
+wide forms take.  Against the CPU oracle, with the tolerances of the parity tests."""
+import numpy as np
+import pytest
+import torch
+
+from helpers import C, O, TOL, WINDOW
+
+pytestmark = pytest.mark.gpu
+
+
+def _gen(seed):
+    return torch.Generator().manual_seed(seed)
+
+
+def _layer(N, d, H, E, R, dtype, seed, act="relu", glu=False, mask_p=None):
+    c = C.LayerCase("edge", 1, N, d, H, E, R=R, dtype=dtype, act=act, glu=glu, seed=seed,
+                    zero_last_bias=glu)
+    return c, C.make_tensors(c)
+
+
+def _dev(t):
+    return None if t is None else t.cuda().contiguous()
+
+
+def _lists(wsp, E):
+    off = wsp.offsets.cpu().numpy()
+    return off, wsp.token_idx[: int(off[E])].cpu().numpy()
+
+
+def _mask(kind, N, E, g):
+    if kind == "one_expert":                  # every token to one expert, the others empty
+        m = torch.zeros(N, E, dtype=torch.bool)
+        m[:, E // 2] = True
+    elif kind == "all":
+        m = torch.ones(N, E, dtype=torch.bool)
+    elif kind == "first_token":               # lists of one row or none
+        m = torch.zeros(N, E, dtype=torch.bool)
+        m[0] = True
+    else:
+        m = torch.rand(N, E, generator=g) < 0.3
+    return m
+
+
+EXPERTS = [  # N, d, H, E, activation, gated
+    (1, 64, 16, 1, "relu", False), (31, 192, 48, 5, "gelu", False), (32, 128, 128, 7, "relu", False),
+    (33, 320, 32, 3, "tanh", False), (64, 768, 128, 4, "relu", False), (65, 128, 80, 6, "relu", False),
+    (127, 256, 128, 2, "leaky_relu", False), (129, 768, 32, 128, "relu", False),
+    (1, 128, 128, 4, "gelu", True), (32, 256, 128, 9, "gelu", True), (65, 192, 64, 3, "gelu", True),
+    (300, 256, 128, 5, "gelu", True),
+]
+
+
+@pytest.mark.parametrize("kind", ["random", "one_expert", "all", "first_token"])
+@pytest.mark.parametrize("N,d,H,E,act,glu", EXPERTS)
+def test_tensor_core_experts(N, d, H, E, act, glu, kind):
+    from d2dmoe_b200 import ops
+    c, t = _layer(N, d, H, E, 128, "bf16", N + d, act, glu)
+    m = _mask(kind, N, E, _gen(N))
+    wsp = ops.Workspace.allocate(N, E, "cuda")
+    wsp.mask_bits[:N].copy_(torch.from_numpy(O.pack_mask(m).view(np.int32)).cuda())
+    ops.compact(wsp, N, E)
+    w1, b1, w2, wu = (_dev(t.get(k)) for k in ("w1", "b1", "w2", "w_up"))
+    if glu:
+        b1 = None
+    packed = ops.prepack_experts(w1, b1, w2, wu)
+    assert packed is not None
+    x2d = _dev(t["x"].reshape(N, d))
+    out = torch.full((N, d), float("nan"), dtype=torch.bfloat16, device="cuda")
+    norms = torch.full((E, N), float("nan"), dtype=torch.bfloat16, device="cuda")
+    ex = O.experts_ffn_exact(t["x"].reshape(N, d), m, t["w1"], None if glu else t["b1"], t["w2"], act,
+                             t.get("w_up") if glu else None)
+    for kw in ({}, dict(norms=norms, norm_layer="output"), dict(norms=norms, norm_layer="intermediate")):
+        ops.experts_ffn(x2d, wsp, w1, b1, w2, act, out, w_up=wu, packed=packed, **kw)
+        wsp.check_status()
+        o = out.cpu().float()
+        assert torch.isfinite(o).all()
+        # k bf16 adds per element, each rounding at the running magnitude
+        assert O.rel_err(o, ex) <= TOL["bf16"] * max(1.0, m.sum(1).max().item() ** 0.5 / 2)
+        if kw:
+            ref = O.expert_activation_norms(t["x"].reshape(N, d), t["w1"], None if glu else t["b1"],
+                                            t["w2"], act, t.get("w_up") if glu else None,
+                                            layer=kw["norm_layer"], ord=2).float()
+            assert O.rel_err(norms.cpu().float(), torch.where(m.t(), ref, 0.0)) <= TOL["bf16"]
+
+
+@pytest.mark.parametrize("E", [8, 24, 128])
+@pytest.mark.parametrize("N", [1, 31, 33, 128, 129, 700, 2048])
+def test_large_router(N, E):
+    """Router 2048 -> 256 -> E: split over clusters for short calls (E = 128: up to 2048 tokens)."""
+    from d2dmoe_b200 import ops
+    d, R, tau = 2048, 256, 0.1
+    c, t = _layer(N, d, 128, E, R, "bf16", N + E)
+    x2d, wa, wb = _dev(t["x"].reshape(N, d)), _dev(t["wa"]), _dev(t["wb"])
+    lb = _dev(t["last_bias"].reshape(-1))
+    packed = ops.prepack_router(wa, wb)
+    wsp = ops.Workspace.allocate(N, E, "cuda")
+    sc = torch.empty(N, E, dtype=torch.bfloat16, device="cuda")
+    out = torch.full((N, d), float("nan"), dtype=torch.bfloat16, device="cuda")
+    for residual in (False, True):
+        ops.router_mask(x2d, wa, wb, tau, wsp, packed=packed, scores_out=sc, last_bias=lb,
+                        add_residual=residual, out_init=out)
+        wsp.check_status()
+        ref = O.router_scores(t["x"].reshape(N, d), t["wa"], t["wb"])
+        assert O.rel_err(sc.cpu(), ref) <= 2.0 ** -7
+        m = O.unpack_mask(wsp.mask_bits[:N].cpu().numpy().view(np.uint32), E)
+        assert torch.equal(m, O.dynk_max_mask(sc.cpu(), tau))
+        want = lb.float().expand(N, d) + (x2d.float() if residual else 0.0)
+        assert torch.equal(out, want.to(torch.bfloat16))
+    # the whole layer: lists of that mask, every row of the output written
+    w1, b1, w2 = _dev(t["w1"]), _dev(t["b1"]), _dev(t["w2"])
+    out.fill_(float("nan"))
+    rt = torch.empty(N, E, dtype=torch.bfloat16, device="cuda")
+    ops.moe_forward(x2d, wa, wb, tau, w1, b1, w2, "relu", out, wsp, last_bias=lb,
+                    router_packed=packed, experts_packed=ops.prepack_experts(w1, b1, w2),
+                    routing_out=rt)
+    wsp.check_status()
+    assert torch.equal(rt.cpu() > 0, m)
+    off, idx = _lists(wsp, E)
+    roff, ridx = O.expert_token_lists(m)
+    assert np.array_equal(off, np.asarray(roff)) and np.array_equal(idx, np.asarray(ridx))
+    ex = O.experts_ffn_exact(t["x"].reshape(N, d), m, t["w1"], t["b1"], t["w2"])
+    assert O.rel_err(out.cpu().float(), ex + t["last_bias"].double()) <= TOL["bf16"]
+
+
+@pytest.mark.parametrize("N,d,H,E,R", [(1, 4, 4, 1, 4), (31, 68, 36, 5, 36), (33, 260, 100, 33, 100),
+                                       (64, 768, 128, 24, 128), (95, 132, 32, 256, 160),
+                                       (257, 64, 64, 40, 64)])
+def test_fp32_layer(N, d, H, E, R):
+    from d2dmoe_b200 import ops
+    c, t = _layer(N, d, H, E, R, "fp32", N + d, act="gelu")
+    x2d, wa, wb = _dev(t["x"].reshape(N, d)), _dev(t["wa"]), _dev(t["wb"])
+    w1, b1, w2, lb = (_dev(t[k]) for k in ("w1", "b1", "w2", "last_bias"))
+    wsp = ops.Workspace.allocate(N, E, "cuda")
+    sc = torch.empty(N, E, device="cuda")
+    ops.router_mask(x2d, wa, wb, 0.3, wsp, scores_out=sc)
+    ref = O.router_scores(t["x"].reshape(N, d), t["wa"], t["wb"])
+    assert O.rel_err(sc.cpu(), ref) <= TOL["fp32"]
+    m = O.unpack_mask(wsp.mask_bits[:N].cpu().numpy().view(np.uint32), E)
+    assert torch.equal(m, O.dynk_max_mask(sc.cpu(), 0.3))
+    assert ((m != O.dynk_max_mask(ref, 0.3)) & ~O.near_threshold(ref, 0.3, WINDOW["fp32"])).sum() == 0
+    for residual in (False, True):
+        out = torch.full((N, d), float("nan"), device="cuda")
+        rt = torch.empty(N, E, device="cuda")
+        ops.moe_forward(x2d, wa, wb, 0.3, w1, b1, w2, "gelu", out, wsp, last_bias=lb.reshape(-1),
+                        add_residual=residual, routing_out=rt)
+        wsp.check_status()
+        assert torch.equal(rt.cpu() > 0, m)
+        ex = O.experts_ffn_exact(t["x"].reshape(N, d), m, t["w1"], t["b1"], t["w2"], "gelu")
+        ex = ex + t["last_bias"].double() + (t["x"].reshape(N, d).double() if residual else 0.0)
+        assert O.rel_err(out.cpu(), ex) <= TOL["fp32"]
+
+
+@pytest.mark.parametrize("dtype,E", [("bf16", 8), ("bf16", 24), ("bf16", 64), ("bf16", 72),
+                                     ("fp32", 4), ("fp32", 24), ("fp32", 32), ("fp32", 36)])
+@pytest.mark.parametrize("N", [1, 127, 129, 300])
+def test_every_mode_is_one_call(N, dtype, E):
+    """topk / dynk / all through the one-call layer: the same mask as the rule kernel alone (which
+    the upstream fixtures pin) on the layer's own scores, its lists, every output row."""
+    import d2dmoe_b200 as D
+    from d2dmoe_b200 import ops
+    c, t = _layer(N, 128, 32, E, 64, dtype, N + E)
+    moe = D.MoeficationMoE("m", c.d, E, True, c.H, torch.nn.ReLU)
+    moe.router = D.MoeficationRouter(c.d, E, width=64, depth=2, bias=False, activation="relu",
+                                     output_activation="abs")
+    moe = moe.to(c.torch_dtype)
+    moe.load_state_dict({"experts.w1": t["w1"], "experts.b1": t["b1"], "experts.w2": t["w2"],
+                         "last_bias": t["last_bias"], "router.layers.0.weight": t["wa"],
+                         "router.layers.2.weight": t["wb"]})
+    moe = moe.cuda().eval()
+    x, x2d = t["x"].cuda(), t["x"].reshape(N, c.d)
+    wsp = ops.Workspace.allocate(N, E, "cuda")
+    sc = torch.empty(N, E, dtype=c.torch_dtype, device="cuda")
+    ops.router_mask(x.reshape(N, c.d), _dev(t["wa"]), _dev(t["wb"]), 0.5, wsp, scores_out=sc,
+                    packed=moe.router.packed())
+    for mode, k, tau in (("topk", 1, None), ("topk", min(3, E), None), ("topk", E, None),
+                         ("dynk", None, 0.0), ("dynk", None, 0.45), ("dynk", None, 2.0),
+                         ("all", None, None)):
+        moe.forward_mode, moe.k, moe.tau = mode, k, tau
+        out, gd = moe(x)
+        got = gd["m"][0].reshape(N, E).cpu() > 0
+        if mode == "all":
+            want = torch.ones(N, E, dtype=torch.bool)
+        else:
+            ops.mask_rule_from_scores(sc, mode, wsp, k=k, tau=tau)
+            want = O.unpack_mask(wsp.mask_bits[:N].cpu().numpy().view(np.uint32), E)
+        assert torch.equal(got, want), (mode, k, tau)
+        w = moe.last_workspace(N, x.device)
+        w.check_status()
+        off, idx = _lists(w, E)
+        roff, ridx = O.expert_token_lists(want)
+        assert np.array_equal(off, np.asarray(roff)) and np.array_equal(idx, np.asarray(ridx))
+        ex = O.experts_ffn_exact(x2d, want, t["w1"], t["b1"], t["w2"]) + t["last_bias"].double()
+        # bf16: k adds, each rounding at the running magnitude
+        slack = max(1.0, want.sum(1).max().item() ** 0.5 / 2) if dtype == "bf16" else 1.0
+        assert O.rel_err(out.reshape(N, c.d).cpu().float(), ex) <= TOL[dtype] * slack
+
+
+@pytest.mark.parametrize("N,E", [(8192, 24), (8193, 24), (4096, 33), (4097, 33), (255, 256), (2100, 128)])
+def test_compaction_with_and_without_table(N, E):
+    from d2dmoe_b200 import ops
+    m = torch.rand(N, E, generator=_gen(E)) < 0.1
+    wsp = ops.Workspace.allocate(N, E, "cuda")
+    wsp.mask_bits[:N].copy_(torch.from_numpy(O.pack_mask(m).view(np.int32)).cuda())
+    ops.compact(wsp, N, E)
+    wsp.check_status()
+    off, idx = _lists(wsp, E)
+    roff, ridx = O.expert_token_lists(m)
+    assert np.array_equal(off, np.asarray(roff)) and np.array_equal(idx, np.asarray(ridx))
