@@ -239,7 +239,7 @@ int d2d_moe_forward_rule(const void* x, const void* wa, const void* wb,
                            aligned(last_bias_opt, 16) && aligned(router_packed_opt, 1024);
   // where the tensor-core expert kernel follows, the rows of tokens with one expert are left to it
   DirectRows dr;
-  const bool may_store = !pre && !add_residual && umma_experts && aligned(last_bias_opt, 16);
+  bool may_store = !pre && !add_residual && umma_experts && aligned(last_bias_opt, 16);
   auto leave_rows = [&]() {
     dr.mask_bits = mask_bits;
     dr.last_bias = last_bias_opt;
@@ -260,13 +260,18 @@ int d2d_moe_forward_rule(const void* x, const void* wa, const void* wb,
     nl += 1;
     lists_ready = rt_done = true;
   } else if (ranked && !scores) {
-    // scores of the fused router for the rule below; its own mask is overwritten there
+    // scores of the fused router for the rule below (its own mask is overwritten there); it also
+    // writes every initial row, at no cost of its own: hardly a token keeps just one expert
     rc = umma_router
              ? launch_router_mask_umma(x, router_packed_opt, thresh_mult, mask_bits,
-                                       scores_scratch, nullptr, nullptr, nullptr, nullptr, true,
-                                       nullptr, N, d, R, E, dev_status, s)
-             : launch_router_mask_simt(x, wa, wb, thresh_mult, mask_bits, scores_scratch, nullptr,
-                                       0, nullptr, N, d, R, E, dtype, dev_status, s);
+                                       scores_scratch, nullptr, last_bias_opt,
+                                       add_residual ? x : nullptr, out_init, true, nullptr, N, d, R,
+                                       E, dev_status, s)
+             : launch_router_mask_simt(x, wa, wb, thresh_mult, mask_bits, scores_scratch,
+                                       last_bias_opt, add_residual, out_init, N, d, R, E, dtype,
+                                       dev_status, s);
+    out_init = nullptr;
+    may_store = false;
     nl += 1;
     scores = scores_scratch;
   }
@@ -287,7 +292,7 @@ int d2d_moe_forward_rule(const void* x, const void* wa, const void* wb,
                                             dev_status, s);
       if (rc != D2D_OK) return rc;
       nl += 1;
-      if (!pre) {
+      if (out_init) {
         rc = launch_init_out(x, last_bias_opt, add_residual, out, N, d, dtype, s);
         nl += 1;
       }

@@ -124,6 +124,18 @@ __device__ __forceinline__ uint4 add_bf16x8(uint4 a, uint4 b) {
 __device__ __forceinline__ void red_add_1(float* p, float a) { atomicAdd(p, a); }
 __device__ __forceinline__ void red_add_1(bf16* p, float a) { atomicAdd(p, __float2bfloat16_rn(a)); }
 
+// bits i (even experts) and 16 + i (odd experts) -> bits 2i and 2i + 1
+__device__ __forceinline__ uint32_t interleave16(uint32_t v) {
+  uint32_t t = (v ^ (v >> 8)) & 0x0000ff00u;
+  v ^= t ^ (t << 8);
+  t = (v ^ (v >> 4)) & 0x00f000f0u;
+  v ^= t ^ (t << 4);
+  t = (v ^ (v >> 2)) & 0x0c0c0c0cu;
+  v ^= t ^ (t << 2);
+  t = (v ^ (v >> 1)) & 0x22222222u;
+  return v ^ t ^ (t << 1);
+}
+
 // 32 x 32 bit matrix, one row per lane, turned over: bit i of lane b's result = bit b of lane i's
 // word (block swaps of size 16, 8, 4, 2, 1)
 __device__ __forceinline__ uint32_t transpose32(uint32_t x, int lane) {

@@ -465,7 +465,20 @@ gate_scores_fused_rows_kernel(const T* __restrict__ scores, float mult, int k, f
   if (w < 4) {
     const T* sv = reinterpret_cast<const T*>(raw);
     uint32_t word[2] = {0u, 0u};
-    if (RULE == 0) {
+    if (RULE == 0 && sizeof(T) == 2) {
+      // pairs throughout: the code is executed once per CTA, so its length is what it costs
+      const __nv_bfloat162* pr = reinterpret_cast<const __nv_bfloat162*>(raw);
+      __nv_bfloat162 m2 = pr[0];
+#pragma unroll
+      for (int q = 1; q < NV * 4; ++q) m2 = __hmax2_nan(m2, pr[q]);
+      const float m = nanmax(__low2float(m2), __high2float(m2));
+      const __nv_bfloat162 thr = __float2bfloat162_rn(__fmul_rn(m, mult));
+#pragma unroll
+      for (int q = 0; q < NV * 4; ++q)
+        word[q >> 4] |= __hge2_mask(pr[q], thr) & (0x00010001u << (q & 15));
+      word[0] = interleave16(word[0]);
+      word[1] = interleave16(word[1]);
+    } else if (RULE == 0) {
       float m = -INFINITY;
 #pragma unroll
       for (int e = 0; e < EMAX; ++e)
@@ -537,13 +550,23 @@ gate_scores_fused_rows_kernel(const T* __restrict__ scores, float mult, int k, f
         __ballot_sync(0xffffffffu, live && __popc(word[0]) + __popc(word[1]) != 1);
     if (lane == 0) rows[w] = todo;
     if (live) {
-      for (int j = 0; j < nw; ++j) mask_bits[t * nw + j] = word[j];
+      mask_bits[t * nw] = word[0];
+      if (nw > 1) mask_bits[t * nw + 1] = word[1];
       if (rt) {
         uint4 one[NV];
-        T* ov = reinterpret_cast<T*>(one);
+        if (sizeof(T) == 2) {
+          uint32_t* ov = reinterpret_cast<uint32_t*>(one);
 #pragma unroll
-        for (int e = 0; e < EMAX; ++e)
-          ov[e] = DT<T>::from_f((word[e >> 5] >> (e & 31)) & 1u ? 1.0f : 0.0f);
+          for (int q = 0; q < NV * 4; ++q) {
+            const uint32_t b = word[q >> 4] >> (2 * (q & 15));
+            ov[q] = (b & 1u) * 0x3f80u | (b & 2u) * (0x3f800000u >> 1);      // bf16 1.0 or 0
+          }
+        } else {
+          T* ov = reinterpret_cast<T*>(one);
+#pragma unroll
+          for (int e = 0; e < EMAX; ++e)
+            ov[e] = DT<T>::from_f((word[e >> 5] >> (e & 31)) & 1u ? 1.0f : 0.0f);
+        }
 #pragma unroll
         for (int q = 0; q < NV; ++q) *(reinterpret_cast<uint4*>(rt + t * E) + q) = one[q];
       }
@@ -572,11 +595,11 @@ all_experts_kernel(uint32_t* __restrict__ mask_bits, T* __restrict__ rt,
   const int nw = (E + 31) / 32;
   grid_launch_dependents();
   grid_dependency_wait();
-  for (int e = 0; e < E; ++e)
-    for (int64_t t = i0; t < N; t += step) {
-      token_idx[e * N + t] = (int32_t)t;
-      if (rt) rt[e * N + t] = DT<T>::from_f(1.f);
-    }
+  const uint32_t n = (uint32_t)N, pairs = n * (uint32_t)E;         // < 2^31
+  for (uint32_t i = (uint32_t)i0; i < pairs; i += (uint32_t)step) {
+    token_idx[i] = (int32_t)(i % n);
+    if (rt) rt[i] = DT<T>::from_f(1.f);
+  }
   for (int64_t i = i0; i < N * nw; i += step) {
     const int j = (int)(i % nw);
     mask_bits[i] = 32 * j + 32 <= E ? 0xffffffffu : (1u << (E - 32 * j)) - 1u;
@@ -799,7 +822,7 @@ int launch_all_experts(uint32_t* mask_bits, void* rt, int32_t* token_idx, int32_
   if (E > 256 || N * (int64_t)E > 0x7fffffffLL) return D2D_ERR_UNSUPPORTED;
   if (out && (d % V != 0 || !al16(out) || !al16(x) || !al16(last_bias)))
     return D2D_ERR_UNSUPPORTED;
-  const int64_t work = out ? (N * (d / V) > N ? N * (d / V) : N) : N;
+  const int64_t work = out && d / V > E ? N * (d / V) : N * E;
   const int grid = grid_for(work, NT, 148 * 8);
   if (dtype == D2D_F32)
     return launch_pdl(all_experts_kernel<float>, dim3((unsigned)grid), dim3(NT), 0, s, mask_bits,

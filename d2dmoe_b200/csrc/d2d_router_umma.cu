@@ -93,18 +93,6 @@ struct Ctl {
   uint32_t init_rows[2][4];
 };
 
-// bits i (even experts) and 16 + i (odd experts) -> bits 2i and 2i + 1
-__device__ __forceinline__ uint32_t interleave16(uint32_t v) {
-  uint32_t t = (v ^ (v >> 8)) & 0x0000ff00u;
-  v ^= t ^ (t << 8);
-  t = (v ^ (v >> 4)) & 0x00f000f0u;
-  v ^= t ^ (t << 4);
-  t = (v ^ (v >> 2)) & 0x0c0c0c0cu;
-  v ^= t ^ (t << 2);
-  t = (v ^ (v >> 1)) & 0x22222222u;
-  return v ^ t ^ (t << 1);
-}
-
 __device__ void role_load(const Params& p, Ctl* c, const CUtensorMap* tmx, uint32_t ring,
                           uint32_t wb, uint32_t stage_bytes) {
   volatile int* af = &c->abort_flag;
