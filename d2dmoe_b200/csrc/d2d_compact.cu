@@ -22,11 +22,7 @@ namespace d2d {
 namespace {
 
 constexpr int NT = 256;
-constexpr int NTS = 256;                 // scatter CTA: one warp per row of 32 tokens
-constexpr int ROWS = 8;                  // rows of 32 tokens per scatter CTA (one per warp)
-constexpr int CHUNK = ROWS * 32;
 constexpr int CTILE = 128;               // granularity of the counts table
-constexpr int TILES_PER_CHUNK = CHUNK / CTILE;
 constexpr int MAX_E = 256;
 
 // one warp = one 128-token tile; lane b ends up with the count of expert 32j+b
@@ -52,11 +48,13 @@ compact_count_kernel(const uint32_t* __restrict__ mask_bits, uint8_t* __restrict
   }
 }
 
-template <bool TABLE>
-__global__ void __launch_bounds__(NTS)
+// ROWS: 32-token rows of a CTA, one per warp
+template <bool TABLE, int ROWS>
+__global__ void __launch_bounds__(32 * ROWS)
 compact_scatter_kernel(const uint32_t* __restrict__ mask_bits, const uint8_t* __restrict__ counts,
                        int32_t* __restrict__ token_idx, int32_t* __restrict__ offsets, int64_t N,
                        int E, int EP, int ntiles, int* dev_status) {
+  constexpr int NTS = 32 * ROWS, CHUNK = 32 * ROWS, TILES_PER_CHUNK = CHUNK / CTILE;
   extern __shared__ int sm[];
   int* cnt = sm;                 // [ROWS][E] -> becomes each row's write base
   int* tot = cnt + ROWS * E;     // [EP]  total per expert, then exclusive offsets
@@ -241,7 +239,6 @@ int launch_compact(const uint32_t* mask_bits, int32_t* token_idx, int32_t* offse
   }
   const int EP = compact_row_cells(E);
   const int64_t ntiles = ceil_div64(N, CTILE);
-  const int64_t nchunks = ceil_div64(N, CHUNK);
   uint8_t* counts = reinterpret_cast<uint8_t*>(counts_ws);
   const bool table = counts_ready || !compact_counts_itself(N, E);
   if (table && !counts_ready) {
@@ -249,10 +246,18 @@ int launch_compact(const uint32_t* mask_bits, int32_t* token_idx, int32_t* offse
                                                                              E, EP);
     if (cudaGetLastError() != cudaSuccess) return D2D_ERR_LAUNCH;
   }
-  const size_t smem = sizeof(int) * ((size_t)ROWS * E + 2 * (size_t)EP);
-  return launch_pdl(table ? compact_scatter_kernel<true> : compact_scatter_kernel<false>,
-                    dim3((unsigned)nchunks), dim3(NTS), smem, s, mask_bits, (const uint8_t*)counts,
-                    token_idx, offsets, N, E, EP, (int)ntiles, dev_status);
+  // Every CTA sweeps the whole table, so with many chunks of 256 tokens the sweeps are what the
+  // launch costs: chunks of 1024 (a quarter of the CTAs, four times the threads for each sweep) once
+  // there are more 256-token chunks than SMs.  (131072 tokens x 128: 21.8 -> 14.7 us; a layer of
+  // 65536 x 96: 124.1 -> 118.9, of 50432 x 24: 87.0 -> 85.7.)
+  const bool big = N > 148 * 256;
+  const int rows = big ? 32 : 8;
+  const int64_t nchunks = ceil_div64(N, 32 * rows);
+  const size_t smem = sizeof(int) * ((size_t)rows * E + 2 * (size_t)EP);
+  auto kernel = table ? (big ? compact_scatter_kernel<true, 32> : compact_scatter_kernel<true, 8>)
+                      : (big ? compact_scatter_kernel<false, 32> : compact_scatter_kernel<false, 8>);
+  return launch_pdl(kernel, dim3((unsigned)nchunks), dim3(32 * rows), smem, s, mask_bits,
+                    (const uint8_t*)counts, token_idx, offsets, N, E, EP, (int)ntiles, dev_status);
 }
 
 }  // namespace d2d

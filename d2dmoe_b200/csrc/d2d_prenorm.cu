@@ -33,6 +33,8 @@ prenorm_init_kernel(const T* __restrict__ x, const T* __restrict__ gamma,
                     const T* __restrict__ last_bias, T* __restrict__ xn, T* __restrict__ out,
                     int64_t N, int d) {
   constexpr int V = 16 / sizeof(T);
+  grid_launch_dependents();
+  grid_dependency_wait();
   const int lane = threadIdx.x & 31;
   const int dv = d / V;                       // vectors per row
   const int nv = (dv + 31) / 32;              // vectors per lane (<= MAXV)
@@ -156,9 +158,9 @@ int launch_prenorm_init(const void* x, const void* gamma, const void* beta, floa
   if (grid < 1) grid = 1;
   const int nv = (d / V + 31) / 32;
 #define D2D_PRENORM_CASE(T_, NV_)                                                              \
-  prenorm_init_kernel<T_, NV_><<<(unsigned)grid, NT, 0, s>>>(                                   \
-      (const T_*)x, (const T_*)gamma, (const T_*)beta, eps, kind, gamma_offset,                 \
-      (const T_*)last_bias, (T_*)xn, (T_*)out, N, d)
+  return launch_pdl(prenorm_init_kernel<T_, NV_>, dim3((unsigned)grid), dim3(NT), 0, s,         \
+                    (const T_*)x, (const T_*)gamma, (const T_*)beta, eps, kind, gamma_offset,   \
+                    (const T_*)last_bias, (T_*)xn, (T_*)out, N, d)
 #define D2D_PRENORM_BY_NV(T_)                                                                  \
   do {                                                                                         \
     if (nv <= 1) D2D_PRENORM_CASE(T_, 1);                                                      \
@@ -172,7 +174,6 @@ int launch_prenorm_init(const void* x, const void* gamma, const void* beta, floa
   else D2D_PRENORM_BY_NV(bf16);
 #undef D2D_PRENORM_BY_NV
 #undef D2D_PRENORM_CASE
-  return cudaGetLastError() == cudaSuccess ? D2D_OK : D2D_ERR_LAUNCH;
 }
 
 }  // namespace d2d
