@@ -246,6 +246,9 @@ int d2d_moe_forward_rule(const void* x, const void* wa, const void* wb,
   };
   bool counts_ready = false, lists_ready = false, rt_done = routing_tensor_opt == nullptr;
   const void* scores = scores_in_opt;
+  ListsOut lists;                  // short calls: written by the kernel that applies the rule
+  lists.token_idx = token_idx;
+  lists.offsets = offsets;
 
   if (rule == D2D_RULE_ALL) {
     rc = launch_all_experts(mask_bits, routing_tensor_opt, token_idx, offsets, x, last_bias_opt,
@@ -281,7 +284,7 @@ int d2d_moe_forward_rule(const void* x, const void* wa, const void* wb,
     // rule + counts table + output init in one launch when the shape allows it
     rc = launch_gate_scores_fused(scores, rule, k, tau, thresh_mult, mask_bits,
                                   routing_tensor_opt, (int32_t*)ws, x, last_bias_opt, add_residual,
-                                  out_init, may_store, N, d, E, dtype, s);
+                                  out_init, may_store, N, d, E, dtype, s, &lists);
     if (rc == D2D_OK) {
       counts_ready = rt_done = true;
       if (may_store) leave_rows();
@@ -301,7 +304,8 @@ int d2d_moe_forward_rule(const void* x, const void* wa, const void* wb,
     // the tensor-core router also fills the compaction's counts table
     rc = launch_router_mask_umma(x, router_packed_opt, thresh_mult, mask_bits, nullptr,
                                  routing_tensor_opt, last_bias_opt, add_residual ? x : nullptr,
-                                 out_init, !may_store, (int32_t*)ws, N, d, R, E, dev_status, s);
+                                 out_init, !may_store, (int32_t*)ws, N, d, R, E, dev_status, s,
+                                 &lists);
     if (may_store) leave_rows();
     counts_ready = !umma_router_splits(N, d, R, E);
     rt_done = true;
@@ -315,7 +319,7 @@ int d2d_moe_forward_rule(const void* x, const void* wa, const void* wb,
     nl += 1;
   }
   if (rc != D2D_OK) return rc;
-  if (!lists_ready) {
+  if (!lists_ready && !lists.written) {
     rc = launch_compact(mask_bits, token_idx, offsets, N, E, (int32_t*)ws, dev_status, s,
                         counts_ready);
     if (rc != D2D_OK) return rc;

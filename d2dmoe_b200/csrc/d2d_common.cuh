@@ -49,22 +49,35 @@ __device__ __forceinline__ void grid_dependency_wait() {
 __device__ __forceinline__ void grid_launch_dependents() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
+// cluster > 0: in clusters of that many CTAs.
 template <typename... KArgs, typename... Args>
-inline int launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
-                      cudaStream_t s, Args... args) {
+inline int launch_pdl_cluster(int cluster, void (*kernel)(KArgs...), dim3 grid, dim3 block,
+                              size_t smem, cudaStream_t s, Args... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
+  if (cluster > 0) {
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = (unsigned)cluster;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cfg.numAttrs = 2;
+  }
   if (cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...) == cudaSuccess) return D2D_OK;
   cudaGetLastError();
   return D2D_ERR_LAUNCH;
+}
+
+template <typename... KArgs, typename... Args>
+inline int launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                      cudaStream_t s, Args... args) {
+  return launch_pdl_cluster(0, kernel, grid, block, smem, s, args...);
 }
 
 // ---- device status word ---------------------------------------------------
@@ -175,11 +188,17 @@ int launch_gate_rule(const void* scores, int rule, int k, float tau, uint32_t* m
 int launch_mask_from_scores(const void* scores, float mult, uint32_t* mask_bits, int64_t N, int E,
                             int dtype, int* dev_status, cudaStream_t s);
 // rule 0: dynk_max with threshold multiplier mult; D2D_RULE_TOPK (k), D2D_RULE_DYNK (tau).
-// direct: initial rows only of tokens not kept by exactly one expert
+// direct: initial rows only of tokens not kept by exactly one expert.  *lists: in, token_idx and
+// offsets may be written here as well (short calls); out, they were
+struct ListsOut {
+  int32_t* token_idx = nullptr;
+  int32_t* offsets = nullptr;
+  bool written = false;
+};
 int launch_gate_scores_fused(const void* scores, int rule, int k, float tau, float mult,
                              uint32_t* mask_bits, void* rt, int32_t* tile_counts, const void* x,
                              const void* last_bias, int add_residual, void* out, bool direct,
-                             int64_t N, int d, int E, int dtype, cudaStream_t s);
+                             int64_t N, int d, int E, int dtype, cudaStream_t s, ListsOut* lists);
 int launch_all_experts(uint32_t* mask_bits, void* rt, int32_t* token_idx, int32_t* offsets,
                        const void* x, const void* last_bias, int add_residual, void* out,
                        int64_t N, int d, int E, int dtype, cudaStream_t s);

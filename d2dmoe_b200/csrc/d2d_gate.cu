@@ -8,6 +8,7 @@
 // Each Linear output is materialised in the tensor dtype T upstream, so the fp32
 // accumulators are rounded to T once after each of the two products, and the
 // threshold is rounded to T before the comparison.
+#include "d2d_cluster_compact.cuh"
 #include "d2d_common.cuh"
 
 namespace d2d {
@@ -439,9 +440,11 @@ gate_scores_fused_rows_kernel(const T* __restrict__ scores, float mult, int k, f
                               uint8_t* __restrict__ tile_counts, int EP,
                               const T* __restrict__ x, const T* __restrict__ last_bias,
                               int add_residual, T* __restrict__ out, int direct, int64_t N, int d,
-                              int E) {
-  __shared__ int cnt[4][64];
+                              int E, int32_t* __restrict__ token_idx,
+                              int32_t* __restrict__ offsets) {
+  __shared__ uint32_t cnt[4][64];        // tokens of a 32-token row that keep an expert, as bits
   __shared__ uint32_t rows[4];
+  __shared__ int scratch[3 * 256];
   constexpr int V = 16 / sizeof(T);
   constexpr int EMAX = NV * V;
   constexpr int NW = (EMAX + 31) / 32;
@@ -572,14 +575,17 @@ gate_scores_fused_rows_kernel(const T* __restrict__ scores, float mult, int k, f
       }
     }
 #pragma unroll
-    for (int j = 0; j < NW; ++j)         // lane b: how many of the warp's tokens keep expert 32j + b
-      cnt[w][32 * j + lane] = __popc(transpose32(word[j], lane));
+    for (int j = 0; j < NW; ++j)         // lane b: which of the warp's tokens keep expert 32j + b
+      cnt[w][32 * j + lane] = transpose32(word[j], lane);
   }
   __syncthreads();
-  for (int e = tid; e < EP; e += NT)
-    tile_counts[(int64_t)blockIdx.x * EP + e] =
-        (uint8_t)(e < E ? cnt[0][e] + cnt[1][e] + cnt[2][e] + cnt[3][e] : 0);
+  if (!token_idx)
+    for (int e = tid; e < EP; e += NT)
+      tile_counts[(int64_t)blockIdx.x * EP + e] =
+          (uint8_t)(e < E ? __popc(cnt[0][e]) + __popc(cnt[1][e]) + __popc(cnt[2][e]) + __popc(cnt[3][e])
+                          : 0);
   if (out && direct) init_tile_rows(x, last_bias, add_residual, out, t0, ntok, d, rows, w, lane);
+  if (token_idx) cluster_compact<NT>(&cnt[0][0], 64, scratch, E, t0, token_idx, offsets);
 }
 
 // Mode 'all' (every expert on every token): mask, routing tensor, lists and offsets, and the
@@ -763,7 +769,7 @@ int launch_gate_rule(const void* scores, int rule, int k, float tau, uint32_t* m
 int launch_gate_scores_fused(const void* scores, int rule, int k, float tau, float mult,
                              uint32_t* mask_bits, void* rt, int32_t* tile_counts, const void* x,
                              const void* last_bias, int add_residual, void* out, bool direct,
-                             int64_t N, int d, int E, int dtype, cudaStream_t s) {
+                             int64_t N, int d, int E, int dtype, cudaStream_t s, ListsOut* lists) {
   const int V = dtype == D2D_F32 ? 4 : 8;
   auto al16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
   if (E > 256 || d % V != 0 || !al16(out) || !al16(x) || !al16(last_bias))
@@ -776,14 +782,18 @@ int launch_gate_scores_fused(const void* scores, int rule, int k, float tau, flo
   const int row_bytes = E * (dtype == D2D_F32 ? 4 : 2);
   const bool rows_form = row_bytes % 16 == 0 && row_bytes <= 128 && al16(scores) &&
                          (rt == nullptr || al16(rt));
+  const bool fused = rows_form && lists && grid <= CLUSTER_TILES;
+  if (fused) lists->written = true;
 #define D2D_ROWS_CASE(T, NVV)                                                                 \
   case NVV: {                                                                                 \
     auto kn = rule == 0               ? gate_scores_fused_rows_kernel<T, NVV, 0>              \
               : rule == D2D_RULE_TOPK ? gate_scores_fused_rows_kernel<T, NVV, D2D_RULE_TOPK>  \
                                       : gate_scores_fused_rows_kernel<T, NVV, D2D_RULE_DYNK>; \
-    return launch_pdl(kn, dim3((unsigned)grid), dim3(NT), 0, s, (const T*)scores, mult, k,    \
-                      tau, mask_bits, (T*)rt, counts, EP, (const T*)x, (const T*)last_bias,   \
-                      add_residual, (T*)out, direct ? 1 : 0, N, d, E);                        \
+    return launch_pdl_cluster(fused ? (int)grid : 0, kn, dim3((unsigned)grid), dim3(NT), 0, s,\
+                              (const T*)scores, mult, k, tau, mask_bits, (T*)rt, counts, EP,  \
+                              (const T*)x, (const T*)last_bias, add_residual, (T*)out,        \
+                              direct ? 1 : 0, N, d, E, fused ? lists->token_idx : nullptr,    \
+                              fused ? lists->offsets : nullptr);                              \
   }
   if (rows_form) {
     if (dtype == D2D_F32) {

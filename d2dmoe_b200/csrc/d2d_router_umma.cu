@@ -21,6 +21,7 @@
 // TMA unit in front of the loads) the second epilogue no longer sits between two tiles.
 #include <cooperative_groups.h>
 
+#include "d2d_cluster_compact.cuh"
 #include "d2d_tmap.cuh"
 #include "d2d_umma_api.cuh"
 #include "d2d_umma_ptx.cuh"
@@ -72,6 +73,8 @@ struct Params {
   bf16* scores;             // optional [N, E]
   bf16* rt_out;             // optional: 0/1 routing tensor [N, E]
   uint8_t* tile_counts;     // optional: bytes [tiles][EP], kept tokens per expert
+  int32_t* token_idx;       // optional (one tile per CTA, all CTAs one cluster): the token lists
+  int32_t* offsets;
   int EP;
   bf16* out_init;           // optional: initial output rows last_bias (+ resid)
   const bf16* last_bias;
@@ -301,7 +304,11 @@ __device__ void role_gate(const Params& p, Ctl* c, uint32_t tmem, int et) {
       __syncwarp();
       ibuf_ph ^= buf;
     }
-    if (p.tile_counts) {
+    if (p.token_idx) {         // (the only tile: both halves of cnt are free)
+#pragma unroll
+      for (int j = 0; j < NW; ++j)
+        c->cnt[0][q4][32 * j + lane] = (int)transpose32(word[j], lane);
+    } else if (p.tile_counts) {
 #pragma unroll
       for (int j = 0; j < NW; ++j)
         c->cnt[buf][q4][32 * j + lane] = __popc(transpose32(word[j], lane));
@@ -452,6 +459,15 @@ router_tiles_kernel(const Params p, const __grid_constant__ CUtensorMap tmx) {
     __syncwarp();
     tc_fence_after();
     tmem_dealloc(tmem, 512);
+  }
+  if (p.token_idx) {
+    uint32_t* rows = reinterpret_cast<uint32_t*>(&c->cnt[0][0][0]);
+    if (*reinterpret_cast<volatile int*>(&c->abort_flag) != 0) {     // nothing a list may rely on
+      for (int i = tid; i < 4 * MAX_E; i += NTHREADS) rows[i] = 0u;
+      __syncthreads();
+    }
+    cluster_compact<NTHREADS>(rows, MAX_E, reinterpret_cast<int*>(smem_raw + (base - raw)), p.E,
+                              (int64_t)blockIdx.x * TILE_M, p.token_idx, p.offsets);
   }
 }
 
@@ -648,6 +664,55 @@ router_cluster_kernel(const Params p, const __grid_constant__ CUtensorMap tmx) {
     }
   }
   cluster.sync();                // the others may still read this CTA's shares
+  if (p.token_idx && rank == 0) {
+    // one tile: its lists from the mask words that the cluster has written (visible since the
+    // barrier), 32 tokens a warp
+    uint32_t* rows = reinterpret_cast<uint32_t*>(smem_raw + (ring - raw));      // [4][MAX_E]
+    int* off = reinterpret_cast<int*>(rows + 4 * MAX_E);
+    if (warp < 4) {
+      const long long t = 32 * warp + lane;
+#pragma unroll
+      for (int j = 0; j < MAX_E / 32; ++j) {
+        const uint32_t word =
+            j < nw && t < p.N ? *const_cast<volatile uint32_t*>(p.mask_bits + t * nw + j) : 0u;
+        rows[warp * MAX_E + 32 * j + lane] = transpose32(word, lane);
+      }
+    }
+    __syncthreads();
+    if (warp == 0) {             // four experts per lane
+      int v[4], s = 0;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int e = 4 * lane + k;
+        v[k] = 0;
+        if (e < p.E)
+          for (int q = 0; q < 4; ++q) v[k] += __popc(rows[q * MAX_E + e]);
+        s += v[k];
+      }
+      int incl = s;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += u;
+      }
+      int run = incl - s;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int e = 4 * lane + k;
+        if (e < p.E) off[e] = p.offsets[e] = run;
+        run += v[k];
+      }
+      if (lane == 31) p.offsets[p.E] = incl;
+    }
+    __syncthreads();
+    for (int i = tid; i < 4 * p.E; i += CL_THREADS) {
+      const int q = i / p.E, e = i - q * p.E;
+      int at = off[e];
+      for (int k = 0; k < q; ++k) at += __popc(rows[k * MAX_E + e]);
+      for (uint32_t m = rows[q * MAX_E + e]; m != 0u; m &= m - 1)
+        p.token_idx[at++] = 32 * q + __ffs(m) - 1;
+    }
+  }
 }
 
 __global__ void prepack_router_kernel(const bf16* __restrict__ wa, const bf16* __restrict__ wb,
@@ -714,7 +779,7 @@ bool umma_router_splits(int64_t N, int d, int R, int E) {
 int launch_router_mask_umma(const void* x, const void* packed, float mult, uint32_t* mask_bits,
                             void* scores, void* rt_out, const void* last_bias, const void* resid,
                             void* out_init, bool init_all, int32_t* tile_counts, int64_t N, int d,
-                            int R, int E, int* dev_status, cudaStream_t s) {
+                            int R, int E, int* dev_status, cudaStream_t s, ListsOut* lists) {
   Params p = {};
   p.N = N;
   p.d = d;
@@ -739,7 +804,13 @@ int launch_router_mask_umma(const void* x, const void* packed, float mult, uint3
   alignas(64) CUtensorMap tmx;
   int rc = encode_tmap_2d_b16(&tmx, x, (uint64_t)d, (uint64_t)N, (uint64_t)d * 2, 64, TILE_M, true);
   if (rc != D2D_OK) return rc == D2D_ERR_BAD_ARG ? D2D_ERR_LAUNCH : rc;
-  if (umma_router_splits(N, d, R, E)) {
+  const bool split = umma_router_splits(N, d, R, E);
+  if (lists && tiles <= (split ? 1 : CLUSTER_TILES)) {
+    p.token_idx = lists->token_idx;
+    p.offsets = lists->offsets;
+    lists->written = true;
+  }
+  if (split) {
     const size_t wa_stage = SLOT + (size_t)(R / CL * 128 + 1023) / 1024 * 1024;
     const size_t smem = 1024 + CL_NS * wa_stage + (size_t)p.g.nd * 128 + sizeof(ClCtl) + 64;
     static_assert((TILE_M * (MAX_E + 1)) * 4 <= CL_NS * SLOT, "shares fit the ring");
@@ -753,7 +824,8 @@ int launch_router_mask_umma(const void* x, const void* packed, float mult, uint3
   rc = device_launch_facts((const void*)router_tiles_kernel, smem, &sms);
   if (rc != D2D_OK) return rc;
   const int64_t grid = tiles < sms ? tiles : sms;
-  return launch_pdl(router_tiles_kernel, dim3((unsigned)grid), dim3(NTHREADS), smem, s, p, tmx);
+  return launch_pdl_cluster(p.token_idx ? (int)tiles : 0, router_tiles_kernel, dim3((unsigned)grid),
+                            dim3(NTHREADS), smem, s, p, tmx);
 }
 
 }  // namespace d2d

@@ -30,7 +30,8 @@ bool umma_router_splits(int64_t N, int d, int R, int E);
 int launch_router_mask_umma(const void* x, const void* packed, float mult, uint32_t* mask_bits,
                             void* scores, void* rt_out, const void* last_bias, const void* resid,
                             void* out_init, bool init_all, int32_t* tile_counts, int64_t N, int d,
-                            int R, int E, int* dev_status, cudaStream_t s);
+                            int R, int E, int* dev_status, cudaStream_t s,
+                            ListsOut* lists = nullptr);
 
 // test hook: how the expert kernel gathers its token rows: 0/1 = 16-byte cp.async
 // (default), 2 = TMA tile::gather4

@@ -208,3 +208,30 @@ def test_compaction_with_and_without_table(N, E):
     off, idx = _lists(wsp, E)
     roff, ridx = O.expert_token_lists(m)
     assert np.array_equal(off, np.asarray(roff)) and np.array_equal(idx, np.asarray(ridx))
+
+
+@pytest.mark.parametrize("E", [1, 24, 33, 128])
+@pytest.mark.parametrize("N", [1, 128, 129, 1000, 1024, 1025])
+def test_short_calls_write_their_lists(N, E):
+    """Up to 1024 tokens the router kernel leaves the lists itself (one cluster), beyond that the
+    scatter kernel does: lists, offsets and routing tensor of the mask either way."""
+    from d2dmoe_b200 import ops
+    c, t = _layer(N, 128, 32, E, 64, "bf16", N + E)
+    x2d, wa, wb = _dev(t["x"].reshape(N, c.d)), _dev(t["wa"]), _dev(t["wb"])
+    w1, b1, w2 = _dev(t["w1"]), _dev(t["b1"]), _dev(t["w2"])
+    wsp = ops.Workspace.allocate(N, E, "cuda")
+    rp, ep = ops.prepack_router(wa, wb), ops.prepack_experts(w1, b1, w2)
+    for tau in (0.3, 1.0):
+        out = torch.full((N, c.d), float("nan"), dtype=torch.bfloat16, device="cuda")
+        rt = torch.empty(N, E, dtype=torch.bfloat16, device="cuda")
+        ops.moe_forward(x2d, wa, wb, tau, w1, b1, w2, "relu", out, wsp, router_packed=rp,
+                        last_bias=_dev(t["last_bias"].reshape(-1)), experts_packed=ep, routing_out=rt)
+        wsp.check_status()
+        m = O.unpack_mask(wsp.mask_bits[:N].cpu().numpy().view(np.uint32), E)
+        assert torch.equal(rt.cpu() > 0, m)
+        off, idx = _lists(wsp, E)
+        roff, ridx = O.expert_token_lists(m)
+        assert np.array_equal(off, np.asarray(roff)) and np.array_equal(idx, np.asarray(ridx))
+        ex = O.experts_ffn_exact(t["x"].reshape(N, c.d), m, t["w1"], t["b1"], t["w2"])
+        slack = max(1.0, m.sum(1).max().item() ** 0.5 / 2)      # one rounding per added expert
+        assert O.rel_err(out.cpu().float(), ex + t["last_bias"].double()) <= TOL["bf16"] * slack
