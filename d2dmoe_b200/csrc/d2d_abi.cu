@@ -356,7 +356,7 @@ int d2d_moe_forward(const void* x, const void* wa, const void* wb, const void* r
 int d2d_last_forward_launches(void) { return g_last_forward_launches; }
 
 int d2d_debug_select_experts_kernel(int which) {
-  umma_debug_select_experts_kernel(which);
+  (void)which;
   return D2D_OK;
 }
 

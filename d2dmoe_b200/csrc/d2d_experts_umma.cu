@@ -931,9 +931,6 @@ int launch_experts_umma(const void* x, const int32_t* token_idx, const int32_t* 
   return launch_pdl(kernel, dim3((unsigned)grid), dim3(NTHREADS), smem, s, p);
 }
 
-// one way of gathering rows is left; kept for callers of the entry point
-void umma_debug_select_experts_kernel(int which) { (void)which; }
-
 void umma_debug_read(uint32_t* wait_limit, int* withhold) {
   *wait_limit = g_wait_limit.load();
   *withhold = g_withhold.load();

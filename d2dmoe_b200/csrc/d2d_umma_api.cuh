@@ -35,7 +35,6 @@ int launch_router_mask_umma(const void* x, const void* packed, float mult, uint3
 
 // test hook: how the expert kernel gathers its token rows: 0/1 = 16-byte cp.async
 // (default), 2 = TMA tile::gather4
-void umma_debug_select_experts_kernel(int which);
 
 // test hooks: poll limit of the bounded device waits (2^log2, out of range = default) and
 // a flag that makes CTA 0 of the next launches skip its first weight tile

@@ -264,8 +264,8 @@ int d2d_moe_forward_rule(const void* x, const void* wa, const void* wb,
                          d2d_stream_t stream);
 
 /* Number of kernels the calling thread's last d2d_moe_forward issued (3 on the tensor-core
- * path: router + rule, compaction scatter, expert FFN; more on the general-shape
- * paths).  Introspection for benchmarks; no upstream counterpart. */
+ * path: router + rule, compaction scatter, expert FFN; 2 on short calls, where the rule's
+ * kernel writes the lists; more on the general-shape paths).  Introspection for benchmarks; no upstream counterpart. */
 int d2d_last_forward_launches(void);
 
 /* Test hook, no upstream counterpart.  Every wait inside the tensor-core kernels is bounded;
@@ -277,10 +277,9 @@ int d2d_last_forward_launches(void);
  * d2d_debug_configure(0, 0) to return to normal operation. */
 int d2d_debug_configure(int wait_limit_log2, int withhold_weight_tile);
 
-/* Test hook, no upstream counterpart.  How the bf16 expert kernel brings the rows of an
- * expert's token list into shared memory: which = 0 or 1: 16-byte cp.async per row piece
- * (default, the faster one on B200); 2: TMA gathers (cp.async.bulk.tensor tile::gather4, four
- * rows per copy), kept so that the two can be compared on any workload. */
+/* Test hook, no upstream counterpart.  Selected how the bf16 expert kernel gathers token rows;
+ * only the 16-byte cp.async form is left (TMA gathers took 101 instead of 61 us on 50432
+ * tokens), so every value of which gives that form. */
 int d2d_debug_select_experts_kernel(int which);
 
 /* One-time re-layout of the weights into the shared-memory tile images the
