@@ -239,6 +239,7 @@ int d2d_moe_forward_rule(const void* x, const void* wa, const void* wb,
                            aligned(last_bias_opt, 16) && aligned(router_packed_opt, 1024);
   // where the tensor-core expert kernel follows, the rows of tokens with one expert are left to it
   DirectRows dr;
+  dr.kept = rule == D2D_RULE_TOPK ? k : rule == D2D_RULE_ALL ? E : rule == D2D_RULE_DYNK ? 6 : 0;
   bool may_store = !pre && !add_residual && umma_experts && aligned(last_bias_opt, 16);
   auto leave_rows = [&]() {
     dr.mask_bits = mask_bits;

@@ -13,6 +13,7 @@ int launch_prepack_experts(const void* w1, const void* b1, const void* w_up, con
 struct DirectRows {
   const uint32_t* mask_bits = nullptr;   // null: every row is added to
   const void* last_bias = nullptr;
+  int kept = 0;                          // experts a token keeps, where the rule fixes it
 };
 int launch_experts_umma(const void* x, const int32_t* token_idx, const int32_t* offsets,
                         const void* packed, void* out, int64_t N, int d, int E, int H, bool glu,

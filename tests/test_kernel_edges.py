@@ -85,6 +85,42 @@ def test_tensor_core_experts(N, d, H, E, act, glu, kind):
             assert O.rel_err(norms.cpu().float(), torch.where(m.t(), ref, 0.0)) <= TOL["bf16"]
 
 
+SHORT = [  # N, d, H, E, activation, gated: around 32 rows of a list, every cluster form, several rounds
+    (1, 128, 32, 3, "relu", False), (31, 256, 64, 24, "gelu", False), (33, 768, 96, 6, "tanh", False),
+    (64, 384, 128, 5, "leaky_relu", False), (65, 2048, 128, 20, "relu", False),
+    (32, 384, 96, 3, "gelu_tanh", True), (33, 640, 32, 9, "gelu", True), (40, 256, 64, 5, "relu", True),
+    (257, 2048, 128, 128, "gelu", True), (512, 2048, 128, 128, "gelu", True),
+]
+
+
+@pytest.mark.parametrize("kind", ["one_expert", "first_token", "few", "random"])
+@pytest.mark.parametrize("N,d,H,E,act,glu", SHORT)
+def test_short_call_experts(N, d, H, E, act, glu, kind):
+    from d2dmoe_b200 import ops
+    c, t = _layer(N, d, H, E, 128, "bf16", N + d, act, glu)
+    g = _gen(N)
+    m = torch.rand(N, E, generator=g) < 2.0 / E if kind == "few" else _mask(kind, N, E, g)
+    if kind == "random" and E > 64:           # lists of up to about 90 rows, the oracle in bounds
+        m &= torch.rand(1, E, generator=g) < 0.2
+    wsp = ops.Workspace.allocate(N, E, "cuda")
+    wsp.mask_bits[:N].copy_(torch.from_numpy(O.pack_mask(m).view(np.int32)).cuda())
+    ops.compact(wsp, N, E)
+    w1, b1, w2, wu = (_dev(t.get(k)) for k in ("w1", "b1", "w2", "w_up"))
+    if glu:
+        b1 = None
+    packed = ops.prepack_experts(w1, b1, w2, wu)
+    x2d = _dev(t["x"].reshape(N, d))
+    out = torch.full((N, d), float("nan"), dtype=torch.bfloat16, device="cuda")
+    ex = O.experts_ffn_exact(t["x"].reshape(N, d), m, t["w1"], None if glu else t["b1"], t["w2"], act,
+                             t.get("w_up") if glu else None)
+    ops.experts_ffn(x2d, wsp, w1, b1, w2, act, out, w_up=wu, packed=packed)
+    wsp.check_status()
+    o = out.cpu().float()
+    assert torch.isfinite(o).all()
+    # k bf16 adds per element, each rounding at the running magnitude
+    assert O.rel_err(o, ex) <= TOL["bf16"] * max(1.0, m.sum(1).max().item() ** 0.5 / 2)
+
+
 @pytest.mark.parametrize("E", [8, 24, 128])
 @pytest.mark.parametrize("N", [1, 31, 33, 128, 129, 700, 2048])
 def test_large_router(N, E):
