@@ -263,6 +263,15 @@ int d2d_moe_forward_rule(const void* x, const void* wa, const void* wb,
     }
     nl += 1;
     lists_ready = rt_done = true;
+  } else if (ranked && !scores && umma_router && umma_router_ranks(N, d, R, E)) {
+    // router and rule in one launch; every row gets its initial value, before the rule is known:
+    // hardly a token keeps just one expert
+    rc = launch_router_mask_umma(x, router_packed_opt, thresh_mult, mask_bits, scores_scratch,
+                                 routing_tensor_opt, last_bias_opt, add_residual ? x : nullptr,
+                                 out_init, true, (int32_t*)ws, N, d, R, E, dev_status, s, &lists,
+                                 rule, k, tau);
+    counts_ready = rt_done = true;
+    nl += 1;
   } else if (ranked && !scores) {
     // scores of the fused router for the rule below (its own mask is overwritten there); it also
     // writes every initial row, at no cost of its own: hardly a token keeps just one expert

@@ -9,6 +9,7 @@
 // accumulators are rounded to T once after each of the two products, and the
 // threshold is rounded to T before the comparison.
 #include "d2d_cluster_compact.cuh"
+#include "d2d_ranked.cuh"
 #include "d2d_common.cuh"
 
 namespace d2d {
@@ -233,9 +234,6 @@ mask_from_scores_kernel(const T* __restrict__ scores, float mult, uint32_t* __re
 //           and every further one while the cumulative share before it (fp32 running sum
 //           in that order, rounded to T per element, as torch.cumsum does) is < T(tau).
 // `before(a, ia, b, ib)`: a precedes b in the descending order used by both rules.
-template <typename T> struct Acc { typedef float type; };
-template <> struct Acc<float> { typedef double type; };
-
 __device__ __forceinline__ bool before(float a, int ia, float b, int ib) {
   const bool an = a != a, bn = b != b;
   if (an || bn) return an && (!bn || ia < ib);
@@ -491,61 +489,7 @@ gate_scores_fused_rows_kernel(const T* __restrict__ scores, float mult, int k, f
       for (int e = 0; e < EMAX; ++e)
         if (e < E && DT<T>::to_f(sv[e]) >= thr) word[e >> 5] |= 1u << (e & 31);
     } else {
-      float v[EMAX];
-#pragma unroll
-      for (int e = 0; e < EMAX; ++e) v[e] = DT<T>::to_f(sv[e]);
-      bool negative = false;
-      if (RULE == D2D_RULE_DYNK) {
-        float s[32];                     // the balanced sum a warp's butterfly makes of 32 lanes
-#pragma unroll
-        for (int l = 0; l < 32; ++l) {
-          s[l] = 0.f;
-#pragma unroll
-          for (int e = l; e < EMAX; e += 32)
-            if (e < E) s[l] += v[e];
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-          for (int l = 0; l < o; ++l) s[l] += s[l + o];
-        const float tot = DT<T>::round(s[0]);
-#pragma unroll
-        for (int e = 0; e < EMAX; ++e) {
-          v[e] = DT<T>::round(v[e] / tot);
-          negative |= e < E && v[e] < 0.f;
-        }
-      }
-      const float tau_t = DT<T>::round(tau);
-      const int most = RULE == D2D_RULE_TOPK ? k : E;
-      uint32_t taken[2] = {0u, 0u};
-      typename Acc<T>::type acc = 0;
-      bool more = true;                  // the expert of the next rank is kept
-      for (int r = 0; r < most; ++r) {
-        float m = 0.f;
-        int best = -1;
-#pragma unroll
-        for (int e = 0; e < EMAX; ++e) {
-          const bool free = e < E && !((taken[e >> 5] >> (e & 31)) & 1u);
-          if (free && (best < 0 || v[e] > m || (v[e] != v[e] && m == m))) {
-            m = v[e];
-            best = e;
-          }
-        }
-        const uint32_t b0 = best < 32 ? 1u << (best & 31) : 0u;
-        const uint32_t b1 = best >= 32 ? 1u << (best & 31) : 0u;
-        taken[0] |= b0;
-        taken[1] |= b1;
-        if (more) {
-          word[0] |= b0;
-          word[1] |= b1;
-        }
-        if (RULE == D2D_RULE_DYNK) {
-          acc += m;
-          more = DT<T>::round((float)acc) < tau_t;
-          // without negative shares the running sum only grows
-          if (!__any_sync(0xffffffffu, more || negative)) break;
-        }
-      }
+      ranked_words<T, EMAX, RULE>(sv, E, k, tau, word);
     }
     const bool live = t < N;
     if (!live) word[0] = word[1] = 0u;

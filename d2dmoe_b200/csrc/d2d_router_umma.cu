@@ -22,6 +22,7 @@
 #include <cooperative_groups.h>
 
 #include "d2d_cluster_compact.cuh"
+#include "d2d_ranked.cuh"
 #include "d2d_tmap.cuh"
 #include "d2d_umma_api.cuh"
 #include "d2d_umma_ptx.cuh"
@@ -69,6 +70,8 @@ struct Params {
   const uint8_t* packed;
   Geo g;
   float mult;
+  int k;                    // ranked rules
+  float tau;
   uint32_t* mask_bits;
   bf16* scores;             // optional [N, E]
   bf16* rt_out;             // optional: 0/1 routing tensor [N, E]
@@ -238,7 +241,7 @@ __device__ __forceinline__ void store_row(bf16* dst, const uint32_t* s, int E) {
 
 // warps 4-7, thread = tile row: the row's scores stay in registers as packed bf16 pairs
 // (NB blocks of 16 experts), so tensor memory is read once and handed back at once
-template <int NB>
+template <int NB, int RULE>
 __device__ void role_gate(const Params& p, Ctl* c, uint32_t tmem, int et) {
   volatile int* af = &c->abort_flag;
   const int tiles = (int)((p.N + TILE_M - 1) / TILE_M);
@@ -275,19 +278,27 @@ __device__ void role_gate(const Params& p, Ctl* c, uint32_t tmem, int et) {
     const float m = nanmax(__low2float(m2), __high2float(m2));
     const __nv_bfloat162 thr = __float2bfloat162_rn(__fmul_rn(m, p.mult));
     if (p.scores && live) store_row<NB>(p.scores + trow * E, s, E);
-    uint32_t word[NW];
+    uint32_t word[RULE != 0 ? 2 : NW];
 #pragma unroll
-    for (int j = 0; j < NW; ++j) word[j] = 0u;
+    for (int j = 0; j < (RULE != 0 ? 2 : NW); ++j) word[j] = 0u;
+    if (RULE != 0) {
+      ranked_words<bf16, NB * 16, RULE>(reinterpret_cast<const bf16*>(s), E, p.k, p.tau, word);
 #pragma unroll
-    for (int q = 0; q < NB * 8; ++q) {
-      const uint32_t k = __hge2_mask(*reinterpret_cast<const __nv_bfloat162*>(&s[q]), thr);
-      word[q >> 4] |= k & (0x00010001u << (q & 15));
-      s[q] = k & 0x3f803f80u;                         // the routing entries: bf16 1.0 or 0
+      for (int q = 0; q < NB * 8; ++q)
+        s[q] = ((word[0] >> (2 * q)) & 1u ? 0x3f80u : 0u) |
+               ((word[0] >> (2 * q + 1)) & 1u ? 0x3f800000u : 0u);
+    } else {
+#pragma unroll
+      for (int q = 0; q < NB * 8; ++q) {
+        const uint32_t k = __hge2_mask(*reinterpret_cast<const __nv_bfloat162*>(&s[q]), thr);
+        word[q >> 4] |= k & (0x00010001u << (q & 15));
+        s[q] = k & 0x3f803f80u;                       // the routing entries: bf16 1.0 or 0
+      }
     }
     int kept = 0;
 #pragma unroll
     for (int j = 0; j < NW; ++j) {
-      word[j] = interleave16(word[j]);
+      if (RULE == 0) word[j] = interleave16(word[j]);
       if (32 * j + 32 > E) word[j] &= (1u << (E - 32 * j)) - 1u;      // E > 32 j
       if (!live) word[j] = 0u;
       kept += __popc(word[j]);
@@ -382,6 +393,8 @@ __device__ void role_init(const Params& p, Ctl* c, int w, int lane) {
   }
 }
 
+// RULE: 0, or D2D_RULE_TOPK / D2D_RULE_DYNK (E <= 32)
+template <int RULE>
 __global__ void __launch_bounds__(NTHREADS, 1)
 router_tiles_kernel(const Params p, const __grid_constant__ CUtensorMap tmx) {
   extern __shared__ uint8_t smem_raw[];
@@ -426,15 +439,20 @@ router_tiles_kernel(const Params p, const __grid_constant__ CUtensorMap tmx) {
   if (warp < 4) {
     role_hidden(p, c, tmem, tid);
   } else if (warp < 8) {
-    switch (p.g.nd >> 4) {
-      case 1: role_gate<1>(p, c, tmem, tid - 128); break;
-      case 2: role_gate<2>(p, c, tmem, tid - 128); break;
-      case 3: role_gate<3>(p, c, tmem, tid - 128); break;
-      case 4: role_gate<4>(p, c, tmem, tid - 128); break;
-      case 5: role_gate<5>(p, c, tmem, tid - 128); break;
-      case 6: role_gate<6>(p, c, tmem, tid - 128); break;
-      case 7: role_gate<7>(p, c, tmem, tid - 128); break;
-      default: role_gate<8>(p, c, tmem, tid - 128); break;
+    if (RULE != 0) {
+      if (p.g.nd == 16) role_gate<1, RULE>(p, c, tmem, tid - 128);
+      else role_gate<2, RULE>(p, c, tmem, tid - 128);
+    } else {
+      switch (p.g.nd >> 4) {
+        case 1: role_gate<1, 0>(p, c, tmem, tid - 128); break;
+        case 2: role_gate<2, 0>(p, c, tmem, tid - 128); break;
+        case 3: role_gate<3, 0>(p, c, tmem, tid - 128); break;
+        case 4: role_gate<4, 0>(p, c, tmem, tid - 128); break;
+        case 5: role_gate<5, 0>(p, c, tmem, tid - 128); break;
+        case 6: role_gate<6, 0>(p, c, tmem, tid - 128); break;
+        case 7: role_gate<7, 0>(p, c, tmem, tid - 128); break;
+        default: role_gate<8, 0>(p, c, tmem, tid - 128); break;
+      }
     }
   } else if (warp == WARP_MMA1) {
     if (elect_one()) role_mma1(p, c, base, stage_bytes, tmem);
@@ -776,10 +794,19 @@ bool umma_router_splits(int64_t N, int d, int R, int E) {
          compact_counts_itself(N, E);
 }
 
+// The ranked rules without a launch of their own (before -> now, per layer:
+// 12608 tokens x 24 experts, topk 2: 42.9 -> 40.4 us; 25216 tokens, topk 4: 90.3 -> 83.5; 197
+// tokens, topk 1: 22.0 -> 20.3).  Beyond 32 scores a thread's registers would not hold them
+// beside their shares.
+bool umma_router_ranks(int64_t N, int d, int R, int E) {
+  return E <= 32 && !umma_router_splits(N, d, R, E);
+}
+
 int launch_router_mask_umma(const void* x, const void* packed, float mult, uint32_t* mask_bits,
                             void* scores, void* rt_out, const void* last_bias, const void* resid,
                             void* out_init, bool init_all, int32_t* tile_counts, int64_t N, int d,
-                            int R, int E, int* dev_status, cudaStream_t s, ListsOut* lists) {
+                            int R, int E, int* dev_status, cudaStream_t s, ListsOut* lists,
+                            int rule, int k, float tau) {
   Params p = {};
   p.N = N;
   p.d = d;
@@ -788,6 +815,8 @@ int launch_router_mask_umma(const void* x, const void* packed, float mult, uint3
   p.packed = (const uint8_t*)packed;
   p.g = router_geo(d, R, E);
   p.mult = mult;
+  p.k = k;
+  p.tau = tau;
   p.mask_bits = mask_bits;
   p.scores = (bf16*)scores;
   p.rt_out = (bf16*)rt_out;
@@ -821,10 +850,13 @@ int launch_router_mask_umma(const void* x, const void* packed, float mult, uint3
   }
   const size_t smem = smem_bytes(p.g);
   int sms = 0;
-  rc = device_launch_facts((const void*)router_tiles_kernel, smem, &sms);
+  auto kernel = rule == D2D_RULE_TOPK   ? router_tiles_kernel<D2D_RULE_TOPK>
+                : rule == D2D_RULE_DYNK ? router_tiles_kernel<D2D_RULE_DYNK>
+                                        : router_tiles_kernel<0>;
+  rc = device_launch_facts((const void*)kernel, smem, &sms);
   if (rc != D2D_OK) return rc;
   const int64_t grid = tiles < sms ? tiles : sms;
-  return launch_pdl_cluster(p.token_idx ? (int)tiles : 0, router_tiles_kernel, dim3((unsigned)grid),
+  return launch_pdl_cluster(p.token_idx ? (int)tiles : 0, kernel, dim3((unsigned)grid),
                             dim3(NTHREADS), smem, s, p, tmx);
 }
 

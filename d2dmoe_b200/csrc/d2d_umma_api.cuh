@@ -32,7 +32,10 @@ int launch_router_mask_umma(const void* x, const void* packed, float mult, uint3
                             void* scores, void* rt_out, const void* last_bias, const void* resid,
                             void* out_init, bool init_all, int32_t* tile_counts, int64_t N, int d,
                             int R, int E, int* dev_status, cudaStream_t s,
-                            ListsOut* lists = nullptr);
+                            ListsOut* lists = nullptr, int rule = 0, int k = 0, float tau = 0.f);
+// whether it applies the ranked rules (rule: D2D_RULE_TOPK with k, D2D_RULE_DYNK with tau) itself: a
+// token's scores are one thread's registers, which ranks up to 32 of them
+bool umma_router_ranks(int64_t N, int d, int R, int E);
 
 // test hook: how the expert kernel gathers its token rows: 0/1 = 16-byte cp.async
 // (default), 2 = TMA tile::gather4

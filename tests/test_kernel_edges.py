@@ -233,6 +233,12 @@ def test_every_mode_is_one_call(N, dtype, E):
         assert O.rel_err(out.reshape(N, c.d).cpu().float(), ex) <= TOL[dtype] * slack
 
 
+@pytest.mark.parametrize("N,E", [(33, 1), (129, 16), (1025, 17), (1025, 31), (1200, 32), (1100, 33)])
+def test_router_ranks_its_scores(N, E):
+    """Up to 32 experts the router applies topk / dynk itself; lists inside and outside the cluster."""
+    test_every_mode_is_one_call(N, "bf16", E)
+
+
 @pytest.mark.parametrize("N,E", [(8192, 24), (8193, 24), (4096, 33), (4097, 33), (255, 256), (2100, 128)])
 def test_compaction_with_and_without_table(N, E):
     from d2dmoe_b200 import ops
