@@ -15,11 +15,13 @@
 
 #include <ATen/ATen.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAException.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/utils/object_ptr.h>
 
 #include <memory>
 #include <vector>
@@ -41,6 +43,9 @@ struct Link {
 struct Plan {
   std::vector<Link> links;
   at::Tensor hold[2];                  // packed router / experts images
+  cudaEvent_t packed = nullptr;        // behind the kernels that wrote them, on `made_on`
+  cudaStream_t made_on = nullptr;
+  std::vector<cudaStream_t> users;     // other streams that have waited for it
   const void *wa = nullptr, *wb = nullptr, *rp = nullptr;
   const void *w1 = nullptr, *b1 = nullptr, *wup = nullptr, *w2 = nullptr, *ep = nullptr;
   const void* last_bias = nullptr;
@@ -48,6 +53,7 @@ struct Plan {
   at::ScalarType dtype = at::kFloat;
   c10::Device device = c10::Device(c10::kCUDA, 0);
   ~Plan() {
+    if (packed) cudaEventDestroy(packed);
     for (Link& l : links) {
       Py_XDECREF(l.dict);
       Py_XDECREF(l.key);
@@ -79,6 +85,26 @@ bool still_valid(const Plan& p, PyObject* const* roots) {
     }
   }
   return !PyErr_Occurred();
+}
+
+bool capturing(cudaStream_t s) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  C10_CUDA_CHECK(cudaStreamIsCapturing(s, &st));
+  return st != cudaStreamCaptureStatusNone;
+}
+
+// Before `s` reads the packed images: it comes behind the kernels that wrote them, and the allocator
+// learns that it uses them.  (A capture cannot depend on work outside it; it starts behind that.)
+void use_on(Plan& p, c10::cuda::CUDAStream s) {
+  if (!p.packed || s.stream() == p.made_on) return;
+  for (cudaStream_t u : p.users)
+    if (u == s.stream()) return;
+  if (capturing(s.stream())) return;
+  C10_CUDA_CHECK(cudaStreamWaitEvent(s.stream(), p.packed, 0));
+  for (const at::Tensor& t : p.hold)
+    if (t.defined()) c10::cuda::CUDACachingAllocator::recordStream(t.storage().data_ptr(), s);
+  if (p.users.size() >= 16) p.users.clear();
+  p.users.push_back(s.stream());
 }
 
 // make_plan(links, (wa, wb, router_packed), (w1, b1, w_up, w2, experts_packed), last_bias, act)
@@ -152,11 +178,20 @@ PyObject* make_plan(PyObject*, PyObject* const* a, Py_ssize_t n) {
   p->last_bias = ptr_of(a[3]);
   p->act = PyLong_AsLong(a[4]);
   if (PyErr_Occurred()) return nullptr;
+  if (p->hold[0].defined() || p->hold[1].defined()) {
+    c10::cuda::CUDAGuard guard(p->device);
+    const cudaStream_t s = c10::cuda::getCurrentCUDAStream(p->device.index()).stream();
+    if (!capturing(s)) {
+      C10_CUDA_CHECK(cudaEventCreateWithFlags(&p->packed, cudaEventDisableTiming));
+      C10_CUDA_CHECK(cudaEventRecord(p->packed, s));
+      p->made_on = s;
+    }
+  }
   return PyCapsule_New(p.release(), kPlan, plan_free);
   END_HANDLE_TH_ERRORS
 }
 
-// buffers of one call: ops.Workspace of (tokens, experts, device), from the module's cache
+// buffers of one call: ops.Workspace of (tokens, experts, device), from a cache of the module's
 struct Buffers {
   void *mask, *idx, *off, *ws, *status;
   size_t ws_bytes;
@@ -164,8 +199,10 @@ struct Buffers {
 
 PyObject* s_get;      // "raw"
 
-bool buffers_of(PyObject* cache, const Plan& p, int64_t N, Buffers* b) {
-  // the cache is a dictionary (tokens, experts, device index) -> Workspace with a miss handler
+// keep: a list that holds on to it, or null
+bool buffers_of(PyObject* cache, const Plan& p, int64_t N, Buffers* b, PyObject* keep = nullptr) {
+  // the cache is a dictionary (tokens, experts, device index) -> Workspace with a miss handler, which
+  // allocates on the current stream
   PyObject* key = Py_BuildValue("(LLi)", (long long)N, (long long)p.E, (int)p.device.index());
   if (!key) return false;
   PyObject* w = PyDict_GetItemWithError(cache, key);       // borrowed
@@ -173,7 +210,9 @@ bool buffers_of(PyObject* cache, const Plan& p, int64_t N, Buffers* b) {
   if (!w && !PyErr_Occurred()) w = made = PyObject_GetItem(cache, key);   // __missing__ allocates
   Py_DECREF(key);
   if (!w) return false;
-  PyObject* raw = PyObject_GetAttr(w, s_get);               // bytes: five addresses and a size
+  PyObject* raw = keep && PyList_Append(keep, w) != 0
+                      ? nullptr
+                      : PyObject_GetAttr(w, s_get);         // bytes: five addresses and a size
   Py_XDECREF(made);                                         // the cache keeps it
   if (!raw) return false;
   const bool ok = PyBytes_Check(raw) && PyBytes_GET_SIZE(raw) == 48;
@@ -229,9 +268,11 @@ PyObject* run_layer(PyObject*, PyObject* const* a, Py_ssize_t n) {
     Py_RETURN_NONE;
   }
   c10::cuda::CUDAGuard guard(p->device);
+  const auto cur = c10::cuda::getCurrentCUDAStream(p->device.index());
+  const auto stream = (d2d_stream_t)cur.stream();
   Buffers b;
   if (!buffers_of(a[3], *p, N, &b)) return nullptr;
-  const auto stream = (d2d_stream_t)c10::cuda::getCurrentCUDAStream(p->device.index()).stream();
+  use_on(*p, cur);
   const int dt = p->dtype == at::kBFloat16 ? D2D_BF16 : D2D_F32;
   const auto opts = x.options();
   at::Tensor out = at::detail::empty_cuda(x.sizes(), opts);
@@ -364,6 +405,20 @@ PyObject* run_host(PyObject*, PyObject* const* a, Py_ssize_t n) {
   }
   const int dt = p->dtype == at::kBFloat16 ? D2D_BF16 : D2D_F32;
   const int64_t B = xh->size(0), per = xh->numel() / B;      // values of one batch entry
+  // `workspaces` is the pipeline's own: allocated and used on the stream of the kernels alone, whatever
+  // the caller's stream is doing, so that one that leaves the cache is reused in stream order
+  const auto run = c10::cuda::getStreamFromExternal(st[1], p->device.index());
+  std::vector<Buffers> bufs((size_t)slices);
+  THPObjectPtr keep(PyList_New(0));
+  if (!keep) return nullptr;
+  {
+    c10::cuda::CUDAStreamGuard on_run(run);
+    for (int64_t i = 0; i < slices; ++i)
+      if (!buffers_of(a[3], *p, (B * (i + 1) / slices - B * i / slices) * per / p->d, &bufs[i],
+                      keep))
+        return nullptr;
+  }
+  use_on(*p, run);
   const size_t es = xh->element_size();
   const char* src = static_cast<const char*>(xh->data_ptr());
   char* dst = static_cast<char*>(oh->data_ptr());
@@ -372,8 +427,7 @@ PyObject* run_host(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const int64_t lo = B * i / slices, hi = B * (i + 1) / slices, N = (hi - lo) * per / p->d;
     const int b = (int)(h->n % kIn), o = (int)(h->n % kOut);
     const size_t bytes = (size_t)((hi - lo) * per) * es, at = (size_t)(lo * per) * es;
-    Buffers buf;
-    if (!buffers_of(a[3], *p, N, &buf)) return nullptr;
+    const Buffers& buf = bufs[i];
     C10_CUDA_CHECK(cudaStreamWaitEvent(st[0], h->in_free[b], 0));
     C10_CUDA_CHECK(cudaMemcpyAsync(stage[b], src + at, bytes, cudaMemcpyHostToDevice, st[0]));
     C10_CUDA_CHECK(cudaEventRecord(h->in_full[b], st[0]));

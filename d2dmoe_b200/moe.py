@@ -84,11 +84,13 @@ class _WorkspaceCache(dict):
 
 
 class _HostBuffers:
-    """Staging buffers and events of ``forward_host``; copies of a module start without them."""
+    """Staging buffers, events and workspaces of ``forward_host``; copies of a module start without
+    them."""
 
-    __slots__ = ("shape", "dtype", "device", "bufs", "pipe", "streams")
+    __slots__ = ("shape", "dtype", "device", "bufs", "pipe", "streams", "wsp")
 
     def __init__(self):
+        self.wsp = _WorkspaceCache()
         self.shape = self.dtype = self.device = self.bufs = self.pipe = self.streams = None
 
     def __deepcopy__(self, memo):
@@ -119,11 +121,21 @@ class _PackedCache:
     A change is seen through the parameter's storage address, shape, dtype and version
     counter, i.e. ``load_state_dict``, ``.to()``, ``copy_`` and other in-place tensor ops.
     Writes that bypass the version counter (``p.data.copy_(...)``, raw pointer writes) are
-    not seen: call ``invalidate()`` (``module.invalidate_packed()``) after those."""
+    not seen: call ``invalidate()`` (``module.invalidate_packed()``) after those.
+
+    A stream that did not write the image waits for the one that did."""
+
+    _made = None                  # (stream that wrote the image, event behind it)
 
     def __init__(self):
         self._key = None
         self._buf = None
+
+    def __deepcopy__(self, memo):
+        return _PackedCache()
+
+    def __reduce__(self):
+        return _PackedCache, ()
 
     def invalidate(self):
         self._key = None
@@ -135,6 +147,15 @@ class _PackedCache:
         if key != self._key:
             self._buf = make()
             self._key = key
+            self._made = None
+            if self._buf is not None and not torch.cuda.is_current_stream_capturing():
+                s = torch.cuda.current_stream(self._buf.device)
+                self._made = s, s.record_event()
+        elif self._made is not None:
+            s = torch.cuda.current_stream(self._buf.device)
+            if s != self._made[0] and not torch.cuda.is_current_stream_capturing():
+                s.wait_event(self._made[1])
+                self._buf.record_stream(s)
         return self._buf
 
 
@@ -776,14 +797,16 @@ class MoeficationMoE(MoELayer):
         for _ in range(2):
             h = self._plan.handle
             if h is not None:
-                r = host.run_host(h, self._modules, self._parameters, self._wsp, hp.pipe, x_host,
+                r = host.run_host(h, self._modules, self._parameters, hp.wsp, hp.pipe, x_host,
                                   out_host, hp.bufs, hp.streams, chunks, rule, 0, self.tau,
                                   self.add_residual_connection, sync)
                 if r is True:
                     return True
                 if r is not None:
                     raise D2DError(r, "d2d_moe_forward")
-            with torch.no_grad():
+            # packed on the stream that will read it, behind what has been done to the weights
+            st[1].wait_stream(torch.cuda.current_stream(dev))
+            with torch.no_grad(), torch.cuda.stream(st[1]):
                 self._plan.handle = self._make_plan()
             if self._plan.handle is None:
                 return False

@@ -1,0 +1,74 @@
+"""Calls of the layer around its kept facts: what a plan, a workspace or a staging buffer is made
+from may change between two calls, on another stream or in another thread."""
+import copy
+
+import pytest
+import torch
+
+from helpers import C, O, TOL
+
+pytestmark = pytest.mark.gpu
+
+
+def _moe(c, t, experts=None, router=None):
+    import d2dmoe_b200 as D
+    moe = D.MoeficationMoE(c.name, c.d, c.E, True, c.H, torch.nn.ReLU)
+    if experts is not None:
+        moe.experts = experts(c.d, c.E, 2, c.H, "without_last", torch.nn.ReLU)
+    moe.router = (router or D.MoeficationRouter)(c.d, c.E, width=c.R, depth=2, bias=False,
+                                                 activation="relu", output_activation="abs")
+    moe = moe.to(c.torch_dtype)
+    moe.load_state_dict({"experts.w1": t["w1"], "experts.b1": t["b1"], "experts.w2": t["w2"],
+                         "last_bias": t["last_bias"], "router.layers.0.weight": t["wa"],
+                         "router.layers.2.weight": t["wb"]})
+    moe = moe.cuda().eval()
+    moe.forward_mode, moe.tau = "dynk_max", c.tau
+    return moe
+
+
+def _case(N=197, dtype="bf16", B=1, **kw):
+    c = C.LayerCase("calls", B, N, 128, 64, 8, R=64, tau=0.3, dtype=dtype, seed=N, **kw)
+    return c, C.make_tensors(c)
+
+
+def _same(moe, x, call="forward"):
+    """The call's result against a layer that has never been called before."""
+    fresh = copy.deepcopy(moe)
+    want, _ = fresh(x)
+    if call == "forward":
+        got, _ = moe(x)
+    elif call == "block":
+        norm = torch.nn.LayerNorm(x.size(-1)).to(x)
+        got, _ = moe.forward_block(x, norm)
+        want, _ = fresh.forward_block(x, norm)
+    else:
+        got = moe.forward_host(x.cpu().pin_memory()).cuda()
+    return O.rel_err(got.float().cpu(), want.float().cpu()) <= TOL["bf16"]
+
+
+def test_forward_host_beside_a_busy_stream():
+    """sync=False: packing, workspaces and kernels depend on nothing the caller's stream is doing.
+    A first call, new slice sizes (more than the cache keeps), changed weights, and forward() calls of
+    the same token counts in between."""
+    import d2dmoe_b200 as D
+    c, t = _case(40, B=24)
+    moe, plain, x = _moe(c, t), _moe(c, t), t["x"].pin_memory()
+    for change in (False, True):
+        if change:
+            with torch.no_grad():
+                moe.experts.w1.mul_(2), plain.experts.w1.mul_(2)
+        want = {b: plain(x[:b].cuda())[0].cpu() for b in range(2, 25)}
+        xd = {b: x[:b].cuda() for b in want}
+        torch.cuda.synchronize()
+        torch.cuda._sleep(100_000_000)
+        got, dev = {}, {}
+        for b in want:
+            got[b] = torch.empty_like(x[:b]).pin_memory()
+            moe.forward_host(x[:b], got[b], chunks=2, sync=False)
+            dev[b] = moe(xd[(b + 1) // 2])[0] if b > 3 else None
+        D.MoeficationMoE.host_synchronize()
+        torch.cuda.synchronize()
+        for b in want:
+            assert O.rel_err(got[b].float(), want[b].float()) <= TOL["bf16"], b
+            if b > 3:
+                assert O.rel_err(dev[b].float().cpu(), want[(b + 1) // 2].float()) <= TOL["bf16"], b
