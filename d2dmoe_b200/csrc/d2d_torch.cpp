@@ -6,10 +6,10 @@
 // calls (weight addresses, shapes, packed copies) are kept in a plan, and a call only checks that
 // the plan still describes the module, allocates the outputs and enters the C ABI.
 //
-// The plan never serves stale weights: each of its links names the dictionary slot a parameter or
-// sub-module sits in, and a call compares what is in the slot now (object, storage address, version
-// counter) with what the plan was made from.  A mismatch returns None and the caller makes a
-// new plan.
+// The plan never serves stale weights: each of its links names the dictionary slot a parameter, a
+// sub-module or a packed image sits in, and a call compares what is in the slot now (object, storage
+// address, version counter) with what the plan was made from.  A mismatch returns None and the caller
+// makes a new plan.  (Writes past the version counter are announced by emptying the image's slot.)
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 

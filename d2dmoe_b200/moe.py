@@ -519,13 +519,16 @@ class MoeficationMoE(MoELayer):
                 links += [(router.layers._modules, i),
                           (router.layers._modules[i]._parameters, "weight")]
             r = (wa, wb, router.packed())
+            links.append((router._packed.__dict__, "_buf"))      # invalidate_packed() empties the slot
         tensors = [t for t in (p["w1"], p["b1"], p["w_up"], p["w2"]) if t is not None]
         if self.bias:
             tensors.append(self.last_bias)
         if any(t.dtype != p["w1"].dtype or t.device != p["w1"].device or not t.is_contiguous()
                for t in tensors + list(r[:2] if r else ())):
             return None
-        return host.make_plan(links, r, (p["w1"], p["b1"], p["w_up"], p["w2"], ex.packed()),
+        packed = ex.packed()
+        links.append((ex._packed.__dict__, "_buf"))
+        return host.make_plan(links, r, (p["w1"], p["b1"], p["w_up"], p["w2"], packed),
                               self.last_bias if self.bias else None, ACT[p["act"]],
                               self._modules, self._parameters)
 

@@ -46,6 +46,19 @@ def _same(moe, x, call="forward"):
     return O.rel_err(got.float().cpu(), want.float().cpu()) <= TOL["bf16"]
 
 
+@pytest.mark.parametrize("call", ["forward", "block", "host"])
+@pytest.mark.parametrize("which", ["experts", "router"])
+def test_invalidate_packed_reaches_every_call(which, call):
+    """Writes through .data leave the version counter alone; invalidate_packed() announces them."""
+    c, t = _case()
+    moe, x = _moe(c, t), t["x"].cuda()
+    assert _same(moe, x, call)
+    p = moe.experts.w2 if which == "experts" else moe.router.layers[0].weight
+    p.data.copy_(torch.roll(p.detach(), 1, 0 if which == "experts" else 1) * 3.0)
+    getattr(moe, which).invalidate_packed()
+    assert _same(moe, x, call)
+
+
 def test_forward_host_beside_a_busy_stream():
     """sync=False: packing, workspaces and kernels depend on nothing the caller's stream is doing.
     A first call, new slice sizes (more than the cache keeps), changed weights, and forward() calls of
