@@ -108,16 +108,17 @@ void use_on(Plan& p, c10::cuda::CUDAStream s) {
 }
 
 // make_plan(links, (wa, wb, router_packed), (w1, b1, w_up, w2, experts_packed), last_bias, act)
-//   links: sequence of (holder, key); holder = a dict, or 0 / 1 for the module's own _modules /
-//   _parameters, which run_layer receives with every call (the plan does not refer to its module)
+//   links: sequence of (holder, key); holder = a dict, or 0 / 1 / 2 for the module's own _modules /
+//   _parameters / __dict__, which run_layer receives with every call (the plan does not refer to its
+//   module)
 PyObject* make_plan(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
-  if (n != 7) {
-    PyErr_SetString(PyExc_TypeError, "make_plan takes 7 arguments");
+  if (n != 8) {
+    PyErr_SetString(PyExc_TypeError, "make_plan takes 8 arguments");
     return nullptr;
   }
   auto p = std::make_unique<Plan>();
-  PyObject* const roots[2] = {a[5], a[6]};
+  PyObject* const roots[3] = {a[5], a[6], a[7]};
   PyObject* seq = PySequence_Fast(a[0], "links");
   if (!seq) return nullptr;
   for (Py_ssize_t i = 0; i < PySequence_Fast_GET_SIZE(seq); ++i) {
@@ -130,7 +131,8 @@ PyObject* make_plan(PyObject*, PyObject* const* a, Py_ssize_t n) {
     }
     Link l = {};
     if (PyLong_Check(holder)) {
-      l.root = PyLong_AsLong(holder) == 1 ? 1 : 0;
+      l.root = (int)PyLong_AsLong(holder);
+      TORCH_CHECK(l.root >= 0 && l.root < 3, "link holder");
     } else {
       Py_INCREF(holder);
       l.dict = holder;
@@ -227,20 +229,20 @@ bool buffers_of(PyObject* cache, const Plan& p, int64_t N, Buffers* b, PyObject*
   return ok;
 }
 
-// run_layer(plan, modules, parameters, workspaces, x, rule, k, tau, residual, scores, norm, capture)
+// run_layer(plan, modules, parameters, attributes, workspaces, x, rule, k, tau, residual, scores, norm, capture)
 //   -> (out, routing[, norms]) | status code (int) | None: the plan does not fit this call
 // rule: D2D_RULE_*; k / tau as that rule reads them (MAX: threshold 1 - tau).
 // scores: None or [.., E] of x's dtype.  norm: None or (kind, gamma, beta|None, eps, gamma_offset):
 // x + layer(norm(x)).  capture: None or (norm layer, ord), with D2D_RULE_ALL.
 PyObject* run_layer(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
-  if (n != 12) {
-    PyErr_SetString(PyExc_TypeError, "run_layer takes 12 arguments");
+  if (n != 13) {
+    PyErr_SetString(PyExc_TypeError, "run_layer takes 13 arguments");
     return nullptr;
   }
   Plan* p = static_cast<Plan*>(PyCapsule_GetPointer(a[0], kPlan));
   if (!p) return nullptr;
-  const at::Tensor* xp = tensor_of(a[4]);
+  const at::Tensor* xp = tensor_of(a[5]);
   if (!xp || !xp->is_cuda() || xp->scalar_type() != p->dtype || xp->device() != p->device ||
       xp->dim() < 1 || xp->size(-1) != p->d || xp->numel() == 0 || !still_valid(*p, a + 1)) {
     if (PyErr_Occurred()) return nullptr;
@@ -248,18 +250,18 @@ PyObject* run_layer(PyObject*, PyObject* const* a, Py_ssize_t n) {
   }
   const at::Tensor x = xp->contiguous();
   const int64_t N = x.numel() / p->d;
-  const int rule = (int)PyLong_AsLong(a[5]);
-  const int k = (int)PyLong_AsLong(a[6]);
+  const int rule = (int)PyLong_AsLong(a[6]);
+  const int k = (int)PyLong_AsLong(a[7]);
   const bool reads_tau = rule == D2D_RULE_MAX || rule == D2D_RULE_DYNK;
-  const double tau = reads_tau ? PyFloat_AsDouble(a[7]) : 0.0;
-  const int residual = PyObject_IsTrue(a[8]);
+  const double tau = reads_tau ? PyFloat_AsDouble(a[8]) : 0.0;
+  const int residual = PyObject_IsTrue(a[9]);
   if (PyErr_Occurred()) return nullptr;
   const float mult = (float)(1.0 - tau);
   const bool ranked = rule == D2D_RULE_TOPK || rule == D2D_RULE_DYNK;
   at::Tensor scores, scratch;
-  const bool given = a[9] != Py_None;
+  const bool given = a[10] != Py_None;
   if (given) {
-    const at::Tensor* sp = tensor_of(a[9]);
+    const at::Tensor* sp = tensor_of(a[10]);
     if (!sp || !sp->is_cuda() || sp->scalar_type() != p->dtype || sp->device() != p->device ||
         sp->numel() != N * p->E)
       Py_RETURN_NONE;
@@ -271,7 +273,7 @@ PyObject* run_layer(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const auto cur = c10::cuda::getCurrentCUDAStream(p->device.index());
   const auto stream = (d2d_stream_t)cur.stream();
   Buffers b;
-  if (!buffers_of(a[3], *p, N, &b)) return nullptr;
+  if (!buffers_of(a[4], *p, N, &b)) return nullptr;
   use_on(*p, cur);
   const int dt = p->dtype == at::kBFloat16 ? D2D_BF16 : D2D_F32;
   const auto opts = x.options();
@@ -285,14 +287,14 @@ PyObject* run_layer(PyObject*, PyObject* const* a, Py_ssize_t n) {
   int res = residual ? 1 : 0, rc = D2D_OK;
   at::Tensor xn, norms;
   int norm_layer = 0, norm_ord = 0;
-  if (a[11] != Py_None) {
-    norm_layer = (int)PyLong_AsLong(PyTuple_GetItem(a[11], 0));
-    norm_ord = (int)PyLong_AsLong(PyTuple_GetItem(a[11], 1));
+  if (a[12] != Py_None) {
+    norm_layer = (int)PyLong_AsLong(PyTuple_GetItem(a[12], 0));
+    norm_ord = (int)PyLong_AsLong(PyTuple_GetItem(a[12], 1));
     if (PyErr_Occurred()) return nullptr;
     norms = at::detail::empty_cuda({p->E, N}, opts);
   }
-  if (a[10] != Py_None) {
-    PyObject* nm = a[10];
+  if (a[11] != Py_None) {
+    PyObject* nm = a[11];
     xn = at::detail::empty_cuda(x.sizes(), opts);
     const long kind = PyLong_AsLong(PyTuple_GetItem(nm, 0));
     const double eps = PyFloat_AsDouble(PyTuple_GetItem(nm, 3));
@@ -366,18 +368,18 @@ PyObject* make_pipe(PyObject*, PyObject* const* a, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
-// run_host(plan, modules, parameters, workspaces, pipe, x_host, out_host, staging (kIn + kOut tensors),
-//          (stream in, stream run, stream out), slices, rule, k, tau, residual, sync)
+// run_host(plan, modules, parameters, attributes, workspaces, pipe, x_host, out_host,
+//          staging (kIn + kOut tensors), (stream in, stream run, stream out), slices, rule, k, tau, residual, sync)
 //   -> True | status code (int) | None: the plan does not fit this call
 // Slice i's copy in, the kernels of slice i - 1 and the copy out of slice i - 2 overlap.  The same
 // pipeline issued from Python took 70 us of host time per slice, more than a slice's copies.
 PyObject* run_host(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
-  TORCH_CHECK(n == 15, "run_host takes 15 arguments");
+  TORCH_CHECK(n == 16, "run_host takes 16 arguments");
   Plan* p = static_cast<Plan*>(PyCapsule_GetPointer(a[0], kPlan));
-  HostPipe* h = static_cast<HostPipe*>(PyCapsule_GetPointer(a[4], kPipe));
+  HostPipe* h = static_cast<HostPipe*>(PyCapsule_GetPointer(a[5], kPipe));
   if (!p || !h) return nullptr;
-  const at::Tensor *xh = tensor_of(a[5]), *oh = tensor_of(a[6]);
+  const at::Tensor *xh = tensor_of(a[6]), *oh = tensor_of(a[7]);
   if (!xh || !oh || xh->scalar_type() != p->dtype || oh->scalar_type() != p->dtype ||
       !xh->is_contiguous() || !oh->is_contiguous() || !oh->is_cpu() || xh->sizes() != oh->sizes() ||
       xh->dim() < 2 || xh->size(-1) != p->d || xh->numel() == 0 || h->device != p->device.index() ||
@@ -386,14 +388,14 @@ PyObject* run_host(PyObject*, PyObject* const* a, Py_ssize_t n) {
     Py_RETURN_NONE;
   }
   void* stage[kIn + kOut];
-  for (int i = 0; i < kIn + kOut; ++i) stage[i] = const_cast<void*>(ptr_of(PyTuple_GetItem(a[7], i)));
+  for (int i = 0; i < kIn + kOut; ++i) stage[i] = const_cast<void*>(ptr_of(PyTuple_GetItem(a[8], i)));
   cudaStream_t st[3];
-  for (int i = 0; i < 3; ++i) st[i] = (cudaStream_t)PyLong_AsVoidPtr(PyTuple_GetItem(a[8], i));
-  const int64_t slices = PyLong_AsLongLong(a[9]);
-  const int rule = (int)PyLong_AsLong(a[10]), k = (int)PyLong_AsLong(a[11]);
+  for (int i = 0; i < 3; ++i) st[i] = (cudaStream_t)PyLong_AsVoidPtr(PyTuple_GetItem(a[9], i));
+  const int64_t slices = PyLong_AsLongLong(a[10]);
+  const int rule = (int)PyLong_AsLong(a[11]), k = (int)PyLong_AsLong(a[12]);
   const bool reads_tau = rule == D2D_RULE_MAX || rule == D2D_RULE_DYNK;
-  const double tau = reads_tau ? PyFloat_AsDouble(a[12]) : 0.0;
-  const int residual = PyObject_IsTrue(a[13]), sync = PyObject_IsTrue(a[14]);
+  const double tau = reads_tau ? PyFloat_AsDouble(a[13]) : 0.0;
+  const int residual = PyObject_IsTrue(a[14]), sync = PyObject_IsTrue(a[15]);
   if (PyErr_Occurred()) return nullptr;
   if ((rule != D2D_RULE_ALL && !p->wa) || (rule != D2D_RULE_ALL && rule != D2D_RULE_MAX))
     Py_RETURN_NONE;
@@ -414,7 +416,7 @@ PyObject* run_host(PyObject*, PyObject* const* a, Py_ssize_t n) {
   {
     c10::cuda::CUDAStreamGuard on_run(run);
     for (int64_t i = 0; i < slices; ++i)
-      if (!buffers_of(a[3], *p, (B * (i + 1) / slices - B * i / slices) * per / p->d, &bufs[i],
+      if (!buffers_of(a[4], *p, (B * (i + 1) / slices - B * i / slices) * per / p->d, &bufs[i],
                       keep))
         return nullptr;
   }

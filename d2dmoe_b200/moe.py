@@ -502,7 +502,9 @@ class MoeficationMoE(MoELayer):
         p = ex.kernel_params()
         if not p["w1"].is_cuda:
             return None
-        links = [(0, "experts"), (0, "router"), (1, "last_bias")]     # (an empty slot is a fact too)
+        # (an empty slot is a fact too)
+        links = [(0, "experts"), (0, "router"), (1, "last_bias"), (2, "bias"),
+                 (ex.__dict__, "activation_str")]
         if type(ex) is B200GluExperts:
             links.append((ex._modules, "layers"))
             for i in ("0", "1", "2"):
@@ -530,7 +532,7 @@ class MoeficationMoE(MoELayer):
         links.append((ex._packed.__dict__, "_buf"))
         return host.make_plan(links, r, (p["w1"], p["b1"], p["w_up"], p["w2"], packed),
                               self.last_bias if self.bias else None, ACT[p["act"]],
-                              self._modules, self._parameters)
+                              self._modules, self._parameters, self.__dict__)
 
     def _run_native(self, x, rule, residual, scores=None, norm=None, capture=None):
         """The layer as one native call -> (out, routing tensor[, norms]), or None when it has
@@ -539,8 +541,8 @@ class MoeficationMoE(MoELayer):
         for _ in range(2):
             h = self._plan.handle
             if h is not None:
-                r = host.run_layer(h, self._modules, self._parameters, self._wsp, x, rule, k,
-                                   self.tau, residual, scores, norm, capture)
+                r = host.run_layer(h, self._modules, self._parameters, self.__dict__, self._wsp, x,
+                                   rule, k, self.tau, residual, scores, norm, capture)
                 if type(r) is tuple:
                     return r
                 if r is not None:
@@ -800,8 +802,8 @@ class MoeficationMoE(MoELayer):
         for _ in range(2):
             h = self._plan.handle
             if h is not None:
-                r = host.run_host(h, self._modules, self._parameters, hp.wsp, hp.pipe, x_host,
-                                  out_host, hp.bufs, hp.streams, chunks, rule, 0, self.tau,
+                r = host.run_host(h, self._modules, self._parameters, self.__dict__, hp.wsp, hp.pipe,
+                                  x_host, out_host, hp.bufs, hp.streams, chunks, rule, 0, self.tau,
                                   self.add_residual_connection, sync)
                 if r is True:
                     return True

@@ -59,6 +59,20 @@ def test_invalidate_packed_reaches_every_call(which, call):
     assert _same(moe, x, call)
 
 
+def test_activation_and_bias_are_read_at_each_call():
+    c, t = _case()
+    moe, x = _moe(c, t), t["x"].cuda()
+    assert _same(moe, x)
+    moe.experts.activation_str = "leaky_relu"
+    moe.experts.b1.data.sub_(4.0)                # (hidden values that the two activations tell apart)
+    moe.experts.invalidate_packed()
+    assert _same(moe, x)
+    moe.last_bias.data.add_(5.0)
+    assert _same(moe, x)
+    moe.bias = False
+    assert _same(moe, x)
+
+
 def test_forward_host_beside_a_busy_stream():
     """sync=False: packing, workspaces and kernels depend on nothing the caller's stream is doing.
     A first call, new slice sizes (more than the cache keeps), changed weights, and forward() calls of
