@@ -511,23 +511,30 @@ class MoeficationMoE(MoELayer):
                 links += [(ex.layers._modules, i), (ex.layers._modules[i]._parameters, "w")]
         else:
             links += [(ex._parameters, k) for k in ("w1", "b1", "w2")]
+        weights = [t for t in (p["w1"], p["b1"], p["w_up"], p["w2"]) if t is not None]
+        if self.bias:
+            weights.append(self.last_bias)
+
+        def plain(tensors):
+            # A weight that is no parameter (pruned, parametrised, replicated) has no slot a link
+            # could watch, and nothing that keeps its storage: it takes the general path.
+            roots = (self._modules, self._parameters, self.__dict__)
+            slots = {id((roots[h] if isinstance(h, int) else h).get(key)) for h, key in links}
+            return all(t.dtype == p["w1"].dtype and t.device == p["w1"].device
+                       and t.is_contiguous() and id(t) in slots for t in tensors)
+
+        if not plain(weights):
+            return None
         r = None
         if type(router) is MoeficationRouter and router.fusable():
             wa, wb = router.layers[0].weight, router.layers[2].weight
-            if wa.dtype != p["w1"].dtype or wa.device != p["w1"].device:
-                return None
             links.append((router._modules, "layers"))
             for i in ("0", "2"):
                 links += [(router.layers._modules, i),
                           (router.layers._modules[i]._parameters, "weight")]
-            r = (wa, wb, router.packed())
-            links.append((router._packed.__dict__, "_buf"))      # invalidate_packed() empties the slot
-        tensors = [t for t in (p["w1"], p["b1"], p["w_up"], p["w2"]) if t is not None]
-        if self.bias:
-            tensors.append(self.last_bias)
-        if any(t.dtype != p["w1"].dtype or t.device != p["w1"].device or not t.is_contiguous()
-               for t in tensors + list(r[:2] if r else ())):
-            return None
+            if plain((wa, wb)):
+                r = (wa, wb, router.packed())
+                links.append((router._packed.__dict__, "_buf"))  # invalidate_packed() empties the slot
         packed = ex.packed()
         links.append((ex._packed.__dict__, "_buf"))
         return host.make_plan(links, r, (p["w1"], p["b1"], p["w_up"], p["w2"], packed),

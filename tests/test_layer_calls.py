@@ -73,6 +73,23 @@ def test_activation_and_bias_are_read_at_each_call():
     assert _same(moe, x)
 
 
+@pytest.mark.parametrize("dtype", ["bf16", "fp32"])
+def test_weights_that_are_no_parameters_are_read_at_each_call(dtype):
+    """Pruning replaces the parameter by a plain attribute that a hook writes anew."""
+    from torch.nn.utils import prune
+    c, t = _case(dtype=dtype)
+    moe, plain, x = _moe(c, t), _moe(c, t), t["x"].cuda()
+    lin = moe.router.layers[0]
+    g = torch.Generator().manual_seed(1)
+    prune.custom_from_mask(lin, "weight", (torch.rand(c.R, c.d, generator=g) < 0.5).cuda())
+    for _ in range(2):
+        with torch.no_grad():
+            lin.weight_orig.copy_(torch.roll(lin.weight_orig, 1, 1))
+            moe.router(x)                        # the hook writes lin.weight
+            plain.router.layers[0].weight.copy_(lin.weight)
+        assert torch.equal(moe(x)[1][c.name][0], plain(x)[1][c.name][0])
+
+
 def test_forward_host_beside_a_busy_stream():
     """sync=False: packing, workspaces and kernels depend on nothing the caller's stream is doing.
     A first call, new slice sizes (more than the cache keeps), changed weights, and forward() calls of
