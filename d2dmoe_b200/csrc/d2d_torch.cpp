@@ -230,7 +230,8 @@ bool buffers_of(PyObject* cache, const Plan& p, int64_t N, Buffers* b, PyObject*
 }
 
 // run_layer(plan, modules, parameters, attributes, workspaces, x, rule, k, tau, residual, scores, norm, capture)
-//   -> (out, routing[, norms]) | status code (int) | None: the plan does not fit this call
+//   -> (out, routing[, norms]) | status code (int) | None: the plan is stale | False: it is as the module
+//   is, but this call takes the general path
 // rule: D2D_RULE_*; k / tau as that rule reads them (MAX: threshold 1 - tau).
 // scores: None or [.., E] of x's dtype.  norm: None or (kind, gamma, beta|None, eps, gamma_offset):
 // x + layer(norm(x)).  capture: None or (norm layer, ord), with D2D_RULE_ALL.
@@ -242,12 +243,14 @@ PyObject* run_layer(PyObject*, PyObject* const* a, Py_ssize_t n) {
   }
   Plan* p = static_cast<Plan*>(PyCapsule_GetPointer(a[0], kPlan));
   if (!p) return nullptr;
-  const at::Tensor* xp = tensor_of(a[5]);
-  if (!xp || !xp->is_cuda() || xp->scalar_type() != p->dtype || xp->device() != p->device ||
-      xp->dim() < 1 || xp->size(-1) != p->d || xp->numel() == 0 || !still_valid(*p, a + 1)) {
+  if (!still_valid(*p, a + 1)) {
     if (PyErr_Occurred()) return nullptr;
     Py_RETURN_NONE;
   }
+  const at::Tensor* xp = tensor_of(a[5]);
+  if (!xp || !xp->is_cuda() || xp->scalar_type() != p->dtype || xp->device() != p->device ||
+      xp->dim() < 1 || xp->size(-1) != p->d || xp->numel() == 0)
+    Py_RETURN_FALSE;
   const at::Tensor x = xp->contiguous();
   const int64_t N = x.numel() / p->d;
   const int rule = (int)PyLong_AsLong(a[6]);
@@ -264,10 +267,10 @@ PyObject* run_layer(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const at::Tensor* sp = tensor_of(a[10]);
     if (!sp || !sp->is_cuda() || sp->scalar_type() != p->dtype || sp->device() != p->device ||
         sp->numel() != N * p->E)
-      Py_RETURN_NONE;
+      Py_RETURN_FALSE;
     scores = sp->contiguous();
   } else if (!p->wa && rule != D2D_RULE_ALL) {
-    Py_RETURN_NONE;
+    Py_RETURN_FALSE;
   }
   c10::cuda::CUDAGuard guard(p->device);
   const auto cur = c10::cuda::getCurrentCUDAStream(p->device.index());
@@ -370,7 +373,7 @@ PyObject* make_pipe(PyObject*, PyObject* const* a, Py_ssize_t n) {
 
 // run_host(plan, modules, parameters, attributes, workspaces, pipe, x_host, out_host,
 //          staging (kIn + kOut tensors), (stream in, stream run, stream out), slices, rule, k, tau, residual, sync)
-//   -> True | status code (int) | None: the plan does not fit this call
+//   -> True | status code (int) | None / False as run_layer
 // Slice i's copy in, the kernels of slice i - 1 and the copy out of slice i - 2 overlap.  The same
 // pipeline issued from Python took 70 us of host time per slice, more than a slice's copies.
 PyObject* run_host(PyObject*, PyObject* const* a, Py_ssize_t n) {
@@ -379,14 +382,15 @@ PyObject* run_host(PyObject*, PyObject* const* a, Py_ssize_t n) {
   Plan* p = static_cast<Plan*>(PyCapsule_GetPointer(a[0], kPlan));
   HostPipe* h = static_cast<HostPipe*>(PyCapsule_GetPointer(a[5], kPipe));
   if (!p || !h) return nullptr;
-  const at::Tensor *xh = tensor_of(a[6]), *oh = tensor_of(a[7]);
-  if (!xh || !oh || xh->scalar_type() != p->dtype || oh->scalar_type() != p->dtype ||
-      !xh->is_contiguous() || !oh->is_contiguous() || !oh->is_cpu() || xh->sizes() != oh->sizes() ||
-      xh->dim() < 2 || xh->size(-1) != p->d || xh->numel() == 0 || h->device != p->device.index() ||
-      !still_valid(*p, a + 1)) {
+  if (!still_valid(*p, a + 1)) {
     if (PyErr_Occurred()) return nullptr;
     Py_RETURN_NONE;
   }
+  const at::Tensor *xh = tensor_of(a[6]), *oh = tensor_of(a[7]);
+  if (!xh || !oh || xh->scalar_type() != p->dtype || oh->scalar_type() != p->dtype ||
+      !xh->is_contiguous() || !oh->is_contiguous() || !oh->is_cpu() || xh->sizes() != oh->sizes() ||
+      xh->dim() < 2 || xh->size(-1) != p->d || xh->numel() == 0 || h->device != p->device.index())
+    Py_RETURN_FALSE;
   void* stage[kIn + kOut];
   for (int i = 0; i < kIn + kOut; ++i) stage[i] = const_cast<void*>(ptr_of(PyTuple_GetItem(a[8], i)));
   cudaStream_t st[3];
@@ -398,7 +402,7 @@ PyObject* run_host(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const int residual = PyObject_IsTrue(a[14]), sync = PyObject_IsTrue(a[15]);
   if (PyErr_Occurred()) return nullptr;
   if ((rule != D2D_RULE_ALL && !p->wa) || (rule != D2D_RULE_ALL && rule != D2D_RULE_MAX))
-    Py_RETURN_NONE;
+    Py_RETURN_FALSE;
   c10::cuda::CUDAGuard guard(p->device);
   const cudaStream_t cur = c10::cuda::getCurrentCUDAStream(p->device.index()).stream();
   if (sync) {                          // what the caller's stream has queued comes first

@@ -526,6 +526,8 @@ class MoeficationMoE(MoELayer):
         if not plain(weights):
             return None
         r = None
+        if isinstance(router, MoeficationRouter):
+            links.append((router.__dict__, "_fusable"))
         if type(router) is MoeficationRouter and router.fusable():
             wa, wb = router.layers[0].weight, router.layers[2].weight
             links.append((router._modules, "layers"))
@@ -552,6 +554,8 @@ class MoeficationMoE(MoELayer):
                                    rule, k, self.tau, residual, scores, norm, capture)
                 if type(r) is tuple:
                     return r
+                if r is False:
+                    return None
                 if r is not None:
                     raise D2DError(r, "d2d_moe_forward")
             with torch.no_grad():
@@ -812,8 +816,8 @@ class MoeficationMoE(MoELayer):
                 r = host.run_host(h, self._modules, self._parameters, self.__dict__, hp.wsp, hp.pipe,
                                   x_host, out_host, hp.bufs, hp.streams, chunks, rule, 0, self.tau,
                                   self.add_residual_connection, sync)
-                if r is True:
-                    return True
+                if type(r) is bool:
+                    return r
                 if r is not None:
                     raise D2DError(r, "d2d_moe_forward")
             # packed on the stream that will read it, behind what has been done to the weights

@@ -90,6 +90,23 @@ def test_weights_that_are_no_parameters_are_read_at_each_call(dtype):
         assert torch.equal(moe(x)[1][c.name][0], plain(x)[1][c.name][0])
 
 
+def test_a_call_that_does_not_fit_keeps_the_plan(monkeypatch):
+    """fp32 scores on a bf16 layer take the general path; the plan stays."""
+    class Scores(torch.nn.Module):
+        def forward(self, x):
+            return torch.linspace(0, 1, 8, device=x.device).expand(*x.shape[:-1], 8)
+    c, t = _case()
+    moe, x = _moe(c, t), t["x"].cuda()
+    moe.router, moe.forward_mode, moe.k = Scores(), "topk", 2
+    made = []
+    make = type(moe)._make_plan
+    monkeypatch.setattr(type(moe), "_make_plan", lambda self: made.append(1) or make(self))
+    for _ in range(3):
+        out, gd = moe(x)
+    assert gd[c.name][0].dtype == torch.float32 and int(gd[c.name][0][..., 6:].sum()) == 2 * c.N
+    assert len(made) == 1
+
+
 def test_forward_host_beside_a_busy_stream():
     """sync=False: packing, workspaces and kernels depend on nothing the caller's stream is doing.
     A first call, new slice sizes (more than the cache keeps), changed weights, and forward() calls of
