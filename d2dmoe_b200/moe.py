@@ -622,25 +622,25 @@ class MoeficationMoE(MoELayer):
                             router_packed=self.router.packed(),
                             experts_packed=self.experts.packed(), routing_out=rt)
             rt = rt.view(*orig_size[:-1], E)
-        elif self.forward_mode == "dynk_max" and not capture:
+        elif self.forward_mode in ("dynk_max", "topk", "dynk") and not capture:
             # any other router: its scores come from device tensor ops, the rule and the
             # rest of the layer from the library
             s = self.router(x) if s is None else s
             s2 = s.reshape(N, E).contiguous()
-            rt = torch.empty(N, E, dtype=s.dtype, device=x.device)
-            ops.moe_forward(x2d, None, None, self.tau, p["w1"], p["b1"], p["w2"], p["act"], out,
-                            wsp, w_up=p["w_up"], scores=s2, last_bias=last_bias,
-                            add_residual=self.add_residual_connection,
-                            experts_packed=self.experts.packed(), routing_out=rt)
+            if self.forward_mode == "dynk_max" and s.dtype == x.dtype:
+                rt = torch.empty(N, E, dtype=s.dtype, device=x.device)
+                ops.moe_forward(x2d, None, None, self.tau, p["w1"], p["b1"], p["w2"], p["act"], out,
+                                wsp, w_up=p["w_up"], scores=s2, last_bias=last_bias,
+                                add_residual=self.add_residual_connection,
+                                experts_packed=self.experts.packed(), routing_out=rt)
+            else:                # stage by stage: the rule reads scores of either dtype
+                self._rule_mask(s2, wsp)
+                ops.compact(wsp, N, E)
+                ops.experts_ffn(x2d, wsp, p["w1"], p["b1"], p["w2"], p["act"], out, w_up=p["w_up"],
+                                packed=self.experts.packed(), last_bias=last_bias,
+                                add_residual=self.add_residual_connection, accumulate=False)
+                rt = ops.expand_mask(wsp, N, E, s.dtype)
             rt = rt.view(*orig_size[:-1], E)
-        elif self.forward_mode in ("topk", "dynk") and not capture:
-            s = self.router(x) if s is None else s
-            self._rule_mask(s.reshape(N, E).contiguous(), wsp)
-            ops.compact(wsp, N, E)
-            ops.experts_ffn(x2d, wsp, p["w1"], p["b1"], p["w2"], p["act"], out, w_up=p["w_up"],
-                            packed=self.experts.packed(), last_bias=last_bias,
-                            add_residual=self.add_residual_connection, accumulate=False)
-            rt = ops.expand_mask(wsp, N, E, s.dtype).view(*orig_size[:-1], E)
         else:
             # mode 'all' (every expert on every token: router training), and any mode while
             # the experts capture their activation norms

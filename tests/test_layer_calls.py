@@ -133,3 +133,30 @@ def test_forward_host_beside_a_busy_stream():
             assert O.rel_err(got[b].float(), want[b].float()) <= TOL["bf16"], b
             if b > 3:
                 assert O.rel_err(dev[b].float().cpu(), want[(b + 1) // 2].float()) <= TOL["bf16"], b
+
+
+@pytest.mark.parametrize("dtype,other", [("bf16", torch.float32), ("fp32", torch.bfloat16)])
+@pytest.mark.parametrize("mode", ["dynk_max", "topk", "dynk"])
+def test_scores_in_another_dtype(mode, dtype, other):
+    """A router whose scores are not of x's dtype (autocast): the rule applies to them as they are."""
+    class Scores(torch.nn.Module):
+        def forward(self, x):
+            return given
+    c, t = _case(dtype=dtype)
+    moe, x = _moe(c, t), t["x"].cuda()
+    given = torch.exp(torch.randn(1, c.N, c.E, generator=torch.Generator().manual_seed(2))).to(other).cuda()
+    moe.router, moe.forward_mode, moe.k = Scores(), mode, 2
+    out, gd = moe(x)
+    rt = gd[c.name][0]
+    s2 = given.reshape(c.N, c.E)
+    if mode == "dynk_max":
+        m = O.dynk_max_mask(s2.cpu(), c.tau)
+    else:
+        from d2dmoe_b200 import ops
+        wsp = ops.Workspace.allocate(c.N, c.E, "cuda")
+        ops.mask_rule_from_scores(s2, mode, wsp, k=2, tau=c.tau)
+        m = ops.expand_mask(wsp, c.N, c.E, other).cpu() > 0
+    assert rt.dtype == other and torch.equal(rt.reshape(c.N, c.E).cpu() > 0, m)
+    ex = O.experts_ffn_exact(t["x"].reshape(c.N, c.d), m, t["w1"], t["b1"], t["w2"])
+    ex = ex + t["last_bias"].double()
+    assert O.rel_err(out.reshape(c.N, c.d).cpu().float(), ex) <= TOL[dtype]
