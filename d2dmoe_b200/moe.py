@@ -497,7 +497,10 @@ class MoeficationMoE(MoELayer):
         """Plan of the one-call layer for the parameters as they are now, or None when the
         modules are not the plain ones of this file or not on a GPU."""
         ex, router = self.experts, self.router
-        if type(ex) not in (B200KernelExperts, B200GluExperts):
+        # (subclasses too, unless they hand out other weights)
+        params = getattr(type(ex), "kernel_params", None)
+        if (params not in (B200KernelExperts.kernel_params, B200GluExperts.kernel_params)
+                or type(ex).packed is not B200KernelExperts.packed):
             return None
         p = ex.kernel_params()
         if not p["w1"].is_cuda:
@@ -505,7 +508,7 @@ class MoeficationMoE(MoELayer):
         # (an empty slot is a fact too)
         links = [(0, "experts"), (0, "router"), (1, "last_bias"), (2, "bias"),
                  (ex.__dict__, "activation_str")]
-        if type(ex) is B200GluExperts:
+        if params is B200GluExperts.kernel_params:
             links.append((ex._modules, "layers"))
             for i in ("0", "1", "2"):
                 links += [(ex.layers._modules, i), (ex.layers._modules[i]._parameters, "w")]
@@ -528,7 +531,8 @@ class MoeficationMoE(MoELayer):
         r = None
         if isinstance(router, MoeficationRouter):
             links.append((router.__dict__, "_fusable"))
-        if type(router) is MoeficationRouter and router.fusable():
+        if (isinstance(router, MoeficationRouter) and router.fusable()
+                and type(router).packed is MoeficationRouter.packed):
             wa, wb = router.layers[0].weight, router.layers[2].weight
             links.append((router._modules, "layers"))
             for i in ("0", "2"):
@@ -578,8 +582,9 @@ class MoeficationMoE(MoELayer):
                 capture = (ops.NORM_OF[capture[0]], capture[1])
         elif router is None or x.numel() == 0:
             return self._forward_general(x)
-        elif (type(router) is not MoeficationRouter or not router._fusable
-              or (rule != ops.RULE_MAX and _hooked(router))):
+        elif (not isinstance(router, MoeficationRouter) or not router.fusable()
+              or (rule != ops.RULE_MAX and (type(router) is not MoeficationRouter
+                                            or _hooked(router)))):
             # (only 'dynk_max' has always skipped the router module's call)
             with torch.no_grad():
                 scores = router(x)
@@ -785,8 +790,8 @@ class MoeficationMoE(MoELayer):
         rule = _RULES.get(self.forward_mode)
         if (rule not in (ops.RULE_MAX, ops.RULE_ALL) or getattr(ex, "_capture", None) is not None
                 or ex._forward_mode not in _KERNEL_MODES or x_host.dim() < 2 or x_host.numel() == 0
-                or (rule == ops.RULE_MAX and not (type(router) is MoeficationRouter
-                                                  and router._fusable))):
+                or (rule == ops.RULE_MAX and not (isinstance(router, MoeficationRouter)
+                                                  and router.fusable()))):
             return False
         B = x_host.shape[0]
         rows = max(B * (i + 1) // chunks - B * i // chunks for i in range(chunks))

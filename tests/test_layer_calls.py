@@ -107,6 +107,25 @@ def test_a_call_that_does_not_fit_keeps_the_plan(monkeypatch):
     assert len(made) == 1
 
 
+def test_subclasses_take_the_fused_path():
+    import d2dmoe_b200 as D
+
+    class Router(D.MoeficationRouter):
+        def forward(self, x):
+            raise AssertionError("'dynk_max' does not call a fusable router")
+
+    class Experts(D.B200KernelExperts):
+        pass
+    c, t = _case()
+    moe, x = _moe(c, t, Experts, Router), t["x"].cuda()
+    plain = _moe(c, t)
+    for call in (lambda m: m(x), lambda m: m.forward_block(x, torch.nn.LayerNorm(c.d).to(x))):
+        got, want = call(moe), call(plain)
+        assert torch.equal(got[1][c.name][0], want[1][c.name][0])
+        assert O.rel_err(got[0].float().cpu(), want[0].float().cpu()) <= TOL["bf16"]
+    assert moe._plan.handle is not None
+
+
 def test_forward_host_beside_a_busy_stream():
     """sync=False: packing, workspaces and kernels depend on nothing the caller's stream is doing.
     A first call, new slice sizes (more than the cache keeps), changed weights, and forward() calls of
