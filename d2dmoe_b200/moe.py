@@ -45,6 +45,9 @@ ACTIVATION_NAME_MAP = {
     "abs": _function_module(torch.abs), "identity": nn.Identity,
 }
 
+# what MoeficationRouter.layers holds where the router kernel computes it
+_FUSABLE_LAYERS = [nn.Linear, nn.ReLU, nn.Linear, ACTIVATION_NAME_MAP["abs"]]
+
 # forward_mode strings of the upstream experts class that mean "the fast GPU path"
 _KERNEL_MODES = ("b200", "triton_atomic", "triton")
 
@@ -354,14 +357,20 @@ MOE_IMPL_MAP = {
 _HOST_STREAMS: dict = {}
 
 
-def _hooked(router) -> bool:
-    """True when a forward hook waits for a call of the router or of one of its layers."""
+def _as_built(router) -> bool:
+    """True when a call of the router module gives what the router kernel computes: the layers of
+    its constructor, nothing replaced, hooked or switched on since, and no autocast."""
     g = nn.modules.module
-    if g._global_forward_hooks or g._global_forward_pre_hooks:
-        return True
-    layers = router._modules["layers"]
-    return any(m._forward_hooks or m._forward_pre_hooks
-               for m in (router, layers, *layers._modules.values()))
+    if (type(router) is not MoeficationRouter or not router._fusable
+            or router.test_override_outputs_p is not None or "forward" in router.__dict__
+            or g._global_forward_hooks or g._global_forward_pre_hooks
+            or torch.is_autocast_enabled("cuda")):
+        return False
+    layers = list(router._modules["layers"]._modules.values())
+    return ([type(m) for m in layers] == _FUSABLE_LAYERS
+            and layers[0]._parameters["bias"] is None and layers[2]._parameters["bias"] is None
+            and not any(m._forward_hooks or m._forward_pre_hooks or "forward" in m.__dict__
+                        for m in (router, *layers)))
 
 
 class MoELayer(nn.Module):
@@ -583,8 +592,7 @@ class MoeficationMoE(MoELayer):
         elif router is None or x.numel() == 0:
             return self._forward_general(x)
         elif (not isinstance(router, MoeficationRouter) or not router.fusable()
-              or (rule != ops.RULE_MAX and (type(router) is not MoeficationRouter
-                                            or _hooked(router)))):
+              or (rule != ops.RULE_MAX and not _as_built(router))):
             # (only 'dynk_max' has always skipped the router module's call)
             with torch.no_grad():
                 scores = router(x)

@@ -126,6 +126,29 @@ def test_subclasses_take_the_fused_path():
     assert moe._plan.handle is not None
 
 
+@pytest.mark.parametrize("how", ["layer", "bias", "forward", "override", "autocast"])
+def test_ranked_rules_call_a_router_that_was_changed(how):
+    """'topk' and 'dynk' rank what the router module returns."""
+    c, t = _case(dtype="fp32" if how == "autocast" else "bf16")
+    moe, x = _moe(c, t), t["x"].cuda()
+    moe.forward_mode, moe.k = "topk", 3
+    r = moe.router
+    if how == "layer":
+        r.layers[1] = torch.nn.Tanh()
+    elif how == "bias":
+        r.layers[2].bias = torch.nn.Parameter(torch.linspace(-9, 9, c.E, dtype=c.torch_dtype).cuda())
+    elif how == "forward":
+        flipped = type(r).forward
+        r.forward = lambda v: 1.0 / (1.0 + flipped(r, v))
+    elif how == "override":
+        r.test_override_outputs_p, r.response_cache = 0.5, {}
+    with torch.no_grad(), torch.autocast("cuda", torch.bfloat16, enabled=how == "autocast"):
+        rt = moe(x)[1][c.name][0]
+        s = r(x)
+    best = torch.zeros_like(s).scatter_(-1, torch.sort(s.float(), dim=-1, descending=True, stable=True)[1][..., :3], 1)
+    assert rt.dtype == s.dtype and torch.equal(rt, best)
+
+
 def test_forward_host_beside_a_busy_stream():
     """sync=False: packing, workspaces and kernels depend on nothing the caller's stream is doing.
     A first call, new slice sizes (more than the cache keeps), changed weights, and forward() calls of
