@@ -305,7 +305,11 @@ PyObject* run_layer(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (PyErr_Occurred()) return nullptr;
     const at::Tensor* gt = tensor_of(PyTuple_GetItem(nm, 1));
     const at::Tensor* bt = tensor_of(PyTuple_GetItem(nm, 2));
-    TORCH_CHECK(gt && gt->numel() == p->d && (!bt || bt->numel() == p->d), "norm parameters");
+    const auto fits = [&](const at::Tensor* t) {
+      return t->numel() == p->d && t->scalar_type() == p->dtype && t->device() == p->device;
+    };
+    TORCH_CHECK(gt && fits(gt) && (!bt || fits(bt)), "norm parameters: ", p->d,
+                " values of x's dtype, on its device");
     const at::Tensor g = gt->contiguous(), bb = bt ? bt->contiguous() : at::Tensor();
     rc = d2d_prenorm_init(xin, g.data_ptr(), bt ? bb.data_ptr() : nullptr, (float)eps, (int)kind,
                           (float)goff, lb, xn.data_ptr(), out.data_ptr(), N, (int)p->d, dt, stream);

@@ -703,8 +703,8 @@ class MoeficationMoE(MoELayer):
         # (affine parameters in another dtype than x -- mixed-precision norms -- keep the
         # framework's own normalisation: the fused pass computes in the dtype of x)
         fused = (na is not None and x.is_cuda and self.forward_mode == "dynk_max"
-                 and na[1].dtype == x.dtype and (na[2] is None or na[2].dtype == x.dtype)
-                 and na[1].device == x.device
+                 and na[1].dtype == x.dtype and na[1].device == x.device
+                 and (na[2] is None or (na[2].dtype == x.dtype and na[2].device == x.device))
                  and getattr(ex, "_capture", None) is None
                  and isinstance(router, MoeficationRouter) and router.fusable()
                  and not self.add_residual_connection

@@ -202,3 +202,13 @@ def test_scores_in_another_dtype(mode, dtype, other):
     ex = O.experts_ffn_exact(t["x"].reshape(c.N, c.d), m, t["w1"], t["b1"], t["w2"])
     ex = ex + t["last_bias"].double()
     assert O.rel_err(out.reshape(c.N, c.d).cpu().float(), ex) <= TOL[dtype]
+
+
+@pytest.mark.parametrize("which", ["weight", "bias"])
+def test_norm_parameters_on_another_device_are_refused(which):
+    c, t = _case()
+    moe, x = _moe(c, t), t["x"].cuda()
+    norm = torch.nn.LayerNorm(c.d).to(x)
+    setattr(norm, which, torch.nn.Parameter(getattr(norm, which).detach().cpu()))
+    with pytest.raises((RuntimeError, ValueError)):
+        moe.forward_block(x, norm)
