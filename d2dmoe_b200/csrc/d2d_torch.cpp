@@ -14,6 +14,7 @@
 #include <Python.h>
 
 #include <ATen/ATen.h>
+#include <ATen/core/CachingHostAllocator.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAException.h>
@@ -429,6 +430,13 @@ PyObject* run_host(PyObject*, PyObject* const* a, Py_ssize_t n) {
         return nullptr;
   }
   use_on(*p, run);
+  // pinned blocks that their owner drops are not handed out again before these copies are done (memory
+  // of another origin is none of the allocator's)
+  const std::pair<const at::Tensor*, cudaStream_t> used[2] = {{xh, st[0]}, {oh, st[2]}};
+  for (const auto& u : used)
+    at::getHostAllocator(at::kCUDA)->record_event(
+        u.first->data_ptr(), u.first->storage().data_ptr().get_context(),
+        c10::cuda::getStreamFromExternal(u.second, p->device.index()).unwrap());
   const size_t es = xh->element_size();
   const char* src = static_cast<const char*>(xh->data_ptr());
   char* dst = static_cast<char*>(oh->data_ptr());

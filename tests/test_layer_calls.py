@@ -212,3 +212,26 @@ def test_norm_parameters_on_another_device_are_refused(which):
     setattr(norm, which, torch.nn.Parameter(getattr(norm, which).detach().cpu()))
     with pytest.raises((RuntimeError, ValueError)):
         moe.forward_block(x, norm)
+
+
+def test_pinned_buffers_dropped_while_the_pipeline_copies():
+    """sync=False: a dropped input is still read, a dropped output still written; neither block may
+    serve a new tensor meanwhile."""
+    import d2dmoe_b200 as D
+    from d2dmoe_b200 import moe as impl
+    c, t = _case(64, B=8)
+    moe = _moe(c, t)
+    want = moe(t["x"].cuda())[0].cpu()
+    out = moe.forward_host(t["x"].pin_memory())
+    assert O.rel_err(out.float(), want.float()) <= TOL["bf16"]
+    out.fill_(0.0)
+    with torch.cuda.stream(impl._HOST_STREAMS[moe.experts.w1.device][0]):
+        torch.cuda._sleep(200_000_000)
+    x = t["x"].pin_memory()
+    moe.forward_host(x, out, sync=False)
+    moe.forward_host(x, torch.empty_like(x).pin_memory(), sync=False)
+    del x
+    new = [torch.full_like(t["x"], 7.0).pin_memory() for _ in range(4)]
+    D.MoeficationMoE.host_synchronize()
+    assert O.rel_err(out.float(), want.float()) <= TOL["bf16"]
+    assert all(bool((v == 7.0).all()) for v in new)
