@@ -90,11 +90,11 @@ class _HostBuffers:
     """Staging buffers, events and workspaces of ``forward_host``; copies of a module start without
     them."""
 
-    __slots__ = ("shape", "dtype", "device", "bufs", "pipe", "streams", "wsp")
+    __slots__ = ("wsp", "staging")
 
     def __init__(self):
         self.wsp = _WorkspaceCache()
-        self.shape = self.dtype = self.device = self.bufs = self.pipe = self.streams = None
+        self.staging = (None,)    # key, buffers, pipe, streams: replaced whole, never changed
 
     def __deepcopy__(self, memo):
         return _HostBuffers()
@@ -805,7 +805,8 @@ class MoeficationMoE(MoELayer):
         rows = max(B * (i + 1) // chunks - B * i // chunks for i in range(chunks))
         shape = (rows,) + tuple(x_host.shape[1:])
         hp = self._host
-        if hp.shape != shape or hp.dtype != x_host.dtype or hp.device != dev:
+        staging = hp.staging      # this call's, whatever another thread puts there meanwhile
+        if staging[0] != (shape, x_host.dtype, dev):
             # Copies and kernels of earlier sync=False calls may still use the old staging
             # buffers: drain the streams before they go back to the allocator (a host wait, but
             # only when the slice shape changes); the allocator is told who uses the new ones.
@@ -820,14 +821,15 @@ class MoeficationMoE(MoELayer):
                 b.record_stream(st[1])
             for b in bufs[2:]:
                 b.record_stream(st[2])
-            hp.shape, hp.dtype, hp.device, hp.bufs = shape, x_host.dtype, dev, tuple(bufs)
-            hp.pipe = host.make_pipe(torch.device(dev).index or 0)
-            hp.streams = tuple(s_.cuda_stream for s_ in st)
+            staging = hp.staging = ((shape, x_host.dtype, dev), tuple(bufs),
+                                    host.make_pipe(torch.device(dev).index or 0),
+                                    tuple(s_.cuda_stream for s_ in st))
+        _, bufs, pipe, streams = staging
         for _ in range(2):
             h = self._plan.handle
             if h is not None:
-                r = host.run_host(h, self._modules, self._parameters, self.__dict__, hp.wsp, hp.pipe,
-                                  x_host, out_host, hp.bufs, hp.streams, chunks, rule, 0, self.tau,
+                r = host.run_host(h, self._modules, self._parameters, self.__dict__, hp.wsp, pipe,
+                                  x_host, out_host, bufs, streams, chunks, rule, 0, self.tau,
                                   self.add_residual_connection, sync)
                 if type(r) is bool:
                     return r

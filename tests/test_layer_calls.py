@@ -235,3 +235,25 @@ def test_pinned_buffers_dropped_while_the_pipeline_copies():
     D.MoeficationMoE.host_synchronize()
     assert O.rel_err(out.float(), want.float()) <= TOL["bf16"]
     assert all(bool((v == 7.0).all()) for v in new)
+
+
+def test_forward_host_keeps_its_buffers_while_another_thread_changes_them(monkeypatch):
+    """A call with other slices, as another thread would make it, between the choice of the staging
+    buffers and their use."""
+    from types import SimpleNamespace
+    from d2dmoe_b200 import moe as impl
+    c, t = _case(40, B=8)
+    moe, x, used = _moe(c, t), t["x"], []
+    real = impl.host
+    monkeypatch.setattr(impl, "host", SimpleNamespace(
+        make_plan=real.make_plan, make_pipe=real.make_pipe, run_layer=real.run_layer,
+        run_host=lambda *a: used.append((tuple(a[6].shape), a[8][0].shape[0])) or True))
+    make = type(moe)._make_plan
+
+    def between(self):
+        monkeypatch.setattr(type(moe), "_make_plan", make)
+        moe.forward_host(x[:2], chunks=2)
+        return make(self)
+    monkeypatch.setattr(type(moe), "_make_plan", between)
+    moe.forward_host(x, chunks=2)
+    assert used == [((2, 40, c.d), 1), ((8, 40, c.d), 4)]
