@@ -475,6 +475,10 @@ class MoeficationMoE(MoELayer):
         self._plan = _Plan()
         self._host = _HostBuffers()
 
+    def __setstate__(self, state):
+        # modules saved whole before these attributes existed
+        super().__setstate__({"_plan": _Plan(), "_host": _HostBuffers(), **state})
+
     # -- routing for the modes that are not fused ---------------------------------
     def gate(self, x):
         """Routing tensor [B,S,E] of 0/1 in the router's dtype for the non-fused modes

@@ -66,6 +66,18 @@ def test_no_cpu_path():
         m.experts(torch.randn(6, 64), torch.ones(6, 4))
 
 
+def test_modules_saved_before_the_call_plans_load():
+    import pickle
+    m = make()
+    m.router = None                       # (its abs module is a local class: not picklable)
+    del m.__dict__["_plan"], m.__dict__["_host"]
+    saved = pickle.dumps(m)
+    m = pickle.loads(saved)
+    assert m._plan.handle is None and m._host.staging == (None,)
+    with pytest.raises(RuntimeError, match="CUDA tensors only"):
+        m(torch.randn(2, 3, 64))
+
+
 def test_matches_upstream_signatures_and_checkpoint():
     ref = load_reference()
     if ref is None:
