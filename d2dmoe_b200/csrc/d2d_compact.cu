@@ -215,11 +215,13 @@ int compact_row_cells(int E) {
   return ep;
 }
 
-// the byte table needs ntiles * EP bytes; this (four bytes per tile and expert) is what
-// d2d_workspace_bytes has always reported and covers it for every E
+// Four bytes per tile and expert, which d2d_workspace_bytes has always reported, hold the byte table of
+// ntiles * EP cells from four experts on; below that its rows of 16 cells are the larger.
 size_t compact_workspace_bytes(int64_t n_max, int E) {
-  const int64_t ntiles = ceil_div64(n_max > 0 ? n_max : 1, CTILE);
-  return (size_t)(ntiles + 1) * (size_t)E * sizeof(int32_t);
+  const size_t ntiles = (size_t)ceil_div64(n_max > 0 ? n_max : 1, CTILE);
+  const size_t reported = (ntiles + 1) * (size_t)E * sizeof(int32_t);
+  const size_t table = E <= MAX_E ? ntiles * (size_t)compact_row_cells(E) : 0;
+  return reported > table ? reported : table;
 }
 
 // short masks are counted by the scatter kernel itself: up to 32 KB every CTA reads them in less

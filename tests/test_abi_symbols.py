@@ -42,6 +42,20 @@ def test_host_only_entry_points():
     assert _capi.lib.d2d_mask_from_scores(None, 0.5, None, 10, 4, 0, None, None) == 1
 
 
+def test_workspace_holds_the_counts_table():
+    """One byte per 128-token tile and expert, rows padded to a power of two of at least 16 cells."""
+    from d2dmoe_b200 import _capi
+    n = ctypes.c_size_t(0)
+    for E in (1, 2, 3, 4, 5, 16, 17, 33, 255, 256):
+        cells = max(16, 1 << (E - 1).bit_length())
+        for N in (0, 1, 128, 129, 1025, 50432, 131072):
+            assert _capi.lib.d2d_workspace_bytes(N, E, ctypes.byref(n)) == 0
+            assert n.value >= -(-N // 128) * cells and n.value >= (-(-max(N, 1) // 128) + 1) * E * 4
+    a = ctypes.c_void_p(0x7f0000000000)                   # never dereferenced
+    need = 394 * 16                                       # 50432 tokens, one expert
+    assert _capi.lib.d2d_compact(a, a, a, 50432, 1, a, need - 16, None, None) == 4   # WORKSPACE
+
+
 def test_misaligned_buffers_are_rejected_before_any_launch():
     """x / out that do not start on a 16-byte boundary (a view with a storage offset) must be
     refused on the host with BAD_ARG: the checks of every stage run before the first launch,

@@ -277,3 +277,28 @@ def test_short_calls_write_their_lists(N, E):
         ex = O.experts_ffn_exact(t["x"].reshape(N, c.d), m, t["w1"], t["b1"], t["w2"])
         slack = max(1.0, m.sum(1).max().item() ** 0.5 / 2)      # one rounding per added expert
         assert O.rel_err(out.cpu().float(), ex + t["last_bias"].double()) <= TOL["bf16"] * slack
+
+
+@pytest.mark.parametrize("E", [1, 2, 3])
+def test_counts_table_of_few_experts_stays_in_the_workspace(E):
+    from d2dmoe_b200 import ops
+    N, d = 50432, 64
+    c, t = _layer(N, d, 16, E, 16, "bf16", E)
+    wsp = ops.Workspace.allocate(N, E, "cuda")
+    need = ops.workspace_bytes(N, E)
+    whole = torch.full((need + 65536,), 0xA5, dtype=torch.uint8, device="cuda")
+    wsp.ws = whole[:need]
+    x2d, wa, wb = _dev(t["x"].reshape(N, d)), _dev(t["wa"]), _dev(t["wb"])
+    w1, b1, w2 = _dev(t["w1"]), _dev(t["b1"]), _dev(t["w2"])
+    out = torch.empty(N, d, dtype=torch.bfloat16, device="cuda")
+    ops.moe_forward(x2d, wa, wb, 0.3, w1, b1, w2, "relu", out, wsp,
+                    router_packed=ops.prepack_router(wa, wb),
+                    experts_packed=ops.prepack_experts(w1, b1, w2))
+    off, idx = _lists(wsp, E)
+    ops.compact(wsp, N, E)
+    wsp.check_status()
+    assert bool((whole[need:] == 0xA5).all())
+    m = O.unpack_mask(wsp.mask_bits[:N].cpu().numpy().view(np.uint32), E)
+    roff, ridx = O.expert_token_lists(m)
+    for o, i in ((off, idx), _lists(wsp, E)):
+        assert np.array_equal(o, np.asarray(roff)) and np.array_equal(i, np.asarray(ridx))
