@@ -196,12 +196,16 @@ compact_scatter_kernel(const uint32_t* __restrict__ mask_bits, const uint8_t* __
   }
   __syncthreads();
   const int32_t row0 = (int32_t)(t - lane);
+  // (a table that does not belong to the mask, left by a router that gave up, must not lead a write
+  // out of the lists)
+  const uint32_t room = (uint32_t)(N * E);
 #pragma unroll
   for (int j = 0; j < MAX_E / 32; ++j) {
     if (j >= nw) break;
     if (32 * j + lane >= E) continue;
-    int32_t* dst = token_idx + cnt[w * E + 32 * j + lane];
-    for (uint32_t m = word[j]; m != 0u; m &= m - 1) *dst++ = row0 + __ffs(m) - 1;
+    uint32_t at = (uint32_t)cnt[w * E + 32 * j + lane];
+    for (uint32_t m = word[j]; m != 0u; m &= m - 1, ++at)
+      if (at < room) token_idx[at] = row0 + __ffs(m) - 1;
   }
 }
 

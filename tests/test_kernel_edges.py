@@ -302,3 +302,30 @@ def test_counts_table_of_few_experts_stays_in_the_workspace(E):
     roff, ridx = O.expert_token_lists(m)
     for o, i in ((off, idx), _lists(wsp, E)):
         assert np.array_equal(o, np.asarray(roff)) and np.array_equal(i, np.asarray(ridx))
+
+
+def test_lists_after_a_router_that_gave_up_stay_in_bounds():
+    """The scatter kernel then meets a counts table that is not the mask's."""
+    from d2dmoe_b200 import _capi, ops
+    N, d, E = 2000, 256, 24
+    c, t = _layer(N, d, 32, E, 64, "bf16", 3)
+    wsp = ops.Workspace.allocate(N, E, "cuda")
+    whole = torch.full((3 * N * E,), -1, dtype=torch.int32, device="cuda")
+    wsp.token_idx = whole[N * E: 2 * N * E]
+    x2d, wa, wb = _dev(t["x"].reshape(N, d)), _dev(t["wa"]), _dev(t["wb"])
+    w1, b1, w2 = _dev(t["w1"]), _dev(t["b1"]), _dev(t["w2"])
+    rp, ep = ops.prepack_router(wa, wb), ops.prepack_experts(w1, b1, w2)
+    out = torch.empty(N, d, dtype=torch.bfloat16, device="cuda")
+    for fill in (0xFF, 0x80, 0x01):
+        wsp.ws.fill_(fill)
+        wsp.mask_bits.fill_(-1)
+        try:
+            assert _capi.lib.d2d_debug_configure(12, 1) == 0
+            ops.moe_forward(x2d, wa, wb, 0.3, w1, b1, w2, "relu", out, wsp, router_packed=rp,
+                            experts_packed=ep)
+            torch.cuda.synchronize()
+        finally:
+            _capi.lib.d2d_debug_configure(0, 0)
+        with pytest.raises(_capi.D2DError, match="TIMEOUT"):
+            wsp.check_status()
+        assert bool((whole[: N * E] == -1).all()) and bool((whole[2 * N * E:] == -1).all())
