@@ -72,9 +72,10 @@ experts_simt_kernel(const T* __restrict__ x, const int32_t* __restrict__ token_i
     int run = 0;
     for (int e = 0; e < E; ++e) {
       tstart[e] = run;
-      const int c = offsets[e + 1] - offsets[e];
-      if (c < 0) { report(dev_status, D2D_ERR_INDEX_RANGE); }
-      run += c > 0 ? (c + TM_ - 1) / TM_ : 0;
+      const int o = offsets[e], o1 = offsets[e + 1];
+      const bool bad = o1 < o || o < 0 || o1 > N * (int64_t)E;
+      if (bad) report(dev_status, D2D_ERR_INDEX_RANGE);
+      run += bad ? 0 : (o1 - o + TM_ - 1) / TM_;        // a bad list is dropped
     }
     tstart[E] = run;
   }

@@ -311,10 +311,10 @@ experts_fp32_kernel(const float* __restrict__ x, const int32_t* __restrict__ tok
 #pragma unroll
     for (int q = 0; q < MAX_E / 32; ++q) {
       const int e = lane * (MAX_E / 32) + q;
-      const int n = e < E ? off[e + 1] - off[e] : 0;
-      if (n < 0 || (e < E && (off[e] < 0 || off[e + 1] > N * (int64_t)E)))
-        report(dev_status, D2D_ERR_INDEX_RANGE);
-      c[q] = n > 0 ? (n + TR - 1) / TR : 0;
+      const bool bad =
+          e < E && (off[e + 1] < off[e] || off[e] < 0 || off[e + 1] > N * (int64_t)E);
+      if (bad) report(dev_status, D2D_ERR_INDEX_RANGE);
+      c[q] = e < E && !bad ? (off[e + 1] - off[e] + TR - 1) / TR : 0;      // a bad list is dropped
       sum += c[q];
     }
     int incl = sum;

@@ -329,3 +329,32 @@ def test_lists_after_a_router_that_gave_up_stay_in_bounds():
         with pytest.raises(_capi.D2DError, match="TIMEOUT"):
             wsp.check_status()
         assert bool((whole[: N * E] == -1).all()) and bool((whole[2 * N * E:] == -1).all())
+
+
+@pytest.mark.parametrize("dtype,glu,norms", [("fp32", False, False), ("fp32", True, False),
+                                             ("fp32", False, True), ("bf16", False, False)])
+@pytest.mark.parametrize("e,value", [(0, -40), (2, 1 << 30), (2, -7), (3, 8 * 4 + 1), (4, 1 << 30)])
+def test_offsets_out_of_range_drop_their_lists(dtype, glu, norms, e, value):
+    """Reported through the status word; the lists on either side of the bad offset are skipped."""
+    from d2dmoe_b200 import _capi, ops
+    N, d, H, E = 8, 64, 32, 4
+    c, t = _layer(N, d, H, E, 16, dtype, 5, "relu", glu)
+    m = torch.ones(N, E, dtype=torch.bool)
+    wsp = ops.Workspace.allocate(N, E, "cuda")
+    off = torch.arange(E + 1, dtype=torch.int32) * N
+    off[e] = value
+    wsp.offsets.copy_(off)
+    wsp.token_idx.copy_(torch.arange(N, dtype=torch.int32).repeat(E))
+    m[:, [i for i in range(E) if off[i] < 0 or off[i + 1] < off[i] or off[i + 1] > N * E]] = False
+    w1, b1, w2, wu = (_dev(t.get(k)) for k in ("w1", "b1", "w2", "w_up"))
+    b1 = None if glu else b1
+    out = torch.empty(N, d, dtype=c.torch_dtype, device="cuda")
+    kw = dict(norms=torch.empty(E, N, device="cuda")) if norms else {}
+    ops.experts_ffn(_dev(t["x"].reshape(N, d)), wsp, w1, b1, w2, "relu", out, w_up=wu,
+                    packed=ops.prepack_experts(w1, b1, w2, wu), **kw)
+    with pytest.raises(_capi.D2DError, match="INDEX_RANGE"):
+        wsp.check_status()
+    ex = O.experts_ffn_exact(t["x"].reshape(N, d), m, t["w1"], None if glu else t["b1"], t["w2"], "relu",
+                             t.get("w_up") if glu else None)
+    # one rounding per added expert
+    assert O.rel_err(out.cpu().float(), ex) <= TOL[dtype]
