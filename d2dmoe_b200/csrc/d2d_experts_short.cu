@@ -215,7 +215,10 @@ __device__ void short_mma(const ShortParams& p, ShortCtl* c, uint32_t ring, uint
       ph ^= ctx;
       ctx ^= 1;
     }
-    if (it == cl) continue;
+    // (A CTA without output columns, d < 128 C, reads no hidden tile.  Nothing would hold hid_full back
+    // until it had seen a phase: its own warps hand the tile on at once, and the others may then
+    // complete the next phase as well, which has the parity of the one before.)
+    if (it == cl || s0 == s1) continue;
     if (!mbar_wait_fast(smem_u32(&c->hid_full), hph, af, p.dev_status)) return;
     hph ^= 1;
     fence_cluster();

@@ -90,17 +90,19 @@ SHORT = [  # N, d, H, E, activation, gated: around 32 rows of a list, every clus
     (64, 384, 128, 5, "leaky_relu", False), (65, 2048, 128, 20, "relu", False),
     (32, 384, 96, 3, "gelu_tanh", True), (33, 640, 32, 9, "gelu", True), (40, 256, 64, 5, "relu", True),
     (257, 2048, 128, 128, "gelu", True), (512, 2048, 128, 128, "gelu", True),
+    # CTAs without output columns (d < 512), more items than clusters
+    (512, 128, 32, 10, "relu", False), (511, 256, 128, 10, "gelu", True), (500, 384, 64, 9, "relu", False),
 ]
 
 
-@pytest.mark.parametrize("kind", ["one_expert", "first_token", "few", "random"])
+@pytest.mark.parametrize("kind", ["one_expert", "first_token", "few", "random", "all"])
 @pytest.mark.parametrize("N,d,H,E,act,glu", SHORT)
 def test_short_call_experts(N, d, H, E, act, glu, kind):
     from d2dmoe_b200 import ops
     c, t = _layer(N, d, H, E, 128, "bf16", N + d, act, glu)
     g = _gen(N)
     m = torch.rand(N, E, generator=g) < 2.0 / E if kind == "few" else _mask(kind, N, E, g)
-    if kind == "random" and E > 64:           # lists of up to about 90 rows, the oracle in bounds
+    if kind in ("random", "all") and E > 64:  # lists of up to about 90 rows, the oracle in bounds
         m &= torch.rand(1, E, generator=g) < 0.2
     wsp = ops.Workspace.allocate(N, E, "cuda")
     wsp.mask_bits[:N].copy_(torch.from_numpy(O.pack_mask(m).view(np.int32)).cuda())
