@@ -406,6 +406,7 @@ __device__ void role_mma1(const Params& p, Ctl* c, uint32_t ring, uint32_t tmem)
     tc_fence_after();
     for (int kc = 0; kc < g.kc1; ++kc) {
       if (!mbar_wait_fast(smem_u32(&c->full[r.s]), r.ph, af, p.dev_status)) return;
+      fence_proxy_async();               // (the token rows are cp.async writes)
       tc_fence_after();
       const uint32_t alo = lo0 + r.s * ((uint32_t)g.stage >> 4), blo = alo + ((uint32_t)g.a_slot >> 4);
 #pragma unroll
