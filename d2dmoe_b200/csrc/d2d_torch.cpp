@@ -44,9 +44,8 @@ struct Link {
 struct Plan {
   std::vector<Link> links;
   at::Tensor hold[2];                  // packed router / experts images
-  cudaEvent_t packed = nullptr;        // behind the kernels that wrote them, on `made_on`
-  cudaStream_t made_on = nullptr;
-  std::vector<cudaStream_t> users;     // other streams that have waited for it
+  PyObject* marks[2] = {};             // behind the kernels that wrote them (capsules of a Mark), or null
+  std::vector<cudaStream_t> users;     // other streams that have waited for those
   const void *wa = nullptr, *wb = nullptr, *rp = nullptr;
   const void *w1 = nullptr, *b1 = nullptr, *wup = nullptr, *w2 = nullptr, *ep = nullptr;
   const void* last_bias = nullptr;
@@ -54,7 +53,7 @@ struct Plan {
   at::ScalarType dtype = at::kFloat;
   c10::Device device = c10::Device(c10::kCUDA, 0);
   ~Plan() {
-    if (packed) cudaEventDestroy(packed);
+    for (PyObject* m : marks) Py_XDECREF(m);
     for (Link& l : links) {
       Py_XDECREF(l.dict);
       Py_XDECREF(l.key);
@@ -94,21 +93,78 @@ bool capturing(cudaStream_t s) {
   return st != cudaStreamCaptureStatusNone;
 }
 
-// Before `s` reads the packed images: it comes behind the kernels that wrote them, and the allocator
-// learns that it uses them.  (A capture cannot depend on work outside it; it starts behind that.)
+// The point of a stream behind the kernels that wrote a packed image.
+struct Mark {
+  cudaEvent_t event = nullptr;
+  cudaStream_t stream = nullptr;
+};
+constexpr const char* kMark = "d2dmoe_b200.mark";
+void mark_free(PyObject* cap) {
+  Mark* m = static_cast<Mark*>(PyCapsule_GetPointer(cap, kMark));
+  cudaEventDestroy(m->event);
+  delete m;
+}
+
+// mark(device index) -> Mark of the current stream, or None while it captures (a graph's event means
+// nothing outside it)
+PyObject* mark(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  TORCH_CHECK(n == 1, "mark(device index)");
+  const auto dev = (c10::DeviceIndex)PyLong_AsLong(a[0]);
+  if (PyErr_Occurred()) return nullptr;
+  c10::cuda::CUDAGuard guard(dev);
+  auto m = std::make_unique<Mark>();
+  m->stream = c10::cuda::getCurrentCUDAStream(dev).stream();
+  if (capturing(m->stream)) Py_RETURN_NONE;
+  C10_CUDA_CHECK(cudaEventCreateWithFlags(&m->event, cudaEventDisableTiming));
+  const cudaError_t err = cudaEventRecord(m->event, m->stream);
+  if (err != cudaSuccess) cudaEventDestroy(m->event);
+  C10_CUDA_CHECK(err);
+  return PyCapsule_New(m.release(), kMark, mark_free);
+  END_HANDLE_TH_ERRORS
+}
+
+// Before `s` reads the image: it comes behind the kernels that wrote it, and the allocator learns that
+// `s` uses it.  (A capture cannot depend on work outside it; it starts behind that.)
+void wait_for(const Mark* m, const at::Tensor& image, c10::cuda::CUDAStream s) {
+  if (s.stream() == m->stream) return;
+  C10_CUDA_CHECK(cudaStreamWaitEvent(s.stream(), m->event, 0));
+  c10::cuda::CUDACachingAllocator::recordStream(image.storage().data_ptr(), s);
+}
+
+// wait_mark(mark, image): the current stream may read the image
+PyObject* wait_mark(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  const at::Tensor* t = n == 2 ? tensor_of(a[1]) : nullptr;
+  TORCH_CHECK(t, "wait_mark(mark, image)");
+  const Mark* m = static_cast<const Mark*>(PyCapsule_GetPointer(a[0], kMark));
+  if (!m) return nullptr;
+  c10::cuda::CUDAGuard guard(t->device());
+  const auto s = c10::cuda::getCurrentCUDAStream(t->device().index());
+  if (s.stream() != m->stream && !capturing(s.stream())) wait_for(m, *t, s);
+  Py_RETURN_NONE;
+  END_HANDLE_TH_ERRORS
+}
+
 void use_on(Plan& p, c10::cuda::CUDAStream s) {
-  if (!p.packed || s.stream() == p.made_on) return;
+  const Mark* m[2];
+  bool other = false;
+  for (int i = 0; i < 2; ++i) {
+    m[i] = p.marks[i] ? static_cast<const Mark*>(PyCapsule_GetPointer(p.marks[i], kMark)) : nullptr;
+    other |= m[i] && m[i]->stream != s.stream();
+  }
+  if (!other) return;
   for (cudaStream_t u : p.users)
     if (u == s.stream()) return;
   if (capturing(s.stream())) return;
-  C10_CUDA_CHECK(cudaStreamWaitEvent(s.stream(), p.packed, 0));
-  for (const at::Tensor& t : p.hold)
-    if (t.defined()) c10::cuda::CUDACachingAllocator::recordStream(t.storage().data_ptr(), s);
+  for (int i = 0; i < 2; ++i)
+    if (m[i]) wait_for(m[i], p.hold[i], s);
   if (p.users.size() >= 16) p.users.clear();
   p.users.push_back(s.stream());
 }
 
-// make_plan(links, (wa, wb, router_packed), (w1, b1, w_up, w2, experts_packed), last_bias, act)
+// make_plan(links, (wa, wb, router_packed, mark), (w1, b1, w_up, w2, experts_packed, mark), last_bias,
+//           act, modules, parameters, attributes)
 //   links: sequence of (holder, key); holder = a dict, or 0 / 1 / 2 for the module's own _modules /
 //   _parameters / __dict__, which run_layer receives with every call (the plan does not refer to its
 //   module)
@@ -161,6 +217,7 @@ PyObject* make_plan(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (const at::Tensor* t = tensor_of(PyTuple_GetItem(r, 2))) {
       p->hold[0] = *t;
       p->rp = t->data_ptr();
+      if (PyObject* m = PyTuple_GetItem(r, 3); m && m != Py_None) p->marks[0] = Py_NewRef(m);
     }
   }
   const at::Tensor* w1 = tensor_of(PyTuple_GetItem(e, 0));
@@ -172,6 +229,7 @@ PyObject* make_plan(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (const at::Tensor* t = tensor_of(PyTuple_GetItem(e, 4))) {
     p->hold[1] = *t;
     p->ep = t->data_ptr();
+    if (PyObject* m = PyTuple_GetItem(e, 5); m && m != Py_None) p->marks[1] = Py_NewRef(m);
   }
   p->E = w1->size(0);
   p->d = w1->size(1);
@@ -181,15 +239,6 @@ PyObject* make_plan(PyObject*, PyObject* const* a, Py_ssize_t n) {
   p->last_bias = ptr_of(a[3]);
   p->act = PyLong_AsLong(a[4]);
   if (PyErr_Occurred()) return nullptr;
-  if (p->hold[0].defined() || p->hold[1].defined()) {
-    c10::cuda::CUDAGuard guard(p->device);
-    const cudaStream_t s = c10::cuda::getCurrentCUDAStream(p->device.index()).stream();
-    if (!capturing(s)) {
-      C10_CUDA_CHECK(cudaEventCreateWithFlags(&p->packed, cudaEventDisableTiming));
-      C10_CUDA_CHECK(cudaEventRecord(p->packed, s));
-      p->made_on = s;
-    }
-  }
   return PyCapsule_New(p.release(), kPlan, plan_free);
   END_HANDLE_TH_ERRORS
 }
@@ -476,6 +525,8 @@ PyObject* run_host(PyObject*, PyObject* const* a, Py_ssize_t n) {
 }
 
 PyMethodDef kMethods[] = {
+    {"mark", (PyCFunction)(void (*)(void))mark, METH_FASTCALL, nullptr},
+    {"wait_mark", (PyCFunction)(void (*)(void))wait_mark, METH_FASTCALL, nullptr},
     {"make_pipe", (PyCFunction)(void (*)(void))make_pipe, METH_FASTCALL, nullptr},
     {"run_host", (PyCFunction)(void (*)(void))run_host, METH_FASTCALL, nullptr},
     {"make_plan", (PyCFunction)(void (*)(void))make_plan, METH_FASTCALL, nullptr},

@@ -128,7 +128,7 @@ class _PackedCache:
 
     A stream that did not write the image waits for the one that did."""
 
-    _made = None                  # (stream that wrote the image, event behind it)
+    mark = None                   # of the stream that wrote the image, behind those kernels
 
     def __init__(self):
         self._key = None
@@ -150,15 +150,9 @@ class _PackedCache:
         if key != self._key:
             self._buf = make()
             self._key = key
-            self._made = None
-            if self._buf is not None and not torch.cuda.is_current_stream_capturing():
-                s = torch.cuda.current_stream(self._buf.device)
-                self._made = s, s.record_event()
-        elif self._made is not None:
-            s = torch.cuda.current_stream(self._buf.device)
-            if s != self._made[0] and not torch.cuda.is_current_stream_capturing():
-                s.wait_event(self._made[1])
-                self._buf.record_stream(s)
+            self.mark = None if self._buf is None else host.mark(self._buf.device.index)
+        elif self.mark is not None:
+            host.wait_mark(self.mark, self._buf)
         return self._buf
 
 
@@ -530,35 +524,34 @@ class MoeficationMoE(MoELayer):
         weights = [t for t in (p["w1"], p["b1"], p["w_up"], p["w2"]) if t is not None]
         if self.bias:
             weights.append(self.last_bias)
-
-        def plain(tensors):
-            # A weight that is no parameter (pruned, parametrised, replicated) has no slot a link
-            # could watch, and nothing that keeps its storage: it takes the general path.
-            roots = (self._modules, self._parameters, self.__dict__)
-            slots = {id((roots[h] if isinstance(h, int) else h).get(key)) for h, key in links}
-            return all(t.dtype == p["w1"].dtype and t.device == p["w1"].device
-                       and t.is_contiguous() and id(t) in slots for t in tensors)
-
-        if not plain(weights):
-            return None
         r = None
         if isinstance(router, MoeficationRouter):
             links.append((router.__dict__, "_fusable"))
-        if (isinstance(router, MoeficationRouter) and router.fusable()
-                and type(router).packed is MoeficationRouter.packed):
-            wa, wb = router.layers[0].weight, router.layers[2].weight
-            links.append((router._modules, "layers"))
-            for i in ("0", "2"):
-                links += [(router.layers._modules, i),
-                          (router.layers._modules[i]._parameters, "weight")]
-            if plain((wa, wb)):
-                r = (wa, wb, router.packed())
-                links.append((router._packed.__dict__, "_buf"))  # invalidate_packed() empties the slot
+            if router.fusable() and type(router).packed is MoeficationRouter.packed:
+                layers = router._modules["layers"]._modules
+                links += [(router._modules, "layers"), (layers, "0"), (layers, "2"),
+                          (layers["0"]._parameters, "weight"), (layers["2"]._parameters, "weight")]
+                r = (layers["0"].weight, layers["2"].weight)
+        # A weight that is no parameter (pruned, parametrised, replicated) has no slot a link
+        # could watch, and nothing that keeps its storage: it takes the general path.
+        roots = (self._modules, self._parameters, self.__dict__)
+        slots = {id((roots[h] if type(h) is int else h).get(key)) for h, key in links}
+        dt, dev = p["w1"].dtype, p["w1"].device
+
+        def plain(tensors):
+            return all(id(t) in slots and t.dtype == dt and t.device == dev and t.is_contiguous()
+                       for t in tensors)
+
+        if not plain(weights):
+            return None
+        if r is not None:
+            r = (*r, router.packed(), router._packed.mark) if plain(r) else None
+            links.append((router._packed.__dict__, "_buf"))      # invalidate_packed() empties the slot
         packed = ex.packed()
         links.append((ex._packed.__dict__, "_buf"))
-        return host.make_plan(links, r, (p["w1"], p["b1"], p["w_up"], p["w2"], packed),
-                              self.last_bias if self.bias else None, ACT[p["act"]],
-                              self._modules, self._parameters, self.__dict__)
+        return host.make_plan(links, r, (p["w1"], p["b1"], p["w_up"], p["w2"], packed,
+                                         ex._packed.mark), self.last_bias if self.bias else None,
+                              ACT[p["act"]], self._modules, self._parameters, self.__dict__)
 
     def _run_native(self, x, rule, residual, scores=None, norm=None, capture=None):
         """The layer as one native call -> (out, routing tensor[, norms]), or None when it has
