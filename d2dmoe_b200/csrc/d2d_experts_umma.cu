@@ -749,17 +749,19 @@ __global__ void prepack_experts_kernel(const bf16* __restrict__ w1, const bf16* 
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n1 + n2 + H;
        i += (long long)gridDim.x * blockDim.x) {
     if (i < n1) {
-      // consecutive threads: consecutive hidden columns (the contiguous direction of W1)
-      const int n = (int)(i % rows1);
-      const int k = (int)((i / rows1) % 64);
+      // consecutive threads: consecutive k, the contiguous direction of the image; the strided reads
+      // hit the cache.  (Along W1's own direction a warp's 2-byte stores go to 32 rows of the image:
+      // 24 experts 768 x 128 53 us instead of 37, 128 gated experts 2048 x 128 825 instead of 504.)
+      const int k = (int)(i % 64);
+      const int n = (int)((i / 64) % rows1);
       const int kc = (int)(i / (64LL * rows1));
       const bf16* src = n < H ? w1 : w_up;
       const bf16 v = src[((long long)e * d + kc * 64 + k) * H + (n < H ? n : n - H)];
       *reinterpret_cast<bf16*>(pe + (long long)kc * g.w1_stage + swz(n, k)) = v;
     } else if (i < n1 + n2) {
       const long long q = i - n1;
-      const int n = (int)(q % g.nd);
-      const int k = (int)((q / g.nd) % 64);
+      const int k = (int)(q % 64);
+      const int n = (int)((q / 64) % g.nd);
       const int k2 = (int)((q / (64LL * g.nd)) % g.kc2);
       const int nci = (int)(q / (64LL * g.nd * g.kc2));
       const int kk = k2 * 64 + k;
