@@ -126,7 +126,7 @@ __device__ void short_gather(const ShortParams& p, ShortCtl* c, uint32_t ring, i
       src[i] = v < 0 ? nullptr : p.x + (size_t)v * p.d + j * 8;
     }
     for (int kc = 0; kc < p.g.kc1; ++kc) {
-      if (!mbar_wait_fast(smem_u32(&c->empty[r.s]), r.ph ^ 1, af, p.dev_status)) return;
+      if (!mbar_wait_warp(smem_u32(&c->empty[r.s]), r.ph ^ 1, af, p.dev_status)) return;
       const uint32_t dst = ring + r.s * p.stage + p.wrows * 128 + r8 * 128 + ((j ^ r8) << 4);
 #pragma unroll
       for (int i = 0; i < 4; ++i)
@@ -158,7 +158,7 @@ __device__ void short_weights(const ShortParams& p, ShortCtl* c, uint32_t ring, 
     const uint8_t* w = p.packed + (more ? (long long)find_item(c, p.E, it).e * g.stride : 0);
     for (int kc = 0; more && kc < g.kc1; ++kc) {
       const uint32_t bar = smem_u32(&c->full[r1.s]);
-      if (!mbar_wait_fast(smem_u32(&c->empty[r1.s]), r1.ph ^ 1, af, p.dev_status)) return;
+      if (!mbar_wait_warp(smem_u32(&c->empty[r1.s]), r1.ph ^ 1, af, p.dev_status)) return;
       if (lane == 0) mbar_arrive_expect_tx(bar, p.wrows * 128);
       __syncwarp();
       if (lane < n1 && !withheld)
@@ -170,7 +170,7 @@ __device__ void short_weights(const ShortParams& p, ShortCtl* c, uint32_t ring, 
     for (int s = s0; wprev && s < s1; ++s)
       for (int k2 = 0; k2 < g.kc2; ++k2) {
         const uint32_t bar = smem_u32(&c->full2[r2.s]);
-        if (!mbar_wait_fast(smem_u32(&c->empty2[r2.s]), r2.ph ^ 1, af, p.dev_status)) return;
+        if (!mbar_wait_warp(smem_u32(&c->empty2[r2.s]), r2.ph ^ 1, af, p.dev_status)) return;
         if (lane == 0) mbar_arrive_expect_tx(bar, SLOT);
         __syncwarp();
         if (lane < n2)
@@ -274,7 +274,7 @@ __device__ void short_epilogues(const ShortParams& p, ShortCtl* c, uint32_t hid,
 #pragma unroll
     for (int q = 0; q < 8; ++q) bb[q] = pack_bf16x2(b1, b1);
 
-    if (!mbar_wait_fast(smem_u32(&c->acc1_full[ctx]), ph, af, p.dev_status)) return;
+    if (!mbar_wait_warp(smem_u32(&c->acc1_full[ctx]), ph, af, p.dev_status)) return;
     tc_fence_after();
     uint32_t v[32];
     tmem_ld32(tmem + 32 * ctx + lanes, v);
@@ -285,7 +285,7 @@ __device__ void short_epilogues(const ShortParams& p, ShortCtl* c, uint32_t hid,
     ph ^= ctx;
     ctx ^= 1;
     // the hidden tile of every CTA has been read by its second product of the item before
-    if (!mbar_wait_fast(smem_u32(&c->hid_free), hph ^ 1, af, p.dev_status)) return;
+    if (!mbar_wait_warp(smem_u32(&c->hid_free), hph ^ 1, af, p.dev_status)) return;
     hph ^= 1;
     fence_cluster();
     if (nh > 0) {                        // (warp-uniform; the last warp's lanes may be partly idle)
@@ -344,7 +344,7 @@ __device__ void short_epilogues(const ShortParams& p, ShortCtl* c, uint32_t hid,
       uint4 bz = make_uint4(0u, 0u, 0u, 0u);
       const int col = cw + (lane & 3) * 8;
       if (direct && p.last_bias) bz = __ldg(reinterpret_cast<const uint4*>(p.last_bias + col));
-      if (!mbar_wait_fast(smem_u32(&c->acc2_full[b2.s]), b2.ph, af, p.dev_status)) return;
+      if (!mbar_wait_warp(smem_u32(&c->acc2_full[b2.s]), b2.ph, af, p.dev_status)) return;
       tc_fence_after();
       tmem_ld32(tmem + 64 + 32 * b2.s + lanes, v);
       tmem_wait_ld();

@@ -193,7 +193,7 @@ __device__ void role_list(const Params& p, Ctl* c, int lane, bool one_window) {
     const int tile = u / parts, part = u - tile * parts;
     Tile* t = &c->tile[r.s];
     if (tile >= total) {
-      if (!mbar_wait_fast(smem_u32(&c->tile_empty[r.s]), r.ph ^ 1, af, p.dev_status)) return;
+      if (!mbar_wait_warp(smem_u32(&c->tile_empty[r.s]), r.ph ^ 1, af, p.dev_status)) return;
       if (lane == 0) t->e = -1;
       __syncwarp();
       mbar_arrive(smem_u32(&c->tile_full[r.s]));
@@ -243,7 +243,7 @@ __device__ void role_list(const Params& p, Ctl* c, int lane, bool one_window) {
 #pragma unroll
     for (int g = 0; g < 4; ++g)          // a lane has rows lane + 32 g
       tok[g] = 32 * g + lane < nrows ? p.token_idx[r0 + 32 * g + lane] : 0;
-    if (!mbar_wait_fast(smem_u32(&c->tile_empty[r.s]), r.ph ^ 1, af, p.dev_status)) return;
+    if (!mbar_wait_warp(smem_u32(&c->tile_empty[r.s]), r.ph ^ 1, af, p.dev_status)) return;
     if (lane == 0) {
       t->e = e;
       t->n0 = part * p.g.nc / parts;
@@ -294,7 +294,7 @@ __device__ void role_gather(const Params& p, Ctl* c, uint32_t ring, int w, int l
   }
   RingPos r = {0, 0}, q = {0, 0};
   for (;; q.next(TILE_RING)) {
-    if (!mbar_wait_fast(smem_u32(&c->tile_full[q.s]), q.ph, af, p.dev_status)) return;
+    if (!mbar_wait_warp(smem_u32(&c->tile_full[q.s]), q.ph, af, p.dev_status)) return;
     if (c->tile[q.s].e < 0) return;
     const int* list = c->tile[q.s].list + w * 32;
     const int v0 = list[0];
@@ -308,7 +308,7 @@ __device__ void role_gather(const Params& p, Ctl* c, uint32_t ring, int w, int l
     if (lane == 0) mbar_arrive(smem_u32(&c->tile_empty[q.s]));
     const bool rows = v0 >= 0;           // warp-uniform
     for (int kc = 0; kc < p.g.kc1; ++kc) {
-      if (!mbar_wait_fast(smem_u32(&c->empty[r.s]), r.ph ^ 1, af, p.dev_status)) return;
+      if (!mbar_wait_warp(smem_u32(&c->empty[r.s]), r.ph ^ 1, af, p.dev_status)) return;
       if (rows) {
         const uint32_t base = ring + r.s * p.g.stage;
 #pragma unroll
@@ -475,16 +475,16 @@ __device__ void role_ep1(const Params& p, Ctl* c, uint32_t tmem, int et) {
   RingPos q = {0, 0};
   uint32_t ctx = 0, ph = 0;
   for (;; q.next(TILE_RING)) {
-    if (!mbar_wait_fast(smem_u32(&c->tile_full[q.s]), q.ph, af, p.dev_status)) return;
+    if (!mbar_wait_warp(smem_u32(&c->tile_full[q.s]), q.ph, af, p.dev_status)) return;
     const Tile* t = &c->tile[q.s];
     const int e = t->e;
     if (e < 0) return;
-    if (!mbar_wait_fast(smem_u32(&c->direct_full[q.s]), q.ph, af, p.dev_status)) return;
+    if (!mbar_wait_warp(smem_u32(&c->direct_full[q.s]), q.ph, af, p.dev_status)) return;
     const uint32_t* bp = t->bias;
     // labels by-product (intermediate layer): this thread's row
     float nacc = 0.f;
     const int ntok = NORM ? t->list[et] : -1;
-    if (!mbar_wait_fast(smem_u32(&c->acc1_full[ctx]), ph, af, p.dev_status)) return;
+    if (!mbar_wait_warp(smem_u32(&c->acc1_full[ctx]), ph, af, p.dev_status)) return;
     tc_fence_after();
     const uint32_t acc = tm_tile<GLU>(tmem, ctx) + lane_base;
     for (int c0 = 0; c0 < p.H; c0 += 16) {
@@ -545,11 +545,11 @@ __device__ void role_drain(const Params& p, Ctl* c, uint32_t stg, uint32_t tmem,
   int turn = wide ? j : 0;                           // group whose step is next
   uint32_t nph = 0;
   for (;; q.next(TILE_RING)) {
-    if (!mbar_wait_fast(smem_u32(&c->tile_full[q.s]), q.ph, af, p.dev_status)) return;
+    if (!mbar_wait_warp(smem_u32(&c->tile_full[q.s]), q.ph, af, p.dev_status)) return;
     const Tile* t = &c->tile[q.s];
     const int e = t->e, n0 = t->n0, n1 = t->n1;
     if (e < 0) return;
-    if (!mbar_wait_fast(smem_u32(&c->direct_full[q.s]), q.ph, af, p.dev_status)) return;
+    if (!mbar_wait_warp(smem_u32(&c->direct_full[q.s]), q.ph, af, p.dev_status)) return;
     const uint32_t direct = t->direct[q4];
     int rt[8];
 #pragma unroll
@@ -573,7 +573,7 @@ __device__ void role_drain(const Params& p, Ctl* c, uint32_t stg, uint32_t tmem,
       if (direct != 0u && p.last_bias)
         bz = __ldg(reinterpret_cast<const uint4*>(p.last_bias + col));
       const uint32_t b = ar.slot(ctx);
-      if (!mbar_wait_fast(smem_u32(&c->acc2_full[b]), ar.at(ctx).ph, af, p.dev_status)) return;
+      if (!mbar_wait_warp(smem_u32(&c->acc2_full[b]), ar.at(ctx).ph, af, p.dev_status)) return;
       tc_fence_after();
       uint32_t v[64];
       const uint32_t acc = ar.column(tmem, ctx, g.nd) + src0;
@@ -629,11 +629,11 @@ __device__ void role_drain(const Params& p, Ctl* c, uint32_t stg, uint32_t tmem,
       // the other group saw the other columns of the same rows
       const uint32_t nf = smem_u32(&c->np_full[q4]), ne = smem_u32(&c->np_empty[q4]);
       if (j == 1) {
-        if (!mbar_wait_fast(ne, nph ^ 1, af, p.dev_status)) return;
+        if (!mbar_wait_warp(ne, nph ^ 1, af, p.dev_status)) return;
         c->npart[q4 * 32 + lane] = nacc;
         mbar_arrive(nf);
       } else {
-        if (!mbar_wait_fast(nf, nph, af, p.dev_status)) return;
+        if (!mbar_wait_warp(nf, nph, af, p.dev_status)) return;
         nacc += c->npart[q4 * 32 + lane];
         mbar_arrive(ne);
         if (mine != -1)

@@ -91,7 +91,7 @@ struct Params {
 struct Ctl {
   unsigned long long full[NS_MAX], empty[NS_MAX];
   unsigned long long wb_full, acc1_full[2], acc1_empty[2], hid_full, g2_done, acc2_empty;
-  unsigned long long init_full[2], init_empty[2];
+  unsigned long long init_full[2], init_empty[2], cnt_full;
   uint32_t tmem_base;
   int abort_flag;
   int wait_limit;           // must follow abort_flag (mbar_wait reads abort_flag[1])
@@ -201,9 +201,9 @@ __device__ void role_hidden(const Params& p, Ctl* c, uint32_t tmem, int et) {
   RingPos a = {0, 0};
   uint32_t ph = 0;
   for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ph ^= 1) {
-    if (!mbar_wait_fast(smem_u32(&c->acc1_full[a.s]), a.ph, af, p.dev_status)) return;
+    if (!mbar_wait_warp(smem_u32(&c->acc1_full[a.s]), a.ph, af, p.dev_status)) return;
     // the previous tile's second product has read the hidden tile
-    if (!mbar_wait_fast(smem_u32(&c->g2_done), ph ^ 1, af, p.dev_status)) return;
+    if (!mbar_wait_warp(smem_u32(&c->g2_done), ph ^ 1, af, p.dev_status)) return;
     tc_fence_after();
     const uint32_t src = tmem + lane_base + a.s * 128, dst = tmem + lane_base + TM_HID;
     for (int c0 = 0; c0 < p.R; c0 += 16) {
@@ -253,7 +253,7 @@ __device__ void role_gate(const Params& p, Ctl* c, uint32_t tmem, int et) {
   for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ph ^= 1, buf ^= 1) {
     const long long trow = (long long)tile * TILE_M + et;
     const bool live = trow < p.N;
-    if (!mbar_wait_fast(smem_u32(&c->g2_done), ph, af, p.dev_status)) return;
+    if (!mbar_wait_warp(smem_u32(&c->g2_done), ph, af, p.dev_status)) return;
     tc_fence_after();
     uint32_t s[NB * 8];
 #pragma unroll
@@ -307,7 +307,7 @@ __device__ void role_gate(const Params& p, Ctl* c, uint32_t tmem, int et) {
     if (p.out_init && !p.init_all) {
       const bool todo = live && kept != 1;
       const uint32_t rows = __ballot_sync(0xffffffffu, todo);
-      if (!mbar_wait_fast(smem_u32(&c->init_empty[buf]), ibuf_ph ^ 1, af, p.dev_status)) return;
+      if (!mbar_wait_warp(smem_u32(&c->init_empty[buf]), ibuf_ph ^ 1, af, p.dev_status)) return;
       if (lane == 0) {
         c->init_rows[buf][q4] = rows;
         mbar_arrive(smem_u32(&c->init_full[buf]));
@@ -323,8 +323,11 @@ __device__ void role_gate(const Params& p, Ctl* c, uint32_t tmem, int et) {
 #pragma unroll
       for (int j = 0; j < NW; ++j)
         c->cnt[buf][q4][32 * j + lane] = __popc(transpose32(word[j], lane));
-      // one barrier per tile: the other half of cnt is written before anybody passes it again
-      asm volatile("bar.sync 1, 128;" ::: "memory");
+      // one barrier per tile: the other half of cnt is written before anybody passes it again (an
+      // mbarrier, because a warp that gave up never comes)
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&c->cnt_full));
+      if (!mbar_wait_warp(smem_u32(&c->cnt_full), ph, af, p.dev_status)) return;
       if (et < p.EP) {
         int n = 0;
         if (et < E)
@@ -355,7 +358,7 @@ __device__ void role_init(const Params& p, Ctl* c, int w, int lane) {
       const long long n = left - 32 * q;
       rows = n >= 32 ? 0xffffffffu : n > 0 ? (1u << n) - 1u : 0u;
     } else {
-      if (!mbar_wait_fast(smem_u32(&c->init_full[buf]), ph, af, p.dev_status)) return;
+      if (!mbar_wait_warp(smem_u32(&c->init_full[buf]), ph, af, p.dev_status)) return;
       share = (c->init_rows[buf][1] | c->init_rows[buf][2] | c->init_rows[buf][3]) == 0u;
       q = share ? 0 : w;
       rows = c->init_rows[buf][q];
@@ -418,6 +421,7 @@ router_tiles_kernel(const Params p, const __grid_constant__ CUtensorMap tmx) {
     mbar_init(smem_u32(&c->hid_full), 128);
     mbar_init(smem_u32(&c->g2_done), 1);
     mbar_init(smem_u32(&c->acc2_empty), 128);
+    mbar_init(smem_u32(&c->cnt_full), 4);
     for (int i = 0; i < 2; ++i) {
       mbar_init(smem_u32(&c->acc1_full[i]), 1);
       mbar_init(smem_u32(&c->acc1_empty[i]), 128);
@@ -598,8 +602,7 @@ router_cluster_kernel(const Params p, const __grid_constant__ CUtensorMap tmx) {
     __syncwarp();
   } else if (warp < 4) {
     const uint32_t lb = (uint32_t)(tid & ~31) << 16;
-    bool ok = __all_sync(0xffffffffu,
-                         mbar_wait_fast(smem_u32(&c->acc1_full), 0, af, p.dev_status));
+    bool ok = mbar_wait_warp(smem_u32(&c->acc1_full), 0, af, p.dev_status);
     if (ok) {
       tc_fence_after();
       for (int c0 = 0; c0 < cw; c0 += 16) {
@@ -612,8 +615,7 @@ router_cluster_kernel(const Params p, const __grid_constant__ CUtensorMap tmx) {
       tmem_wait_st();
       tc_fence_before();
       mbar_arrive(smem_u32(&c->hid_full));
-      ok = __all_sync(0xffffffffu,
-                      mbar_wait_fast(smem_u32(&c->acc2_full), 0, af, p.dev_status));
+      ok = mbar_wait_warp(smem_u32(&c->acc2_full), 0, af, p.dev_status);
     }
     if (ok) {                    // (both products are done: the ring is free)
       tc_fence_after();

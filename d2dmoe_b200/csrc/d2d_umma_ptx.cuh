@@ -80,6 +80,27 @@ __device__ __forceinline__ bool mbar_wait_fast(uint32_t bar, uint32_t parity,
   if (mbar_try_wait(bar, parity)) return true;
   return mbar_wait(bar, parity, abort_flag, dev_status);
 }
+// The same for a whole converged warp, which polls, goes on and gives up as one: no lane stands at a
+// warp-wide instruction that another has left behind.
+static __device__ __noinline__ bool mbar_poll_warp(uint32_t bar, uint32_t parity,
+                                                   volatile int* abort_flag, int* dev_status) {
+  const uint32_t limit = (uint32_t)abort_flag[1];
+  for (uint32_t i = 0; i < limit; ++i) {
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    if (i > 64) {
+      __nanosleep(i > 4096 ? 256 : 32);
+      if ((i & 63) == 0 && __any_sync(0xffffffffu, *abort_flag)) return false;
+    }
+  }
+  *abort_flag = 1;
+  report(dev_status, D2D_ERR_TIMEOUT);
+  return false;
+}
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag,
+                                               int* dev_status) {
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  return mbar_poll_warp(bar, parity, abort_flag, dev_status);
+}
 __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t bytes,
                                          uint32_t bar) {
   asm volatile(

@@ -360,3 +360,56 @@ def test_offsets_out_of_range_drop_their_lists(dtype, glu, norms, e, value):
                              t.get("w_up") if glu else None)
     # one rounding per added expert
     assert O.rel_err(out.cpu().float(), ex) <= TOL[dtype]
+
+
+@pytest.mark.parametrize("limit", [8, 12])
+@pytest.mark.parametrize("form,N,d,H,E,R,glu", [
+    ("short", 197, 256, 64, 16, 64, False), ("short", 64, 2048, 128, 32, 64, True),
+    ("short", 500, 128, 32, 9, 64, False), ("long", 2000, 256, 64, 16, 64, False),
+    ("long", 2000, 128, 128, 5, 64, True), ("norms", 700, 256, 64, 6, 64, False),
+    ("router", 2000, 768, 32, 24, 128, False), ("router", 2000, 256, 32, 100, 256, False),
+    ("cluster", 300, 2048, 32, 24, 256, False)])
+def test_every_form_gives_up_and_the_next_call_is_clean(form, N, d, H, E, R, glu, limit):
+    """A slice of weights that never arrives: each role leaves as whole warps, the launch ends and
+    reports, and the same call right afterwards gives what it gave before."""
+    from d2dmoe_b200 import _capi, ops
+    c, t = _layer(N, d, H, E, R, "bf16", N + d, "relu", glu)
+    x2d, wa, wb = _dev(t["x"].reshape(N, d)), _dev(t["wa"]), _dev(t["wb"])
+    w1, b1, w2, wu = (_dev(t.get(k)) for k in ("w1", "b1", "w2", "w_up"))
+    b1 = None if glu else b1
+    wsp = ops.Workspace.allocate(N, E, "cuda")
+    out = torch.empty(N, d, dtype=torch.bfloat16, device="cuda")
+    if form in ("router", "cluster"):
+        packed, lb = ops.prepack_router(wa, wb), _dev(t["last_bias"].reshape(-1))
+
+        def call():
+            ops.router_mask(x2d, wa, wb, 0.3, wsp, packed=packed, out_init=out, last_bias=lb)
+            return wsp.mask_bits[:N].clone(), out.clone()
+    else:
+        m = torch.rand(N, E, generator=_gen(N)) < (0.02 if E > 16 else 0.1)
+        wsp.mask_bits[:N].copy_(torch.from_numpy(O.pack_mask(m).view(np.int32)).cuda())
+        ops.compact(wsp, N, E)
+        packed = ops.prepack_experts(w1, b1, w2, wu)
+        kw = dict(norms=torch.empty(E, N, dtype=torch.bfloat16, device="cuda")) if form == "norms" else {}
+
+        def call():
+            ops.experts_ffn(x2d, wsp, w1, b1, w2, "relu", out, w_up=wu, packed=packed, **kw)
+            return (out.clone(),)
+    ref = call()
+    wsp.check_status()
+    try:
+        assert _capi.lib.d2d_debug_configure(limit, 1) == 0
+        call()
+        torch.cuda.synchronize()                     # returns
+        with pytest.raises(_capi.D2DError, match="TIMEOUT"):
+            wsp.check_status()
+    finally:
+        _capi.lib.d2d_debug_configure(0, 0)
+    out.fill_(float("nan"))
+    got = call()
+    wsp.check_status()
+    for a, b in zip(got, ref):
+        if a.dtype == torch.int32:
+            assert torch.equal(a, b)
+        else:      # the order of the adds is free: one rounding each
+            assert O.rel_err(a.float().cpu(), b.float().cpu()) <= TOL["bf16"]
