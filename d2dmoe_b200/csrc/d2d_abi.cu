@@ -366,8 +366,7 @@ int d2d_moe_forward(const void* x, const void* wa, const void* wb, const void* r
 int d2d_last_forward_launches(void) { return g_last_forward_launches; }
 
 int d2d_debug_select_experts_kernel(int which) {
-  (void)which;
-  return D2D_OK;
+  return which == 0 || which == 1 ? D2D_OK : D2D_ERR_UNSUPPORTED;
 }
 
 int d2d_debug_configure(int wait_limit_log2, int withhold_weight_tile) {

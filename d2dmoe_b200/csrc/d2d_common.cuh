@@ -103,7 +103,7 @@ __device__ __forceinline__ float activate(float h, int act) {
 }
 
 // ---- vector reductions into global memory ---------------------------------
-// fp32: one 16-byte red per 4 values.  bf16: packed pairs, 8 or 16 bytes per red.
+// fp32: one 16-byte red per 4 values.  bf16: packed pairs, 8 bytes per red.
 __device__ __forceinline__ void red_add_v4(float* p, float a, float b, float c, float d) {
   asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c),
                "f"(d)
@@ -118,13 +118,7 @@ __device__ __forceinline__ void red_add_v4(bf16* p, float a, float b, float c, f
   asm volatile("red.global.add.noftz.v2.bf16x2 [%0], {%1, %2};" ::"l"(p), "r"(lo), "r"(hi)
                : "memory");
 }
-__device__ __forceinline__ void red_add_bf16x8(bf16* p, uint32_t a, uint32_t b, uint32_t c,
-                                               uint32_t d) {
-  asm volatile("red.global.add.noftz.v4.bf16x2 [%0], {%1, %2, %3, %4};" ::"l"(p), "r"(a), "r"(b),
-               "r"(c), "r"(d)
-               : "memory");
-}
-// eight bf16 pairs-wise sums, each rounded once
+// eight bf16 sums in pairs, each rounded once
 __device__ __forceinline__ uint4 add_bf16x8(uint4 a, uint4 b) {
   uint4 r;
   const __nv_bfloat162* x = reinterpret_cast<const __nv_bfloat162*>(&a);

@@ -19,16 +19,6 @@ int encode_tmap_2d_b16(CUtensorMap* map, const void* base, uint64_t inner, uint6
 
 #ifdef __CUDACC__
 namespace umma {
-// rows r0..r3 (any four rows of the tensor), box_inner elements from column c0 each, to four
-// consecutive 128-byte rows at dst; completes 4 * box_inner * 2 bytes on the barrier
-__device__ __forceinline__ void tma_gather4(uint32_t dst, const CUtensorMap* map, int c0, int r0,
-                                            int r1, int r2, int r3, uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.tile::gather4.mbarrier::complete_tx::bytes "
-      "[%0], [%1, {%2, %3, %4, %5, %6}], [%7];" ::"r"(dst),
-      "l"(map), "r"(c0), "r"(r0), "r"(r1), "r"(r2), "r"(r3), "r"(bar)
-      : "memory");
-}
 // one box at (column c0, row r0); rows past the tensor's end arrive as zeros
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int c0, int r0,
                                             uint32_t bar) {

@@ -37,9 +37,6 @@ int launch_router_mask_umma(const void* x, const void* packed, float mult, uint3
 // token's scores are one thread's registers, which ranks up to 32 of them
 bool umma_router_ranks(int64_t N, int d, int R, int E);
 
-// test hook: how the expert kernel gathers its token rows: 0/1 = 16-byte cp.async
-// (default), 2 = TMA tile::gather4
-
 // test hooks: poll limit of the bounded device waits (2^log2, out of range = default) and
 // a flag that makes CTA 0 of the next launches skip its first weight tile
 void umma_debug_configure(int wait_limit_log2, int withhold_weight_tile);

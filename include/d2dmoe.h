@@ -277,9 +277,9 @@ int d2d_last_forward_launches(void);
  * d2d_debug_configure(0, 0) to return to normal operation. */
 int d2d_debug_configure(int wait_limit_log2, int withhold_weight_tile);
 
-/* Test hook, no upstream counterpart.  Selected how the bf16 expert kernel gathers token rows;
- * only the 16-byte cp.async form is left (TMA gathers took 101 instead of 61 us on 50432
- * tokens), so every value of which gives that form. */
+/* Test hook, no upstream counterpart: how the bf16 expert kernel gathers token rows.  0 and 1 are the
+ * 16-byte cp.async form, the only one there is (TMA gathers took 101 instead of 61 us on 50432
+ * tokens); any other value returns D2D_ERR_UNSUPPORTED. */
 int d2d_debug_select_experts_kernel(int which);
 
 /* One-time re-layout of the weights into the shared-memory tile images the

@@ -20,16 +20,3 @@ def pytest_collection_modifyitems(config, items):
     for it in items:
         if "gpu" in it.keywords:
             it.add_marker(skip)
-
-
-@pytest.fixture(scope="session", autouse=True)
-def _experts_kernel_choice():
-    """D2D_TEST_EXPERTS_KERNEL=2 runs the whole suite with the bf16 expert kernel gathering
-    its token rows by TMA (tile::gather4) instead of the default 16-byte cp.async, so that
-    every parity case reaches both row paths."""
-    import os
-    which = int(os.environ.get("D2D_TEST_EXPERTS_KERNEL", "0"))
-    if which:
-        from d2dmoe_b200 import _capi
-        _capi.lib.d2d_debug_select_experts_kernel(which)
-    yield

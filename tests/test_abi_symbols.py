@@ -78,6 +78,7 @@ def test_misaligned_buffers_are_rejected_before_any_launch():
                              None, 0, 1, a(base), 256, 768, 24, 128, 0, 1, None, None)
     assert rc == 1
     assert lib.d2d_debug_configure(0, 0) == 0
+    assert [lib.d2d_debug_select_experts_kernel(w) for w in (0, 1, 2)] == [0, 0, 2]   # UNSUPPORTED
 
 
 def test_argument_checks_of_the_block_level_and_label_entry_points():
