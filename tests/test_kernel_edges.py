@@ -124,9 +124,9 @@ def test_short_call_experts(N, d, H, E, act, glu, kind):
 
 
 @pytest.mark.parametrize("E", [8, 24, 128])
-@pytest.mark.parametrize("N", [1, 31, 33, 128, 129, 700, 2048])
+@pytest.mark.parametrize("N", [1, 31, 33, 128, 129, 700, 1920, 1921, 2048])
 def test_large_router(N, E):
-    """Router 2048 -> 256 -> E: split over clusters for short calls (E = 128: up to 2048 tokens)."""
+    """Router 2048 -> 256 -> E: split over clusters for short calls (up to 15 tiles, 1920 tokens)."""
     from d2dmoe_b200 import ops
     d, R, tau = 2048, 256, 0.1
     c, t = _layer(N, d, 128, E, R, "bf16", N + E)
