@@ -239,6 +239,7 @@ int d2d_moe_forward_rule(const void* x, const void* wa, const void* wb,
                            aligned(last_bias_opt, 16) && aligned(router_packed_opt, 1024);
   // where the tensor-core expert kernel follows, the rows of tokens with one expert are left to it
   DirectRows dr;
+  // (the cumulative rule's share is not known here: six)
   dr.kept = rule == D2D_RULE_TOPK ? k : rule == D2D_RULE_ALL ? E : rule == D2D_RULE_DYNK ? 6 : 0;
   bool may_store = !pre && !add_residual && umma_experts && aligned(last_bias_opt, 16);
   auto leave_rows = [&]() {
@@ -264,8 +265,8 @@ int d2d_moe_forward_rule(const void* x, const void* wa, const void* wb,
     nl += 1;
     lists_ready = rt_done = true;
   } else if (ranked && !scores && umma_router && umma_router_ranks(N, d, R, E)) {
-    // router and rule in one launch; every row gets its initial value, before the rule is known:
-    // hardly a token keeps just one expert
+    // router and rule in one launch; every row gets its initial value, before the rule is known
+    // (nearly every token keeps several experts, unless k is 1: then the rows are written twice)
     rc = launch_router_mask_umma(x, router_packed_opt, thresh_mult, mask_bits, scores_scratch,
                                  routing_tensor_opt, last_bias_opt, add_residual ? x : nullptr,
                                  out_init, true, (int32_t*)ws, N, d, R, E, dev_status, s, &lists,
@@ -274,7 +275,7 @@ int d2d_moe_forward_rule(const void* x, const void* wa, const void* wb,
     nl += 1;
   } else if (ranked && !scores) {
     // scores of the fused router for the rule below (its own mask is overwritten there); it also
-    // writes every initial row, at no cost of its own: hardly a token keeps just one expert
+    // writes every initial row, as above
     rc = umma_router
              ? launch_router_mask_umma(x, router_packed_opt, thresh_mult, mask_bits,
                                        scores_scratch, nullptr, last_bias_opt,

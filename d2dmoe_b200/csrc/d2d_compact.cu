@@ -9,9 +9,10 @@
 //   count   : counts[tile][e] = tokens of the 128-token tile that keep expert e, one BYTE
 //             per cell (a tile holds at most 128 tokens), rows padded to EP cells
 //             (skipped when the router kernel already wrote the table)
-//   scatter : one CTA per 256 tokens sweeps the byte table with 16-byte loads (sum over all
-//             tiles = the expert totals, sum over earlier tiles = its own base), scans the
-//             totals over the experts and writes its token indices.
+//   scatter : one CTA per 256 tokens (1024 on long calls) sweeps the byte table with 16-byte loads
+//             (sum over all tiles = the expert totals, sum over earlier tiles = its own base), scans
+//             the totals over the experts and writes its token indices.  Short masks have no
+//             table: every CTA counts the whole mask itself.
 // Every CTA reads the whole table, but at one byte per cell that is 12 KB for a ViT-B/16
 // layer (394 tiles x 32) and 128 KB for 131072 tokens x 128 experts, out of L2.
 // Integer work, bit-exact by construction; HBM traffic is the mask (read twice)

@@ -483,16 +483,18 @@ __global__ void __launch_bounds__(NT, 2) experts_short_kernel(const ShortParams 
 int cluster_of(int H, bool glu) { return H % (glu ? 64 : 32) == 0 ? 4 : 2; }
 
 // Items that a call is taken to have, from what the host knows: every expert's last tile, and the
-// full ones.  kept: experts per token (0: not fixed by the rule).
+// full ones.  kept: experts per token; where the rule does not fix it (0), four, more than a threshold
+// rule keeps in use (1.3 to 2.3 at tau_cfg 0.9), so that the items rather fit than not.
 long long items_of(int64_t N, int E, int kept) {
   const long long pairs = N * (long long)(kept > 0 ? kept : 4);
   return (pairs < E ? pairs : E) + pairs / TN;
 }
 
-// Clusters of four that run at once with two CTAs an SM: 71 of 74 (a cluster's SMs are one GPC's).
-// One that has to wait for a place starts 9 us late, so calls that may have an item for every
-// cluster launch 69; those that do not launch 74, of which the last ones find nothing to do (measured
-// 19.8 instead of 21.0 us per layer on 197 tokens, 24 experts).
+// Up to 70 clusters of four run at once with two CTAs an SM (a cluster's SMs are one GPC's): 128 tokens,
+// 128 gated experts take 54.3 us with 66, 68, 69 or 70 clusters and 58.4 with 71, 72 or 74, where one
+// waits for a place.  Calls that may have an item for every cluster launch 69.  Those that do not launch
+// 74, of which the last ones find nothing to do, whichever waits (197 tokens, 24 experts, us per layer:
+// 19.3 instead of 20.4).
 constexpr int ALL_CLUSTERS = 74, SAFE_CLUSTERS = 69, FEW_ITEMS = 64;
 
 template <bool GLU>
@@ -515,13 +517,17 @@ int launch(const ShortParams& p, int act, bool few, cudaStream_t s) {
 
 }  // namespace
 
-// Which calls.  One round of clusters is faster than the form for long lists (layer, us, before ->
-// now: 197 tokens x 24 experts 23.4 -> 19.8, 394 tokens 26.8 -> 23.9), a second round
-// is not (788 tokens 29.4 -> 31.6; 96 experts x 32, 192 tokens 28.1 -> 28.9): the items have to fit.
+// Which calls.  One round of clusters is faster than the form for long lists, a second round of small
+// experts is not: the items have to fit.  Layer, us, long form -> this one:
+//   24 experts x 128, d 768 (0.4 MB an expert):  32 tokens 21.3 -> 17.8, 256 24.1 -> 19.5
+//   96 of them:                   32 tokens 24.2 -> 20.5, 128 27.8 -> 25.9, 256 30.5 -> 31.1, 512 30.4 -> 31.8
 // Experts of a megabyte and more are bound by their stream, which is read by every CTA that has a
-// share of a list's output there and once here: up to four tokens per expert, however many
-// items (d 2048, 128 gated experts x 128: 32 tokens 42.5 -> 34.1, 64 tokens 53.2 -> 36.4, 128 tokens
-// 67 -> 54, 512 tokens 79 -> 66; 1024 tokens 79 -> 81).
+// share of a list's output there and once here: up to four tokens per expert (two kept each), however
+// many items.  Per layer, 64 experts:
+//   gated 2048 x 128 (1.5 MB):  32 tokens 40.1 -> 31.8, 256 60.2 -> 42.8, 512 62.5 -> 59.1
+//   2048 x 128 (1.0 MB):        32 tokens 32.1 -> 27.3, 256 41.1 -> 33.5, 512 41.1 -> 45.1
+//   below the line, gated 1024 x 128 (0.75 MB): 32 tokens 31.2 -> 24.0, 256 37.0 -> 27.9, 512 39.7 -> 36.2
+// It would pay for smaller experts too: the line is on the safe side.
 bool experts_short_supported(int64_t N, int d, int E, int H, bool glu, int kept) {
   if (N < 1 || N > 512 || d % 128 != 0 || H % 32 != 0 || H > 128) return false;
   if (items_of(N, E, kept) <= ALL_CLUSTERS) return true;

@@ -8,9 +8,7 @@
 // What bounds it: latency, not a unit.  A hand-over from the tensor pipe to a waiting thread
 // (commit, mbarrier, wake-up) takes about 300 cycles and one back to the issuing thread as much
 // again, an M = 128, K = 16 instruction N/2 + 43 cycles with A in shared memory and N/2 + 10 with
-// A in tensor memory.  The previous form (hidden tile in shared memory, two accumulator-2
-// buffers, separate draining and writing warps) ran 21k cycles per tile with no pipe above 30 %.
-// Hence here
+// A in tensor memory; the tensor pipe and DRAM are busy below 30 % of the time.  Hence
 //   * the hidden tile replaces accumulator 1 in place: the second product reads its A operand
 //     from tensor memory, and no shared memory is spent on it (rings of 128 + 48 KB);
 //   * two tiles are in work at once: the first product of one runs while the second product of
@@ -20,7 +18,7 @@
 //     some 300 cycles besides the products, so few and large ones;
 //   * eight warps drain accumulator 2, each 64 columns of its 32 rows and on its own (convert,
 //     transpose through its own 4 KB, add or store whole 128-byte lines), in straight-line
-//     code: with twenty warps in eight different loops instruction fetch is what a branch costs;
+//     code: with twenty warps in eight different loops instruction fetch is what a branch costs
 //     (sixteen warps with 32 columns each: 59.6 instead of 56.5 us on the 50432-token layer);
 //   * the lists are cut into equal tiles of a size that fills the last round of the persistent
 //     grid; where there are fewer tiles than SMs the output columns are split as well;
@@ -51,7 +49,12 @@ constexpr int NTHREADS = 640;
 constexpr int WARP_DRAIN0 = 4, WARP_GATHER0 = 12, WARP_MMA1 = 16, WARP_MMA2 = 17, WARP_W = 18;
 constexpr int TILE_RING = 4;                  // tiles known ahead of the slowest role
 constexpr int TILE_READERS = 4 + 8 + 4 + 1 + 1 + 2;   // warps 0-15, both products, both weight streams
-constexpr long long L2_WEIGHTS = 32 << 20;    // weights up to this size are taken to stay in L2
+// Weights up to this size are taken to stay in L2 beside a window's rows.  Layer, us, windows / one
+// window: up to 48 MB of weights the two are alike on 32768 and 65536 tokens (66.6 / 66.2 with 9 MB,
+// 94.9 / 93.7 with 48) and windows win on 131072 (243.7 / 263.9 with 48 MB); from 96 MB on one window
+// wins (432 / 412 on 131072 tokens, 273 / 248 on 32768 with 192 MB).  Where between 48 and 96 MB they
+// meet has not been measured.
+constexpr long long L2_WEIGHTS = 32 << 20;
 
 struct Params {
   const bf16* x;

@@ -13,7 +13,8 @@
 //   experts  an item is (expert, 32 rows of its list, 32 hidden columns); it adds its share of the
 //            second product to the output rows.  In fp32 nothing is rounded between the
 //            slices, so no exchange is needed; the price is one add of the output rows per slice.
-// Measured (1576 tokens x 768, 24 experts x 128, router 128): see the launch rule below.
+// Measured (1576 tokens x 768, 24 experts x 128, router 128): router 23.7, experts 52.9 us, the layer 78.5
+// as a graph replay; with the general-shape kernels 34.2, 80.5 and 115.
 #include <cooperative_groups.h>
 
 #include "d2d_common.cuh"

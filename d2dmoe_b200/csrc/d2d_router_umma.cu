@@ -15,10 +15,8 @@
 //
 // Bound: HBM.  A layer reads x once; the initial rows are written only for tokens whose row
 // the expert kernel has to ADD to (more than one expert, or none): a token kept by exactly
-// one expert gets its row from that expert's store.  Compared with the form that shared its
-// tile loop with the expert kernel (hidden tile in shared memory, separate rings for x and Wa,
-// Wb streamed per tile, eight warps each doing both epilogues, every initial row written by the
-// TMA unit in front of the loads) the second epilogue no longer sits between two tiles.
+// one expert gets its row from that expert's store.  The two epilogues are different warps, so
+// that the second one does not sit between two tiles.
 #include <cooperative_groups.h>
 
 #include "d2d_cluster_compact.cuh"
@@ -802,10 +800,10 @@ bool umma_router_splits(int64_t N, int d, int R, int E) {
          compact_counts_itself(N, E);
 }
 
-// The ranked rules without a launch of their own (before -> now, per layer:
-// 12608 tokens x 24 experts, topk 2: 42.9 -> 40.4 us; 25216 tokens, topk 4: 90.3 -> 83.5; 197
-// tokens, topk 1: 22.0 -> 20.3).  Beyond 32 scores a thread's registers would not hold them
-// beside their shares.
+// The ranked rules without a launch of their own (layer of 24 experts x 128, us, own launch -> in the
+// router): 197 tokens, topk 1 21.8 -> 20.6; 12608 tokens, topk 2 47.2 -> 45.3, topk 8 88.8 -> 83.2,
+// dynk 71.1 -> 69.2; 25216 tokens, topk 4 92.6 -> 88.4.  Beyond 32 scores a thread's registers would
+// not hold them beside their shares.
 bool umma_router_ranks(int64_t N, int d, int R, int E) {
   return E <= 32 && !umma_router_splits(N, d, R, E);
 }

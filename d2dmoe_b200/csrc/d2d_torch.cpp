@@ -1,8 +1,8 @@
 // Native host path of the module forwards: one call from Python per layer call.
 //
-// A layer call launches three or four kernels that take 20 to 100 us together; preparing it in
-// Python (attribute walks, argument checks, thirty ctypes conversions) took 55 to 60 us, so every
-// call below about 10k tokens was bound by the host.  Here the facts that do not change between
+// A layer call launches two to four kernels that take 20 to 100 us together; prepared in Python
+// (attribute walks, argument checks, thirty ctypes conversions: 55 to 60 us) every call below about
+// 10k tokens would be bound by the host.  Here the facts that do not change between
 // calls (weight addresses, shapes, packed copies) are kept in a plan, and a call only checks that
 // the plan still describes the module, allocates the outputs and enters the C ABI.
 //
@@ -279,7 +279,8 @@ bool buffers_of(PyObject* cache, const Plan& p, int64_t N, Buffers* b, PyObject*
   return ok;
 }
 
-// run_layer(plan, modules, parameters, attributes, workspaces, x, rule, k, tau, residual, scores, norm, capture)
+// run_layer(plan, modules, parameters, attributes, workspaces, x, rule, k, tau, residual, scores, norm,
+//           capture)
 //   -> (out, routing[, norms]) | status code (int) | None: the plan is stale | False: it is as the module
 //   is, but this call takes the general path
 // rule: D2D_RULE_*; k / tau as that rule reads them (MAX: threshold 1 - tau).
@@ -426,10 +427,11 @@ PyObject* make_pipe(PyObject*, PyObject* const* a, Py_ssize_t n) {
 }
 
 // run_host(plan, modules, parameters, attributes, workspaces, pipe, x_host, out_host,
-//          staging (kIn + kOut tensors), (stream in, stream run, stream out), slices, rule, k, tau, residual, sync)
+//          staging (kIn + kOut tensors), (stream in, stream run, stream out), slices, rule, k, tau,
+//          residual, sync)
 //   -> True | status code (int) | None / False as run_layer
-// Slice i's copy in, the kernels of slice i - 1 and the copy out of slice i - 2 overlap.  The same
-// pipeline issued from Python took 70 us of host time per slice, more than a slice's copies.
+// Slice i's copy in, the kernels of slice i - 1 and the copy out of slice i - 2 overlap.  (Issued from
+// Python it takes 70 us of host time per slice, more than a slice's copies.)
 PyObject* run_host(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   TORCH_CHECK(n == 16, "run_host takes 16 arguments");

@@ -433,9 +433,9 @@ class MoeficationMoE(MoELayer):
 
     ``forward(x[B,S,d]) -> (out[B,S,d], {name: (routing_tensor[B,S,E],)})`` with
     ``forward_mode`` in {'all','topk','dynk','dynk_max'}, ``tau``/``k`` read at call
-    time.  In 'dynk_max' mode with a D2DMoE router the whole layer is one library call
-    (router + rule -> bit mask -> token lists -> expert FFN with scatter-add); other
-    modes compute the routing tensor with device tensor ops and share the rest.
+    time.  In every mode the whole layer is one native call (router + rule -> bit mask ->
+    token lists -> expert FFN with scatter-add); a router that is not the D2DMoE form runs as
+    the module it is and hands over its scores.
     ``tau`` keeps the upstream meaning: expert e runs iff score_e >= max_e(score)*(1.0-tau).
     """
 
@@ -473,10 +473,11 @@ class MoeficationMoE(MoELayer):
         # modules saved whole before these attributes existed
         super().__setstate__({"_plan": _Plan(), "_host": _HostBuffers(), **state})
 
-    # -- routing for the modes that are not fused ---------------------------------
+    # -- routing alone ------------------------------------------------------------
     def gate(self, x):
-        """Routing tensor [B,S,E] of 0/1 in the router's dtype for the non-fused modes
-        (architectures/moe/moefication.py:54-88), on the device."""
+        """Routing tensor [B,S,E] of 0/1 in the router's dtype
+        (architectures/moe/moefication.py:54-88), on the device: the router as a module, then
+        the rule's kernel."""
         if self.forward_mode == "all":
             return torch.ones(x.size(0), x.size(1), self.num_experts, dtype=x.dtype,
                               device=x.device)
