@@ -786,17 +786,19 @@ int launch_prepack_router(const void* wa, const void* wb, void* packed, int d, i
   return cudaGetLastError() == cudaSuccess ? D2D_OK : D2D_ERR_LAUNCH;
 }
 
-// The cluster form: one cluster of eight per tile, as many tiles as clusters run at once (15: the SMs
-// of a cluster are one GPC's; a sixteenth waits for the first to end), and a Wa worth splitting; it
-// writes no counts table, so the mask has to be short enough for the scatter kernel to count itself.
-// Layer of 24 experts x 32, us, one CTA per tile -> cluster:
+// The cluster form: one cluster of eight per tile, and a Wa worth splitting; it writes no counts table,
+// so the mask has to be short enough for the scatter kernel to count itself.  Fifteen clusters run at
+// once (the SMs of a cluster are one GPC's); a sixteenth waits for one to end, which only the largest
+// Wa still pay for.  Layer of 24 experts x 32, us, one CTA per tile -> cluster:
 //   2048 x 256 (512 K values):    32 tokens 30.5 -> 25.6, 1024 46.2 -> 37.4, 1800 54.4 -> 44.8, 2048 54.8 -> 55.1
+//                                 (128 gated experts x 128, 2048 tokens: 121 -> 116)
 //   2048 x 128 / 1024 x 256 (256 K): 32 tokens 25.8 -> 25.4 / 20.8 -> 18.1, 1024 41.6 -> 37.0 / 30.7 -> 26.8,
-//                                    2048 50.3 -> 55.0 / 35.4 -> 38.1
+//                                    2048 50.3 -> 55.0 / 35.4 -> 38.1; 1536 x 256 with 2048 45.0 -> 46.5
 //   below the line: 768 x 256 (192 K) 32 tokens 18.8 -> 16.7, 1024 26.4 -> 23.9; 768 x 128 (96 K) 18.9 -> 19.0
 //   with 197, 24.2 -> 23.6 with 1024.  It would pay from about 128 K on.
 bool umma_router_splits(int64_t N, int d, int R, int E) {
-  return N <= 15 * TILE_M && (int64_t)d * R >= 256 * 1024 && R % (16 * CL) == 0 &&
+  const int64_t wa = (int64_t)d * R;
+  return wa >= 256 * 1024 && N <= (wa >= 512 * 1024 ? 16 : 15) * TILE_M && R % (16 * CL) == 0 &&
          compact_counts_itself(N, E);
 }
 

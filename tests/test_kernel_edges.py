@@ -124,11 +124,12 @@ def test_short_call_experts(N, d, H, E, act, glu, kind):
 
 
 @pytest.mark.parametrize("E", [8, 24, 128])
-@pytest.mark.parametrize("N", [1, 31, 33, 128, 129, 700, 1920, 1921, 2048])
-def test_large_router(N, E):
-    """Router 2048 -> 256 -> E: split over clusters for short calls (up to 15 tiles, 1920 tokens)."""
+@pytest.mark.parametrize("N,d", [(n, 2048) for n in (1, 31, 33, 128, 129, 700, 1921, 2048, 2049)] +
+                         [(1920, 1024), (1921, 1024)])
+def test_large_router(N, d, E):
+    """Router d -> 256 -> E: split over clusters for short calls (up to 16 tiles, d < 2048 up to 15)."""
     from d2dmoe_b200 import ops
-    d, R, tau = 2048, 256, 0.1
+    R, tau = 256, 0.1
     c, t = _layer(N, d, 128, E, R, "bf16", N + E)
     x2d, wa, wb = _dev(t["x"].reshape(N, d)), _dev(t["wa"]), _dev(t["wb"])
     lb = _dev(t["last_bias"].reshape(-1))
