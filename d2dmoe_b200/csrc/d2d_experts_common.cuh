@@ -9,8 +9,7 @@ namespace umma {
 
 constexpr int MAX_E = 128;
 constexpr int NS_MAX = 8, NS2_MAX = 8;        // stages of the two rings (upper bounds)
-constexpr int STG = 8 * 4096;                 // transposition blocks of the drain warps
-constexpr int SMEM_TILES = 220 * 1024;        // both rings + STG
+constexpr int SMEM_TILES = 220 * 1024;        // both rings
 
 struct Geo {
   int kc1;         // d / 64
@@ -38,10 +37,10 @@ inline Geo experts_geo(int d, int H, bool glu, long long n) {
   g.a_slot = n <= 32 ? SLOT / 4 : n <= 64 ? SLOT / 2 : SLOT;
   g.stage = g.a_slot + g.w1_stage;
   g.w2_piece = g.nd * 128;
-  // at least three W2 pieces, then as many stages of the first ring as fit, the rest for W2
-  const int ns = (SMEM_TILES - STG - 3 * g.w2_piece) / g.stage;
+  // 48 KB of W2 pieces, then as many stages of the first ring as fit, the rest for W2
+  const int ns = (SMEM_TILES - 48 * 1024) / g.stage;
   g.ns = ns < NS_MAX ? ns : NS_MAX;
-  const int ns2 = (SMEM_TILES - STG - g.ns * g.stage) / g.w2_piece;
+  const int ns2 = (SMEM_TILES - g.ns * g.stage) / g.w2_piece;
   g.ns2 = ns2 < NS2_MAX ? ns2 : NS2_MAX;
   g.w1_bytes = (long long)g.kc1 * g.w1_stage;
   g.bias_off = g.w1_bytes + (long long)g.nc * g.kc2 * g.w2_piece;
@@ -81,8 +80,15 @@ __device__ __forceinline__ void ep1_pairs(const uint32_t* v, const uint32_t* u, 
   }
 }
 
+// Row n of a packed W2 piece holds this output column of the piece: in each block of 32 the two 2-bit
+// fields above the lowest bit change places, so that column 8 f + 2 l + i of the accumulator, which
+// the fragment loads give to lane l of a row, is output column 8 l + 2 f + i.
+__host__ __device__ __forceinline__ int out_column(int n) {
+  return (n & ~30) | ((n & 6) << 2) | ((n >> 2) & 6);
+}
+
 // t >= 0: add; t < -1: store; -1: nothing (predicated, no branch)
-__device__ __forceinline__ void put_row(bf16* p, int t, uint4 add, uint4 st) {
+__device__ __forceinline__ void put_row(void* p, int t, uint4 add, uint4 st) {
   asm volatile(
       "{\n\t.reg .pred a, b;\n\t"
       "setp.ge.s32 a, %1, 0;\n\t"
@@ -91,6 +97,16 @@ __device__ __forceinline__ void put_row(bf16* p, int t, uint4 add, uint4 st) {
       "@b st.global.v4.b32 [%0], {%6, %7, %8, %9};\n\t}" ::"l"(p),
       "r"(t), "r"(add.x), "r"(add.y), "r"(add.z), "r"(add.w), "r"(st.x), "r"(st.y), "r"(st.z),
       "r"(st.w)
+      : "memory");
+}
+
+// t >= 0: add
+__device__ __forceinline__ void add_row(void* p, int t, uint4 v) {
+  asm volatile(
+      "{\n\t.reg .pred a;\n\t"
+      "setp.ge.s32 a, %1, 0;\n\t"
+      "@a red.global.add.noftz.v4.bf16x2 [%0], {%2, %3, %4, %5};\n\t}" ::"l"(p),
+      "r"(t), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w)
       : "memory");
 }
 

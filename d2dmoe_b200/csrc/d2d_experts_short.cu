@@ -354,7 +354,7 @@ __device__ void short_epilogues(const ShortParams& p, ShortCtl* c, uint32_t hid,
       b2.next(NACC2);
 #pragma unroll
       for (int t = 0; t < 32; ++t)
-        asm volatile("st.shared.b16 [%0], %1;" ::"r"(blk + t * 64 + lane * 2),
+        asm volatile("st.shared.b16 [%0], %1;" ::"r"(blk + t * 64 + out_column(lane) * 2),
                      "h"((uint16_t)pack_bf16x2(__uint_as_float(v[t]), 0.f))
                      : "memory");
       __syncwarp();

@@ -16,10 +16,8 @@
 //   * the second product works in steps of 128 output columns (64 where d or the tensor memory
 //     does not allow it) over two or more accumulator-2 buffers: a step costs its issuing thread
 //     some 300 cycles besides the products, so few and large ones;
-//   * eight warps drain accumulator 2, each 64 columns of its 32 rows and on its own (convert,
-//     transpose through its own 4 KB, add or store whole 128-byte lines), in straight-line
-//     code: with twenty warps in eight different loops instruction fetch is what a branch costs
-//     (sixteen warps with 32 columns each: 59.6 instead of 56.5 us on the 50432-token layer);
+//   * eight warps drain accumulator 2, each 64 columns of its 32 rows and on its own, from
+//     registers to whole 128-byte lines of the output;
 //   * the lists are cut into equal tiles of a size that fills the last round of the persistent
 //     grid; where there are fewer tiles than SMs the output columns are split as well;
 //   * where the weights of all experts stay in L2, the tiles are taken window by window of the
@@ -526,21 +524,71 @@ __device__ __forceinline__ void role_ep1_act(const Params& p, Ctl* c, uint32_t t
   }
 }
 
+// 16 rows x 64 columns of fragments as bf16 pairs: w[row rl or rl + 8][block of 32 columns][4 pairs]
+template <bool NORM>
+__device__ __forceinline__ void frag_pairs(const uint32_t* v, uint32_t (&w)[2][2][4], float* nacc, int nord) {
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+#pragma unroll
+      for (int h = 0; h < 4; ++h) {
+        const uint32_t* f = v + 16 * k + 4 * h + 2 * i;
+        w[i][k][h] = pack_bf16x2(__uint_as_float(f[0]), __uint_as_float(f[1]));
+        if (NORM) {
+          const float lo = __uint_as_float(w[i][k][h] << 16),
+                      hi = __uint_as_float(w[i][k][h] & 0xffff0000u);
+          nacc[i] += nord == 1 ? fabsf(lo) + fabsf(hi) : fmaf(lo, lo, hi * hi);
+        }
+      }
+}
+
+// The lanes of an even row give its second block for the first one of the next row: eight lanes have a
+// row's 128 bytes (even rows' lanes the first block's).  All exchanges come before the first write.
+template <bool DIRECT>
+__device__ __forceinline__ void put_rows(uint32_t (&w)[2][2][4], const int* rt, uint8_t* o,
+                                         uint32_t row_bytes, uint4 bz, int odd) {
+  uint32_t got[2][4];
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int h = 0; h < 4; ++h)
+      got[i][h] = __shfl_xor_sync(0xffffffffu, odd ? w[i][0][h] : w[i][1][h], 4);
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {        // k = 0: the even row
+      uint32_t x[4];
+#pragma unroll
+      for (int h = 0; h < 4; ++h) x[h] = odd == k ? w[i][k][h] : got[i][h];
+      const uint4 val = make_uint4(x[0], x[1], x[2], x[3]);
+      const int r = rt[2 * i + k];
+      uint8_t* const row = o + (uint64_t)((uint32_t)r & 0x7fffffffu) * row_bytes;
+      if (DIRECT) put_row(row, r, val, add_bf16x8(bz, val));
+      else add_row(row, r, val);
+    }
+}
+
 // Warps 4-11: warp q4 of group j has rows 32 q4 .. +31 and 64 columns: with 128-column steps the two
 // groups share each one, with 64-column steps they take every other one.
-// Thread = row out of tensor memory; through the warp's own 4 KB the 64 columns are turned into
-// 8 lanes per row, so that one instruction covers 4 whole 128-byte lines of the output.
-template <bool GLU, bool NORM>
-__device__ void role_drain(const Params& p, Ctl* c, uint32_t stg, uint32_t tmem, int j, int q4,
-                           int lane) {
+// The loads take the accumulator as fragments of 8 rows x 8 columns (four lanes a row, two columns
+// each); W2's columns are packed in the order (out_column) that gives a lane eight neighbouring
+// ones of each 32-column block, and the lanes of two rows trade a block, so that eight of them have
+// 128 bytes of one row: whole lines leave an SM at 25 bytes per clock where they are added, half lines at
+// 20 (stored: 32 and 29; 148 CTAs, rows of 1536 bytes).  A transposition through shared memory took
+// 1250 cycles a step with nothing written, this 730 (950 where rows are stored as well).
+// What bounds a tile of the two-layer form is now the way between SM and L2: 128 rows added, gathered
+// and 384 KB of weights take 8.3, 2.8 and 5.5 thousand cycles alone and 12.9 together.
+// DIRECT: rows of tokens with one expert are stored, see DirectRows
+template <bool GLU, bool NORM, bool DIRECT>
+__device__ void role_drain(const Params& p, Ctl* c, uint32_t tmem, int j, int q4, int lane) {
   volatile int* af = &c->abort_flag;
   const Geo& g = p.g;
-  const uint32_t blk = stg + (j * 4 + q4) * 4096;
-  const uint32_t wr = blk + lane * 128, x7 = lane & 7;
-  const int rl = lane >> 3, pl = lane & 7;
+  const int rl = lane >> 2, ql = lane & 3, odd = rl & 1;
   const int nord = p.norm_ord;
   const bool wide = g.nd == 128;
   const int col0 = wide ? 64 * j : 0;                // my columns of a step
+  const uint32_t row_bytes = 2 * (uint32_t)p.d;
   const uint32_t src0 = ((uint32_t)(q4 * 32) << 16) + col0;
   Acc2Ring<GLU> ar;
   RingPos q = {0, 0};
@@ -553,17 +601,17 @@ __device__ void role_drain(const Params& p, Ctl* c, uint32_t stg, uint32_t tmem,
     const int e = t->e, n0 = t->n0, n1 = t->n1;
     if (e < 0) return;
     if (!mbar_wait_warp(smem_u32(&c->direct_full[q.s]), q.ph, af, p.dev_status)) return;
-    const uint32_t direct = t->direct[q4];
-    int rt[8];
+    const uint32_t direct = DIRECT ? t->direct[q4] : 0u;
+    int rt[8];                           // rows 8 (i / 2) + (rl & ~1) + i % 2; sign bit: stored
 #pragma unroll
-    for (int it = 0; it < 8; ++it) {     // sign bit: the row is stored
-      const uint32_t v = (uint32_t)t->list[q4 * 32 + it * 4 + rl];
-      rt[it] = (int)(v | (((direct >> (it * 4 + rl)) & 1u) << 31));
+    for (int i = 0; i < 8; ++i) {
+      const int r = 8 * (i >> 1) + (rl & 6) + (i & 1);
+      rt[i] = (int)((uint32_t)t->list[q4 * 32 + r] | (((direct >> r) & 1u) << 31));
     }
-    const int mine = NORM ? t->list[q4 * 32 + lane] : -1;
+    const int mine = NORM ? t->list[q4 * 32 + 8 * ql + rl] : -1;
     __syncwarp();
     if (lane == 0) mbar_arrive(smem_u32(&c->tile_empty[q.s]));
-    float nacc = 0.f;
+    float nacc[4] = {0.f, 0.f, 0.f, 0.f};
     for (int n = n0; n < n1; ++n) {
       const bool skip = turn != j;
       if (!wide) turn ^= 1;
@@ -571,57 +619,30 @@ __device__ void role_drain(const Params& p, Ctl* c, uint32_t stg, uint32_t tmem,
         ar.next(ctx, g.nd);
         continue;
       }
-      const int col = n * g.nd + col0 + pl * 8;
+      const int col = n * g.nd + col0 + 32 * odd + 8 * ql;
+      uint8_t* const o = reinterpret_cast<uint8_t*>(p.out + col);
       uint4 bz = make_uint4(0u, 0u, 0u, 0u);
-      if (direct != 0u && p.last_bias)
+      if (DIRECT && p.last_bias)
         bz = __ldg(reinterpret_cast<const uint4*>(p.last_bias + col));
       const uint32_t b = ar.slot(ctx);
       if (!mbar_wait_warp(smem_u32(&c->acc2_full[b]), ar.at(ctx).ph, af, p.dev_status)) return;
       tc_fence_after();
-      uint32_t v[64];
       const uint32_t acc = ar.column(tmem, ctx, g.nd) + src0;
-      tmem_ld32(acc, v);
-      tmem_ld32(acc + 32, v + 32);
-      tmem_wait_ld();
+      ar.next(ctx, g.nd);
+      // 16 rows at a time (64 values more would spill): the second half's load runs while the first
+      // half is written out
+      uint32_t v[32], w[2][2][4];
+      tmem_ld_frag64(acc, v);
+      tmem_wait_ld32(v);
+      frag_pairs<NORM>(v, w, nacc, nord);
+      tmem_ld_frag64(acc + (16u << 16), v);
+      put_rows<DIRECT>(w, rt, o, row_bytes, bz, odd);
+      tmem_wait_ld32(v);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&c->acc2_empty[b]));
-      ar.next(ctx, g.nd);
-#pragma unroll
-      for (int pc = 0; pc < 8; ++pc) {      // piece XOR row: conflict-free 16-byte stores
-        uint32_t ww[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-          ww[k] = pack_bf16x2(__uint_as_float(v[8 * pc + 2 * k]),
-                              __uint_as_float(v[8 * pc + 2 * k + 1]));
-        st_shared_v4(wr + ((pc ^ x7) << 4), ww[0], ww[1], ww[2], ww[3]);
-        if (NORM) {
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            const float lo = __uint_as_float(ww[k] << 16), hi = __uint_as_float(ww[k] & 0xffff0000u);
-            nacc += nord == 1 ? fabsf(lo) + fabsf(hi) : fmaf(lo, lo, hi * hi);
-          }
-        }
-      }
-      __syncwarp();
-      uint4 val[8];
-#pragma unroll
-      for (int it = 0; it < 8; ++it) {
-        const int rr = it * 4 + rl;
-        val[it] = ld_shared_v4(blk + rr * 128 + ((pl ^ (rr & 7)) << 4));
-      }
-      __syncwarp();
-      bf16* o = p.out + col;
-      if (direct != 0u) {
-#pragma unroll
-        for (int it = 0; it < 8; ++it)
-          put_row(o + (size_t)(rt[it] & 0x7fffffff) * p.d, rt[it], val[it],
-                  add_bf16x8(bz, val[it]));
-      } else {
-#pragma unroll
-        for (int it = 0; it < 8; ++it)
-          put_row(o + (size_t)(rt[it] & 0x7fffffff) * p.d, rt[it], val[it], val[it]);
-      }
+      frag_pairs<NORM>(v, w, nacc + 2, nord);
+      put_rows<DIRECT>(w, rt + 4, o, row_bytes, bz, odd);
     }
     // every read of this tile's tensor memory by this warp is done
     if (GLU) {
@@ -629,19 +650,26 @@ __device__ void role_drain(const Params& p, Ctl* c, uint32_t stg, uint32_t tmem,
       if (lane == 0) mbar_arrive(smem_u32(&c->ctx_free[ctx]));
     }
     if (NORM) {
-      // the other group saw the other columns of the same rows
+      // a row's four lanes, then the other group, which saw the other columns: lane = row 8 ql + rl
+      float sum = 0.f;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        nacc[i] += __shfl_xor_sync(0xffffffffu, nacc[i], 1);
+        nacc[i] += __shfl_xor_sync(0xffffffffu, nacc[i], 2);
+        if (ql == i) sum = nacc[i];
+      }
       const uint32_t nf = smem_u32(&c->np_full[q4]), ne = smem_u32(&c->np_empty[q4]);
       if (j == 1) {
         if (!mbar_wait_warp(ne, nph ^ 1, af, p.dev_status)) return;
-        c->npart[q4 * 32 + lane] = nacc;
+        c->npart[q4 * 32 + lane] = sum;
         mbar_arrive(nf);
       } else {
         if (!mbar_wait_warp(nf, nph, af, p.dev_status)) return;
-        nacc += c->npart[q4 * 32 + lane];
+        sum += c->npart[q4 * 32 + lane];
         mbar_arrive(ne);
         if (mine != -1)
           p.norms[(long long)e * p.N + mine] =
-              __float2bfloat16_rn(nord == 1 ? nacc : sqrtf(nacc));
+              __float2bfloat16_rn(nord == 1 ? sum : sqrtf(sum));
       }
       nph ^= 1;
     }
@@ -659,8 +687,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) experts_tiles_kernel(const Params
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t ring = (raw + 1023u) & ~1023u;
   const uint32_t ring2 = ring + p.g.ns * p.g.stage;
-  const uint32_t stg = ring2 + p.g.ns2 * p.g.w2_piece;
-  Ctl* c = reinterpret_cast<Ctl*>(smem_raw + (stg - raw) + STG);
+  Ctl* c = reinterpret_cast<Ctl*>(smem_raw + (ring2 - raw) + p.g.ns2 * p.g.w2_piece);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // Programmatic dependent launch: see router_tiles_kernel.
   grid_launch_dependents();
@@ -707,7 +734,10 @@ __global__ void __launch_bounds__(NTHREADS, 1) experts_tiles_kernel(const Params
     role_ep1_act<GLU, NORM == D2D_NORM_OF_INTERMEDIATE>(p, c, tmem, tid);
   } else if (warp < WARP_GATHER0) {
     const int w = warp - WARP_DRAIN0;
-    role_drain<GLU, NORM == D2D_NORM_OF_OUTPUT>(p, c, stg, tmem, w >> 2, w & 3, lane);
+    if (NORM != D2D_NORM_OF_OUTPUT && p.mask_bits)
+      role_drain<GLU, false, true>(p, c, tmem, w >> 2, w & 3, lane);
+    else
+      role_drain<GLU, NORM == D2D_NORM_OF_OUTPUT, false>(p, c, tmem, w >> 2, w & 3, lane);
   } else if (warp < WARP_MMA1) {
     role_gather(p, c, ring, warp - WARP_GATHER0, lane);
     cp_async_wait_all();
@@ -768,7 +798,7 @@ __global__ void prepack_experts_kernel(const bf16* __restrict__ w1, const bf16* 
       const int k2 = (int)((q / (64LL * g.nd)) % g.kc2);
       const int nci = (int)(q / (64LL * g.nd * g.kc2));
       const int kk = k2 * 64 + k;
-      const bf16 v = kk < H ? w2[((long long)e * H + kk) * d + nci * g.nd + n] : zero;
+      const bf16 v = kk < H ? w2[((long long)e * H + kk) * d + nci * g.nd + out_column(n)] : zero;
       *reinterpret_cast<bf16*>(pe + g.w1_bytes + (long long)(nci * g.kc2 + k2) * g.w2_piece +
                                swz(n, k)) = v;
     } else {
@@ -836,7 +866,7 @@ int launch_experts_umma(const void* x, const int32_t* token_idx, const int32_t* 
   p.norm_ord = nc.ord;
   umma_debug_read(&p.wait_limit, &p.withhold);
   const size_t smem =
-      1024 + (size_t)p.g.ns * p.g.stage + (size_t)p.g.ns2 * p.g.w2_piece + STG + sizeof(Ctl) + 64;
+      1024 + (size_t)p.g.ns * p.g.stage + (size_t)p.g.ns2 * p.g.w2_piece + sizeof(Ctl) + 64;
   auto kernel = glu ? (p.norm_layer == 0                          ? experts_tiles_kernel<true, 0>
                        : p.norm_layer == D2D_NORM_OF_INTERMEDIATE ? experts_tiles_kernel<true, 1>
                                                                   : experts_tiles_kernel<true, 2>)
