@@ -41,7 +41,9 @@ const char* d2d_strerror(int status) {
 
 int d2d_workspace_bytes(int64_t n_max, int E, size_t* bytes) {
   if (!bytes || n_max < 0 || E < 1) return D2D_ERR_BAD_ARG;
-  *bytes = align_up(compact_workspace_bytes(n_max, E), 256);
+  const size_t counts = compact_workspace_bytes(n_max, E);
+  const size_t table = E <= 128 ? mask_table_bytes(n_max, E) : 0;     // (the tensor-core kernels' limit)
+  *bytes = align_up(counts > table ? counts : table, 256);
   return D2D_OK;
 }
 
@@ -156,8 +158,9 @@ static int experts_ffn_impl(const void* x, const int32_t* token_idx, const int32
   }
   if (experts_packed_opt && umma_experts_supported(d, E, H, w_up_opt != nullptr, dtype) &&
       aligned(experts_packed_opt, 1024))
-    return launch_experts_umma(x, token_idx, offsets, experts_packed_opt, out, N, d, E, H,
-                               w_up_opt != nullptr, act, dev_status, s, nc);
+    return launch_experts_umma(x, const_cast<int32_t*>(token_idx), const_cast<int32_t*>(offsets),
+                               experts_packed_opt, out, N, d, E, H, w_up_opt != nullptr, act,
+                               dev_status, s, nc);
   return launch_experts_simt(x, token_idx, offsets, w1, b1_opt, w_up_opt, w2, out, N, d, E, H, act,
                              dtype, dev_status, s, nc);
 }
@@ -251,6 +254,11 @@ int d2d_moe_forward_rule(const void* x, const void* wa, const void* wb,
   ListsOut lists;                  // short calls: written by the kernel that applies the rule
   lists.token_idx = token_idx;
   lists.offsets = offsets;
+  // long calls: the expert kernel makes the lists from a table that the rule's kernel leaves (a workspace
+  // as large as d2d_workspace_bytes used to ask for takes the launch of its own that this saves)
+  if (umma_experts && N * (int64_t)E <= 0x7fffffffLL && N <= TABLE_MAX_TILES * 128 &&
+      ws_bytes >= mask_table_bytes(N, E))
+    lists.table = ws;
 
   if (rule == D2D_RULE_ALL) {
     rc = launch_all_experts(mask_bits, routing_tensor_opt, token_idx, offsets, x, last_bias_opt,
@@ -330,7 +338,7 @@ int d2d_moe_forward_rule(const void* x, const void* wa, const void* wb,
     nl += 1;
   }
   if (rc != D2D_OK) return rc;
-  if (!lists_ready && !lists.written) {
+  if (!lists_ready && !lists.written && !lists.tabled) {
     rc = launch_compact(mask_bits, token_idx, offsets, N, E, (int32_t*)ws, dev_status, s,
                         counts_ready);
     if (rc != D2D_OK) return rc;
@@ -342,9 +350,12 @@ int d2d_moe_forward_rule(const void* x, const void* wa, const void* wb,
     nl += 1;
   }
   g_last_forward_launches = nl + 1;
-  if (umma_experts)
+  if (umma_experts) {
+    const MaskTable mt = lists.tabled ? mask_table(ws, N, E) : MaskTable();
     return launch_experts_umma(x, token_idx, offsets, experts_packed_opt, out, N, d, E, H,
-                               w_up_opt != nullptr, act, dev_status, s, nc, dr);
+                               w_up_opt != nullptr, act, dev_status, s, nc, dr,
+                               lists.tabled ? &mt : nullptr);
+  }
   return launch_experts_simt(x, token_idx, offsets, w1, b1_opt, w_up_opt, w2, out, N, d, E, H, act,
                              dtype, dev_status, s, nc);
 }

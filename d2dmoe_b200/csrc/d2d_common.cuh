@@ -188,7 +188,22 @@ struct ListsOut {
   int32_t* token_idx = nullptr;
   int32_t* offsets = nullptr;
   bool written = false;
+  void* table = nullptr;       // in: memory for a mask table that may be written instead (long calls)
+  bool tabled = false;         // out: it was
 };
+
+// What an expert kernel that makes its own lists reads: the counts table of the compaction, and the mask
+// turned over, per 128-token tile and expert the four words whose bit t says that token 32 q + t of the
+// tile keeps the expert.  A tile's entries lie together: whole sectors are written at once.
+struct MaskTable {
+  uint8_t* counts;             // [ntiles][EP]
+  uint4* words;                // [ntiles][E]
+  int ntiles, EP;
+};
+constexpr int TABLE_CHUNKS = 15;                       // parts in which its readers count it,
+constexpr int64_t TABLE_MAX_TILES = 511 * TABLE_CHUNKS;    // each with 16-bit sums
+MaskTable mask_table(void* mem, int64_t N, int E);
+size_t mask_table_bytes(int64_t N, int E);
 int launch_gate_scores_fused(const void* scores, int rule, int k, float tau, float mult,
                              uint32_t* mask_bits, void* rt, int32_t* tile_counts, const void* x,
                              const void* last_bias, int add_residual, void* out, bool direct,

@@ -220,6 +220,18 @@ int compact_row_cells(int E) {
   return ep;
 }
 
+MaskTable mask_table(void* mem, int64_t N, int E) {
+  MaskTable t;
+  t.ntiles = (int)ceil_div64(N, CTILE);
+  t.EP = compact_row_cells(E);
+  t.counts = static_cast<uint8_t*>(mem);
+  t.words = reinterpret_cast<uint4*>(t.counts + (size_t)t.ntiles * t.EP);
+  return t;
+}
+size_t mask_table_bytes(int64_t N, int E) {
+  return (size_t)ceil_div64(N, CTILE) * ((size_t)compact_row_cells(E) + 16 * (size_t)E);
+}
+
 // Four bytes per tile and expert, which d2d_workspace_bytes has always reported, hold the byte table of
 // ntiles * EP cells from four experts on; below that its rows of 16 cells are the larger.
 size_t compact_workspace_bytes(int64_t n_max, int E) {

@@ -9,7 +9,7 @@ namespace umma {
 
 constexpr int MAX_E = 128;
 constexpr int NS_MAX = 8, NS2_MAX = 8;        // stages of the two rings (upper bounds)
-constexpr int SMEM_TILES = 220 * 1024;        // both rings
+constexpr int SMEM_TILES = 212 * 1024;        // both rings
 
 struct Geo {
   int kc1;         // d / 64

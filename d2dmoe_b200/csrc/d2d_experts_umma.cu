@@ -20,6 +20,8 @@
 //     registers to whole 128-byte lines of the output;
 //   * the lists are cut into equal tiles of a size that fills the last round of the persistent
 //     grid; where there are fewer tiles than SMs the output columns are split as well;
+//   * on long calls there are no lists before this kernel: the gather warps find a tile's rows in a table
+//     that the router leaves (50432 tokens 95.1 -> 88.4 us per layer, 12608 x 12 narrow experts 39.6 -> 35.6);
 //   * where the weights of all experts stay in L2, the tiles are taken window by window of the
 //     token range, all experts of a window next to each other, so that a row of x is read and
 //     a row of out is added to in L2 by every expert but the first; last window first, because
@@ -60,8 +62,9 @@ struct Params {
   int d, E, H, act;
   const uint8_t* packed;
   Geo g;
-  const int32_t* token_idx;
-  const int32_t* offsets;
+  int32_t* token_idx;
+  int32_t* offsets;
+  MaskTable mt;                // words null: the lists are there; else they are made here from the table
   bf16* out;
   const uint32_t* mask_bits;   // optional: see DirectRows
   const bf16* last_bias;
@@ -75,7 +78,8 @@ struct Params {
 struct Tile {
   int e;                           // expert; -1: no more tiles
   int n0, n1;                      // steps of the second product
-  int pad;
+  int r0, nrows;                   // its part of token_idx
+  int first, from, seen;           // mask table: place in the expert's list, tile and count to look from
   uint32_t direct[4];              // rows that are stored instead of added to
   int list[TILE_M];                // tokens, -1: no row
   uint32_t bias[64];               // b1 of the expert as bf16 pairs
@@ -84,12 +88,14 @@ struct Tile {
 struct Ctl {
   unsigned long long full[NS_MAX], empty[NS_MAX], full2[NS2_MAX], empty2[NS2_MAX];
   unsigned long long acc1_full[2], ctx_free[2], hid_full[2], acc2_full[6], acc2_empty[6];
-  unsigned long long tile_full[TILE_RING], direct_full[TILE_RING], tile_empty[TILE_RING];
-  unsigned long long np_full[4], np_empty[4];
+  unsigned long long tile_full[TILE_RING], bias_full[TILE_RING], rows_full[TILE_RING], tile_empty[TILE_RING];
+  unsigned long long np_full[4], np_empty[4], tot_full;
   uint32_t tmem_base;
   int abort_flag;
   int wait_limit;                  // must follow abort_flag (mbar_wait reads abort_flag[1])
   float npart[TILE_M];             // norm terms that the other drain group saw
+  alignas(16) int chunk[TABLE_CHUNKS][MAX_E];   // mask table: tokens per expert of a fifteenth of the tiles
+  alignas(16) int tot[MAX_E];                   // and of all
   alignas(16) Tile tile[TILE_RING];
 };
 
@@ -122,192 +128,398 @@ struct Acc2Ring {
 // ---------------------------------------------------------------------------
 // roles
 // ---------------------------------------------------------------------------
-// Warp 19: cuts the lists into tiles, finds the ones of this CTA and hands them to the other roles
-// with their row lists, then the expert's bias and which rows are stored (tokens that one expert
-// keeps): those loads depend on the list's, and only the epilogue warps wait for them.
+__device__ __forceinline__ int chunk_start(const MaskTable& t, int w) { return w * t.ntiles / TABLE_CHUNKS; }
+
+// Warps 0-11 and 16-18: tokens per expert in the warp's fifteenth of the counts table.  A lane has 16 cells of every
+// so many rows, summed as pairs of 16-bit halves (a chunk has at most 511 tiles of 128 tokens).  (Called
+// without `live` before the table is there: see role_list.)
+__device__ __forceinline__ void count_chunk(const Params& p, Ctl* c, int w, int lane, bool live) {
+  const MaskTable& t = p.mt;
+  const int per = t.EP >> 4, step = 32 / per, g = lane & (per - 1);      // lanes per row, rows at once
+  const int t1 = chunk_start(t, w + 1);
+  uint32_t acc[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
+#pragma unroll 1
+  for (int t0 = chunk_start(t, w) + lane / per; t0 < t1; t0 += 4 * step) {
+    uint4 x[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      x[u] = make_uint4(0u, 0u, 0u, 0u);
+      if (live && t0 + u * step < t1)
+        x[u] = *(reinterpret_cast<const uint4*>(t.counts + (size_t)(t0 + u * step) * t.EP) + g);
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const uint32_t v[4] = {x[u].x, x[u].y, x[u].z, x[u].w};
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        acc[2 * k] += v[k] & 0x00ff00ffu;
+        acc[2 * k + 1] += (v[k] >> 8) & 0x00ff00ffu;
+      }
+    }
+  }
+#pragma unroll 1
+  for (int o = 16; o >= per; o >>= 1)
+#pragma unroll
+    for (int q = 0; q < 8; ++q) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], o);
+  if (lane < per)
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int4 v = make_int4(acc[2 * k] & 0xffff, acc[2 * k + 1] & 0xffff, acc[2 * k] >> 16,
+                               acc[2 * k + 1] >> 16);
+      int* tot = &c->tot[16 * g + 4 * k];
+      *reinterpret_cast<int4*>(&c->chunk[w][16 * g + 4 * k]) = v;
+      if (!live) continue;
+      if (v.x) atomicAdd(tot, v.x);
+      if (v.y) atomicAdd(tot + 1, v.y);
+      if (v.z) atomicAdd(tot + 2, v.z);
+      if (v.w) atomicAdd(tot + 3, v.w);
+    }
+  __syncwarp();
+  if (live && lane == 0) mbar_arrive(smem_u32(&c->tot_full));
+}
+
+__device__ __forceinline__ int warp_scan(int v, int lane) {      // inclusive
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, v, o);
+    if (lane >= o) v += u;
+  }
+  return v;
+}
+
+// position of the r-th one of m
+__device__ __forceinline__ int select_bit(uint32_t m, int r) {
+  int at = 0;
+#pragma unroll
+  for (int s = 16; s > 0; s >>= 1) {
+    const int n = __popc((m >> at) & ((1u << s) - 1u));
+    if (r >= n) {
+      r -= n;
+      at += s;
+    }
+  }
+  return at;
+}
+
+// Where token `first` of expert e's list is: the counted chunk says from which tile on to look and how many
+// tokens come before it.
+__device__ __forceinline__ void find_chunk(const MaskTable& t, const Ctl* c, int e, int first, int lane,
+                                           int& tile, int& seen) {
+  const int n = lane < TABLE_CHUNKS ? c->chunk[lane][e] : 0, incl = warp_scan(n, lane);
+  const uint32_t past = __ballot_sync(0xffffffffu, incl > first);
+  const int w = past != 0u ? __ffs(past) - 1 : TABLE_CHUNKS;
+  seen = __shfl_sync(0xffffffffu, incl - n, w & 31);
+  tile = chunk_start(t, w);
+}
+// the same to the tile, from the counts table
+__device__ __forceinline__ void find_tile(const MaskTable& t, int e, int first, int lane, int& tile, int& seen) {
+#pragma unroll 1
+  for (; tile < t.ntiles; tile += 32) {
+    const int n = tile + lane < t.ntiles ? t.counts[(size_t)(tile + lane) * t.EP + e] : 0;
+    const int incl = warp_scan(n, lane);
+    const uint32_t past = __ballot_sync(0xffffffffu, seen + incl > first);
+    const int w = past != 0u ? __ffs(past) - 1 : 31;
+    seen += __shfl_sync(0xffffffffu, past != 0u ? incl - n : incl, w);
+    if (past != 0u) {
+      tile += w;
+      return;
+    }
+  }
+}
+// expert e's words of 96 tiles, three per lane
+constexpr int LOOK = 3;
+__device__ __forceinline__ void load_words(const MaskTable& t, int E, int e, int tile, int lane, bool live,
+                                           uint4* x) {
+#pragma unroll
+  for (int k = 0; k < LOOK; ++k) {
+    x[k] = make_uint4(0u, 0u, 0u, 0u);
+    if (live && tile + 32 * k + lane < t.ntiles)
+      x[k] = t.words[(size_t)(tile + 32 * k + lane) * E + e];
+  }
+}
+
+// Row `row` of a tile out of the mask table, -1 where it is none (row >= nrows).  A lane has one tile's words
+// (x: those of the 96 tiles from t->from on), and a row looks for the lane, the word and the bit that it
+// is: no loop over bits, as many steps for one token in a hundred as for one in four.  A table that is
+// not the mask's, left by a router that gave up, gives -1.
+__device__ __forceinline__ int find_token(const Params& p, const Tile* t, uint4* x, int row, int lane, bool live) {
+  const MaskTable& mt = p.mt;
+  const int first = t->first, end = first + t->nrows;
+  int tile = t->from, seen = t->seen, tok = -1;
+#pragma unroll 1
+  for (;;) {
+#pragma unroll 1
+    for (int k = 0; k < LOOK && tile < mt.ntiles && seen < end; ++k, tile += 32) {
+      const uint4 y = k == 0 ? x[0] : k == 1 ? x[1] : x[2];
+      const int c0 = __popc(y.x), c1 = c0 + __popc(y.y), c2 = c1 + __popc(y.z), n = c2 + __popc(y.w);
+      const int incl = warp_scan(n, lane), all = __shfl_sync(0xffffffffu, incl, 31);
+      int r = first + row - seen, at = 0;
+      const bool mine = r >= 0 && r < all && first + row < end;
+      seen += all;
+      if (live && !__any_sync(0xffffffffu, mine)) continue;
+#pragma unroll
+      for (int s = 16; s > 0; s >>= 1)   // lanes whose tokens all come before r
+        if (__shfl_sync(0xffffffffu, incl, at + s - 1) <= r) at += s;
+      at = min(at, 31);
+      const int en = __shfl_sync(0xffffffffu, c0 | c1 << 8 | c2 << 16, at);      // (at most 96 each)
+      r -= __shfl_sync(0xffffffffu, incl - n, at);
+      const int e0 = en & 255, e1 = en >> 8 & 255, e2 = en >> 16;
+      const uint32_t w0 = __shfl_sync(0xffffffffu, y.x, at), w1 = __shfl_sync(0xffffffffu, y.y, at),
+                     w2 = __shfl_sync(0xffffffffu, y.z, at), w3 = __shfl_sync(0xffffffffu, y.w, at);
+      const int q = (r >= e0) + (r >= e1) + (r >= e2);
+      const uint32_t w = q == 0 ? w0 : q == 1 ? w1 : q == 2 ? w2 : w3;
+      r -= q == 0 ? 0 : q == 1 ? e0 : q == 2 ? e1 : e2;
+      if (mine) tok = (tile + at) * 128 + 32 * q + select_bit(w, r);
+    }
+    if (!live || tile >= mt.ntiles || seen >= end) return tok;
+    load_words(mt, p.E, t->e, tile, lane, live, x);
+  }
+}
+
+// Warp 19: cuts the lists into tiles and hands the ones of this CTA to the other roles: expert, part of the
+// list, then its bias.  The rows themselves are found by the gather warps.  Without lists (the mask table in
+// their place) the experts' totals are counted here; a launch of its own for the lists took 4.3 us
+// (8.5 for 50432 tokens).
 //
 // Tiles have S rows at most, S as small as the number of rounds of the grid allows:
 // T = sum ceil(n_e / S) <= rows / S + E, so R rounds of G CTAs are enough for S = rows / (R G - E),
 // and R is the least with S <= 128.  (524 rows per SM: five tiles of about 109 rows per CTA
 // instead of four of 128 and one of 12.)  An expert's tiles are equal.
-// The first pass over the set-up runs on no rows, while the previous kernel drains: instructions
-// executed for the first time cost some 20 cycles each, and everything waits for the first tile.
+// The first pass runs, while the previous kernel drains, up to the first tile of a list of one
+// row: instructions that are executed for the first time cost some 20 cycles each, and everything
+// waits for the first tile.  So do the first passes of count_chunk and of the gather warps.
 __device__ void role_list(const Params& p, Ctl* c, int lane, bool one_window) {
   volatile int* af = &c->abort_flag;
-  const int nw = (p.E + 31) >> 5;
-  int off[5], n[4], nt[4], total = 0, rounds = 1;
+  const int E = p.E, G = gridDim.x;
+  const bool tabled = p.mt.words != nullptr;
 #pragma unroll 1
   for (int pass = 0; pass < 2; ++pass) {
-    if (pass) grid_dependency_wait();
-    const int E = pass ? p.E : 0;
+    const bool live = pass != 0;
+    if (live) grid_dependency_wait();
+    int off[5], n[4], nt[4];             // experts 4 lane .. + 3
+    if (tabled) {
+      if (live && !mbar_wait_warp(smem_u32(&c->tot_full), 0, af, p.dev_status)) return;
+      const int4 v = *reinterpret_cast<const int4*>(&c->tot[4 * lane]);
+      n[0] = 4 * lane < E ? v.x : 0;
+      n[1] = 4 * lane + 1 < E ? v.y : 0;
+      n[2] = 4 * lane + 2 < E ? v.z : 0;
+      n[3] = 4 * lane + 3 < E ? v.w : 0;
+      const int sum = n[0] + n[1] + n[2] + n[3];
+      off[0] = warp_scan(sum, lane) - sum;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) off[q + 1] = off[q] + n[q];
+    } else {
+#pragma unroll
+      for (int q = 0; q < 5; ++q) off[q] = live && 4 * lane + q <= E ? p.offsets[4 * lane + q] : 0;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int e = 4 * lane + q;
+        const bool bad = off[q + 1] < off[q] || off[q] < 0 || off[q + 1] > p.N * (long long)E;
+        n[q] = e < E && !bad ? off[q + 1] - off[q] : 0;
+        if (e < E && bad) report(p.dev_status, D2D_ERR_INDEX_RANGE);
+      }
+    }
+    if (!live) n[0] = lane == 0 ? 1 : 0;
     int rows = 0, used = 0;
     bool all_n = true;                   // every expert of this lane lists exactly N tokens
 #pragma unroll
-    for (int q = 0; q < 5; ++q) {
-      const int e = 4 * lane + q;
-      off[q] = e <= E && E > 0 ? p.offsets[e] : 0;
-    }
-#pragma unroll
     for (int q = 0; q < 4; ++q) {
-      const int e = 4 * lane + q;
-      const bool bad = off[q + 1] < off[q] || off[q] < 0 || off[q + 1] > p.N * (long long)p.E;
-      n[q] = e < E && !bad ? off[q + 1] - off[q] : 0;
-      if (e < E && bad) report(p.dev_status, D2D_ERR_INDEX_RANGE);
-      all_n = all_n && (e >= E || n[q] == p.N);
+      all_n = all_n && (4 * lane + q >= E || n[q] == p.N);
       rows += n[q];
       used += n[q] > 0 ? 1 : 0;
     }
     rows = __reduce_add_sync(0xffffffffu, rows);
     used = __reduce_add_sync(0xffffffffu, used);
-    const float G = (float)gridDim.x;
-    const float R = ceilf(((float)rows * (1.0f / TILE_M) + (float)used) / G);
+    const float R = ceilf(__fdividef((float)rows * (1.0f / TILE_M) + (float)used, (float)G));
     const int S =                        // (never more rows than a stage has room for)
-        max(32, min(p.g.a_slot >> 7, (int)ceilf((float)rows / fmaxf(R * G - (float)used, 1.0f))));
-    const float inv = 1.0f / (float)S;
+        max(32, min(p.g.a_slot >> 7,
+                    (int)ceilf(__fdividef((float)rows, fmaxf(R * (float)G - (float)used, 1.0f)))));
+    const uint32_t inv = 0xffffffffu / (uint32_t)S + 1u;      // ceil(2^32 / S)
     int sum = 0;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {        // ceil(n / S): float quotient, exact correction
-      nt[q] = (int)((float)n[q] * inv);
-      while ((long long)nt[q] * S < n[q]) ++nt[q];
-      while (nt[q] > 0 && (long long)(nt[q] - 1) * S >= n[q]) --nt[q];
+    for (int q = 0; q < 4; ++q) {        // ceil(n / S): n < 2^31, so at most one too many
+      nt[q] = (int)__umulhi((uint32_t)n[q] + (uint32_t)S - 1u, inv);
+      if (nt[q] > 0 && (uint32_t)(nt[q] - 1) * (uint32_t)S >= (uint32_t)n[q]) --nt[q];
       sum += nt[q];
     }
-    total = __reduce_add_sync(0xffffffffu, sum);
+    const int total = __reduce_add_sync(0xffffffffu, sum);
     // windows: one per round of the grid, or a single one (expert by expert) where each window
     // would stream all the weights again; with every expert on every token they pay all the same
-    rounds = one_window && !__all_sync(0xffffffffu, all_n) ? 1 : max(1, (int)R);
-  }
-  // fewer than half as many tiles as CTAs: split the output columns (the first product is
-  // repeated, the second product, W2 and the output are shared out)
-  int parts = 1;
-  if (total > 0 && 2 * total <= (int)gridDim.x && p.norm_layer == 0)
-    parts = min((int)gridDim.x / total, p.g.nc);
-  const float inv_rounds = 1.0f / (float)rounds;
+    const int rounds = one_window && !__all_sync(0xffffffffu, all_n) ? 1 : max(1, (int)R);
+    // fewer than half as many tiles as CTAs: split the output columns (the first product is
+    // repeated, the second product, W2 and the output are shared out)
+    int parts = 1;
+    if (total > 0 && 2 * total <= G && p.norm_layer == 0) parts = min(G / total, p.g.nc);
+    const float inv_rounds = __fdividef(1.0f, (float)rounds);
 
-  // the current window's tiles of my experts: lo .. hi - 1
-  int lo[4], hi[4], w = rounds, start = 0, count = 0, incl = 0;
+    // the current window's tiles of my experts: lo .. hi - 1
+    int lo[4], hi[4], w = rounds, start = 0, count = 0, incl = 0;
 #pragma unroll
-  for (int q = 0; q < 4; ++q) lo[q] = nt[q];
-  RingPos r = {0, 0};
+    for (int q = 0; q < 4; ++q) lo[q] = nt[q];
+    RingPos r = {0, 0};
 #pragma unroll 1
-  for (int u = blockIdx.x;; u += gridDim.x, r.next(TILE_RING)) {
-    const int tile = u / parts, part = u - tile * parts;
-    Tile* t = &c->tile[r.s];
-    if (tile >= total) {
-      if (!mbar_wait_warp(smem_u32(&c->tile_empty[r.s]), r.ph ^ 1, af, p.dev_status)) return;
-      if (lane == 0) t->e = -1;
-      __syncwarp();
-      mbar_arrive(smem_u32(&c->tile_full[r.s]));
-      return;
-    }
-    while (tile >= start + count) {
-      start += count;
-      --w;
-      int mine = 0;
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        hi[q] = lo[q];
-        lo[q] = w == 0 ? 0 : min(hi[q], (int)((float)nt[q] * ((float)w * inv_rounds)));
-        mine += hi[q] - lo[q];
+    for (int u = live ? blockIdx.x : 0;; u += G, r.next(TILE_RING)) {
+      const int tile = parts == 1 ? u : u / parts, part = parts == 1 ? 0 : u - tile * parts;
+      Tile* t = &c->tile[r.s];
+      if (tile >= total) {
+        if (!mbar_wait_warp(smem_u32(&c->tile_empty[r.s]), r.ph ^ 1, af, p.dev_status)) return;
+        if (lane == 0) t->e = -1;
+        __syncwarp();
+        mbar_arrive(smem_u32(&c->tile_full[r.s]));
+        break;
       }
-      incl = mine;
+      while (tile >= start + count) {
+        start += count;
+        --w;
+        int mine = 0;
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += v;
-      }
-      count = __shfl_sync(0xffffffffu, incl, 31);
-    }
-    const int owner = __ffs(__ballot_sync(0xffffffffu, incl > tile - start)) - 1;
-    int e = 0, r0 = 0, nrows = 0;
-    if (lane == owner) {
-      int k = tile - start - (incl - (hi[0] + hi[1] + hi[2] + hi[3] - lo[0] - lo[1] - lo[2] - lo[3]));
-      bool found = false;
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int m = hi[q] - lo[q];
-        if (!found && k < m) {
-          found = true;
-          e = 4 * lane + q;
-          const int size = (n[q] + nt[q] - 1) / nt[q];
-          const int first = (lo[q] + k) * size;
-          r0 = off[q] + first;
-          nrows = min(size, n[q] - first);      // (may be negative where the last tiles are empty)
+        for (int q = 0; q < 4; ++q) {
+          hi[q] = lo[q];
+          lo[q] = w == 0 ? 0 : min(hi[q], (int)((float)nt[q] * ((float)w * inv_rounds)));
+          mine += hi[q] - lo[q];
         }
-        if (!found) k -= m;
+        incl = warp_scan(mine, lane);
+        count = __shfl_sync(0xffffffffu, incl, 31);
       }
-    }
-    e = __shfl_sync(0xffffffffu, e, owner);
-    r0 = __shfl_sync(0xffffffffu, r0, owner);
-    nrows = __shfl_sync(0xffffffffu, nrows, owner);
-    int tok[4];
+      const int owner = __ffs(__ballot_sync(0xffffffffu, incl > tile - start)) - 1;
+      int e = 0, first = 0, r0 = 0, nrows = 0;
+      if (lane == owner) {
+        int k = tile - start - (incl - (hi[0] + hi[1] + hi[2] + hi[3] - lo[0] - lo[1] - lo[2] - lo[3]));
+        int len = 0, tiles = 1;
+        bool found = false;
 #pragma unroll
-    for (int g = 0; g < 4; ++g)          // a lane has rows lane + 32 g
-      tok[g] = 32 * g + lane < nrows ? p.token_idx[r0 + 32 * g + lane] : 0;
-    if (!mbar_wait_warp(smem_u32(&c->tile_empty[r.s]), r.ph ^ 1, af, p.dev_status)) return;
-    if (lane == 0) {
-      t->e = e;
-      t->n0 = part * p.g.nc / parts;
-      t->n1 = (part + 1) * p.g.nc / parts;
-    }
-#pragma unroll
-    for (int g = 0; g < 4; ++g) {
-      if (tok[g] < 0 || tok[g] >= p.N) {
-        report(p.dev_status, D2D_ERR_INDEX_RANGE);
-        tok[g] = -1;
+        for (int q = 0; q < 4; ++q) {
+          const int m = hi[q] - lo[q];
+          if (!found && k < m) {
+            found = true;
+            e = 4 * lane + q;
+            first = lo[q] + k;
+            len = n[q];
+            tiles = nt[q];
+            r0 = off[q];
+          }
+          if (!found) k -= m;
+        }
+        const int size = (len + tiles - 1) / tiles;
+        first *= size;
+        r0 += first;
+        nrows = min(size, len - first);  // (may be negative where the last tiles are empty)
       }
-      if (32 * g + lane >= nrows) tok[g] = -1;
-      t->list[32 * g + lane] = tok[g];
+      e = __shfl_sync(0xffffffffu, e, owner);
+      first = __shfl_sync(0xffffffffu, first, owner);
+      int from = 0, seen = 0;
+      if (tabled) {
+        find_chunk(p.mt, c, e, first, lane, from, seen);
+        if (u != (int)blockIdx.x && live) find_tile(p.mt, e, first, lane, from, seen);   // (not urgent)
+      }
+      if (live && !mbar_wait_warp(smem_u32(&c->tile_empty[r.s]), r.ph ^ 1, af, p.dev_status)) return;
+      if (lane == owner) {
+        t->e = e;
+        t->n0 = part * p.g.nc / parts;
+        t->n1 = (part + 1) * p.g.nc / parts;
+        t->r0 = r0;
+        t->nrows = nrows;
+        t->first = first;
+        t->from = from;
+        t->seen = seen;
+      }
+      __syncwarp();
+      if (live) mbar_arrive(smem_u32(&c->tile_full[r.s]));
+      const float4 b1 = 4 * lane < p.H
+                            ? __ldg(reinterpret_cast<const float4*>(
+                                  p.packed + (long long)e * p.g.stride + p.g.bias_off) + lane)
+                            : make_float4(0.f, 0.f, 0.f, 0.f);
+      t->bias[2 * lane] = pack_bf16x2(b1.x, b1.y);
+      t->bias[2 * lane + 1] = pack_bf16x2(b1.z, b1.w);
+      if (!live) break;
+      mbar_arrive(smem_u32(&c->bias_full[r.s]));
     }
-    __syncwarp();
-    mbar_arrive(smem_u32(&c->tile_full[r.s]));
-    const float4 b1 = 4 * lane < p.H
-                          ? __ldg(reinterpret_cast<const float4*>(
-                                p.packed + (long long)e * p.g.stride + p.g.bias_off) + lane)
-                          : make_float4(0.f, 0.f, 0.f, 0.f);
+    if (tabled && live && blockIdx.x == 0) {
 #pragma unroll
-    for (int g = 0; g < 4; ++g) {
-      int kept = 0;
-      if (p.mask_bits && tok[g] >= 0)
-        for (int q = 0; q < nw; ++q) kept += __popc(p.mask_bits[(long long)tok[g] * nw + q]);
-      const uint32_t d = __ballot_sync(0xffffffffu, kept == 1);
-      if (lane == 0) t->direct[g] = d;
+      for (int q = 0; q < 4; ++q)
+        if (4 * lane + q < E) p.offsets[4 * lane + q] = off[q];
+      if (lane == 31) p.offsets[E] = off[4];
+      if (lane == 31 && off[4] > p.N * (long long)E) report(p.dev_status, D2D_ERR_INDEX_RANGE);
     }
-    t->bias[2 * lane] = pack_bf16x2(b1.x, b1.y);
-    t->bias[2 * lane + 1] = pack_bf16x2(b1.z, b1.w);
-    __syncwarp();
-    mbar_arrive(smem_u32(&c->direct_full[r.s]));
   }
 }
 
-// Warps 12-15: rows of x by 16-byte cp.async (4 rows x 128 bytes per warp instruction, software
-// swizzle; a TMA gather spends a request per 128-byte row and was 1.6 times slower).  Rows past
+// Warps 12-15: warp w has rows 32 w .. + 31 of a tile.  It finds their tokens (the list's, or out of the
+// mask table, whose part of the list it then writes), says which of them are stored, and copies their
+// rows of x by 16-byte cp.async (4 rows x 128 bytes per warp instruction, software swizzle; a TMA
+// gather spends a request per 128-byte row and was 1.6 times slower).  Rows past
 // the list's end repeat the 32-row group's first one, a group without rows loads nothing: what
 // their slots hold reaches only accumulator rows nobody reads.
+// (Beside the traffic of the kernel a load takes some thousand cycles: the mask words of a tile travel
+// while its rows are copied, and so do the next tile's table words where that tile is known by then.)
 __device__ void role_gather(const Params& p, Ctl* c, uint32_t ring, int w, int lane) {
   volatile int* af = &c->abort_flag;
-  const int j = lane & 7;
+  const int j = lane & 7, row = w * 32 + lane;
+  const int nw = (p.E + 31) >> 5;
+  const bool tabled = p.mt.words != nullptr;
   uint32_t dstoff[8];
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
-    const int row = w * 32 + i * 4 + (lane >> 3);
-    dstoff[i] = (row >> 3) * 1024 + (row & 7) * 128 + ((j ^ (row & 7)) << 4);
+    const int rr = w * 32 + i * 4 + (lane >> 3);
+    dstoff[i] = (rr >> 3) * 1024 + (rr & 7) * 128 + ((j ^ (rr & 7)) << 4);
   }
   RingPos r = {0, 0}, q = {0, 0};
-  for (;; q.next(TILE_RING)) {
-    if (!mbar_wait_warp(smem_u32(&c->tile_full[q.s]), q.ph, af, p.dev_status)) return;
-    if (c->tile[q.s].e < 0) return;
-    const int* list = c->tile[q.s].list + w * 32;
-    const int v0 = list[0];
+  uint4 x[LOOK];
+  x[0] = x[1] = x[2] = make_uint4(0u, 0u, 0u, 0u);
+  bool live = false, ahead = true;       // ahead: this tile's first loads are on their way
+#pragma unroll 1
+  for (;;) {
+    Tile* t = &c->tile[q.s];
+    if (live) {
+      if (!mbar_wait_warp(smem_u32(&c->tile_full[q.s]), q.ph, af, p.dev_status)) return;
+      if (t->e < 0) return;
+    }
+    const int e = live ? t->e : 0, nrows = live ? t->nrows : 0, at = live ? t->r0 + row : 0;
+    if (!ahead) {
+      if (tabled) load_words(p.mt, p.E, e, t->from, lane, live, x);
+      else x[0].x = row < nrows ? p.token_idx[at] : 0;
+    }
+    int tok = (int)x[0].x;
+    if (tabled) tok = find_token(p, t, x, row, lane, live);
+    if (row < nrows && (tok < 0 || tok >= p.N)) {
+      report(p.dev_status, D2D_ERR_INDEX_RANGE);
+      tok = -1;
+    }
+    if (row >= nrows) tok = -1;
+    if (live) t->list[row] = tok;
+    // (in bounds whatever the table says)
+    if (tabled && tok >= 0 && t->n0 == 0 && (uint32_t)at < (uint32_t)(p.N * p.E)) p.token_idx[at] = tok;
+    uint32_t mask[4] = {0u, 0u, 0u, 0u};
+    if (p.mask_bits && tok >= 0)
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (k < nw) mask[k] = p.mask_bits[(long long)tok * nw + k];
+    const int v0 = __shfl_sync(0xffffffffu, tok, 0);
     const bf16* src[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      const int v = list[i * 4 + (lane >> 3)];
+      const int v = __shfl_sync(0xffffffffu, tok, i * 4 + (lane >> 3));
       src[i] = p.x + (size_t)max(v < 0 ? v0 : v, 0) * p.d + j * 8;
     }
-    __syncwarp();
-    if (lane == 0) mbar_arrive(smem_u32(&c->tile_empty[q.s]));
+    if (!live) {                         // the previous kernel's results from here on
+      grid_dependency_wait();
+      live = true;
+      ahead = false;
+      continue;
+    }
+    const RingPos q0 = q;
+    q.next(TILE_RING);
+    ahead = false;
+    if (__all_sync(0xffffffffu, mbar_test_wait(smem_u32(&c->tile_full[q.s]), q.ph))) {
+      const Tile* t1 = &c->tile[q.s];
+      if (t1->e >= 0) {
+        ahead = true;
+        if (tabled) load_words(p.mt, p.E, t1->e, t1->from, lane, true, x);
+        else x[0].x = row < t1->nrows ? p.token_idx[t1->r0 + row] : 0;
+      }
+    }
     const bool rows = v0 >= 0;           // warp-uniform
+#pragma unroll 1
     for (int kc = 0; kc < p.g.kc1; ++kc) {
       if (!mbar_wait_warp(smem_u32(&c->empty[r.s]), r.ph ^ 1, af, p.dev_status)) return;
       if (rows) {
@@ -317,6 +529,14 @@ __device__ void role_gather(const Params& p, Ctl* c, uint32_t ring, int w, int l
       }
       cp_async_arrive_noinc(smem_u32(&c->full[r.s]));
       r.next(p.g.ns);
+    }
+    const uint32_t d = __ballot_sync(
+        0xffffffffu, __popc(mask[0]) + __popc(mask[1]) + __popc(mask[2]) + __popc(mask[3]) == 1);
+    if (lane == 0) c->tile[q0.s].direct[w] = d;
+    __syncwarp();
+    if (lane == 0) {
+      mbar_arrive(smem_u32(&c->rows_full[q0.s]));
+      mbar_arrive(smem_u32(&c->tile_empty[q0.s]));
     }
   }
 }
@@ -480,10 +700,11 @@ __device__ void role_ep1(const Params& p, Ctl* c, uint32_t tmem, int et) {
     const Tile* t = &c->tile[q.s];
     const int e = t->e;
     if (e < 0) return;
-    if (!mbar_wait_warp(smem_u32(&c->direct_full[q.s]), q.ph, af, p.dev_status)) return;
+    if (!mbar_wait_warp(smem_u32(&c->bias_full[q.s]), q.ph, af, p.dev_status)) return;
     const uint32_t* bp = t->bias;
     // labels by-product (intermediate layer): this thread's row
     float nacc = 0.f;
+    if (NORM && !mbar_wait_warp(smem_u32(&c->rows_full[q.s]), q.ph, af, p.dev_status)) return;
     const int ntok = NORM ? t->list[et] : -1;
     if (!mbar_wait_warp(smem_u32(&c->acc1_full[ctx]), ph, af, p.dev_status)) return;
     tc_fence_after();
@@ -600,7 +821,7 @@ __device__ void role_drain(const Params& p, Ctl* c, uint32_t tmem, int j, int q4
     const Tile* t = &c->tile[q.s];
     const int e = t->e, n0 = t->n0, n1 = t->n1;
     if (e < 0) return;
-    if (!mbar_wait_warp(smem_u32(&c->direct_full[q.s]), q.ph, af, p.dev_status)) return;
+    if (!mbar_wait_warp(smem_u32(&c->rows_full[q.s]), q.ph, af, p.dev_status)) return;
     const uint32_t direct = DIRECT ? t->direct[q4] : 0u;
     int rt[8];                           // rows 8 (i / 2) + (rl & ~1) + i % 2; sign bit: stored
 #pragma unroll
@@ -692,6 +913,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) experts_tiles_kernel(const Params
   // Programmatic dependent launch: see router_tiles_kernel.
   grid_launch_dependents();
 
+  if (tid < MAX_E) c->tot[tid] = 0;
   if (tid == 0) {
     for (int i = 0; i < NS_MAX; ++i) {
       mbar_init(smem_u32(&c->full[i]), 129);          // 128 gather threads, one weight copy
@@ -708,12 +930,14 @@ __global__ void __launch_bounds__(NTHREADS, 1) experts_tiles_kernel(const Params
     }
     for (int i = 0; i < TILE_RING; ++i) {
       mbar_init(smem_u32(&c->tile_full[i]), 32);
-      mbar_init(smem_u32(&c->direct_full[i]), 32);
+      mbar_init(smem_u32(&c->bias_full[i]), 32);
+      mbar_init(smem_u32(&c->rows_full[i]), 4);
       mbar_init(smem_u32(&c->tile_empty[i]), TILE_READERS);
       mbar_init(smem_u32(&c->np_full[i]), 32);
       mbar_init(smem_u32(&c->np_empty[i]), 32);
     }
     static_assert(TILE_RING == 4, "np barriers: one per row quarter");
+    mbar_init(smem_u32(&c->tot_full), TABLE_CHUNKS);
     for (int i = 0; i < 6; ++i) {
       mbar_init(smem_u32(&c->acc2_full[i]), 1);
       mbar_init(smem_u32(&c->acc2_empty[i]), p.g.nd >> 4);    // four warps per 64 columns
@@ -728,7 +952,13 @@ __global__ void __launch_bounds__(NTHREADS, 1) experts_tiles_kernel(const Params
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = c->tmem_base;
-  if (warp <= WARP_W) grid_dependency_wait();
+  // (the list and gather warps wait for the previous kernel in their roles)
+  if (warp < WARP_GATHER0 || (warp >= WARP_MMA1 && warp <= WARP_W)) {
+    const int w = warp < WARP_GATHER0 ? warp : warp - (WARP_MMA1 - WARP_GATHER0);
+    if (p.mt.words) count_chunk(p, c, w, lane, false);
+    grid_dependency_wait();
+    if (p.mt.words) count_chunk(p, c, w, lane, true);
+  }
 
   if (warp < WARP_DRAIN0) {
     role_ep1_act<GLU, NORM == D2D_NORM_OF_INTERMEDIATE>(p, c, tmem, tid);
@@ -840,10 +1070,11 @@ int launch_prepack_experts(const void* w1, const void* b1, const void* w_up, con
   return cudaGetLastError() == cudaSuccess ? D2D_OK : D2D_ERR_LAUNCH;
 }
 
-int launch_experts_umma(const void* x, const int32_t* token_idx, const int32_t* offsets,
+int launch_experts_umma(const void* x, int32_t* token_idx, int32_t* offsets,
                         const void* packed, void* out, int64_t N, int d, int E, int H, bool glu,
-                        int act, int* dev_status, cudaStream_t s, NormCapture nc, DirectRows dr) {
-  if (!nc.norms && experts_short_supported(N, d, E, H, glu, dr.kept))
+                        int act, int* dev_status, cudaStream_t s, NormCapture nc, DirectRows dr,
+                        const MaskTable* mt) {
+  if (!nc.norms && !mt && experts_short_supported(N, d, E, H, glu, dr.kept))
     return launch_experts_short(x, token_idx, offsets, packed, out, N, d, E, H, glu, act, dev_status,
                                 s, dr);
   Params p = {};
@@ -857,6 +1088,7 @@ int launch_experts_umma(const void* x, const int32_t* token_idx, const int32_t* 
   p.g = experts_geo(d, H, glu, N);
   p.token_idx = token_idx;
   p.offsets = offsets;
+  if (mt) p.mt = *mt;
   p.out = (bf16*)out;
   p.mask_bits = dr.mask_bits;
   p.last_bias = (const bf16*)dr.last_bias;

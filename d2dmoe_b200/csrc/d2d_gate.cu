@@ -439,7 +439,7 @@ gate_scores_fused_rows_kernel(const T* __restrict__ scores, float mult, int k, f
                               const T* __restrict__ x, const T* __restrict__ last_bias,
                               int add_residual, T* __restrict__ out, int direct, int64_t N, int d,
                               int E, int32_t* __restrict__ token_idx,
-                              int32_t* __restrict__ offsets) {
+                              int32_t* __restrict__ offsets, const MaskTable mt) {
   __shared__ uint32_t cnt[4][64];        // tokens of a 32-token row that keep an expert, as bits
   __shared__ uint32_t rows[4];
   __shared__ int scratch[3 * 256];
@@ -523,6 +523,8 @@ gate_scores_fused_rows_kernel(const T* __restrict__ scores, float mult, int k, f
       cnt[w][32 * j + lane] = transpose32(word[j], lane);
   }
   __syncthreads();
+  if (mt.words && tid < E)
+    mt.words[(int64_t)blockIdx.x * E + tid] = make_uint4(cnt[0][tid], cnt[1][tid], cnt[2][tid], cnt[3][tid]);
   if (!token_idx)
     for (int e = tid; e < EP; e += NT)
       tile_counts[(int64_t)blockIdx.x * EP + e] =
@@ -728,6 +730,12 @@ int launch_gate_scores_fused(const void* scores, int rule, int k, float tau, flo
                          (rt == nullptr || al16(rt));
   const bool fused = rows_form && lists && grid <= CLUSTER_TILES;
   if (fused) lists->written = true;
+  MaskTable mt = {};
+  if (rows_form && lists && lists->table && !fused) {
+    mt = mask_table(lists->table, N, E);
+    counts = mt.counts;
+    lists->tabled = true;
+  }
 #define D2D_ROWS_CASE(T, NVV)                                                                 \
   case NVV: {                                                                                 \
     auto kn = rule == 0               ? gate_scores_fused_rows_kernel<T, NVV, 0>              \
@@ -737,7 +745,7 @@ int launch_gate_scores_fused(const void* scores, int rule, int k, float tau, flo
                               (const T*)scores, mult, k, tau, mask_bits, (T*)rt, counts, EP,  \
                               (const T*)x, (const T*)last_bias, add_residual, (T*)out,        \
                               direct ? 1 : 0, N, d, E, fused ? lists->token_idx : nullptr,    \
-                              fused ? lists->offsets : nullptr);                              \
+                              fused ? lists->offsets : nullptr, mt);                          \
   }
   if (rows_form) {
     if (dtype == D2D_F32) {

@@ -77,6 +77,7 @@ struct Params {
   int32_t* token_idx;       // optional (one tile per CTA, all CTAs one cluster): the token lists
   int32_t* offsets;
   int EP;
+  MaskTable mt;             // words null: none
   bf16* out_init;           // optional: initial output rows last_bias (+ resid)
   const bf16* last_bias;
   const bf16* resid;
@@ -93,7 +94,7 @@ struct Ctl {
   uint32_t tmem_base;
   int abort_flag;
   int wait_limit;           // must follow abort_flag (mbar_wait reads abort_flag[1])
-  int cnt[2][4][MAX_E];     // kept tokens per expert of a 32-token row group
+  int cnt[2][4][MAX_E];     // per expert, the tokens of a 32-token row group that keep it: number or bits
   uint32_t init_rows[2][4];
 };
 
@@ -319,8 +320,10 @@ __device__ void role_gate(const Params& p, Ctl* c, uint32_t tmem, int et) {
         c->cnt[0][q4][32 * j + lane] = (int)transpose32(word[j], lane);
     } else if (p.tile_counts) {
 #pragma unroll
-      for (int j = 0; j < NW; ++j)
-        c->cnt[buf][q4][32 * j + lane] = __popc(transpose32(word[j], lane));
+      for (int j = 0; j < NW; ++j) {
+        const uint32_t col = transpose32(word[j], lane);
+        c->cnt[buf][q4][32 * j + lane] = p.mt.words ? (int)col : __popc(col);
+      }
       // one barrier per tile: the other half of cnt is written before anybody passes it again (an
       // mbarrier, because a warp that gave up never comes)
       __syncwarp();
@@ -328,8 +331,16 @@ __device__ void role_gate(const Params& p, Ctl* c, uint32_t tmem, int et) {
       if (!mbar_wait_warp(smem_u32(&c->cnt_full), ph, af, p.dev_status)) return;
       if (et < p.EP) {
         int n = 0;
-        if (et < E)
-          n = c->cnt[buf][0][et] + c->cnt[buf][1][et] + c->cnt[buf][2][et] + c->cnt[buf][3][et];
+        if (et < E) {
+          const int a = c->cnt[buf][0][et], b = c->cnt[buf][1][et], cc = c->cnt[buf][2][et],
+                    dd = c->cnt[buf][3][et];
+          if (p.mt.words) {
+            p.mt.words[(long long)tile * E + et] = make_uint4(a, b, cc, dd);
+            n = __popc(a) + __popc(b) + __popc(cc) + __popc(dd);
+          } else {
+            n = a + b + cc + dd;
+          }
+        }
         p.tile_counts[(long long)tile * p.EP + et] = (uint8_t)n;
       }
     }
@@ -842,6 +853,11 @@ int launch_router_mask_umma(const void* x, const void* packed, float mult, uint3
   int rc = encode_tmap_2d_b16(&tmx, x, (uint64_t)d, (uint64_t)N, (uint64_t)d * 2, 64, TILE_M, true);
   if (rc != D2D_OK) return rc == D2D_ERR_BAD_ARG ? D2D_ERR_LAUNCH : rc;
   const bool split = umma_router_splits(N, d, R, E);
+  if (lists && lists->table && !split && tiles > CLUSTER_TILES) {
+    p.mt = mask_table(lists->table, N, E);
+    p.tile_counts = p.mt.counts;
+    lists->tabled = true;
+  }
   if (lists && tiles <= (split ? 1 : CLUSTER_TILES)) {
     p.token_idx = lists->token_idx;
     p.offsets = lists->offsets;

@@ -15,10 +15,12 @@ struct DirectRows {
   const void* last_bias = nullptr;
   int kept = 0;                          // experts a token keeps, where the rule fixes it
 };
-int launch_experts_umma(const void* x, const int32_t* token_idx, const int32_t* offsets,
+// mt: there are no lists yet; the kernel makes them from the table and writes them as well
+int launch_experts_umma(const void* x, int32_t* token_idx, int32_t* offsets,
                         const void* packed, void* out, int64_t N, int d, int E, int H, bool glu,
                         int act, int* dev_status, cudaStream_t s,
-                        NormCapture nc = NormCapture(), DirectRows dr = DirectRows());
+                        NormCapture nc = NormCapture(), DirectRows dr = DirectRows(),
+                        const MaskTable* mt = nullptr);
 
 bool umma_router_supported(int d, int R, int E, int dtype);
 size_t umma_router_packed_bytes(int d, int R, int E);

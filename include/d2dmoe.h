@@ -66,7 +66,8 @@ int d2d_abi_version(void);
 const char* d2d_strerror(int status);
 
 /* Bytes of caller-owned workspace d2d_compact / d2d_moe_forward need for up to
- * n_max tokens.  (The upstream path allocates its scratch inside every call:
+ * n_max tokens.  (d2d_moe_forward also takes the (ceil(n_max/128) + 1) * 4E bytes of earlier versions,
+ * at the price of a launch that writes the lists.)  (The upstream path allocates its scratch inside every call:
  * architectures/moe/moe_impls.py:15,190.) */
 int d2d_workspace_bytes(int64_t n_max, int E, size_t* bytes /* host */);
 
@@ -263,9 +264,9 @@ int d2d_moe_forward_rule(const void* x, const void* wa, const void* wb,
                          void* routing_tensor_opt, void* norms_opt, int norm_layer, int norm_ord,
                          d2d_stream_t stream);
 
-/* Number of kernels the calling thread's last d2d_moe_forward issued (3 on the tensor-core
- * path: router + rule, compaction scatter, expert FFN; 2 on short calls, where the rule's
- * kernel writes the lists; more on the general-shape paths).  Introspection for benchmarks; no upstream counterpart. */
+/* Number of kernels the calling thread's last d2d_moe_forward issued (2 on the tensor-core
+ * path: router + rule, expert FFN; the lists come from the first on short calls and from the second on
+ * long ones; 3 where ws has no room for the table between them; more on the general-shape paths).  Introspection for benchmarks; no upstream counterpart. */
 int d2d_last_forward_launches(void);
 
 /* Test hook, no upstream counterpart.  Every wait inside the tensor-core kernels is bounded;

@@ -414,3 +414,40 @@ def test_every_form_gives_up_and_the_next_call_is_clean(form, N, d, H, E, R, glu
             assert torch.equal(a, b)
         else:      # the order of the adds is free: one rounding each
             assert O.rel_err(a.float().cpu(), b.float().cpu()) <= TOL["bf16"]
+
+
+# N: tiles past the lists' cluster (1024 tokens) to more than one look at the table (96 tiles), ragged
+# ends; E: one to eight 16-cell groups of counts; tau: a token in a hundred to nearly every one
+@pytest.mark.parametrize("N,E,tau", [(1025, 1, 0.3), (1153, 5, 1.0), (1151, 24, 0.2), (2049, 33, 0.9), (5000, 64, 0.02),
+                                     (12801, 97, 0.1), (20011, 128, 0.0), (20000, 16, 0.6)])
+def test_lists_made_by_the_expert_kernel(N, E, tau):
+    """Lists and offsets of a long call, from the table that the router (or the rule on given scores)
+    leaves, against those of the scatter kernel, which a workspace without room for the table gets."""
+    from d2dmoe_b200 import ops
+    d, H, R = 64, 16, 16
+    c, t = _layer(N, d, H, E, R, "bf16", N + E)
+    x2d, wa, wb = _dev(t["x"].reshape(N, d)), _dev(t["wa"]), _dev(t["wb"])
+    w1, b1, w2 = _dev(t["w1"]), _dev(t["b1"]), _dev(t["w2"])
+    rp, ep = ops.prepack_router(wa, wb), ops.prepack_experts(w1, b1, w2)
+    scores = torch.rand(N, E, generator=_gen(N), dtype=torch.float32).to(torch.bfloat16).cuda()
+    for given in (None, scores):
+        got = []
+        for room in (True, False):
+            wsp = ops.Workspace.allocate(N, E, "cuda")
+            if not room:
+                wsp.ws = wsp.ws[: -(-N // 128) * max(16, 1 << (E - 1).bit_length(), 4 * E) + 4 * E]
+            wsp.token_idx.fill_(-1)
+            out = torch.empty(N, d, dtype=torch.bfloat16, device="cuda")
+            ops.moe_forward(x2d, None if given is not None else wa, None if given is not None else wb, tau, w1,
+                            b1, w2, "relu", out, wsp, scores=given, experts_packed=ep,
+                            router_packed=None if given is not None else rp)
+            wsp.check_status()
+            got.append((_lists(wsp, E), out, wsp.mask_bits[:N].clone(), wsp.token_idx.clone()))
+        (l0, o0, m0, i0), (l1, o1, m1, i1) = got
+        assert torch.equal(m0, m1) and np.array_equal(l0[0], l1[0]) and np.array_equal(l0[1], l1[1])
+        assert torch.equal(i0, i1)                       # nothing behind the lists either
+        roff, ridx = O.expert_token_lists(O.unpack_mask(m0.cpu().numpy().view(np.uint32), E))
+        assert np.array_equal(l0[0], np.asarray(roff)) and np.array_equal(l0[1], np.asarray(ridx))
+        # the order of the adds is free: one rounding per expert of a token
+        k = float(l0[0][-1]) / N
+        assert O.rel_err(o0.float().cpu(), o1.float().cpu()) <= TOL["bf16"] * max(1.0, k ** 0.5 / 2)
