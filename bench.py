@@ -820,7 +820,7 @@ def run_ours(args):
                 "api": "MoeficationMoE.forward_host (pinned host x -> pinned host out, 2 slices "
                        "per layer, layers pipelined); bytes are per rank"},
         # kernels per layer call: what the library counted for the last d2d_moe_forward
-        # (router + rule + routing tensor, compaction scatter, expert FFN)
+        # (router + rule + routing tensor, expert FFN with the lists)
         "gpu_launches": steps * stack.layers * launches_per_layer,
         "clocks": clocks, "check": check,
     }

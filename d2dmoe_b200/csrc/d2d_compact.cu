@@ -5,7 +5,8 @@
 // The sort only serves to bring each expert's tokens to the front of its column;
 // a compaction gives the same set per expert, here in ascending token order.
 //
-// Two launches:
+// Two launches, for the calls whose lists neither the rule's kernel (short ones) nor the expert kernel
+// (long ones, from the same counts table and the words beside it) makes:
 //   count   : counts[tile][e] = tokens of the 128-token tile that keep expert e, one BYTE
 //             per cell (a tile holds at most 128 tokens), rows padded to EP cells
 //             (skipped when the router kernel already wrote the table)

@@ -285,16 +285,17 @@ __device__ __forceinline__ int find_token(const Params& p, const Tile* t, uint4*
 // T = sum ceil(n_e / S) <= rows / S + E, so R rounds of G CTAs are enough for S = rows / (R G - E),
 // and R is the least with S <= 128.  (524 rows per SM: five tiles of about 109 rows per CTA
 // instead of four of 128 and one of 12.)  An expert's tiles are equal.
-// The first pass runs, while the previous kernel drains, up to the first tile of a list of one
-// row: instructions that are executed for the first time cost some 20 cycles each, and everything
-// waits for the first tile.  So do the first passes of count_chunk and of the gather warps.
+// Behind a router (the mask table) a first pass runs, while that drains, up to the first tile of a list of
+// one row: instructions that are executed for the first time cost some 20 cycles each, and
+// everything waits for the first tile.  So do the first passes of count_chunk and of the gather warps.
+// (50432 tokens 80.2 -> 76.9 us per layer; behind the kernel of mode 'all', which is over before, 50.6 ->
+// 52.7.  The other roles' code is warm too late: with such passes of theirs 79.7.)
 __device__ void role_list(const Params& p, Ctl* c, int lane, bool one_window) {
   volatile int* af = &c->abort_flag;
   const int E = p.E, G = gridDim.x;
   const bool tabled = p.mt.words != nullptr;
 #pragma unroll 1
-  for (int pass = 0; pass < 2; ++pass) {
-    const bool live = pass != 0;
+  for (bool live = tabled ? first_pass() : in_earnest(), last = live;; live = in_earnest(), last = true) {
     if (live) grid_dependency_wait();
     int off[5], n[4], nt[4];             // experts 4 lane .. + 3
     if (tabled) {
@@ -441,6 +442,7 @@ __device__ void role_list(const Params& p, Ctl* c, int lane, bool one_window) {
       if (lane == 31) p.offsets[E] = off[4];
       if (lane == 31 && off[4] > p.N * (long long)E) report(p.dev_status, D2D_ERR_INDEX_RANGE);
     }
+    if (last) return;
   }
 }
 
@@ -466,7 +468,9 @@ __device__ void role_gather(const Params& p, Ctl* c, uint32_t ring, int w, int l
   RingPos r = {0, 0}, q = {0, 0};
   uint4 x[LOOK];
   x[0] = x[1] = x[2] = make_uint4(0u, 0u, 0u, 0u);
-  bool live = false, ahead = true;       // ahead: this tile's first loads are on their way
+  bool live = tabled ? first_pass() : in_earnest();
+  bool ahead = tabled;                   // this tile's first loads are on their way
+  if (!tabled) grid_dependency_wait();
 #pragma unroll 1
   for (;;) {
     Tile* t = &c->tile[q.s];
@@ -503,7 +507,7 @@ __device__ void role_gather(const Params& p, Ctl* c, uint32_t ring, int w, int l
     }
     if (!live) {                         // the previous kernel's results from here on
       grid_dependency_wait();
-      live = true;
+      live = in_earnest();
       ahead = false;
       continue;
     }
@@ -955,9 +959,16 @@ __global__ void __launch_bounds__(NTHREADS, 1) experts_tiles_kernel(const Params
   // (the list and gather warps wait for the previous kernel in their roles)
   if (warp < WARP_GATHER0 || (warp >= WARP_MMA1 && warp <= WARP_W)) {
     const int w = warp < WARP_GATHER0 ? warp : warp - (WARP_MMA1 - WARP_GATHER0);
-    if (p.mt.words) count_chunk(p, c, w, lane, false);
-    grid_dependency_wait();
-    if (p.mt.words) count_chunk(p, c, w, lane, true);
+    if (p.mt.words) {
+      bool live = first_pass();
+#pragma unroll 1
+      for (int pass = 0; pass < 2; ++pass, live = in_earnest()) {
+        if (live) grid_dependency_wait();
+        count_chunk(p, c, w, lane, live);
+      }
+    } else {
+      grid_dependency_wait();
+    }
   }
 
   if (warp < WARP_DRAIN0) {

@@ -98,6 +98,16 @@ struct Ctl {
   uint32_t init_rows[2][4];
 };
 
+// Whether a role begins in earnest.  Where the kernel also writes the lists (up to eight tiles, one
+// each) it does: the previous call's kernels are over too soon for a first pass without effect (197 tokens
+// 21.2 -> 22.1 us per layer with one); long calls gain by it (12608 tokens x 24 52.3 -> 48.2, 50432 80.0
+// -> 77.3, 65536 x 96 114.4 -> 106.1).
+__device__ __forceinline__ bool first_run(const Params& p) {
+  if (!p.token_idx) return first_pass();
+  grid_dependency_wait();
+  return in_earnest();
+}
+
 __device__ void role_load(const Params& p, Ctl* c, const CUtensorMap* tmx, uint32_t ring,
                           uint32_t wb, uint32_t stage_bytes) {
   volatile int* af = &c->abort_flag;
@@ -106,22 +116,31 @@ __device__ void role_load(const Params& p, Ctl* c, const CUtensorMap* tmx, uint3
   const uint32_t wb_bytes = (uint32_t)(g.kc2 * g.nd * 128);
   bool withheld = (p.withhold & 1) != 0 && blockIdx.x == 0;
   RingPos r = {0, 0};
-  bool first = true;
-  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-    for (int kc = 0; kc < g.kc1; ++kc) {
-      if (!mbar_wait_fast(smem_u32(&c->empty[r.s]), r.ph ^ 1, af, p.dev_status)) return;
+  bool first = true, run = first_run(p);
+  for (int tile = blockIdx.x; tile < tiles;) {
+    const int slices = run ? g.kc1 : 1;
+    for (int kc = 0; kc < slices; ++kc) {
+      if (run && !mbar_wait_fast(smem_u32(&c->empty[r.s]), r.ph ^ 1, af, p.dev_status)) return;
       const uint32_t bar = smem_u32(&c->full[r.s]), dst = ring + r.s * stage_bytes;
-      mbar_arrive_expect_tx(bar, SLOT + g.wa_bytes);
-      tma_load_2d(dst, tmx, kc * 64, tile * TILE_M, bar);
-      if (withheld) withheld = false;
-      else bulk_g2s(dst + SLOT, p.packed + (long long)kc * g.wa_bytes, g.wa_bytes, bar);
-      r.next(g.ns);
+      mbar_arrive_expect_tx(bar, SLOT + g.wa_bytes, run);
+      tma_load_2d(dst, tmx, kc * 64, tile * TILE_M, bar, run);
+      bulk_g2s(dst + SLOT, p.packed + (long long)kc * g.wa_bytes, g.wa_bytes, bar, run && !withheld);
+      if (run) {
+        withheld = false;
+        r.next(g.ns);
+      }
     }
     if (first) {           // after the first tile's stages: Wb is needed only behind its hidden tile
-      first = false;
+      first = !run;
       const uint32_t bar = smem_u32(&c->wb_full);
-      mbar_arrive_expect_tx(bar, wb_bytes);
-      bulk_g2s(wb, p.packed + g.w1_bytes, wb_bytes, bar);
+      mbar_arrive_expect_tx(bar, wb_bytes, run);
+      bulk_g2s(wb, p.packed + g.w1_bytes, wb_bytes, bar, run);
+    }
+    if (run) {
+      tile += gridDim.x;
+    } else {
+      grid_dependency_wait();
+      run = in_earnest();
     }
   }
 }
@@ -136,23 +155,29 @@ __device__ void role_mma1(const Params& p, Ctl* c, uint32_t ring, uint32_t stage
   const uint32_t hi = (uint32_t)(d0 >> 32), lo0 = (uint32_t)d0;
   const int nacc = p.R <= 128 ? 2 : 1;
   RingPos r = {0, 0}, a = {0, 0};
-  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-    if (!mbar_wait_fast(smem_u32(&c->acc1_empty[a.s]), a.ph ^ 1, af, p.dev_status)) return;
+  bool run = first_run(p);
+  for (int tile = blockIdx.x; tile < tiles;) {
+    if (run && !mbar_wait_fast(smem_u32(&c->acc1_empty[a.s]), a.ph ^ 1, af, p.dev_status)) return;
     tc_fence_after();
     const uint32_t acc = tmem + a.s * 128;
-    for (int kc = 0; kc < g.kc1; ++kc) {
-      if (!mbar_wait_fast(smem_u32(&c->full[r.s]), r.ph, af, p.dev_status)) return;
+    const int slices = run ? g.kc1 : 1;
+    for (int kc = 0; kc < slices; ++kc) {
+      if (run && !mbar_wait_fast(smem_u32(&c->full[r.s]), r.ph, af, p.dev_status)) return;
       tc_fence_after();
       const uint32_t alo = lo0 + r.s * (stage_bytes >> 4), blo = alo + (SLOT >> 4);
 #pragma unroll
       for (uint32_t k = 0; k < 4; ++k)
         umma_bf16(acc, ((uint64_t)hi << 32) | (alo + 2 * k), ((uint64_t)hi << 32) | (blo + 2 * k),
-                  idesc, (kc | k) != 0);
-      umma_commit(smem_u32(&c->empty[r.s]));
-      r.next(g.ns);
+                  idesc, (kc | k) != 0, run);
+      umma_commit(smem_u32(&c->empty[r.s]), run);
+      if (run) r.next(g.ns);
     }
-    umma_commit(smem_u32(&c->acc1_full[a.s]));
-    a.next(nacc);
+    umma_commit(smem_u32(&c->acc1_full[a.s]), run);
+    if (run) {
+      a.next(nacc);
+      tile += gridDim.x;
+    }
+    run = in_earnest();
   }
 }
 
@@ -165,18 +190,26 @@ __device__ void role_mma2(const Params& p, Ctl* c, uint32_t wb, uint32_t tmem) {
   const uint32_t hi = (uint32_t)(d0 >> 32), lo0 = (uint32_t)d0;
   const int ksteps = p.R >> 4;
   uint32_t ph = 0;
-  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ph ^= 1) {
-    if (tile == (int)blockIdx.x &&
-        !mbar_wait_fast(smem_u32(&c->wb_full), 0, af, p.dev_status))
-      return;
-    if (!mbar_wait_fast(smem_u32(&c->acc2_empty), ph ^ 1, af, p.dev_status)) return;
-    if (!mbar_wait_fast(smem_u32(&c->hid_full), ph, af, p.dev_status)) return;
+  bool run = first_run(p);
+  for (int tile = blockIdx.x; tile < tiles;) {
+    if (run) {
+      if (tile == (int)blockIdx.x &&
+          !mbar_wait_fast(smem_u32(&c->wb_full), 0, af, p.dev_status))
+        return;
+      if (!mbar_wait_fast(smem_u32(&c->acc2_empty), ph ^ 1, af, p.dev_status)) return;
+      if (!mbar_wait_fast(smem_u32(&c->hid_full), ph, af, p.dev_status)) return;
+    }
     tc_fence_after();
     for (int k = 0; k < ksteps; ++k)
       umma_bf16_ta(tmem + TM_ACC2, tmem + TM_HID + 8 * k,
                    ((uint64_t)hi << 32) | (lo0 + (uint32_t)(k >> 2) * (g.nd * 8) + 2 * (k & 3)),
-                   idesc, k != 0);
-    umma_commit(smem_u32(&c->g2_done));
+                   idesc, k != 0, run);
+    umma_commit(smem_u32(&c->g2_done), run);
+    if (run) {
+      tile += gridDim.x;
+      ph ^= 1;
+    }
+    run = in_earnest();
   }
 }
 
@@ -199,10 +232,14 @@ __device__ void role_hidden(const Params& p, Ctl* c, uint32_t tmem, int et) {
   const int nacc = p.R <= 128 ? 2 : 1;
   RingPos a = {0, 0};
   uint32_t ph = 0;
-  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ph ^= 1) {
-    if (!mbar_wait_warp(smem_u32(&c->acc1_full[a.s]), a.ph, af, p.dev_status)) return;
-    // the previous tile's second product has read the hidden tile
-    if (!mbar_wait_warp(smem_u32(&c->g2_done), ph ^ 1, af, p.dev_status)) return;
+  bool run = first_run(p);
+#pragma unroll 1
+  for (int tile = blockIdx.x; tile < tiles;) {
+    if (run) {
+      if (!mbar_wait_warp(smem_u32(&c->acc1_full[a.s]), a.ph, af, p.dev_status)) return;
+      // the previous tile's second product has read the hidden tile
+      if (!mbar_wait_warp(smem_u32(&c->g2_done), ph ^ 1, af, p.dev_status)) return;
+    }
     tc_fence_after();
     const uint32_t src = tmem + lane_base + a.s * 128, dst = tmem + lane_base + TM_HID;
     for (int c0 = 0; c0 < p.R; c0 += 16) {
@@ -214,9 +251,14 @@ __device__ void role_hidden(const Params& p, Ctl* c, uint32_t tmem, int et) {
     }
     tmem_wait_st();
     tc_fence_before();
-    mbar_arrive(smem_u32(&c->acc1_empty[a.s]));
-    mbar_arrive(smem_u32(&c->hid_full));
-    a.next(nacc);
+    mbar_arrive(smem_u32(&c->acc1_empty[a.s]), run);
+    mbar_arrive(smem_u32(&c->hid_full), run);
+    if (run) {
+      a.next(nacc);
+      tile += gridDim.x;
+      ph ^= 1;
+    }
+    run = in_earnest();
   }
 }
 
@@ -249,10 +291,12 @@ __device__ void role_gate(const Params& p, Ctl* c, uint32_t tmem, int et) {
   const int nw = (E + 31) >> 5;                       // == NW
   const uint32_t lane_base = (uint32_t)(et & ~31) << 16;
   uint32_t ph = 0, buf = 0, ibuf_ph = 0;
-  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ph ^= 1, buf ^= 1) {
+  bool run = first_run(p);                    // first pass: as if no row were there
+#pragma unroll 1
+  for (int tile = blockIdx.x; tile < tiles;) {
     const long long trow = (long long)tile * TILE_M + et;
-    const bool live = trow < p.N;
-    if (!mbar_wait_warp(smem_u32(&c->g2_done), ph, af, p.dev_status)) return;
+    const bool live = run && trow < p.N;
+    if (run && !mbar_wait_warp(smem_u32(&c->g2_done), ph, af, p.dev_status)) return;
     tc_fence_after();
     uint32_t s[NB * 8];
 #pragma unroll
@@ -268,7 +312,7 @@ __device__ void role_gate(const Params& p, Ctl* c, uint32_t tmem, int et) {
       }
     }
     tc_fence_before();
-    mbar_arrive(smem_u32(&c->acc2_empty));
+    mbar_arrive(smem_u32(&c->acc2_empty), run);
     // columns past E have zero weights, hence score 0: no effect on a maximum of magnitudes
     __nv_bfloat162 m2 = *reinterpret_cast<const __nv_bfloat162*>(&s[0]);
 #pragma unroll
@@ -281,7 +325,8 @@ __device__ void role_gate(const Params& p, Ctl* c, uint32_t tmem, int et) {
 #pragma unroll
     for (int j = 0; j < (RULE != 0 ? 2 : NW); ++j) word[j] = 0u;
     if (RULE != 0) {
-      ranked_words<bf16, NB * 16, RULE>(reinterpret_cast<const bf16*>(s), E, p.k, p.tau, word);
+      ranked_words<bf16, NB * 16, RULE>(reinterpret_cast<const bf16*>(s), run ? E : 1, run ? p.k : 1, p.tau,
+                                        word);
 #pragma unroll
       for (int q = 0; q < NB * 8; ++q)
         s[q] = ((word[0] >> (2 * q)) & 1u ? 0x3f80u : 0u) |
@@ -306,13 +351,13 @@ __device__ void role_gate(const Params& p, Ctl* c, uint32_t tmem, int et) {
     if (p.out_init && !p.init_all) {
       const bool todo = live && kept != 1;
       const uint32_t rows = __ballot_sync(0xffffffffu, todo);
-      if (!mbar_wait_warp(smem_u32(&c->init_empty[buf]), ibuf_ph ^ 1, af, p.dev_status)) return;
+      if (run && !mbar_wait_warp(smem_u32(&c->init_empty[buf]), ibuf_ph ^ 1, af, p.dev_status)) return;
       if (lane == 0) {
         c->init_rows[buf][q4] = rows;
-        mbar_arrive(smem_u32(&c->init_full[buf]));
+        mbar_arrive(smem_u32(&c->init_full[buf]), run);
       }
       __syncwarp();
-      ibuf_ph ^= buf;
+      if (run) ibuf_ph ^= buf;
     }
     if (p.token_idx) {         // (the only tile: both halves of cnt are free)
 #pragma unroll
@@ -327,24 +372,77 @@ __device__ void role_gate(const Params& p, Ctl* c, uint32_t tmem, int et) {
       // one barrier per tile: the other half of cnt is written before anybody passes it again (an
       // mbarrier, because a warp that gave up never comes)
       __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&c->cnt_full));
-      if (!mbar_wait_warp(smem_u32(&c->cnt_full), ph, af, p.dev_status)) return;
+      if (lane == 0) mbar_arrive(smem_u32(&c->cnt_full), run);
+      if (run && !mbar_wait_warp(smem_u32(&c->cnt_full), ph, af, p.dev_status)) return;
       if (et < p.EP) {
         int n = 0;
         if (et < E) {
           const int a = c->cnt[buf][0][et], b = c->cnt[buf][1][et], cc = c->cnt[buf][2][et],
                     dd = c->cnt[buf][3][et];
           if (p.mt.words) {
-            p.mt.words[(long long)tile * E + et] = make_uint4(a, b, cc, dd);
+            if (run) p.mt.words[(long long)tile * E + et] = make_uint4(a, b, cc, dd);
             n = __popc(a) + __popc(b) + __popc(cc) + __popc(dd);
           } else {
             n = a + b + cc + dd;
           }
         }
-        p.tile_counts[(long long)tile * p.EP + et] = (uint8_t)n;
+        if (run) p.tile_counts[(long long)tile * p.EP + et] = (uint8_t)n;
       }
     }
     if (p.rt_out && live) store_row<NB>(p.rt_out + trow * E, s, E);
+    if (run) {
+      tile += gridDim.x;
+      ph ^= 1;
+      buf ^= 1;
+    } else {
+      grid_dependency_wait();
+      run = in_earnest();
+    }
+  }
+}
+
+// warps 12-15 where every row is initialised with the layer's own input: out of the stages of the first
+// product, which then wait for these warps as well.  Warp w has rows 32 w .. + 31.  (Read
+// again from memory, eight rows at a time: 12608 x 768 took 26 thousand cycles, twice the rest of the tile.)
+__device__ void role_init_stages(const Params& p, Ctl* c, uint32_t ring, uint32_t stage_bytes, int w,
+                                 int lane) {
+  volatile int* af = &c->abort_flag;
+  const int tiles = (int)((p.N + TILE_M - 1) / TILE_M), j = lane & 7, r4 = lane >> 3;
+  RingPos r = {0, 0};
+  bool run = first_run(p);
+#pragma unroll 1
+  for (int tile = blockIdx.x; tile < tiles;) {
+    const long long row0 = (long long)tile * TILE_M + 32 * w + r4;
+    const int slices = run ? p.g.kc1 : 1;
+#pragma unroll 1
+    for (int kc = 0; kc < slices; ++kc) {
+      uint4 bz = make_uint4(0u, 0u, 0u, 0u), v[8];
+      if (run) {
+        if (p.last_bias) bz = __ldg(reinterpret_cast<const uint4*>(p.last_bias) + kc * 8 + j);
+        if (!mbar_wait_warp(smem_u32(&c->full[r.s]), r.ph, af, p.dev_status)) return;
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int row = 32 * w + 4 * i + r4;
+        v[i] = ld_shared_v4(ring + r.s * stage_bytes + (row >> 3) * 1024 + (row & 7) * 128 +
+                            ((j ^ (row & 7)) << 4));
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (run && row0 + 4 * i < p.N)
+          *(reinterpret_cast<uint4*>(p.out_init + (row0 + 4 * i) * p.d) + kc * 8 + j) =
+              add_bf16x8(bz, v[i]);
+      // behind the stores, which have waited for what was loaded: an arrival does not wait for loads under way
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&c->empty[r.s]), run);
+      if (run) r.next(p.g.ns);
+    }
+    if (run) {
+      tile += gridDim.x;
+    } else {
+      grid_dependency_wait();
+      run = in_earnest();
+    }
   }
 }
 
@@ -356,11 +454,15 @@ __device__ void role_init(const Params& p, Ctl* c, int w, int lane) {
   const int tiles = (int)((p.N + TILE_M - 1) / TILE_M);
   const int v8 = p.d >> 3;
   uint32_t ph = 0, buf = 0;
-  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ph ^= buf, buf ^= 1) {
+  bool run = first_run(p);                    // first pass: one row that is neither read nor written
+#pragma unroll 1
+  for (int tile = blockIdx.x; tile < tiles;) {
     bool share = false;
     int q = w;
     uint32_t rows;
-    if (p.init_all) {                  // no need to know what the gate says
+    if (!run) {
+      rows = 1u;
+    } else if (p.init_all) {           // no need to know what the gate says
       const long long left = p.N - (long long)tile * TILE_M;
       share = left <= 32;
       q = share ? 0 : w;
@@ -374,15 +476,15 @@ __device__ void role_init(const Params& p, Ctl* c, int w, int lane) {
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&c->init_empty[buf]));
     }
-    if (rows == 0u) continue;
     const long long row0 = (long long)tile * TILE_M + 32 * q;
-    const int step = share ? 128 : 32;
-    for (int c8 = lane + (share ? 32 * w : 0); c8 < v8; c8 += step) {
+    const int step = share ? 128 : 32, c8n = rows == 0u ? 0 : run ? v8 : 32;
+#pragma unroll 1
+    for (int c8 = lane + (share ? 32 * w : 0); c8 < c8n; c8 += step) {
       uint4 bz = make_uint4(0u, 0u, 0u, 0u);
-      if (p.last_bias) bz = __ldg(reinterpret_cast<const uint4*>(p.last_bias) + c8);
+      if (p.last_bias && run) bz = __ldg(reinterpret_cast<const uint4*>(p.last_bias) + c8);
       if (!p.resid) {
         for (uint32_t m = rows; m != 0u; m &= m - 1)
-          *(reinterpret_cast<uint4*>(p.out_init + (row0 + __ffs(m) - 1) * p.d) + c8) = bz;
+          if (run) *(reinterpret_cast<uint4*>(p.out_init + (row0 + __ffs(m) - 1) * p.d) + c8) = bz;
         continue;
       }
       for (uint32_t m = rows; m != 0u;) {
@@ -390,7 +492,7 @@ __device__ void role_init(const Params& p, Ctl* c, int w, int lane) {
         int rr[8];
 #pragma unroll
         for (int u = 0; u < 8; ++u) {        // eight rows in flight
-          rr[u] = m != 0u ? __ffs(m) - 1 : -1;
+          rr[u] = m != 0u && run ? __ffs(m) - 1 : -1;
           m &= m - 1;
           if (rr[u] >= 0)
             xv[u] = __ldg(reinterpret_cast<const uint4*>(p.resid + (row0 + rr[u]) * p.d) + c8);
@@ -401,6 +503,14 @@ __device__ void role_init(const Params& p, Ctl* c, int w, int lane) {
             *(reinterpret_cast<uint4*>(p.out_init + (row0 + rr[u]) * p.d) + c8) =
                 add_bf16x8(bz, xv[u]);
       }
+    }
+    if (run) {
+      tile += gridDim.x;
+      ph ^= buf;
+      buf ^= 1;
+    } else {
+      grid_dependency_wait();
+      run = in_earnest();
     }
   }
 }
@@ -424,7 +534,7 @@ router_tiles_kernel(const Params p, const __grid_constant__ CUtensorMap tmx) {
   if (tid == 0) {
     for (int i = 0; i < NS_MAX; ++i) {
       mbar_init(smem_u32(&c->full[i]), 1);
-      mbar_init(smem_u32(&c->empty[i]), 1);
+      mbar_init(smem_u32(&c->empty[i]), p.out_init && p.init_all && p.resid ? 5 : 1);
     }
     mbar_init(smem_u32(&c->wb_full), 1);
     mbar_init(smem_u32(&c->hid_full), 128);
@@ -446,9 +556,9 @@ router_tiles_kernel(const Params p, const __grid_constant__ CUtensorMap tmx) {
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  grid_dependency_wait();
   const uint32_t tmem = c->tmem_base;
 
+  // (roles that touch global memory wait for the previous kernel behind their first pass)
   if (warp < 4) {
     role_hidden(p, c, tmem, tid);
   } else if (warp < 8) {
@@ -477,7 +587,8 @@ router_tiles_kernel(const Params p, const __grid_constant__ CUtensorMap tmx) {
     if (elect_one()) role_load(p, c, &tmx, base, wb, stage_bytes);
     __syncwarp();
   } else if (warp >= WARP_INIT0 && p.out_init) {
-    role_init(p, c, warp - WARP_INIT0, tid & 31);
+    if (p.init_all && p.resid) role_init_stages(p, c, base, stage_bytes, warp - WARP_INIT0, tid & 31);
+    else role_init(p, c, warp - WARP_INIT0, tid & 31);
   }
 
   // A launch that gave up may still have copies and MMAs in flight that use this CTA's
@@ -492,6 +603,7 @@ router_tiles_kernel(const Params p, const __grid_constant__ CUtensorMap tmx) {
     tmem_dealloc(tmem, 512);
   }
   if (p.token_idx) {
+    grid_dependency_wait();
     uint32_t* rows = reinterpret_cast<uint32_t*>(&c->cnt[0][0][0]);
     if (*reinterpret_cast<volatile int*>(&c->abort_flag) != 0) {     // nothing a list may rely on
       for (int i = tid; i < 4 * MAX_E; i += NTHREADS) rows[i] = 0u;

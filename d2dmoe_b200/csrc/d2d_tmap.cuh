@@ -21,11 +21,12 @@ int encode_tmap_2d_b16(CUtensorMap* map, const void* base, uint64_t inner, uint6
 namespace umma {
 // one box at (column c0, row r0); rows past the tensor's end arrive as zeros
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int c0, int r0,
-                                            uint32_t bar) {
+                                            uint32_t bar, bool run = true) {
   asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
-      "[%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
-      "l"(map), "r"(c0), "r"(r0), "r"(bar)
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %5, 0;\n\t"
+      "@p cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
+      "[%0], [%1, {%2, %3}], [%4];\n\t}" ::"r"(dst),
+      "l"(map), "r"(c0), "r"(r0), "r"(bar), "r"((int)run)
       : "memory");
 }
 }  // namespace umma

@@ -448,6 +448,7 @@ def test_lists_made_by_the_expert_kernel(N, E, tau):
         assert torch.equal(i0, i1)                       # nothing behind the lists either
         roff, ridx = O.expert_token_lists(O.unpack_mask(m0.cpu().numpy().view(np.uint32), E))
         assert np.array_equal(l0[0], np.asarray(roff)) and np.array_equal(l0[1], np.asarray(ridx))
-        # the order of the adds is free: one rounding per expert of a token
-        k = float(l0[0][-1]) / N
-        assert O.rel_err(o0.float().cpu(), o1.float().cpu()) <= TOL["bf16"] * max(1.0, k ** 0.5 / 2)
+        # the order of the adds is free: either side rounds once per expert of a token, half an ulp (2^-9) of
+        # a running sum each; a token whose hidden layer is all zero ties all experts and keeps them
+        kmax = int(O.unpack_mask(m0.cpu().numpy().view(np.uint32), E).sum(1).max())
+        assert O.rel_err(o0.float().cpu(), o1.float().cpu()) <= kmax * 2.0 ** -8
