@@ -98,16 +98,22 @@ struct Ctl {
   uint32_t init_rows[2][4];
 };
 
-// Whether a role begins in earnest.  Where the kernel also writes the lists (up to eight tiles, one
-// each) it does: the previous call's kernels are over too soon for a first pass without effect (197 tokens
-// 21.2 -> 22.1 us per layer with one); long calls gain by it (12608 tokens x 24 52.3 -> 48.2, 50432 80.0
-// -> 77.3, 65536 x 96 114.4 -> 106.1).
-__device__ __forceinline__ bool first_run(const Params& p) {
-  if (!p.token_idx) return first_pass();
+// WARM: a role's first pass is without effect.  Where the kernel also writes the lists (up to eight tiles,
+// one each) there is none: the previous call's kernels are over too soon for it, and its branches alone
+// make a call whose code is executed once longer (197 tokens 21.2 -> 22.4 us per layer).  Long calls
+// gain by it (12608 tokens x 24 52.3 -> 48.2, 50432 80.0 -> 77.3, 65536 x 96 114.4 -> 106.1).
+template <bool WARM>
+__device__ __forceinline__ bool first_run() {
+  if (WARM) return first_pass();
   grid_dependency_wait();
-  return in_earnest();
+  return true;
+}
+template <bool WARM>
+__device__ __forceinline__ bool next_run() {
+  return WARM ? in_earnest() : true;
 }
 
+template <bool WARM>
 __device__ void role_load(const Params& p, Ctl* c, const CUtensorMap* tmx, uint32_t ring,
                           uint32_t wb, uint32_t stage_bytes) {
   volatile int* af = &c->abort_flag;
@@ -116,7 +122,7 @@ __device__ void role_load(const Params& p, Ctl* c, const CUtensorMap* tmx, uint3
   const uint32_t wb_bytes = (uint32_t)(g.kc2 * g.nd * 128);
   bool withheld = (p.withhold & 1) != 0 && blockIdx.x == 0;
   RingPos r = {0, 0};
-  bool first = true, run = first_run(p);
+  bool first = true, run = first_run<WARM>();
   for (int tile = blockIdx.x; tile < tiles;) {
     const int slices = run ? g.kc1 : 1;
     for (int kc = 0; kc < slices; ++kc) {
@@ -140,11 +146,12 @@ __device__ void role_load(const Params& p, Ctl* c, const CUtensorMap* tmx, uint3
       tile += gridDim.x;
     } else {
       grid_dependency_wait();
-      run = in_earnest();
+      run = next_run<WARM>();
     }
   }
 }
 
+template <bool WARM>
 __device__ void role_mma1(const Params& p, Ctl* c, uint32_t ring, uint32_t stage_bytes,
                           uint32_t tmem) {
   volatile int* af = &c->abort_flag;
@@ -155,7 +162,7 @@ __device__ void role_mma1(const Params& p, Ctl* c, uint32_t ring, uint32_t stage
   const uint32_t hi = (uint32_t)(d0 >> 32), lo0 = (uint32_t)d0;
   const int nacc = p.R <= 128 ? 2 : 1;
   RingPos r = {0, 0}, a = {0, 0};
-  bool run = first_run(p);
+  bool run = first_run<WARM>();
   for (int tile = blockIdx.x; tile < tiles;) {
     if (run && !mbar_wait_fast(smem_u32(&c->acc1_empty[a.s]), a.ph ^ 1, af, p.dev_status)) return;
     tc_fence_after();
@@ -177,10 +184,11 @@ __device__ void role_mma1(const Params& p, Ctl* c, uint32_t ring, uint32_t stage
       a.next(nacc);
       tile += gridDim.x;
     }
-    run = in_earnest();
+    run = next_run<WARM>();
   }
 }
 
+template <bool WARM>
 __device__ void role_mma2(const Params& p, Ctl* c, uint32_t wb, uint32_t tmem) {
   volatile int* af = &c->abort_flag;
   const Geo& g = p.g;
@@ -190,7 +198,7 @@ __device__ void role_mma2(const Params& p, Ctl* c, uint32_t wb, uint32_t tmem) {
   const uint32_t hi = (uint32_t)(d0 >> 32), lo0 = (uint32_t)d0;
   const int ksteps = p.R >> 4;
   uint32_t ph = 0;
-  bool run = first_run(p);
+  bool run = first_run<WARM>();
   for (int tile = blockIdx.x; tile < tiles;) {
     if (run) {
       if (tile == (int)blockIdx.x &&
@@ -209,7 +217,7 @@ __device__ void role_mma2(const Params& p, Ctl* c, uint32_t wb, uint32_t tmem) {
       tile += gridDim.x;
       ph ^= 1;
     }
-    run = in_earnest();
+    run = next_run<WARM>();
   }
 }
 
@@ -225,6 +233,7 @@ __device__ __forceinline__ void relu_pairs(const uint32_t* v, uint32_t* w) {
 }
 
 // warps 0-3, thread = tile row = TMEM lane: hidden tile = bf16 relu of accumulator 1
+template <bool WARM>
 __device__ void role_hidden(const Params& p, Ctl* c, uint32_t tmem, int et) {
   volatile int* af = &c->abort_flag;
   const int tiles = (int)((p.N + TILE_M - 1) / TILE_M);
@@ -232,7 +241,7 @@ __device__ void role_hidden(const Params& p, Ctl* c, uint32_t tmem, int et) {
   const int nacc = p.R <= 128 ? 2 : 1;
   RingPos a = {0, 0};
   uint32_t ph = 0;
-  bool run = first_run(p);
+  bool run = first_run<WARM>();
 #pragma unroll 1
   for (int tile = blockIdx.x; tile < tiles;) {
     if (run) {
@@ -258,7 +267,7 @@ __device__ void role_hidden(const Params& p, Ctl* c, uint32_t tmem, int et) {
       tile += gridDim.x;
       ph ^= 1;
     }
-    run = in_earnest();
+    run = next_run<WARM>();
   }
 }
 
@@ -282,7 +291,7 @@ __device__ __forceinline__ void store_row(bf16* dst, const uint32_t* s, int E) {
 
 // warps 4-7, thread = tile row: the row's scores stay in registers as packed bf16 pairs
 // (NB blocks of 16 experts), so tensor memory is read once and handed back at once
-template <int NB, int RULE>
+template <int NB, int RULE, bool WARM>
 __device__ void role_gate(const Params& p, Ctl* c, uint32_t tmem, int et) {
   volatile int* af = &c->abort_flag;
   const int tiles = (int)((p.N + TILE_M - 1) / TILE_M);
@@ -291,7 +300,7 @@ __device__ void role_gate(const Params& p, Ctl* c, uint32_t tmem, int et) {
   const int nw = (E + 31) >> 5;                       // == NW
   const uint32_t lane_base = (uint32_t)(et & ~31) << 16;
   uint32_t ph = 0, buf = 0, ibuf_ph = 0;
-  bool run = first_run(p);                    // first pass: as if no row were there
+  bool run = first_run<WARM>();                    // first pass: as if no row were there
 #pragma unroll 1
   for (int tile = blockIdx.x; tile < tiles;) {
     const long long trow = (long long)tile * TILE_M + et;
@@ -396,7 +405,7 @@ __device__ void role_gate(const Params& p, Ctl* c, uint32_t tmem, int et) {
       buf ^= 1;
     } else {
       grid_dependency_wait();
-      run = in_earnest();
+      run = next_run<WARM>();
     }
   }
 }
@@ -404,12 +413,13 @@ __device__ void role_gate(const Params& p, Ctl* c, uint32_t tmem, int et) {
 // warps 12-15 where every row is initialised with the layer's own input: out of the stages of the first
 // product, which then wait for these warps as well.  Warp w has rows 32 w .. + 31.  (Read
 // again from memory, eight rows at a time: 12608 x 768 took 26 thousand cycles, twice the rest of the tile.)
+template <bool WARM>
 __device__ void role_init_stages(const Params& p, Ctl* c, uint32_t ring, uint32_t stage_bytes, int w,
                                  int lane) {
   volatile int* af = &c->abort_flag;
   const int tiles = (int)((p.N + TILE_M - 1) / TILE_M), j = lane & 7, r4 = lane >> 3;
   RingPos r = {0, 0};
-  bool run = first_run(p);
+  bool run = first_run<WARM>();
 #pragma unroll 1
   for (int tile = blockIdx.x; tile < tiles;) {
     const long long row0 = (long long)tile * TILE_M + 32 * w + r4;
@@ -441,7 +451,7 @@ __device__ void role_init_stages(const Params& p, Ctl* c, uint32_t ring, uint32_
       tile += gridDim.x;
     } else {
       grid_dependency_wait();
-      run = in_earnest();
+      run = next_run<WARM>();
     }
   }
 }
@@ -449,12 +459,13 @@ __device__ void role_init_stages(const Params& p, Ctl* c, uint32_t ring, uint32_
 // warps 12-15: the initial rows of the tile's tokens that ask for one.  Warp w has rows 32 w .. + 31;
 // where only the first 32 have any (a call of few tokens) the warps share a row instead, every
 // fourth 512-byte piece each (32 tokens x 2048: 12 -> 4 us).
+template <bool WARM>
 __device__ void role_init(const Params& p, Ctl* c, int w, int lane) {
   volatile int* af = &c->abort_flag;
   const int tiles = (int)((p.N + TILE_M - 1) / TILE_M);
   const int v8 = p.d >> 3;
   uint32_t ph = 0, buf = 0;
-  bool run = first_run(p);                    // first pass: one row that is neither read nor written
+  bool run = first_run<WARM>();                    // first pass: one row that is neither read nor written
 #pragma unroll 1
   for (int tile = blockIdx.x; tile < tiles;) {
     bool share = false;
@@ -510,13 +521,13 @@ __device__ void role_init(const Params& p, Ctl* c, int w, int lane) {
       buf ^= 1;
     } else {
       grid_dependency_wait();
-      run = in_earnest();
+      run = next_run<WARM>();
     }
   }
 }
 
-// RULE: 0, or D2D_RULE_TOPK / D2D_RULE_DYNK (E <= 32)
-template <int RULE>
+// RULE: 0, or D2D_RULE_TOPK / D2D_RULE_DYNK (E <= 32).  WARM: see first_run
+template <int RULE, bool WARM>
 __global__ void __launch_bounds__(NTHREADS, 1)
 router_tiles_kernel(const Params p, const __grid_constant__ CUtensorMap tmx) {
   extern __shared__ uint8_t smem_raw[];
@@ -560,35 +571,35 @@ router_tiles_kernel(const Params p, const __grid_constant__ CUtensorMap tmx) {
 
   // (roles that touch global memory wait for the previous kernel behind their first pass)
   if (warp < 4) {
-    role_hidden(p, c, tmem, tid);
+    role_hidden<WARM>(p, c, tmem, tid);
   } else if (warp < 8) {
     if (RULE != 0) {
-      if (p.g.nd == 16) role_gate<1, RULE>(p, c, tmem, tid - 128);
-      else role_gate<2, RULE>(p, c, tmem, tid - 128);
+      if (p.g.nd == 16) role_gate<1, RULE, WARM>(p, c, tmem, tid - 128);
+      else role_gate<2, RULE, WARM>(p, c, tmem, tid - 128);
     } else {
       switch (p.g.nd >> 4) {
-        case 1: role_gate<1, 0>(p, c, tmem, tid - 128); break;
-        case 2: role_gate<2, 0>(p, c, tmem, tid - 128); break;
-        case 3: role_gate<3, 0>(p, c, tmem, tid - 128); break;
-        case 4: role_gate<4, 0>(p, c, tmem, tid - 128); break;
-        case 5: role_gate<5, 0>(p, c, tmem, tid - 128); break;
-        case 6: role_gate<6, 0>(p, c, tmem, tid - 128); break;
-        case 7: role_gate<7, 0>(p, c, tmem, tid - 128); break;
-        default: role_gate<8, 0>(p, c, tmem, tid - 128); break;
+        case 1: role_gate<1, 0, WARM>(p, c, tmem, tid - 128); break;
+        case 2: role_gate<2, 0, WARM>(p, c, tmem, tid - 128); break;
+        case 3: role_gate<3, 0, WARM>(p, c, tmem, tid - 128); break;
+        case 4: role_gate<4, 0, WARM>(p, c, tmem, tid - 128); break;
+        case 5: role_gate<5, 0, WARM>(p, c, tmem, tid - 128); break;
+        case 6: role_gate<6, 0, WARM>(p, c, tmem, tid - 128); break;
+        case 7: role_gate<7, 0, WARM>(p, c, tmem, tid - 128); break;
+        default: role_gate<8, 0, WARM>(p, c, tmem, tid - 128); break;
       }
     }
   } else if (warp == WARP_MMA1) {
-    if (elect_one()) role_mma1(p, c, base, stage_bytes, tmem);
+    if (elect_one()) role_mma1<WARM>(p, c, base, stage_bytes, tmem);
     __syncwarp();
   } else if (warp == WARP_MMA2) {
-    if (elect_one()) role_mma2(p, c, wb, tmem);
+    if (elect_one()) role_mma2<WARM>(p, c, wb, tmem);
     __syncwarp();
   } else if (warp == WARP_LOAD) {
-    if (elect_one()) role_load(p, c, &tmx, base, wb, stage_bytes);
+    if (elect_one()) role_load<WARM>(p, c, &tmx, base, wb, stage_bytes);
     __syncwarp();
   } else if (warp >= WARP_INIT0 && p.out_init) {
-    if (p.init_all && p.resid) role_init_stages(p, c, base, stage_bytes, warp - WARP_INIT0, tid & 31);
-    else role_init(p, c, warp - WARP_INIT0, tid & 31);
+    if (p.init_all && p.resid) role_init_stages<WARM>(p, c, base, stage_bytes, warp - WARP_INIT0, tid & 31);
+    else role_init<WARM>(p, c, warp - WARP_INIT0, tid & 31);
   }
 
   // A launch that gave up may still have copies and MMAs in flight that use this CTA's
@@ -986,9 +997,12 @@ int launch_router_mask_umma(const void* x, const void* packed, float mult, uint3
   }
   const size_t smem = smem_bytes(p.g);
   int sms = 0;
-  auto kernel = rule == D2D_RULE_TOPK   ? router_tiles_kernel<D2D_RULE_TOPK>
-                : rule == D2D_RULE_DYNK ? router_tiles_kernel<D2D_RULE_DYNK>
-                                        : router_tiles_kernel<0>;
+  auto kernel = rule == D2D_RULE_TOPK   ? (p.token_idx ? router_tiles_kernel<D2D_RULE_TOPK, false>
+                                                       : router_tiles_kernel<D2D_RULE_TOPK, true>)
+                : rule == D2D_RULE_DYNK ? (p.token_idx ? router_tiles_kernel<D2D_RULE_DYNK, false>
+                                                       : router_tiles_kernel<D2D_RULE_DYNK, true>)
+                                        : (p.token_idx ? router_tiles_kernel<0, false>
+                                                       : router_tiles_kernel<0, true>);
   rc = device_launch_facts((const void*)kernel, smem, &sms);
   if (rc != D2D_OK) return rc;
   const int64_t grid = tiles < sms ? tiles : sms;
