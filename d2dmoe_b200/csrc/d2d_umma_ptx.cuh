@@ -257,12 +257,6 @@ __device__ __forceinline__ void tmem_wait_ld32(uint32_t* v) {
                    "+r"(v[30]), "+r"(v[31])
                ::"memory");
 }
-__device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c,
-                                             uint32_t d) {
-  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c),
-               "r"(d)
-               : "memory");
-}
 
 // One lane of a converged warp.  Unlike a test on the lane id, elect.sync tells the
 // compiler that exactly one thread runs the guarded code, so warp-uniform operands of

@@ -452,3 +452,21 @@ def test_lists_made_by_the_expert_kernel(N, E, tau):
         # a running sum each; a token whose hidden layer is all zero ties all experts and keeps them
         kmax = int(O.unpack_mask(m0.cpu().numpy().view(np.uint32), E).sum(1).max())
         assert O.rel_err(o0.float().cpu(), o1.float().cpu()) <= kmax * 2.0 ** -8
+
+
+@pytest.mark.parametrize("bias", [True, False])
+@pytest.mark.parametrize("N,d", [(1, 64), (129, 768), (1025, 512), (18945, 768), (20011, 128)])
+def test_initial_rows_of_a_residual_layer(N, d, bias):
+    """x + last_bias, one rounding, exactly: the rows come out of the stages of the router's first product (one
+    stage to several laps of the ring, one tile to two per CTA, a last tile of one row)."""
+    from d2dmoe_b200 import ops
+    E, R = 12, 128
+    c, t = _layer(N, d, 16, E, R, "bf16", N + d)
+    x2d, wa, wb = _dev(t["x"].reshape(N, d)), _dev(t["wa"]), _dev(t["wb"])
+    lb = _dev(t["last_bias"].reshape(-1)) if bias else None
+    packed, wsp = ops.prepack_router(wa, wb), ops.Workspace.allocate(N, E, "cuda")
+    for _ in range(8):
+        out = torch.full((N, d), float("nan"), dtype=torch.bfloat16, device="cuda")
+        ops.router_mask(x2d, wa, wb, 0.3, wsp, packed=packed, out_init=out, last_bias=lb, add_residual=True)
+        wsp.check_status()
+        assert torch.equal(out, x2d + lb if bias else x2d + 0)
