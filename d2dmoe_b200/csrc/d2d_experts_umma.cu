@@ -426,7 +426,7 @@ __device__ void role_list(const Params& p, Ctl* c, int lane, bool one_window) {
       }
       __syncwarp();
       if (live) mbar_arrive(smem_u32(&c->tile_full[r.s]));
-      const float4 b1 = 4 * lane < p.H
+      const float4 b1 = live && 4 * lane < p.H         // (no global read before the wait)
                             ? __ldg(reinterpret_cast<const float4*>(
                                   p.packed + (long long)e * p.g.stride + p.g.bias_off) + lane)
                             : make_float4(0.f, 0.f, 0.f, 0.f);
