@@ -442,7 +442,9 @@ __device__ void role_init_stages(const Params& p, Ctl* c, uint32_t ring, uint32_
         if (run && row0 + 4 * i < p.N)
           *(reinterpret_cast<uint4*>(p.out_init + (row0 + 4 * i) * p.d) + kc * 8 + j) =
               add_bf16x8(bz, v[i]);
-      // behind the stores, which have waited for what was loaded: an arrival does not wait for loads under way
+      // behind the stores, which have waited for what was loaded: an arrival does not wait for loads under way;
+      // and the next copy into the stage is the async proxy's
+      fence_proxy_async();
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&c->empty[r.s]), run);
       if (run) r.next(p.g.ns);
