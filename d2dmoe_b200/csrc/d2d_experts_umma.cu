@@ -204,8 +204,8 @@ __device__ __forceinline__ int select_bit(uint32_t m, int r) {
 // Where token `first` of expert e's list is: the counted chunk says from which tile on to look and how many
 // tokens come before it.
 __device__ __forceinline__ void find_chunk(const MaskTable& t, const Ctl* c, int e, int first, int lane,
-                                           int& tile, int& seen) {
-  const int n = lane < TABLE_CHUNKS ? c->chunk[lane][e] : 0, incl = warp_scan(n, lane);
+                                           bool live, int& tile, int& seen) {
+  const int n = live && lane < TABLE_CHUNKS ? c->chunk[lane][e] : 0, incl = warp_scan(n, lane);
   const uint32_t past = __ballot_sync(0xffffffffu, incl > first);
   const int w = past != 0u ? __ffs(past) - 1 : TABLE_CHUNKS;
   seen = __shfl_sync(0xffffffffu, incl - n, w & 31);
@@ -244,8 +244,9 @@ __device__ __forceinline__ void load_words(const MaskTable& t, int E, int e, int
 // not the mask's, left by a router that gave up, gives -1.
 __device__ __forceinline__ int find_token(const Params& p, const Tile* t, uint4* x, int row, int lane, bool live) {
   const MaskTable& mt = p.mt;
-  const int first = t->first, end = first + t->nrows;
-  int tile = t->from, seen = t->seen, tok = -1;
+  // (first pass: one row from the table's start on, whatever the list warp is writing meanwhile)
+  const int first = live ? t->first : 0, end = live ? first + t->nrows : 1;
+  int tile = live ? t->from : 0, seen = live ? t->seen : 0, tok = -1;
 #pragma unroll 1
   for (;;) {
 #pragma unroll 1
@@ -300,7 +301,9 @@ __device__ void role_list(const Params& p, Ctl* c, int lane, bool one_window) {
     int off[5], n[4], nt[4];             // experts 4 lane .. + 3
     if (tabled) {
       if (live && !mbar_wait_warp(smem_u32(&c->tot_full), 0, af, p.dev_status)) return;
-      const int4 v = *reinterpret_cast<const int4*>(&c->tot[4 * lane]);
+      // (first pass: one row of expert 0, whatever the counting warps are adding meanwhile)
+      int4 v = make_int4(lane == 0 ? 1 : 0, 0, 0, 0);
+      if (live) v = *reinterpret_cast<const int4*>(&c->tot[4 * lane]);
       n[0] = 4 * lane < E ? v.x : 0;
       n[1] = 4 * lane + 1 < E ? v.y : 0;
       n[2] = 4 * lane + 2 < E ? v.z : 0;
@@ -320,7 +323,6 @@ __device__ void role_list(const Params& p, Ctl* c, int lane, bool one_window) {
         if (e < E && bad) report(p.dev_status, D2D_ERR_INDEX_RANGE);
       }
     }
-    if (!live) n[0] = lane == 0 ? 1 : 0;
     int rows = 0, used = 0;
     bool all_n = true;                   // every expert of this lane lists exactly N tokens
 #pragma unroll
@@ -410,7 +412,7 @@ __device__ void role_list(const Params& p, Ctl* c, int lane, bool one_window) {
       first = __shfl_sync(0xffffffffu, first, owner);
       int from = 0, seen = 0;
       if (tabled) {
-        find_chunk(p.mt, c, e, first, lane, from, seen);
+        find_chunk(p.mt, c, e, first, lane, live, from, seen);
         if (u != (int)blockIdx.x && live) find_tile(p.mt, e, first, lane, from, seen);   // (not urgent)
       }
       if (live && !mbar_wait_warp(smem_u32(&c->tile_empty[r.s]), r.ph ^ 1, af, p.dev_status)) return;
