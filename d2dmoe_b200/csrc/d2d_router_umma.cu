@@ -183,8 +183,10 @@ __device__ void role_mma1(const Params& p, Ctl* c, uint32_t ring, uint32_t stage
     if (run) {
       a.next(nacc);
       tile += gridDim.x;
+    } else {
+      grid_dependency_wait();
+      run = next_run<WARM>();
     }
-    run = next_run<WARM>();
   }
 }
 
@@ -216,8 +218,10 @@ __device__ void role_mma2(const Params& p, Ctl* c, uint32_t wb, uint32_t tmem) {
     if (run) {
       tile += gridDim.x;
       ph ^= 1;
+    } else {
+      grid_dependency_wait();
+      run = next_run<WARM>();
     }
-    run = next_run<WARM>();
   }
 }
 
@@ -266,8 +270,10 @@ __device__ void role_hidden(const Params& p, Ctl* c, uint32_t tmem, int et) {
       a.next(nacc);
       tile += gridDim.x;
       ph ^= 1;
+    } else {
+      grid_dependency_wait();
+      run = next_run<WARM>();
     }
-    run = next_run<WARM>();
   }
 }
 
@@ -571,7 +577,7 @@ router_tiles_kernel(const Params p, const __grid_constant__ CUtensorMap tmx) {
   tc_fence_after();
   const uint32_t tmem = c->tmem_base;
 
-  // (roles that touch global memory wait for the previous kernel behind their first pass)
+  // (every role waits for the previous kernel behind its first pass: its bounded waits count from there on)
   if (warp < 4) {
     role_hidden<WARM>(p, c, tmem, tid);
   } else if (warp < 8) {

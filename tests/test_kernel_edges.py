@@ -470,3 +470,34 @@ def test_initial_rows_of_a_residual_layer(N, d, bias):
         ops.router_mask(x2d, wa, wb, 0.3, wsp, packed=packed, out_init=out, last_bias=lb, add_residual=True)
         wsp.check_status()
         assert torch.equal(out, x2d + lb if bias else x2d + 0)
+
+
+@pytest.mark.parametrize("N,resid", [(1100, False), (2000, True), (20011, False)])
+def test_waits_begin_when_the_previous_kernel_is_over(N, resid):
+    """A router call behind one that takes some 80 ms to give up: its bounded waits (a few ms here) are for its own
+    copies and products, not for the kernel in front of it, whose blocks it may start beside."""
+    from d2dmoe_b200 import _capi, ops
+    d, E, R = 256, 24, 64
+    c, t = _layer(N, d, 32, E, R, "bf16", N)
+    x2d, wa, wb = _dev(t["x"].reshape(N, d)), _dev(t["wa"]), _dev(t["wb"])
+    packed = ops.prepack_router(wa, wb)
+    first, then = ops.Workspace.allocate(N, E, "cuda"), ops.Workspace.allocate(N, E, "cuda")
+    out = torch.empty(N, d, dtype=torch.bfloat16, device="cuda")
+
+    def call(wsp):
+        ops.router_mask(x2d, wa, wb, 0.3, wsp, packed=packed, out_init=out, add_residual=resid)
+    call(then)
+    ref = then.mask_bits[:N].clone()
+    then.check_status()
+    try:
+        assert _capi.lib.d2d_debug_configure(18, 1) == 0
+        call(first)
+        assert _capi.lib.d2d_debug_configure(14, 0) == 0
+        call(then)
+        torch.cuda.synchronize()
+    finally:
+        _capi.lib.d2d_debug_configure(0, 0)
+    with pytest.raises(_capi.D2DError, match="TIMEOUT"):
+        first.check_status()
+    then.check_status()
+    assert torch.equal(then.mask_bits[:N], ref)
