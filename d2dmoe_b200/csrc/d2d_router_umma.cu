@@ -98,10 +98,10 @@ struct Ctl {
   uint32_t init_rows[2][4];
 };
 
-// WARM: a role's first pass is without effect.  Where the kernel also writes the lists (up to eight tiles,
-// one each) there is none: the previous call's kernels are over too soon for it, and its branches alone
-// make a call whose code is executed once longer (197 tokens 21.2 -> 22.4 us per layer).  Long calls
-// gain by it (12608 tokens x 24 52.3 -> 48.2, 50432 80.0 -> 77.3, 65536 x 96 114.4 -> 106.1).
+// WARM: a role's first pass is without effect.  Calls of up to eight tiles have none: a layer's previous
+// kernels are over too soon for it, and its branches alone make a call whose code is executed once longer
+// (197 tokens 21.2 -> 22.4 us per layer call; the router alone, replayed, 5.46 -> 5.63, 1024 tokens 5.47 -> 5.81).
+// Long calls gain by it (12608 tokens x 24 52.3 -> 48.2, 50432 80.0 -> 77.3, 65536 x 96 114.4 -> 106.1).
 template <bool WARM>
 __device__ __forceinline__ bool first_run() {
   if (WARM) return first_pass();
@@ -1005,12 +1005,13 @@ int launch_router_mask_umma(const void* x, const void* packed, float mult, uint3
   }
   const size_t smem = smem_bytes(p.g);
   int sms = 0;
-  auto kernel = rule == D2D_RULE_TOPK   ? (p.token_idx ? router_tiles_kernel<D2D_RULE_TOPK, false>
-                                                       : router_tiles_kernel<D2D_RULE_TOPK, true>)
-                : rule == D2D_RULE_DYNK ? (p.token_idx ? router_tiles_kernel<D2D_RULE_DYNK, false>
-                                                       : router_tiles_kernel<D2D_RULE_DYNK, true>)
-                                        : (p.token_idx ? router_tiles_kernel<0, false>
-                                                       : router_tiles_kernel<0, true>);
+  const bool warm = tiles > CLUSTER_TILES;
+  auto kernel = rule == D2D_RULE_TOPK   ? (warm ? router_tiles_kernel<D2D_RULE_TOPK, true>
+                                                : router_tiles_kernel<D2D_RULE_TOPK, false>)
+                : rule == D2D_RULE_DYNK ? (warm ? router_tiles_kernel<D2D_RULE_DYNK, true>
+                                                : router_tiles_kernel<D2D_RULE_DYNK, false>)
+                                        : (warm ? router_tiles_kernel<0, true>
+                                                : router_tiles_kernel<0, false>);
   rc = device_launch_facts((const void*)kernel, smem, &sms);
   if (rc != D2D_OK) return rc;
   const int64_t grid = tiles < sms ? tiles : sms;
