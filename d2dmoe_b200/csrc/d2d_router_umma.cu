@@ -382,7 +382,7 @@ __device__ void role_gate(const Params& p, Ctl* c, uint32_t tmem, int et) {
 #pragma unroll
       for (int j = 0; j < NW; ++j) {
         const uint32_t col = transpose32(word[j], lane);
-        c->cnt[buf][q4][32 * j + lane] = p.mt.words ? (int)col : __popc(col);
+        c->cnt[buf][q4][32 * j + lane] = WARM && p.mt.words ? (int)col : __popc(col);
       }
       // one barrier per tile: the other half of cnt is written before anybody passes it again (an
       // mbarrier, because a warp that gave up never comes)
@@ -394,7 +394,7 @@ __device__ void role_gate(const Params& p, Ctl* c, uint32_t tmem, int et) {
         if (et < E) {
           const int a = c->cnt[buf][0][et], b = c->cnt[buf][1][et], cc = c->cnt[buf][2][et],
                     dd = c->cnt[buf][3][et];
-          if (p.mt.words) {
+          if (WARM && p.mt.words) {
             if (run) p.mt.words[(long long)tile * E + et] = make_uint4(a, b, cc, dd);
             n = __popc(a) + __popc(b) + __popc(cc) + __popc(dd);
           } else {
@@ -534,8 +534,9 @@ __device__ void role_init(const Params& p, Ctl* c, int w, int lane) {
   }
 }
 
-// RULE: 0, or D2D_RULE_TOPK / D2D_RULE_DYNK (E <= 32).  WARM: see first_run
-template <int RULE, bool WARM>
+// RULE: 0, or D2D_RULE_TOPK / D2D_RULE_DYNK (E <= 32).  WARM: see first_run.  STAGES: initial rows by
+// role_init_stages (as a branch in one kernel it cost the calls without it 0.4 us, 197 tokens 19.5 -> 20.0)
+template <int RULE, bool WARM, bool STAGES>
 __global__ void __launch_bounds__(NTHREADS, 1)
 router_tiles_kernel(const Params p, const __grid_constant__ CUtensorMap tmx) {
   extern __shared__ uint8_t smem_raw[];
@@ -553,7 +554,7 @@ router_tiles_kernel(const Params p, const __grid_constant__ CUtensorMap tmx) {
   if (tid == 0) {
     for (int i = 0; i < NS_MAX; ++i) {
       mbar_init(smem_u32(&c->full[i]), 1);
-      mbar_init(smem_u32(&c->empty[i]), p.out_init && p.init_all && p.resid ? 5 : 1);
+      mbar_init(smem_u32(&c->empty[i]), STAGES ? 5 : 1);
     }
     mbar_init(smem_u32(&c->wb_full), 1);
     mbar_init(smem_u32(&c->hid_full), 128);
@@ -606,7 +607,7 @@ router_tiles_kernel(const Params p, const __grid_constant__ CUtensorMap tmx) {
     if (elect_one()) role_load<WARM>(p, c, &tmx, base, wb, stage_bytes);
     __syncwarp();
   } else if (warp >= WARP_INIT0 && p.out_init) {
-    if (p.init_all && p.resid) role_init_stages<WARM>(p, c, base, stage_bytes, warp - WARP_INIT0, tid & 31);
+    if (STAGES) role_init_stages<WARM>(p, c, base, stage_bytes, warp - WARP_INIT0, tid & 31);
     else role_init<WARM>(p, c, warp - WARP_INIT0, tid & 31);
   }
 
@@ -1005,13 +1006,14 @@ int launch_router_mask_umma(const void* x, const void* packed, float mult, uint3
   }
   const size_t smem = smem_bytes(p.g);
   int sms = 0;
-  const bool warm = tiles > CLUSTER_TILES;
-  auto kernel = rule == D2D_RULE_TOPK   ? (warm ? router_tiles_kernel<D2D_RULE_TOPK, true>
-                                                : router_tiles_kernel<D2D_RULE_TOPK, false>)
-                : rule == D2D_RULE_DYNK ? (warm ? router_tiles_kernel<D2D_RULE_DYNK, true>
-                                                : router_tiles_kernel<D2D_RULE_DYNK, false>)
-                                        : (warm ? router_tiles_kernel<0, true>
-                                                : router_tiles_kernel<0, false>);
+  const bool warm = tiles > CLUSTER_TILES, stages = out_init && init_all && resid;
+#define D2D_ROUTER_OF(RULE)                                                                         \
+  (warm ? (stages ? router_tiles_kernel<RULE, true, true> : router_tiles_kernel<RULE, true, false>) \
+        : (stages ? router_tiles_kernel<RULE, false, true> : router_tiles_kernel<RULE, false, false>))
+  auto kernel = rule == D2D_RULE_TOPK   ? D2D_ROUTER_OF(D2D_RULE_TOPK)
+                : rule == D2D_RULE_DYNK ? D2D_ROUTER_OF(D2D_RULE_DYNK)
+                                        : D2D_ROUTER_OF(0);
+#undef D2D_ROUTER_OF
   rc = device_launch_facts((const void*)kernel, smem, &sms);
   if (rc != D2D_OK) return rc;
   const int64_t grid = tiles < sms ? tiles : sms;
