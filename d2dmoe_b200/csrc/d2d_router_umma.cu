@@ -98,10 +98,13 @@ struct Ctl {
   uint32_t init_rows[2][4];
 };
 
-// WARM: a role's first pass is without effect.  Calls of up to eight tiles have none: a layer's previous
-// kernels are over too soon for it, and its branches alone make a call whose code is executed once longer
-// (197 tokens 21.2 -> 22.4 us per layer call; the router alone, replayed, 5.46 -> 5.63, 1024 tokens 5.47 -> 5.81).
-// Long calls gain by it (12608 tokens x 24 52.3 -> 48.2, 50432 80.0 -> 77.3, 65536 x 96 114.4 -> 106.1).
+// WARM: a role's first pass is without effect.  Where the kernel also writes the lists (up to eight tiles,
+// one each) there is none: the previous call's kernels are over too soon for it, and its branches alone
+// make a call whose code is executed once longer (197 tokens 21.2 -> 22.4 us per layer).  Long calls
+// gain by it (12608 tokens x 24 52.3 -> 48.2, 50432 80.0 -> 77.3, 65536 x 96 114.4 -> 106.1), and so do short ones
+// that leave the lists to other kernels, which are there to be waited for (replayed, without / with it: 24
+// experts stage by stage 1024 tokens 26.5 / 25.0, 256 21.5 / 20.4, 64 19.6 / 20.4, 32 19.0 / 18.5; top-4 of 96 1024 tokens
+// 62.7 / 61.4, 128 59.4 / 58.0, 64 55.0 / 55.6; nothing but routers one after another 5.5 / 5.8).
 template <bool WARM>
 __device__ __forceinline__ bool first_run() {
   if (WARM) return first_pass();
@@ -1006,7 +1009,7 @@ int launch_router_mask_umma(const void* x, const void* packed, float mult, uint3
   }
   const size_t smem = smem_bytes(p.g);
   int sms = 0;
-  const bool warm = tiles > CLUSTER_TILES, stages = out_init && init_all && resid;
+  const bool warm = !p.token_idx, stages = out_init && init_all && resid;
 #define D2D_ROUTER_OF(RULE)                                                                         \
   (warm ? (stages ? router_tiles_kernel<RULE, true, true> : router_tiles_kernel<RULE, true, false>) \
         : (stages ? router_tiles_kernel<RULE, false, true> : router_tiles_kernel<RULE, false, false>))
