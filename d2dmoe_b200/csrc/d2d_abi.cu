@@ -344,6 +344,8 @@ int d2d_moe_forward_rule(const void* x, const void* wa, const void* wb,
     if (rc != D2D_OK) return rc;
     nl += compact_counts_itself(N, E) || counts_ready ? 1 : 2;    // [count,] scatter
   }
+  // behind the kernels of mode 'all' and of the routing tensor there is nothing to be waited for
+  dr.warm = rule != D2D_RULE_ALL && rt_done;
   if (!rt_done) {                  // paths whose first kernel does not write the routing tensor
     rc = launch_expand_mask(mask_bits, routing_tensor_opt, N, E, dtype, s);
     if (rc != D2D_OK) return rc;

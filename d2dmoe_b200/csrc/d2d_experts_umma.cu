@@ -71,6 +71,7 @@ struct Params {
   int* dev_status;
   uint32_t wait_limit;         // polls per bounded wait
   int withhold;                // test hook: CTA 0 never loads its first weight tile
+  bool warm;                   // list and gather warps: a first pass without data, see role_list
   bf16* norms;                 // optional: [E, N] norms of each computed pair's activations
   int norm_layer, norm_ord;    // D2D_NORM_OF_INTERMEDIATE / D2D_NORM_OF_OUTPUT (0: none); 1 or 2
 };
@@ -286,23 +287,26 @@ __device__ __forceinline__ int find_token(const Params& p, const Tile* t, uint4*
 // T = sum ceil(n_e / S) <= rows / S + E, so R rounds of G CTAs are enough for S = rows / (R G - E),
 // and R is the least with S <= 128.  (524 rows per SM: five tiles of about 109 rows per CTA
 // instead of four of 128 and one of 12.)  An expert's tiles are equal.
-// Behind a router (the mask table) a first pass runs, while that drains, up to the first tile of a list of
-// one row: instructions that are executed for the first time cost some 20 cycles each, and
-// everything waits for the first tile.  So do the first passes of count_chunk and of the gather warps.
-// (50432 tokens 80.2 -> 76.9 us per layer; behind the kernel of mode 'all', which is over before, 50.6 ->
-// 52.7.  The other roles' code is warm too late: with such passes of theirs 79.7.)
+// Where the previous kernel lets this one start early (router, rule on given scores, scatter: p.warm) a first
+// pass runs, while that drains, up to the first tile of a list of one row: instructions that are executed
+// for the first time cost some 20 cycles each, and everything waits for the first tile.  So do the first
+// passes of count_chunk and of the gather warps.  Single calls: behind a router 50432 tokens 80.2 -> 76.9 us per
+// layer; replayed: behind a scatter 1024 tokens x 128 gated 83.8 -> 79.3, 50432 84.7 -> 81.3, 1920 tokens x 64
+// of 2048 x 128 56.7 -> 52.4.  Behind a kernel that is over before, it only comes later: mode 'all' 50.6 -> 52.7, behind
+// the routing tensor's own kernel 61.0 -> 62.5 (top-4 of 96, 1024 tokens).  (The other roles' code is warm
+// too late: with such passes of theirs 79.7.)
 __device__ void role_list(const Params& p, Ctl* c, int lane, bool one_window) {
   volatile int* af = &c->abort_flag;
   const int E = p.E, G = gridDim.x;
   const bool tabled = p.mt.words != nullptr;
 #pragma unroll 1
-  for (bool live = tabled ? first_pass() : in_earnest(), last = live;; live = in_earnest(), last = true) {
+  for (bool live = p.warm ? first_pass() : in_earnest(), last = live;; live = in_earnest(), last = true) {
     if (live) grid_dependency_wait();
     int off[5], n[4], nt[4];             // experts 4 lane .. + 3
     if (tabled) {
       if (live && !mbar_wait_warp(smem_u32(&c->tot_full), 0, af, p.dev_status)) return;
-      // (first pass: one row of expert 0, whatever the counting warps are adding meanwhile)
-      int4 v = make_int4(lane == 0 ? 1 : 0, 0, 0, 0);
+      // (first pass: nothing that the counting warps are adding meanwhile)
+      int4 v = make_int4(0, 0, 0, 0);
       if (live) v = *reinterpret_cast<const int4*>(&c->tot[4 * lane]);
       n[0] = 4 * lane < E ? v.x : 0;
       n[1] = 4 * lane + 1 < E ? v.y : 0;
@@ -323,6 +327,7 @@ __device__ void role_list(const Params& p, Ctl* c, int lane, bool one_window) {
         if (e < E && bad) report(p.dev_status, D2D_ERR_INDEX_RANGE);
       }
     }
+    if (!live) n[0] = lane == 0 ? 1 : 0;
     int rows = 0, used = 0;
     bool all_n = true;                   // every expert of this lane lists exactly N tokens
 #pragma unroll
@@ -470,9 +475,9 @@ __device__ void role_gather(const Params& p, Ctl* c, uint32_t ring, int w, int l
   RingPos r = {0, 0}, q = {0, 0};
   uint4 x[LOOK];
   x[0] = x[1] = x[2] = make_uint4(0u, 0u, 0u, 0u);
-  bool live = tabled ? first_pass() : in_earnest();
-  bool ahead = tabled;                   // this tile's first loads are on their way
-  if (!tabled) grid_dependency_wait();
+  bool live = p.warm ? first_pass() : in_earnest();
+  bool ahead = p.warm;                   // this tile's first loads are on their way (none in a first pass)
+  if (live) grid_dependency_wait();
 #pragma unroll 1
   for (;;) {
     Tile* t = &c->tile[q.s];
@@ -1102,6 +1107,7 @@ int launch_experts_umma(const void* x, int32_t* token_idx, int32_t* offsets,
   p.token_idx = token_idx;
   p.offsets = offsets;
   if (mt) p.mt = *mt;
+  p.warm = dr.warm;
   p.out = (bf16*)out;
   p.mask_bits = dr.mask_bits;
   p.last_bias = (const bf16*)dr.last_bias;

@@ -14,6 +14,7 @@ struct DirectRows {
   const uint32_t* mask_bits = nullptr;   // null: every row is added to
   const void* last_bias = nullptr;
   int kept = 0;                          // experts a token keeps, where the rule fixes it
+  bool warm = false;                     // the previous kernel lets this one start early: see role_list
 };
 // mt: there are no lists yet; the kernel makes them from the table and writes them as well
 int launch_experts_umma(const void* x, int32_t* token_idx, int32_t* offsets,
