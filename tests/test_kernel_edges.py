@@ -416,21 +416,37 @@ def test_every_form_gives_up_and_the_next_call_is_clean(form, N, d, H, E, R, glu
             assert O.rel_err(a.float().cpu(), b.float().cpu()) <= TOL["bf16"]
 
 
+U = 2.0 ** -8          # bf16 holds 8 bits: a rounding changes a value by at most this share of it
+
+
+def _magnitudes(x2d, m, w1, b1, w2):
+    """Per token and column: sum over its experts of |h W2| and of (|x W1| + |b1|) |W2|, in fp32."""
+    S, A = torch.zeros_like(x2d, dtype=torch.float32), torch.zeros_like(x2d, dtype=torch.float32)
+    x, m = x2d.float(), m.to(x2d.device)
+    for e in range(w1.shape[0]):
+        a, b, w = x @ w1[e].float(), b1[e].float(), w2[e].float()
+        S += m[:, e : e + 1] * ((a + b).relu() @ w).abs()
+        A += m[:, e : e + 1] * ((a.abs() + b.abs()) @ w.abs())
+    return S, A
+
+
 # N: tiles past the lists' cluster (1024 tokens) to more than one look at the table (96 tiles), ragged
 # ends; E: one to eight 16-cell groups of counts; tau: a token in a hundred to nearly every one
 @pytest.mark.parametrize("N,E,tau", [(1025, 1, 0.3), (1153, 5, 1.0), (1151, 24, 0.2), (2049, 33, 0.9), (5000, 64, 0.02),
-                                     (12801, 97, 0.1), (20011, 128, 0.0), (20000, 16, 0.6)])
+                                     (12801, 97, 0.1), (20011, 128, 0.0), (20000, 16, 0.6), (1025, 8, 0.7), (9001, 40, 0.2)])
 def test_lists_made_by_the_expert_kernel(N, E, tau):
-    """Lists and offsets of a long call, from the table that the router (or the rule on given scores)
-    leaves, against those of the scatter kernel, which a workspace without room for the table gets."""
-    from d2dmoe_b200 import ops
+    """Lists and offsets of a long call, from the table that the router (or the rule on given scores of whole
+    16-byte rows, some of them NaN) leaves, against those of the scatter kernel, which a workspace without room
+    for the table gets.  The number of launches tells that the two arms are the two forms."""
+    from d2dmoe_b200 import _capi, ops
     d, H, R = 64, 16, 16
     c, t = _layer(N, d, H, E, R, "bf16", N + E)
     x2d, wa, wb = _dev(t["x"].reshape(N, d)), _dev(t["wa"]), _dev(t["wb"])
     w1, b1, w2 = _dev(t["w1"]), _dev(t["b1"]), _dev(t["w2"])
     rp, ep = ops.prepack_router(wa, wb), ops.prepack_experts(w1, b1, w2)
     scores = torch.rand(N, E, generator=_gen(N), dtype=torch.float32).to(torch.bfloat16).cuda()
-    for given in (None, scores):
+    scores[5::97] = float("nan")
+    for given in (None, scores) if E % 8 == 0 and E <= 64 else (None,):
         got = []
         for room in (True, False):
             wsp = ops.Workspace.allocate(N, E, "cuda")
@@ -441,17 +457,94 @@ def test_lists_made_by_the_expert_kernel(N, E, tau):
             ops.moe_forward(x2d, None if given is not None else wa, None if given is not None else wb, tau, w1,
                             b1, w2, "relu", out, wsp, scores=given, experts_packed=ep,
                             router_packed=None if given is not None else rp)
+            assert _capi.lib.d2d_last_forward_launches() == (2 if room else 3)
             wsp.check_status()
             got.append((_lists(wsp, E), out, wsp.mask_bits[:N].clone(), wsp.token_idx.clone()))
         (l0, o0, m0, i0), (l1, o1, m1, i1) = got
         assert torch.equal(m0, m1) and np.array_equal(l0[0], l1[0]) and np.array_equal(l0[1], l1[1])
         assert torch.equal(i0, i1)                       # nothing behind the lists either
-        roff, ridx = O.expert_token_lists(O.unpack_mask(m0.cpu().numpy().view(np.uint32), E))
+        m = O.unpack_mask(m0.cpu().numpy().view(np.uint32), E)
+        roff, ridx = O.expert_token_lists(m)
         assert np.array_equal(l0[0], np.asarray(roff)) and np.array_equal(l0[1], np.asarray(ridx))
-        # the order of the adds is free: either side rounds once per expert of a token, half an ulp (2^-9) of
-        # a running sum each; a token whose hidden layer is all zero ties all experts and keeps them
-        kmax = int(O.unpack_mask(m0.cpu().numpy().view(np.uint32), E).sum(1).max())
-        assert O.rel_err(o0.float().cpu(), o1.float().cpu()) <= kmax * 2.0 ** -8
+        if given is not None:
+            assert not m[5::97].any() and m[:5].any(1).all()
+        # Both arms add the same bf16 contributions in an order of their own: each of a token's k - 1 adds rounds by
+        # U of a running sum, which is at most S and what the contributions are rounded by (4 times U
+        # of A, see below).  One add: equal.
+        S, A = _magnitudes(x2d, m, w1, b1, w2)
+        k = m.sum(1, keepdim=True).cuda()
+        lim = 1.02 * 2 * (k - 1).clamp(min=0) * U * (S + 4 * U * A)
+        diff = (o0.float() - o1.float()).abs()
+        assert bool((diff <= lim).all()), ((diff - lim).max(), (diff * (k == 1)).max())
+        # against the exact sum: x W1, its sum with b1 and the hidden value are rounded (3 times U of A at
+        # most), then each contribution and each add (U of S, at most A)
+        ex = O.experts_ffn_exact(x2d.cpu(), m, w1.cpu(), b1.cpu(), w2.cpu(), "relu").cuda()
+        assert bool(((o0.double() - ex).abs() <= 1.02 * (3 + 1 + k) * U * A).all())
+
+
+@pytest.mark.parametrize("N,launches", [(511 * 15 * 128, 2), (511 * 15 * 128 + 1, 3)])
+def test_lists_of_the_longest_calls(N, launches):
+    """Every expert on every token: the 16-bit sums of the table's fifteen parts at their largest (511 tiles of
+    128 tokens), and the first call that is too long for them."""
+    from d2dmoe_b200 import _capi, ops
+    d, H, E, R = 64, 16, 8, 16
+    c, t = _layer(64, d, H, E, R, "bf16", 3)
+    x2d = _dev(t["x"].reshape(64, d)).repeat(-(-N // 64), 1)[:N].contiguous()
+    wa, wb, w1, b1, w2 = (_dev(t[n]) for n in ("wa", "wb", "w1", "b1", "w2"))
+    wsp, out = ops.Workspace.allocate(N, E, "cuda"), torch.empty_like(x2d)
+    wsp.token_idx.fill_(-1)
+    ops.moe_forward(x2d, wa, wb, 1.0, w1, b1, w2, "relu", out, wsp, experts_packed=ops.prepack_experts(w1, b1, w2),
+                    router_packed=ops.prepack_router(wa, wb))
+    assert _capi.lib.d2d_last_forward_launches() == launches
+    wsp.check_status()
+    each = torch.arange(N, dtype=torch.int32, device="cuda")
+    assert torch.equal(wsp.offsets, torch.arange(E + 1, dtype=torch.int32, device="cuda") * N)
+    assert torch.equal(wsp.token_idx.view(E, N), each.expand(E, N))
+    m = torch.ones(64, E, dtype=torch.bool)
+    ex = O.experts_ffn_exact(t["x"].reshape(64, d), m, t["w1"], t["b1"], t["w2"], "relu").cuda()
+    _, A = _magnitudes(x2d[:64], m, w1, b1, w2)
+    lim = (1.02 * (4 + E) * U * A).repeat(-(-N // 64), 1)[:N]        # as above
+    assert bool(((out.double() - ex.repeat(-(-N // 64), 1)[:N]).abs() <= lim).all())
+
+
+@pytest.mark.parametrize("N,E,glu", [(2000, 16, False), (5000, 24, True)])
+def test_layer_gives_up_over_a_table_that_is_not_the_masks(N, E, glu):
+    """Router and experts both miss a slice of weights, and where the router leaves nothing the table holds more
+    tokens than there are: the call ends and reports, nothing is written past the lists, the next one is right."""
+    from d2dmoe_b200 import _capi, ops
+    d, H, R = 256, 64, 64
+    c, t = _layer(N, d, H, E, R, "bf16", N, "relu", glu)
+    x2d, wa, wb = _dev(t["x"].reshape(N, d)), _dev(t["wa"]), _dev(t["wb"])
+    w1, b1, w2, wu = (_dev(t.get(k)) for k in ("w1", "b1", "w2", "w_up"))
+    b1 = None if glu else b1
+    rp, ep = ops.prepack_router(wa, wb), ops.prepack_experts(w1, b1, w2, wu)
+    wsp = ops.Workspace.allocate(N, E, "cuda")
+    whole = torch.full((2 * N * E,), -1, dtype=torch.int32, device="cuda")
+    wsp.token_idx = whole[: N * E]
+    out = torch.empty(N, d, dtype=torch.bfloat16, device="cuda")
+
+    def call():
+        ops.moe_forward(x2d, wa, wb, 0.2, w1, b1, w2, "relu", out, wsp, w_up=wu, experts_packed=ep, router_packed=rp)
+        assert _capi.lib.d2d_last_forward_launches() == 2
+    call()
+    wsp.check_status()
+    ref, lists = out.clone(), _lists(wsp, E)
+    wsp.ws.fill_(255)
+    try:
+        assert _capi.lib.d2d_debug_configure(12, 1) == 0
+        call()
+        torch.cuda.synchronize()                     # returns
+    finally:
+        _capi.lib.d2d_debug_configure(0, 0)
+    with pytest.raises(_capi.D2DError, match="TIMEOUT"):
+        wsp.check_status()
+    assert bool((whole[N * E :] == -1).all())
+    out.fill_(float("nan"))
+    call()
+    wsp.check_status()
+    got = _lists(wsp, E)
+    assert np.array_equal(got[0], lists[0]) and np.array_equal(got[1], lists[1])
+    assert O.rel_err(out.float().cpu(), ref.float().cpu()) <= TOL["bf16"]      # (the order of the adds is free)
 
 
 @pytest.mark.parametrize("bias", [True, False])
