@@ -66,9 +66,9 @@ int d2d_abi_version(void);
 const char* d2d_strerror(int status);
 
 /* Bytes of caller-owned workspace d2d_compact / d2d_moe_forward need for up to
- * n_max tokens.  (d2d_moe_forward also takes the (ceil(n_max/128) + 1) * 4E bytes of earlier versions,
- * at the price of a launch that writes the lists.)  (The upstream path allocates its scratch inside every call:
- * architectures/moe/moe_impls.py:15,190.) */
+ * n_max tokens.  (d2d_moe_forward also takes the max((t + 1) * 4E, t * max(16, p)) bytes of earlier versions,
+ * t = ceil(n_max/128) and p the least power of two >= E, at the price of a launch that writes the lists.)
+ * (The upstream path allocates its scratch inside every call: architectures/moe/moe_impls.py:15,190.) */
 int d2d_workspace_bytes(int64_t n_max, int E, size_t* bytes /* host */);
 
 /* Router MLP fused with the dynamic-k rule.
@@ -266,7 +266,10 @@ int d2d_moe_forward_rule(const void* x, const void* wa, const void* wb,
 
 /* Number of kernels the calling thread's last d2d_moe_forward issued (2 on the tensor-core
  * path: router + rule, expert FFN; the lists come from the first on short calls and from the second on
- * long ones; 3 where ws has no room for the table between them; more on the general-shape paths).  Introspection for benchmarks; no upstream counterpart. */
+ * long ones).  A third one writes the lists where ws has no room for the table between the two, past 981120
+ * tokens, where clusters split the router (2 to 16 tiles of 128 tokens at d * R >= 256 K) and where the rows of
+ * given scores are not whole 16-byte vectors of at most 128 bytes; more on the general-shape paths.
+ * Introspection for benchmarks; no upstream counterpart. */
 int d2d_last_forward_launches(void);
 
 /* Test hook, no upstream counterpart.  Every wait inside the tensor-core kernels is bounded;
@@ -288,7 +291,9 @@ int d2d_debug_select_experts_kernel(int which);
  * parameters in place (architectures/moe/moe_impls.py:137-146,276-284); here the
  * module owns a packed copy and refreshes it when the parameters change.
  * *_bytes returns 0 bytes when the shape has no tensor-core path.  `packed` must be
- * 1024-byte aligned. */
+ * 1024-byte aligned.  A packed buffer is valid with the library build that made it and with no other: the
+ * order inside it may change without its size or D2D_ABI_VERSION changing (W2's columns have done so), and
+ * nothing in it tells.  Do not store one; pack again after loading the weights. */
 int d2d_prepack_experts_bytes(int d, int E, int H, int glu, int dtype, size_t* bytes /* host */);
 int d2d_prepack_experts(const void* w1, const void* b1_opt, const void* w_up_opt, const void* w2,
                         void* packed, int d, int E, int H, int dtype, d2d_stream_t stream);
