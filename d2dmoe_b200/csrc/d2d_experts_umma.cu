@@ -10,7 +10,7 @@
 // again, an M = 128, K = 16 instruction N/2 + 43 cycles with A in shared memory and N/2 + 10 with
 // A in tensor memory; the tensor pipe and DRAM are busy below 30 % of the time.  Hence
 //   * the hidden tile replaces accumulator 1 in place: the second product reads its A operand
-//     from tensor memory, and no shared memory is spent on it (rings of 128 + 48 KB);
+//     from tensor memory, and no shared memory is spent on it (rings of 160 + 48 KB);
 //   * two tiles are in work at once: the first product of one runs while the second product of
 //     the other runs and is written out;
 //   * the second product works in steps of 128 output columns (64 where d or the tensor memory
@@ -21,7 +21,8 @@
 //   * the lists are cut into equal tiles of a size that fills the last round of the persistent
 //     grid; where there are fewer tiles than SMs the output columns are split as well;
 //   * on long calls there are no lists before this kernel: the gather warps find a tile's rows in a table
-//     that the router leaves (50432 tokens 95.1 -> 88.4 us per layer, 12608 x 12 narrow experts 39.6 -> 35.6);
+//     that the router leaves (single calls: 50432 tokens 95.1 -> 88.4 us per layer, 12608 x 12 narrow experts
+//     39.6 -> 35.6; 131072 gated tokens gain nothing: scatter 12.3 -> 0, this kernel 587 -> 601, see role_gather);
 //   * where the weights of all experts stay in L2, the tiles are taken window by window of the
 //     token range, all experts of a window next to each other, so that a row of x is read and
 //     a row of out is added to in L2 by every expert but the first; last window first, because
@@ -32,8 +33,9 @@
 // half (256 columns): gate at 0, up at H, hidden in place at 0, and once epilogue 1 is done
 // three 64-column accumulator-2 buffers from 64 on.
 //
-// Warps: 0-3 epilogue 1; 4-11 drain; 12-15 row gather (cp.async); 16 first product; 17 second
-// product; 18 weights (bulk copies); 19 the tiles and their row lists.
+// Warps: 0-3 epilogue 1; 4-11 drain; 12-15 a tile's rows: tokens and gather (cp.async); 16 first product;
+// 17 second product; 18 weights (bulk copies); 19 cuts the lists into tiles.  On calls with a mask table 0-11
+// and 16-18 count it first.
 //
 // Every wait is bounded: when one runs out the kernel records D2D_ERR_TIMEOUT in the status word,
 // all roles leave their loops, TMEM is freed and the kernel returns.
@@ -290,7 +292,7 @@ __device__ __forceinline__ int find_token(const Params& p, const Tile* t, uint4*
 // Where the previous kernel lets this one start early (router, rule on given scores, scatter: p.warm) a first
 // pass runs, while that drains, up to the first tile of a list of one row: instructions that are executed
 // for the first time cost some 20 cycles each, and everything waits for the first tile.  So do the first
-// passes of count_chunk and of the gather warps.  Single calls: behind a router 50432 tokens 80.2 -> 76.9 us per
+// passes of count_chunk and of the gather warps.  Queued calls: behind a router 50432 tokens 80.2 -> 76.9 us per
 // layer; replayed: behind a scatter 1024 tokens x 128 gated 83.8 -> 79.3, 50432 84.7 -> 81.3, 1920 tokens x 64
 // of 2048 x 128 56.7 -> 52.4.  Behind a kernel that is over before, it only comes later: mode 'all' 50.6 -> 52.7, behind
 // the routing tensor's own kernel 61.0 -> 62.5 (top-4 of 96, 1024 tokens).  (The other roles' code is warm
@@ -460,7 +462,9 @@ __device__ void role_list(const Params& p, Ctl* c, int lane, bool one_window) {
 // the list's end repeat the 32-row group's first one, a group without rows loads nothing: what
 // their slots hold reaches only accumulator rows nobody reads.
 // (Beside the traffic of the kernel a load takes some thousand cycles: the mask words of a tile travel
-// while its rows are copied, and so do the next tile's table words where that tile is known by then.)
+// while its rows are copied, and so do the next tile's table words where that tile is known by then.  The
+// selection itself stands between two tiles' copies: a gated expert with two rows per 128-token tile makes it
+// search 64 of those for one of its own.)
 __device__ void role_gather(const Params& p, Ctl* c, uint32_t ring, int w, int lane) {
   volatile int* af = &c->abort_flag;
   const int j = lane & 7, row = w * 32 + lane;

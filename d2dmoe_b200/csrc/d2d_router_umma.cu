@@ -100,8 +100,8 @@ struct Ctl {
 
 // WARM: a role's first pass is without effect.  Where the kernel also writes the lists (up to eight tiles,
 // one each) there is none: the previous call's kernels are over too soon for it, and its branches alone
-// make a call whose code is executed once longer (197 tokens 21.2 -> 22.4 us per layer).  Long calls
-// gain by it (12608 tokens x 24 52.3 -> 48.2, 50432 80.0 -> 77.3, 65536 x 96 114.4 -> 106.1), and so do short ones
+// make a call whose code is executed once longer (single calls, 197 tokens 21.2 -> 22.4 us per layer).  Long calls
+// gain by it (queued, 12608 tokens x 24 52.3 -> 48.2, 50432 80.0 -> 77.3, 65536 x 96 114.4 -> 106.1), and so do short ones
 // that leave the lists to other kernels, which are there to be waited for (replayed, without / with it: 24
 // experts stage by stage 1024 tokens 26.5 / 25.0, 256 21.5 / 20.4, 64 19.6 / 20.4, 32 19.0 / 18.5; top-4 of 96 1024 tokens
 // 62.7 / 61.4, 128 59.4 / 58.0, 64 55.0 / 55.6; nothing but routers one after another 5.5 / 5.8).
