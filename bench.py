@@ -40,10 +40,11 @@ sys.path.insert(0, str(ROOT))
 
 HEADLINE = "vit_b16"
 HEADLINE_TAU = 0.9
-# dram__bytes_read.sum + dram__bytes_write.sum of one expert-kernel launch of the headline
-# workload at tau_cfg 0.9 (50432 tokens, one layer), from the ncu capture summarised in
-# profiles/layer_kernels_vit_b16_tau0.9.md (117.3 MB read + 26.3 MB written)
-NCU_EXPERTS_TRAFFIC_BYTES = 143.6e6
+# dram__bytes_read.sum + dram__bytes_write.sum of one staged expert-kernel launch (ready lists, every row
+# added to: what the roofline object times) of the headline workload at tau_cfg 0.9 (50432 tokens, one
+# layer), from the ncu capture summarised in profiles/layer_kernels_vit_b16_tau0.9.md (165.6 MB read + 24.4 MB
+# written, mean of two)
+NCU_EXPERTS_TRAFFIC_BYTES = 189.9e6
 FALLBACK_PEAKS = {"hbm_gbs": 6650.0, "bf16_tflops": 1590.0, "bf16_tflops_sustained": 1400.0}
 
 BF16, FP32 = torch.bfloat16, torch.float32
