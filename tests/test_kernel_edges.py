@@ -165,7 +165,8 @@ def test_large_router(N, d, E):
 
 @pytest.mark.parametrize("N,d,H,E,R", [(1, 4, 4, 1, 4), (31, 68, 36, 5, 36), (33, 260, 100, 33, 100),
                                        (64, 768, 128, 24, 128), (95, 132, 32, 256, 160),
-                                       (257, 64, 64, 40, 64)])
+                                       (257, 64, 64, 40, 64), (191, 256, 32, 1, 64), (192, 320, 96, 1, 128),
+                                       (225, 4, 4, 1, 4), (417, 132, 100, 2, 36), (385, 516, 44, 2, 64)])
 def test_fp32_layer(N, d, H, E, R):
     from d2dmoe_b200 import ops
     c, t = _layer(N, d, H, E, R, "fp32", N + d, act="gelu")
