@@ -21,7 +21,8 @@ std::mutex g_dev_lock;
 
 }  // namespace
 
-// The opt-in (cudaFuncSetAttribute) holds for the current device only, as does the SM count.
+// The opt-in (cudaFuncSetAttribute) holds for the current device only, as does the SM count.  kernel null: only that
+// count.
 int device_launch_facts(const void* kernel, size_t smem, int* sms) {
   int dev = -1;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= MAX_DEVICES) {
@@ -38,6 +39,7 @@ int device_launch_facts(const void* kernel, size_t smem, int* sms) {
     return D2D_ERR_NO_DEVICE;
   }
   if (sms) *sms = f.sms;
+  if (!kernel) return D2D_OK;
   int i = 0;
   while (i < f.n && f.optin[i].kernel != kernel) ++i;
   if (i == f.n || f.optin[i].smem < smem) {

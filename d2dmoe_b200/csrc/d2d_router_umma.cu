@@ -19,6 +19,8 @@
 // that the second one does not sit between two tiles.
 #include <cooperative_groups.h>
 
+#include <algorithm>
+
 #include "d2d_cluster_compact.cuh"
 #include "d2d_ranked.cuh"
 #include "d2d_tmap.cuh"
@@ -82,6 +84,8 @@ struct Params {
   const bf16* last_bias;
   const bf16* resid;
   int init_all;             // every row; 0: rows not kept by exactly one expert
+  int ctas;                 // that take tiles
+  bf16* help_init;          // optional: every initial row, by the CTAs behind those (then out_init is null)
   int* dev_status;
   uint32_t wait_limit;
   int withhold;             // test hook: CTA 0 never loads its first weight slice
@@ -146,7 +150,7 @@ __device__ void role_load(const Params& p, Ctl* c, const CUtensorMap* tmx, uint3
       bulk_g2s(wb, p.packed + g.w1_bytes, wb_bytes, bar, run);
     }
     if (run) {
-      tile += gridDim.x;
+      tile += p.ctas;
     } else {
       grid_dependency_wait();
       run = next_run<WARM>();
@@ -185,7 +189,7 @@ __device__ void role_mma1(const Params& p, Ctl* c, uint32_t ring, uint32_t stage
     umma_commit(smem_u32(&c->acc1_full[a.s]), run);
     if (run) {
       a.next(nacc);
-      tile += gridDim.x;
+      tile += p.ctas;
     } else {
       grid_dependency_wait();
       run = next_run<WARM>();
@@ -219,7 +223,7 @@ __device__ void role_mma2(const Params& p, Ctl* c, uint32_t wb, uint32_t tmem) {
                    idesc, k != 0, run);
     umma_commit(smem_u32(&c->g2_done), run);
     if (run) {
-      tile += gridDim.x;
+      tile += p.ctas;
       ph ^= 1;
     } else {
       grid_dependency_wait();
@@ -271,7 +275,7 @@ __device__ void role_hidden(const Params& p, Ctl* c, uint32_t tmem, int et) {
     mbar_arrive(smem_u32(&c->hid_full), run);
     if (run) {
       a.next(nacc);
-      tile += gridDim.x;
+      tile += p.ctas;
       ph ^= 1;
     } else {
       grid_dependency_wait();
@@ -409,7 +413,7 @@ __device__ void role_gate(const Params& p, Ctl* c, uint32_t tmem, int et) {
     }
     if (p.rt_out && live) store_row<NB>(p.rt_out + trow * E, s, E);
     if (run) {
-      tile += gridDim.x;
+      tile += p.ctas;
       ph ^= 1;
       buf ^= 1;
     } else {
@@ -459,7 +463,7 @@ __device__ void role_init_stages(const Params& p, Ctl* c, uint32_t ring, uint32_
       if (run) r.next(p.g.ns);
     }
     if (run) {
-      tile += gridDim.x;
+      tile += p.ctas;
     } else {
       grid_dependency_wait();
       run = next_run<WARM>();
@@ -527,7 +531,7 @@ __device__ void role_init(const Params& p, Ctl* c, int w, int lane) {
       }
     }
     if (run) {
-      tile += gridDim.x;
+      tile += p.ctas;
       ph ^= buf;
       buf ^= 1;
     } else {
@@ -537,9 +541,45 @@ __device__ void role_init(const Params& p, Ctl* c, int w, int lane) {
   }
 }
 
-// RULE: 0, or D2D_RULE_TOPK / D2D_RULE_DYNK (E <= 32).  WARM: see first_run.  STAGES: initial rows by
-// role_init_stages (as a branch in one kernel it cost the calls without it 0.4 us, 197 tokens 19.5 -> 20.0)
-template <int RULE, bool WARM, bool STAGES>
+// Calls of few tiles: the other CTAs of the grid write every initial row while the tiles are computed.  A tile's
+// own CTA knows only behind its gate which rows want one, and 47 rows (of 128, 24 experts at 0.9) at an SM's 30
+// bytes a clock then keep the next kernel waiting for 3 us; that the expert kernel writes some of these rows
+// again costs nothing here.
+__device__ __forceinline__ void help_init_rows(const Params& p) {
+  const int v8 = p.d >> 3, helpers = (int)gridDim.x - p.ctas, h = (int)blockIdx.x - p.ctas;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const long long row0 = p.N * h / helpers, row1 = p.N * (h + 1) / helpers;
+  grid_dependency_wait();
+  for (int c8 = lane; c8 < v8; c8 += 32) {
+    uint4 bz = make_uint4(0u, 0u, 0u, 0u);
+    if (p.last_bias) bz = __ldg(reinterpret_cast<const uint4*>(p.last_bias) + c8);
+    if (!p.resid) {
+      for (long long t = row0 + warp; t < row1; t += NTHREADS / 32)
+        *(reinterpret_cast<uint4*>(p.help_init + t * p.d) + c8) = bz;
+      continue;
+    }
+    for (long long t = row0 + warp; t < row1; t += 4 * (NTHREADS / 32)) {
+      uint4 v[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u)          // four rows in flight
+        if (t + u * (NTHREADS / 32) < row1)
+          v[u] = __ldg(reinterpret_cast<const uint4*>(p.resid + (t + u * (NTHREADS / 32)) * p.d) + c8);
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (t + u * (NTHREADS / 32) < row1)
+          *(reinterpret_cast<uint4*>(p.help_init + (t + u * (NTHREADS / 32)) * p.d) + c8) =
+              add_bf16x8(bz, v[u]);
+    }
+  }
+}
+
+// Initial rows: by warps of the tile's CTA, by those out of the stages of the first product, or by CTAs of their
+// own.  Kernels of their own, because a call of few tiles executes the code once: as a branch in one kernel
+// the second form cost the calls without it 0.4 us (197 tokens 19.5 -> 20.0), the third one as much.
+enum { INIT_TILE, INIT_STAGES, INIT_OTHERS };
+
+// RULE: 0, or D2D_RULE_TOPK / D2D_RULE_DYNK (E <= 32).  WARM: see first_run
+template <int RULE, bool WARM, int INIT>
 __global__ void __launch_bounds__(NTHREADS, 1)
 router_tiles_kernel(const Params p, const __grid_constant__ CUtensorMap tmx) {
   extern __shared__ uint8_t smem_raw[];
@@ -554,10 +594,14 @@ router_tiles_kernel(const Params p, const __grid_constant__ CUtensorMap tmx) {
   // runs (it waits for this grid before it reads anything); this CTA initialises its barriers
   // while the previous kernel drains and reads global memory only after the wait below.
   grid_launch_dependents();
+  if (INIT == INIT_OTHERS && (int)blockIdx.x >= p.ctas) {
+    help_init_rows(p);
+    return;
+  }
   if (tid == 0) {
     for (int i = 0; i < NS_MAX; ++i) {
       mbar_init(smem_u32(&c->full[i]), 1);
-      mbar_init(smem_u32(&c->empty[i]), STAGES ? 5 : 1);
+      mbar_init(smem_u32(&c->empty[i]), INIT == INIT_STAGES ? 5 : 1);
     }
     mbar_init(smem_u32(&c->wb_full), 1);
     mbar_init(smem_u32(&c->hid_full), 128);
@@ -609,9 +653,11 @@ router_tiles_kernel(const Params p, const __grid_constant__ CUtensorMap tmx) {
   } else if (warp == WARP_LOAD) {
     if (elect_one()) role_load<WARM>(p, c, &tmx, base, wb, stage_bytes);
     __syncwarp();
-  } else if (warp >= WARP_INIT0 && p.out_init) {
-    if (STAGES) role_init_stages<WARM>(p, c, base, stage_bytes, warp - WARP_INIT0, tid & 31);
-    else role_init<WARM>(p, c, warp - WARP_INIT0, tid & 31);
+  } else if (INIT != INIT_OTHERS && warp >= WARP_INIT0 && p.out_init) {
+    if (INIT == INIT_STAGES)
+      role_init_stages<WARM>(p, c, base, stage_bytes, warp - WARP_INIT0, tid & 31);
+    else
+      role_init<WARM>(p, c, warp - WARP_INIT0, tid & 31);
   }
 
   // A launch that gave up may still have copies and MMAs in flight that use this CTA's
@@ -1009,18 +1055,37 @@ int launch_router_mask_umma(const void* x, const void* packed, float mult, uint3
   }
   const size_t smem = smem_bytes(p.g);
   int sms = 0;
-  const bool warm = !p.token_idx, stages = out_init && init_all && resid;
-#define D2D_ROUTER_OF(RULE)                                                                         \
-  (warm ? (stages ? router_tiles_kernel<RULE, true, true> : router_tiles_kernel<RULE, true, false>) \
-        : (stages ? router_tiles_kernel<RULE, false, true> : router_tiles_kernel<RULE, false, false>))
+  rc = device_launch_facts(nullptr, 0, &sms);
+  if (rc != D2D_OK) return rc;
+  const int64_t ctas = tiles < sms ? tiles : sms;
+  p.ctas = (int)ctas;
+  // Initial rows by the SMs that have no tile, see help_init_rows, where those are at least a quarter, or half
+  // if the rows of x are read for them.  Layer, us, by the tiles' own CTAs / by others (replayed): 197 tokens x 24
+  // experts 19.4 / 17.4, 1100 24.3 / 21.0, 6304 28.1 / 26.0, 13 000 x 96 39.6 / 37.4, 12 608 36.8 / 36.7, 13 500 x
+  // 128 gated 150 / 144; with 123 tiles 38.7 / 44.0.  Residual: 788 21.9 / 19.3, 9456 26.6 / 24.5, 12 608 29.1 / 29.7.
+  // (Short calls, one cluster: up to six more clusters, which are all there at once.)
+  const int64_t more = p.token_idx ? tiles * std::min<int64_t>((sms - tiles) / tiles, 6) : sms - ctas;
+  // Rows that all start from last_bias (ranked rules) stay with the tile: they are written before its gate.
+  // (Top-4 of 24, 12 608 tokens 46.4 / 47.3.)
+  const bool help = out_init && (resid || !init_all) && 4 * tiles <= (resid ? 2 : 3) * sms && more > 0;
+  if (help) {
+    p.help_init = p.out_init;
+    p.out_init = nullptr;
+  }
+  const bool warm = !p.token_idx, stages = warm && p.out_init && init_all && resid;
+#define D2D_ROUTER_OF(RULE)                                                    \
+  (help ? (warm ? router_tiles_kernel<RULE, true, INIT_OTHERS>                 \
+                : router_tiles_kernel<RULE, false, INIT_OTHERS>)               \
+        : stages ? router_tiles_kernel<RULE, true, INIT_STAGES>                \
+                 : (warm ? router_tiles_kernel<RULE, true, INIT_TILE>          \
+                         : router_tiles_kernel<RULE, false, INIT_TILE>))
   auto kernel = rule == D2D_RULE_TOPK   ? D2D_ROUTER_OF(D2D_RULE_TOPK)
                 : rule == D2D_RULE_DYNK ? D2D_ROUTER_OF(D2D_RULE_DYNK)
                                         : D2D_ROUTER_OF(0);
 #undef D2D_ROUTER_OF
-  rc = device_launch_facts((const void*)kernel, smem, &sms);
+  rc = device_launch_facts((const void*)kernel, smem, nullptr);
   if (rc != D2D_OK) return rc;
-  const int64_t grid = tiles < sms ? tiles : sms;
-  return launch_pdl_cluster(p.token_idx ? (int)tiles : 0, kernel, dim3((unsigned)grid),
+  return launch_pdl_cluster(p.token_idx ? (int)tiles : 0, kernel, dim3((unsigned)(ctas + (help ? more : 0))),
                             dim3(NTHREADS), smem, s, p, tmx);
 }
 

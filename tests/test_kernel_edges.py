@@ -566,6 +566,33 @@ def test_initial_rows_of_a_residual_layer(N, d, bias):
         assert torch.equal(out, x2d + lb if bias else x2d + 0)
 
 
+@pytest.mark.parametrize("bias", [True, False])
+@pytest.mark.parametrize("N,d", [(1, 64), (127, 768), (130, 2048), (1024, 64), (1025, 320), (14208, 64), (14209, 64)])
+def test_initial_rows_by_other_blocks(N, d, bias):
+    """last_bias in every row, exactly, from the blocks that have no tile (one tile, one cluster of eight, more;
+    either side of the rule's line at 111 tiles), and the layer over them."""
+    from d2dmoe_b200 import ops
+    E, R = 3, 16
+    c, t = _layer(N, d, 16, E, R, "bf16", N + d)
+    x2d, wa, wb = _dev(t["x"].reshape(N, d)), _dev(t["wa"]), _dev(t["wb"])
+    w1, b1, w2 = _dev(t["w1"]), _dev(t["b1"]), _dev(t["w2"])
+    lb = _dev(t["last_bias"].reshape(-1)) if bias else None
+    packed, wsp = ops.prepack_router(wa, wb), ops.Workspace.allocate(N, E, "cuda")
+    out = torch.full((N, d), float("nan"), dtype=torch.bfloat16, device="cuda")
+    ops.router_mask(x2d, wa, wb, 0.3, wsp, packed=packed, out_init=out, last_bias=lb)
+    wsp.check_status()
+    assert torch.equal(out, lb.expand(N, d) if bias else torch.zeros_like(out))
+    for residual in (False, True):
+        out.fill_(float("nan"))
+        ops.moe_forward(x2d, wa, wb, 0.3, w1, b1, w2, "relu", out, wsp, last_bias=lb, router_packed=packed,
+                        experts_packed=ops.prepack_experts(w1, b1, w2), add_residual=residual)
+        wsp.check_status()
+        m = O.unpack_mask(wsp.mask_bits[:N].cpu().numpy().view(np.uint32), E)
+        ex = O.experts_ffn_exact(t["x"].reshape(N, d), m, t["w1"], t["b1"], t["w2"])
+        ex = ex + (t["last_bias"].double() if bias else 0.0) + (t["x"].reshape(N, d).double() if residual else 0.0)
+        assert O.rel_err(out.cpu().float(), ex) <= TOL["bf16"]
+
+
 @pytest.mark.parametrize("N,resid", [(1100, False), (2000, True), (20011, False)])
 def test_waits_begin_when_the_previous_kernel_is_over(N, resid):
     """A router call behind one that takes some 80 ms to give up: its bounded waits (a few ms here) are for its own
