@@ -40,9 +40,11 @@ prenorm_init_kernel(const T* __restrict__ x, const T* __restrict__ gamma,
   const int nv = (dv + 31) / 32;              // vectors per lane (<= MAXV)
   const int64_t warps = (int64_t)gridDim.x * (NT / 32);
   // Short rows (<= 4 vectors per lane) keep the NEXT row's loads in flight while the current
-  // row is reduced and written: one row per warp at a time leaves too few bytes in flight.
+  // row is reduced and written: one row per warp at a time leaves too few bytes in flight.  gamma, beta and
+  // last_bias are loaded once, with the first row instead of behind its statistics.
   constexpr bool PREFETCH = MAXV_ <= 4;
   uint4 raw[MAXV_], nxt[PREFETCH ? MAXV_ : 1];
+  uint4 pg[PREFETCH ? MAXV_ : 1], pb[PREFETCH ? MAXV_ : 1], pl[PREFETCH ? MAXV_ : 1];
   int64_t row = (int64_t)blockIdx.x * (NT / 32) + (threadIdx.x >> 5);
   if (PREFETCH && row < N) {
     const uint4* xr = reinterpret_cast<const uint4*>(x + row * d);
@@ -50,6 +52,16 @@ prenorm_init_kernel(const T* __restrict__ x, const T* __restrict__ gamma,
     for (int i = 0; i < MAXV_; ++i) {
       const int c = lane + 32 * i;
       if (i < nv && c < dv) raw[i] = __ldg(xr + c);
+    }
+#pragma unroll
+    for (int i = 0; i < MAXV_; ++i) {
+      const int c = lane + 32 * i;
+      pb[i] = pl[i] = make_uint4(0u, 0u, 0u, 0u);
+      if (i < nv && c < dv) {
+        pg[i] = __ldg(reinterpret_cast<const uint4*>(gamma) + c);
+        if (beta) pb[i] = __ldg(reinterpret_cast<const uint4*>(beta) + c);
+        if (last_bias) pl[i] = __ldg(reinterpret_cast<const uint4*>(last_bias) + c);
+      }
     }
   }
   for (; row < N; row += warps) {
@@ -115,10 +127,14 @@ prenorm_init_kernel(const T* __restrict__ x, const T* __restrict__ gamma,
     for (int i = 0; i < MAXV_; ++i) {
       const int c = lane + 32 * i;
       if (i < nv && c < dv) {
-        const uint4 gv = __ldg(reinterpret_cast<const uint4*>(gamma) + c);
-        uint4 bv = make_uint4(0u, 0u, 0u, 0u), lb = make_uint4(0u, 0u, 0u, 0u);
-        if (beta) bv = __ldg(reinterpret_cast<const uint4*>(beta) + c);
-        if (last_bias) lb = __ldg(reinterpret_cast<const uint4*>(last_bias) + c);
+        uint4 gv, bv = make_uint4(0u, 0u, 0u, 0u), lb = make_uint4(0u, 0u, 0u, 0u);
+        if (PREFETCH) {
+          gv = pg[i], bv = pb[i], lb = pl[i];
+        } else {
+          gv = __ldg(reinterpret_cast<const uint4*>(gamma) + c);
+          if (beta) bv = __ldg(reinterpret_cast<const uint4*>(beta) + c);
+          if (last_bias) lb = __ldg(reinterpret_cast<const uint4*>(last_bias) + c);
+        }
         const T* e = reinterpret_cast<const T*>(&raw[i]);
         const T* g = reinterpret_cast<const T*>(&gv);
         const T* b = reinterpret_cast<const T*>(&bv);
@@ -153,10 +169,15 @@ int launch_prenorm_init(const void* x, const void* gamma, const void* beta, floa
   if (d % V != 0 || d / V > 32 * MAXV) return D2D_ERR_UNSUPPORTED;
   if (!al16(x) || !al16(gamma) || !al16(beta) || !al16(last_bias) || !al16(xn) || !al16(out))
     return D2D_ERR_BAD_ARG;
-  int64_t grid = ceil_div64(N, NT / 32);
-  if (grid > 148 * 16) grid = 148 * 16;
-  if (grid < 1) grid = 1;
+  // Short rows: four CTAs per SM at most, so that a warp has several rows for one reading of the parameters.
+  // Half a block of d = 768, us, parameters read for each row in 16 CTAs per SM / this (in 2, 6 per SM): 788 tokens
+  // 27.1 / 26.5 (26.5, 26.4), 7289 42.1 / 41.0 (41.4, 42.4), 17 730 55.2 / 51.1 (52.4, 52.5), 49 250 117.6 / 112.9
+  // (114.7, 112.2).
   const int nv = (d / V + 31) / 32;
+  const int64_t most = nv <= 4 ? 148 * 4 : 148 * 16;
+  int64_t grid = ceil_div64(N, NT / 32);
+  if (grid > most) grid = most;
+  if (grid < 1) grid = 1;
 #define D2D_PRENORM_CASE(T_, NV_)                                                              \
   return launch_pdl(prenorm_init_kernel<T_, NV_>, dim3((unsigned)grid), dim3(NT), 0, s,         \
                     (const T_*)x, (const T_*)gamma, (const T_*)beta, eps, kind, gamma_offset,   \
