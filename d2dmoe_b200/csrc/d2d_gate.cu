@@ -8,6 +8,8 @@
 // Each Linear output is materialised in the tensor dtype T upstream, so the fp32
 // accumulators are rounded to T once after each of the two products, and the
 // threshold is rounded to T before the comparison.
+#include <algorithm>
+
 #include "d2d_cluster_compact.cuh"
 #include "d2d_ranked.cuh"
 #include "d2d_common.cuh"
@@ -431,7 +433,8 @@ gate_scores_fused_kernel(const T* __restrict__ scores, float mult,
 // (order of equal values, NaN, summation and rounding as in gate_rule_kernel, which ranks every
 // expert against every other with one warp per token: 15 us for 12608 tokens x 24, before counts,
 // routing tensor and initial rows.)
-template <typename T, int NV, int RULE>
+// OTHERS: the tiles are the first `ctas` blocks; those behind them write every initial row meanwhile.
+template <typename T, int NV, int RULE, bool OTHERS>
 __global__ void __launch_bounds__(NT)
 gate_scores_fused_rows_kernel(const T* __restrict__ scores, float mult, int k, float tau,
                               uint32_t* __restrict__ mask_bits, T* __restrict__ rt,
@@ -439,7 +442,7 @@ gate_scores_fused_rows_kernel(const T* __restrict__ scores, float mult, int k, f
                               const T* __restrict__ x, const T* __restrict__ last_bias,
                               int add_residual, T* __restrict__ out, int direct, int64_t N, int d,
                               int E, int32_t* __restrict__ token_idx,
-                              int32_t* __restrict__ offsets, const MaskTable mt) {
+                              int32_t* __restrict__ offsets, const MaskTable mt, int ctas) {
   __shared__ uint32_t cnt[4][64];        // tokens of a 32-token row that keep an expert, as bits
   __shared__ uint32_t rows[4];
   __shared__ int scratch[3 * 256];
@@ -452,6 +455,14 @@ gate_scores_fused_rows_kernel(const T* __restrict__ scores, float mult, int k, f
   const int ntok = (int)min((int64_t)128, N - t0);
   grid_launch_dependents();
   grid_dependency_wait();
+  if (OTHERS) {
+    if ((int)blockIdx.x >= ctas) {
+      const int64_t n = (int64_t)gridDim.x - ctas, h = (int64_t)blockIdx.x - ctas, r0 = N * h / n;
+      init_tile_rows(x, last_bias, add_residual, out, r0, (int)(N * (h + 1) / n - r0), d, nullptr, w, lane);
+      return;
+    }
+    out = nullptr;
+  }
   // this lane's score row first: the loads fly while initial output rows are issued
   const int64_t t = t0 + w * 32 + lane;
   uint4 raw[NV];
@@ -736,16 +747,29 @@ int launch_gate_scores_fused(const void* scores, int rule, int k, float tau, flo
     counts = mt.counts;
     lists->tabled = true;
   }
+  // Few tiles: blocks of their own, of some 16 rows, write every initial row while the rule is applied, which alone
+  // knows the rows that want one (as in the tensor-core router).  Layer of 24 experts on given scores, us, by
+  // the tiles' blocks / by others: 20 tokens 14.8 / 14.2, 180 17.3 / 14.2, 2000 24.7 / 19.8, 9000 27.7 / 23.8, 15 000
+  // 34.0 / 31.7, 18 000 (141 tiles) 34.7 / 33.2, 32 768 42.9 / 49.0; top-2, where all rows want one, 2000 35.6 / 20.4,
+  // 18 000 55 / 39.8.  Instances of their own: as a branch it cost
+  // the 32 768 tokens 0.7 us.  (One cluster: up to six more clusters.)
+  const int64_t more = fused ? grid * std::min<int64_t>((148 - grid) / grid, 6)
+                             : std::min<int64_t>(std::max<int64_t>(N / 16, 2 * 148), 4 * 148);
+  const bool others = out && rows_form && grid <= 148 && more > 0;
+  const int64_t blocks = others ? grid + more : grid;
+#define D2D_ROWS_OF(T, NVV, RULE)                                                             \
+  (others ? gate_scores_fused_rows_kernel<T, NVV, RULE, true>                                 \
+          : gate_scores_fused_rows_kernel<T, NVV, RULE, false>)
 #define D2D_ROWS_CASE(T, NVV)                                                                 \
   case NVV: {                                                                                 \
-    auto kn = rule == 0               ? gate_scores_fused_rows_kernel<T, NVV, 0>              \
-              : rule == D2D_RULE_TOPK ? gate_scores_fused_rows_kernel<T, NVV, D2D_RULE_TOPK>  \
-                                      : gate_scores_fused_rows_kernel<T, NVV, D2D_RULE_DYNK>; \
-    return launch_pdl_cluster(fused ? (int)grid : 0, kn, dim3((unsigned)grid), dim3(NT), 0, s,\
+    auto kn = rule == 0               ? D2D_ROWS_OF(T, NVV, 0)                                \
+              : rule == D2D_RULE_TOPK ? D2D_ROWS_OF(T, NVV, D2D_RULE_TOPK)                    \
+                                      : D2D_ROWS_OF(T, NVV, D2D_RULE_DYNK);                   \
+    return launch_pdl_cluster(fused ? (int)grid : 0, kn, dim3((unsigned)blocks), dim3(NT), 0, s,\
                               (const T*)scores, mult, k, tau, mask_bits, (T*)rt, counts, EP,  \
                               (const T*)x, (const T*)last_bias, add_residual, (T*)out,        \
                               direct ? 1 : 0, N, d, E, fused ? lists->token_idx : nullptr,    \
-                              fused ? lists->offsets : nullptr, mt);                          \
+                              fused ? lists->offsets : nullptr, mt, (int)grid);               \
   }
   if (rows_form) {
     if (dtype == D2D_F32) {
@@ -763,6 +787,7 @@ int launch_gate_scores_fused(const void* scores, int rule, int k, float tau, flo
     }
   }
 #undef D2D_ROWS_CASE
+#undef D2D_ROWS_OF
   if (rule != 0) return D2D_ERR_UNSUPPORTED;
   if (dtype == D2D_F32)
     return launch_pdl(gate_scores_fused_kernel<float>, dim3((unsigned)grid), dim3(NT), 0, s,

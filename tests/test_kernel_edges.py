@@ -593,6 +593,32 @@ def test_initial_rows_by_other_blocks(N, d, bias):
         assert O.rel_err(out.cpu().float(), ex) <= TOL["bf16"]
 
 
+@pytest.mark.parametrize("dtype,E", [("bf16", 24), ("fp32", 8)])
+@pytest.mark.parametrize("N", [1, 127, 1024, 1025, 18944, 18945])
+def test_initial_rows_beside_given_scores(N, dtype, E):
+    """The same where the scores are given (one tile, one cluster of eight, more; either side of the rule's line at
+    148 tiles)."""
+    from d2dmoe_b200 import ops
+    d = 64
+    c, t = _layer(N, d, 16, E, 16, dtype, N + E)
+    dt = t["x"].dtype
+    x2d, w1, b1, w2 = _dev(t["x"].reshape(N, d)), _dev(t["w1"]), _dev(t["b1"]), _dev(t["w2"])
+    lb = _dev(t["last_bias"].reshape(-1))
+    scores = torch.rand(N, E, generator=_gen(N)).to(dt)
+    packed = ops.prepack_experts(w1, b1, w2) if dtype == "bf16" else None
+    wsp = ops.Workspace.allocate(N, E, "cuda")
+    m = O.dynk_max_mask(scores, 0.1)
+    ex = O.experts_ffn_exact(t["x"].reshape(N, d), m, t["w1"], t["b1"], t["w2"]) + t["last_bias"].double()
+    for residual in (False, True):
+        out = torch.full((N, d), float("nan"), dtype=dt, device="cuda")
+        ops.moe_forward(x2d, None, None, 0.1, w1, b1, w2, "relu", out, wsp, last_bias=lb, scores=_dev(scores),
+                        experts_packed=packed, add_residual=residual)
+        wsp.check_status()
+        assert torch.equal(O.unpack_mask(wsp.mask_bits[:N].cpu().numpy().view(np.uint32), E), m)
+        want = ex + (t["x"].reshape(N, d).double() if residual else 0.0)
+        assert O.rel_err(out.cpu().float(), want) <= TOL[dtype]
+
+
 @pytest.mark.parametrize("N,resid", [(1100, False), (2000, True), (20011, False)])
 def test_waits_begin_when_the_previous_kernel_is_over(N, resid):
     """A router call behind one that takes some 80 ms to give up: its bounded waits (a few ms here) are for its own
