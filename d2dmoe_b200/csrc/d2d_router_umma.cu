@@ -1059,15 +1059,15 @@ int launch_router_mask_umma(const void* x, const void* packed, float mult, uint3
   if (rc != D2D_OK) return rc;
   const int64_t ctas = tiles < sms ? tiles : sms;
   p.ctas = (int)ctas;
-  // Initial rows by the SMs that have no tile, see help_init_rows, where those are at least a quarter, or half
-  // if the rows of x are read for them.  Layer, us, by the tiles' own CTAs / by others (replayed): 197 tokens x 24
+  // Initial rows by the SMs that have no tile, see help_init_rows, where those are at least a quarter; half if
+  // the rows of x are read for them; seven eighths where every row starts from last_bias (ranked rules: the
+  // tile's own warps write those before its gate).  Layer, us, by the tiles' own CTAs / by others: 197 tokens x 24
   // experts 19.4 / 17.4, 1100 24.3 / 21.0, 6304 28.1 / 26.0, 13 000 x 96 39.6 / 37.4, 12 608 36.8 / 36.7, 13 500 x
   // 128 gated 150 / 144; with 123 tiles 38.7 / 44.0.  Residual: 788 21.9 / 19.3, 9456 26.6 / 24.5, 12 608 29.1 / 29.7.
+  // Top-k: 591 23.3 / 20.7, 985 26.9 / 24.5, 2167 27.1 / 26.5, 5319 35.0 / 35.3, 12 608 47.3 / 48.4.
   // (Short calls, one cluster: up to six more clusters, which are all there at once.)
   const int64_t more = p.token_idx ? tiles * std::min<int64_t>((sms - tiles) / tiles, 6) : sms - ctas;
-  // Rows that all start from last_bias (ranked rules) stay with the tile: they are written before its gate.
-  // (Top-4 of 24, 12 608 tokens 46.4 / 47.3.)
-  const bool help = out_init && (resid || !init_all) && 4 * tiles <= (resid ? 2 : 3) * sms && more > 0;
+  const bool help = out_init && more > 0 && tiles <= (resid ? sms / 2 : init_all ? sms / 8 : 3 * sms / 4);
   if (help) {
     p.help_init = p.out_init;
     p.out_init = nullptr;
