@@ -3,10 +3,10 @@
 // d2d_experts_umma.cu (architectures/moe/moe_impls.py:93-180, 244-301).
 //
 // What bounds it: the weight stream (an SM takes 64 bytes per clock) and, in the form for long lists,
-// instructions whose 128 rows are mostly padding: N / 2 + 43 cycles for K = 16 whatever the rows,
+// instructions whose 128 rows are mostly padding: N / 2 cycles for K = 16 whatever the rows,
 // N = 2 H of a gated expert, repeated by every CTA that has a share of the output columns.  Hence
 //   * both products are transposed: the WEIGHTS are the 128 rows of the instruction and the (up to
-//     32) tokens its columns, 59 cycles; the packed images serve as the A operand as they are;
+//     32) tokens its columns, 48 cycles (some 70 issued); the packed images serve as the A operand as they are;
 //   * a cluster of C CTAs has an expert: each takes H / C of its hidden columns over all of d,
 //     pushes its hidden slice into the others' shared memory and then takes its share of
 //     the output columns with the whole hidden tile.  No weight is read twice, no partial sum is

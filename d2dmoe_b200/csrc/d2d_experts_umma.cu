@@ -7,8 +7,8 @@
 //
 // What bounds it: latency, not a unit.  A hand-over from the tensor pipe to a waiting thread
 // (commit, mbarrier, wake-up) takes about 300 cycles and one back to the issuing thread as much
-// again, an M = 128, K = 16 instruction N/2 + 43 cycles with A in shared memory and N/2 + 10 with
-// A in tensor memory; the tensor pipe and DRAM are busy below 30 % of the time.  Hence
+// again; an M = 128, K = 16 instruction takes 64 cycles at N = 128, a role's wait, four of them and a
+// commit 280; the tensor pipe and DRAM are busy below 30 % of the time.  Hence
 //   * the hidden tile replaces accumulator 1 in place: the second product reads its A operand
 //     from tensor memory, and no shared memory is spent on it (rings of 160 + 48 KB);
 //   * two tiles are in work at once: the first product of one runs while the second product of
