@@ -813,8 +813,9 @@ __device__ __forceinline__ void put_rows(uint32_t (&w)[2][2][4], const int* rt, 
 // 128 bytes of one row: whole lines leave an SM at 25 bytes per clock where they are added, half lines at
 // 20 (stored: 32 and 29; 148 CTAs, rows of 1536 bytes).  A transposition through shared memory took
 // 1250 cycles a step with nothing written, this 730 (950 where rows are stored as well).
-// What bounds a tile of the two-layer form is now the way between SM and L2: 128 rows added, gathered
-// and 384 KB of weights take 8.3, 2.8 and 5.5 thousand cycles alone and 12.9 together.
+// What bounds a tile of the two-layer form is this role: 1850 cycles a 128-column step, some 1350 of them the
+// write path's backlog (26 bytes a clock and SM, rows stored and added mixed), 1550 with nothing else
+// travelling.  A register that spills here waits behind the writes.
 // DIRECT: rows of tokens with one expert are stored, see DirectRows
 template <bool GLU, bool NORM, bool DIRECT>
 __device__ void role_drain(const Params& p, Ctl* c, uint32_t tmem, int j, int q4, int lane) {

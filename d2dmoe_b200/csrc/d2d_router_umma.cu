@@ -2,7 +2,7 @@
 //     s = |bf16(relu(bf16(x Wa^T)) Wb^T)|,  keep e iff s_e >= bf16(max s * mult)
 // (architectures/moe/moefication.py:328-330 and :80-85), written as mask bits, the 0/1 routing
 // tensor and the compaction's counts table; the same CTA writes the initial rows of the layer
-// output that the expert kernel will add to.
+// output that the expert kernel will add to (where few SMs have a tile: the others, help_init_rows).
 //
 // One persistent CTA per SM, 16 warps, one 128-token tile after another:
 //   warp 10     one thread loads stages (a 128-row x 64-column TMA box of x and the matching 64-deep
