@@ -370,3 +370,37 @@ def test_prenorm_init_shapes_against_the_oracle(dtype, kind):
             assert O.rel_err(xn.cpu().float(), ref) <= tol, (d, n)
             want = (x.float() + lb.float()).to(dtype).float()
             assert torch.equal(init.cpu().float(), want), (d, n)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype,d,lines", [
+    # blocks of eight rows, the last ones before the kernel's form or grid changes on a device of 148 SMs
+    (torch.bfloat16, 248, (592,)), (torch.bfloat16, 512, (222, 592, 1775, 4735)),
+    (torch.bfloat16, 768, (222, 592, 1775, 4735)), (torch.bfloat16, 1000, (222, 592, 1775, 4735)),
+    (torch.float32, 128, (592, 4735)), (torch.float32, 252, (592, 2367)),
+    (torch.float32, 384, (222, 592, 1775, 2367)), (torch.float32, 508, (222, 592, 1775, 2367))])
+def test_prenorm_warps_with_several_rows(dtype, d, lines):
+    """Every form that keeps gamma, beta and last_bias from one row of a warp to the next, on either side of the
+    row counts at which form or grid changes; layer norm, then RMSNorm without last_bias."""
+    from d2dmoe_b200 import ops
+    tol = 2e-6 if dtype == torch.float32 else 2.0 ** -8
+    g = torch.Generator().manual_seed(d)
+    x = (torch.randn(8 * max(lines) + 1, d, generator=g) * 1.7 + 0.4).to(dtype)
+    gamma = (1.0 + 0.1 * torch.randn(d, generator=g)).to(dtype)
+    beta, lb = ((0.1 * torch.randn(d, generator=g)).to(dtype) for _ in range(2))
+    ln, rms = O.prenorm(x, gamma, beta, 1e-6, "layer", 0.0).float(), O.prenorm(x, gamma, None, 1e-6, "rms", 1.0).float()
+    xd, gd, bd, ld = x.cuda(), gamma.cuda(), beta.cuda(), lb.cuda()
+    want = (x.float() + lb.float()).to(dtype)
+    for n in sorted({8 * b + e for b in lines for e in (0, 1)}):
+        xn, init = torch.full_like(xd[:n], float("nan")), torch.full_like(xd[:n], float("nan"))
+        ops.prenorm_init(xd[:n], gd, bd, 1e-6, ops.NORM_LAYER, xn, init, last_bias=ld)
+        assert O.rel_err(xn.cpu().float(), ln[:n]) <= tol, n
+        # relative per row: one row among thousands with another's statistics or parameters is seen
+        err = (xn.cpu().float() - ln[:n]).norm(dim=1) / ln[:n].norm(dim=1)
+        assert err.max() <= 4 * tol, (n, int(err.argmax()))
+        assert torch.equal(init.cpu(), want[:n]), n
+        xn.fill_(float("nan"))
+        ops.prenorm_init(xd[:n], gd, None, 1e-6, ops.NORM_RMS, xn, init, gamma_offset=1.0)
+        err = (xn.cpu().float() - rms[:n]).norm(dim=1) / rms[:n].norm(dim=1)
+        assert err.max() <= 4 * tol, (n, int(err.argmax()))
+        assert torch.equal(init.cpu(), x[:n]), n
