@@ -359,7 +359,7 @@ int d2d_moe_forward_rule(const void* x, const void* wa, const void* wb,
                                lists.tabled ? &mt : nullptr);
   }
   return launch_experts_simt(x, token_idx, offsets, w1, b1_opt, w_up_opt, w2, out, N, d, E, H, act,
-                             dtype, dev_status, s, nc);
+                             dtype, dev_status, s, nc, rule == D2D_RULE_DYNK ? 0 : dr.kept);
 }
 
 int d2d_moe_forward(const void* x, const void* wa, const void* wb, const void* router_packed_opt,

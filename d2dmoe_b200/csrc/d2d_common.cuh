@@ -238,10 +238,11 @@ int launch_router_fp32(const void* x, const void* wa, const void* wb, float mult
                        cudaStream_t s);
 int launch_experts_fp32(const void* x, const int32_t* token_idx, const int32_t* offsets,
                         const void* w1, const void* b1, const void* w2, void* out, int64_t N, int d,
-                        int E, int H, int act, int* dev_status, cudaStream_t s);
+                        int E, int H, int act, int* dev_status, cudaStream_t s, int kept);
+// kept: experts that a token keeps, 0 where the rule leaves it open
 int launch_experts_simt(const void* x, const int32_t* token_idx, const int32_t* offsets,
                         const void* w1, const void* b1, const void* w_up, const void* w2,
                         void* out, int64_t N, int d, int E, int H, int act, int dtype,
-                        int* dev_status, cudaStream_t s, NormCapture nc = NormCapture());
+                        int* dev_status, cudaStream_t s, NormCapture nc = NormCapture(), int kept = 0);
 
 }  // namespace d2d

@@ -369,12 +369,12 @@ int launch_t(const void* x, const int32_t* token_idx, const int32_t* offsets, co
 int launch_experts_simt(const void* x, const int32_t* token_idx, const int32_t* offsets,
                         const void* w1, const void* b1, const void* w_up, const void* w2,
                         void* out, int64_t N, int d, int E, int H, int act, int dtype,
-                        int* dev_status, cudaStream_t s, NormCapture nc) {
+                        int* dev_status, cudaStream_t s, NormCapture nc, int kept) {
   if (E > MAX_E) return D2D_ERR_UNSUPPORTED;
   if (dtype == D2D_F32) {
     if (!w_up && !nc.norms) {
       const int rc = launch_experts_fp32(x, token_idx, offsets, w1, b1, w2, out, N, d, E, H, act,
-                                         dev_status, s);
+                                         dev_status, s, kept);
       if (rc != D2D_ERR_UNSUPPORTED) return rc;
     }
     return w_up ? launch_t<float, true>(x, token_idx, offsets, w1, b1, w_up, w2, out, N, d, E, H,

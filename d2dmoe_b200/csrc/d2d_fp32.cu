@@ -22,6 +22,8 @@
 // 6304 209 -> 171.
 #include <cooperative_groups.h>
 
+#include <algorithm>
+
 #include "d2d_common.cuh"
 
 namespace d2d {
@@ -47,6 +49,11 @@ struct Tiling {
   static constexpr int STAGE = A_FLOATS + KW * TH;        // floats of a warp's stage
   static constexpr int PART = TR * TH;                    // a warp's sums
   static constexpr int FLOATS = 4 * (ST * STAGE + PART);  // of a CTA
+  // CTAs per SM of the experts' grid.  (16 rows: the tables of 64 experts and more leave room for four at a time; the
+  // fifth then follows the first that is done.  A grid of four, us, five / four: 64 experts 197 tokens 48.6 / 46.2,
+  // 1576 74.6 / 77.3, 6304 205 / 198, 12 608 358 / 370; 96 experts x 32 197 tokens 32.1 / 34.6; 128 experts 788 69.8 / 82.5;
+  // 64 of d = 2048 4096 tokens 383 / 420.)
+  static constexpr int CTAS = MR == 4 ? 5 : 3;
   static_assert(W2_ROWS * 64 <= STAGE, "a stage holds a piece of W2");
 };
 
@@ -394,7 +401,7 @@ router_fp32_kernel(const float* __restrict__ x, const float* __restrict__ wa,
 // experts
 // ---------------------------------------------------------------------------
 template <int MR>
-__global__ void __launch_bounds__(NT, MR == 4 ? 5 : 3)
+__global__ void __launch_bounds__(NT, Tiling<MR>::CTAS)
 experts_fp32_kernel(const float* __restrict__ x, const int32_t* __restrict__ token_idx,
                     const int32_t* __restrict__ offsets, const float* __restrict__ w1,
                     const float* __restrict__ b1, const float* __restrict__ w2,
@@ -593,15 +600,14 @@ bool al16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 template <int MR>
 int launch_experts(const float* x, const int32_t* token_idx, const int32_t* offsets, const float* w1,
                    const float* b1, const float* w2, float* out, int64_t N, int d, int E, int H,
-                   int act, int* dev_status, cudaStream_t s) {
+                   int act, int* dev_status, int sms, cudaStream_t s) {
   using T = Tiling<MR>;
   const size_t smem = sizeof(float) * (size_t)T::FLOATS + 2 * sizeof(int) * (size_t)(E + 1);
-  int sms = 0;
-  const int rc = device_launch_facts((const void*)experts_fp32_kernel<MR>, smem, &sms);
+  const int rc = device_launch_facts((const void*)experts_fp32_kernel<MR>, smem, nullptr);
   if (rc != D2D_OK) return rc;
   // at most one item per TR rows of an expert and slice, plus a partial one
   const int64_t most = (ceil_div64(N * (int64_t)E, T::TR) + E) * ceil_div(H, TH);
-  const int64_t ctas = (int64_t)(MR == 4 ? 5 : 3) * sms, grid = most < ctas ? most : ctas;
+  const int64_t ctas = (int64_t)T::CTAS * sms, grid = most < ctas ? most : ctas;
   return launch_pdl(experts_fp32_kernel<MR>, dim3((unsigned)grid), dim3(NT), smem, s, x, token_idx,
                     offsets, w1, b1, w2, out, N, d, E, H, act, dev_status);
 }
@@ -630,18 +636,34 @@ int launch_router_fp32(const void* x, const void* wa, const void* wb, float mult
                     (float*)out_init, N, d, R, E);
 }
 
-// Rows of an item: 16, which is what spreads a small call over the SMs, or 32 where every expert may be
-// expected to fill several (halves the weights' way from L2 and what a warp reads per FMA).  Layer of 24
-// experts, us, 16 / 32 rows: 788 tokens 52.0 / 59.9, 1576 54.6 / 62.3, 3152 101 / 108, 6304 184 / 171 (with 3.5
-// experts a token instead of 1.5: 52.1 / 60.5, 86.5 / 96.7, 164 / 164, 301 / 283).
+// Rows of an item: 16, which is what spreads a small call over the SMs, or 32 (halves the weights' way from L2 and
+// what a warp reads per FMA) where lists are long or, if kept is known (experts a token keeps; 0: the threshold's
+// 1.5), where 32 rows take fewer rounds of the CTAs that run at a time (such a round takes a tenth longer).
+// Layer of 24 experts, us, 16 / 32 rows, mean length of a list in brackets:
+//   threshold    1576 tokens (98) 53.7 / 57.8, 3152 (197) 102 / 107, 4700 (294) 147 / 134, 6304 (394) 184 / 170
+//   top-2        1200 (100) 56 / 62, 1576 (131) 85 / 66, 1900 (158) 82 / 86, 2700 (225) 99 / 107, 3152 (263) 122 / 109
+//   top-4        700 (117) 54 / 59, 1200 (200) 89 / 96, 1576 (263) 112 / 97, 2700 (450) 165 / 162, 5200 (867) 298 / 270
+//   all experts  200 65 / 72, 260 90 / 75, 330 99 / 101, 400 111 / 108, 788 218 / 206, 4000 1028 / 936
 int launch_experts_fp32(const void* x, const int32_t* token_idx, const int32_t* offsets,
                         const void* w1, const void* b1, const void* w2, void* out, int64_t N, int d,
-                        int E, int H, int act, int* dev_status, cudaStream_t s) {
+                        int E, int H, int act, int* dev_status, cudaStream_t s, int kept) {
   if (d % 4 || H % 4 || E > MAX_E || !al16(x) || !al16(w1) || !al16(w2) || !al16(out))
     return D2D_ERR_UNSUPPORTED;
-  auto launch = N >= 192 * (int64_t)E ? launch_experts<8> : launch_experts<4>;
+  int sms = 0;
+  const int rc = device_launch_facts(nullptr, 0, &sms);
+  if (rc != D2D_OK) return rc;
+  const int64_t pairs = kept ? N * kept : N * 3 / 2;
+  auto rounds = [&](int rows, int ctas) {      // half a tile more for each list; a twentieth left over is none
+    const int64_t tiles = kept == E ? E * ceil_div64(N, rows) : pairs / rows + E / 2;
+    const int64_t slots = (int64_t)ctas * sms, items = tiles * ceil_div(H, TH);
+    return std::max<int64_t>(ceil_div64(items - slots / 20, slots), 1);
+  };
+  const bool rows32 = kept ? pairs >= 400 * (int64_t)E ||
+                                 11 * rounds(32, Tiling<8>::CTAS) <= 10 * rounds(16, Tiling<4>::CTAS)
+                           : pairs >= 288 * (int64_t)E;
+  auto launch = rows32 ? launch_experts<8> : launch_experts<4>;
   return launch((const float*)x, token_idx, offsets, (const float*)w1, (const float*)b1,
-                (const float*)w2, (float*)out, N, d, E, H, act, dev_status, s);
+                (const float*)w2, (float*)out, N, d, E, H, act, dev_status, sms, s);
 }
 
 }  // namespace d2d

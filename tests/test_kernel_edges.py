@@ -648,3 +648,29 @@ def test_waits_begin_when_the_previous_kernel_is_over(N, resid):
         first.check_status()
     then.check_status()
     assert torch.equal(then.mask_bits[:N], ref)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode,k,E,N", [("topk", 2, 5, 95), ("topk", 2, 5, 999), ("topk", 4, 5, 500), ("all", 5, 5, 399),
+                                        ("all", 5, 5, 400), ("dynk", 0, 5, 961), ("dynk_max", 0, 5, 959),
+                                        ("dynk_max", 0, 5, 960), ("topk", 2, 24, 1463), ("topk", 2, 24, 1464),
+                                        ("all", 24, 24, 240), ("all", 24, 24, 241), ("all", 24, 24, 289)])
+def test_fp32_items_of_several_ragged_lists(mode, k, E, N):
+    """Item sizes of 16 and of 32 rows over several experts with ragged lists, on either side of the
+    lines of the rule that chooses between them (mean list of 288 or 400 rows; rounds of CTAs)."""
+    import d2dmoe_b200 as D
+    d, H = 132, 100
+    c, t = _layer(N, d, H, E, 36, "fp32", N + k)
+    moe = D.MoeficationMoE("m", d, E, True, H, torch.nn.ReLU)
+    moe.router = D.MoeficationRouter(d, E, width=36, depth=2, bias=False, activation="relu", output_activation="abs")
+    moe.load_state_dict({"experts.w1": t["w1"], "experts.b1": t["b1"], "experts.w2": t["w2"], "last_bias": t["last_bias"],
+                         "router.layers.0.weight": t["wa"], "router.layers.2.weight": t["wb"]})
+    moe = moe.cuda().eval()
+    moe.forward_mode, moe.k, moe.tau = mode, k, 0.6
+    with torch.no_grad():
+        out, gating = moe(_dev(t["x"]))
+    m = gating["m"][0].reshape(N, E).cpu() > 0
+    if mode in ("topk", "all"):
+        assert (m.sum(1) == (k if mode == "topk" else E)).all()
+    ex = O.experts_ffn_exact(t["x"].reshape(N, d), m, t["w1"], t["b1"], t["w2"]) + t["last_bias"].double()
+    assert O.rel_err(out.reshape(N, d).cpu(), ex) <= TOL["fp32"]
