@@ -674,3 +674,24 @@ def test_fp32_items_of_several_ragged_lists(mode, k, E, N):
         assert (m.sum(1) == (k if mode == "topk" else E)).all()
     ex = O.experts_ffn_exact(t["x"].reshape(N, d), m, t["w1"], t["b1"], t["w2"]) + t["last_bias"].double()
     assert O.rel_err(out.reshape(N, d).cpu(), ex) <= TOL["fp32"]
+
+
+@pytest.mark.parametrize("tau,N", [(0.02, 47 * 128), (0.02, 47 * 128 + 1), (0.0, 41 * 128), (0.0, 41 * 128 + 1),
+                                   (1.0, 111 * 128), (1.0, 111 * 128 + 1)])
+def test_who_writes_initial_rows_by_the_threshold(tau, N):
+    """The blocks without a tile write them up to a line that follows the threshold (no share of the tokens expected
+    to keep several experts, a small one, all): the layer on either side of it, on a device of 148 SMs."""
+    from d2dmoe_b200 import ops
+    E, R, d = 3, 16, 64
+    c, t = _layer(N, d, 16, E, R, "bf16", N)
+    x2d, wa, wb = _dev(t["x"].reshape(N, d)), _dev(t["wa"]), _dev(t["wb"])
+    w1, b1, w2, lb = _dev(t["w1"]), _dev(t["b1"]), _dev(t["w2"]), _dev(t["last_bias"].reshape(-1))
+    wsp = ops.Workspace.allocate(N, E, "cuda")
+    out = torch.full((N, d), float("nan"), dtype=torch.bfloat16, device="cuda")
+    ops.moe_forward(x2d, wa, wb, tau, w1, b1, w2, "relu", out, wsp, last_bias=lb, router_packed=ops.prepack_router(wa, wb),
+                    experts_packed=ops.prepack_experts(w1, b1, w2))
+    wsp.check_status()
+    m = O.unpack_mask(wsp.mask_bits[:N].cpu().numpy().view(np.uint32), E)
+    assert (m.sum(1) == E).all() if tau == 1.0 else (m.sum(1) >= 1).all()
+    ex = O.experts_ffn_exact(t["x"].reshape(N, d), m, t["w1"], t["b1"], t["w2"]) + t["last_bias"].double()
+    assert O.rel_err(out.cpu().float(), ex) <= TOL["bf16"]
