@@ -747,15 +747,19 @@ int launch_gate_scores_fused(const void* scores, int rule, int k, float tau, flo
     counts = mt.counts;
     lists->tabled = true;
   }
-  // Few tiles: blocks of their own, of some 16 rows, write every initial row while the rule is applied, which alone
-  // knows the rows that want one (as in the tensor-core router).  Layer of 24 experts on given scores, us, by
-  // the tiles' blocks / by others: 20 tokens 14.8 / 14.2, 180 17.3 / 14.2, 2000 24.7 / 19.8, 9000 27.7 / 23.8, 15 000
-  // 34.0 / 31.7, 18 000 (141 tiles) 34.7 / 33.2, 32 768 42.9 / 49.0; top-2, where all rows want one, 2000 35.6 / 20.4,
-  // 18 000 55 / 39.8.  Instances of their own: as a branch it cost
-  // the 32 768 tokens 0.7 us.  (One cluster: up to six more clusters.)
-  const int64_t more = fused ? grid * std::min<int64_t>((148 - grid) / grid, 6)
-                             : std::min<int64_t>(std::max<int64_t>(N / 16, 2 * 148), 4 * 148);
-  const bool others = out && rows_form && grid <= 148 && more > 0;
+  // No more tiles than SMs: blocks of their own (two to four per SM, of 16 rows between those; one cluster: up to six
+  // more clusters) write every initial row while the rule is applied, which alone knows the rows that want one (as in
+  // the tensor-core router, but with 8 to 24 experts of d = 256 to 2048 at mult 0.9 and 0.995 no size lost by it).
+  // Layer of 24 experts on given scores, us, by the tiles' blocks / by others: 20 tokens 14.8 / 14.2, 180 17.3 / 14.2,
+  // 2000 24.7 / 19.8, 9000 27.7 / 23.8, 15 000 34.0 / 31.7, 18 000 (141 tiles) 34.7 / 33.2, 32 768 42.9 / 49.0; nearly all
+  // tokens with one expert 18 011 32.3 / 31.4; residual 18 907 60.4 / 38.4; top-2, where all rows want one, 2000 35.6 / 20.4,
+  // 18 000 55 / 39.8.  Instances of their own: as a branch it cost the 32 768 tokens 0.7 us.
+  int sms = 0;
+  const int facts = device_launch_facts(nullptr, 0, &sms);
+  if (facts != D2D_OK) return facts;
+  const int64_t more = fused ? grid * std::min<int64_t>((sms - grid) / grid, 6)
+                             : std::min<int64_t>(std::max<int64_t>(N / 16, 2 * sms), 4 * sms);
+  const bool others = out && rows_form && grid <= sms && more > 0;
   const int64_t blocks = others ? grid + more : grid;
 #define D2D_ROWS_OF(T, NVV, RULE)                                                             \
   (others ? gate_scores_fused_rows_kernel<T, NVV, RULE, true>                                 \
