@@ -695,3 +695,69 @@ def test_who_writes_initial_rows_by_the_threshold(tau, N):
     assert (m.sum(1) == E).all() if tau == 1.0 else (m.sum(1) >= 1).all()
     ex = O.experts_ffn_exact(t["x"].reshape(N, d), m, t["w1"], t["b1"], t["w2"]) + t["last_bias"].double()
     assert O.rel_err(out.cpu().float(), ex) <= TOL["bf16"]
+
+
+@pytest.mark.parametrize("N", [18 * 128, 18 * 128 + 1, 74 * 128, 74 * 128 + 1])
+def test_initial_rows_at_the_other_lines(N):
+    """Every row from last_bias (ranked rules, the router's own call: 18 tiles) or with the layer's input added (74
+    tiles): the rows themselves, exactly, and top-k and dynk layers, on a device of 148 SMs."""
+    from d2dmoe_b200 import ops
+    import d2dmoe_b200 as D
+    E, R, d, H = 4, 16, 64, 16
+    c, t = _layer(N, d, H, E, R, "bf16", N)
+    x2d, wa, wb, lb = _dev(t["x"].reshape(N, d)), _dev(t["wa"]), _dev(t["wb"]), _dev(t["last_bias"].reshape(-1))
+    packed, wsp = ops.prepack_router(wa, wb), ops.Workspace.allocate(N, E, "cuda")
+    for residual in (False, True):
+        out = torch.full((N, d), float("nan"), dtype=torch.bfloat16, device="cuda")
+        ops.router_mask(x2d, wa, wb, 0.3, wsp, packed=packed, out_init=out, last_bias=lb, add_residual=residual)
+        wsp.check_status()
+        assert torch.equal(out, x2d + lb if residual else lb.expand(N, d))
+        for mode, k in (("topk", 1), ("topk", 3), ("dynk", 0)):
+            moe = D.MoeficationMoE("m", d, E, True, H, torch.nn.ReLU, add_residual_connection=residual)
+            moe.router = D.MoeficationRouter(d, E, width=R, depth=2, bias=False, activation="relu", output_activation="abs")
+            moe = moe.bfloat16()
+            moe.load_state_dict({"experts.w1": t["w1"], "experts.b1": t["b1"], "experts.w2": t["w2"],
+                                 "last_bias": t["last_bias"], "router.layers.0.weight": t["wa"],
+                                 "router.layers.2.weight": t["wb"]})
+            moe = moe.cuda().eval()
+            moe.forward_mode, moe.k, moe.tau = mode, k, 0.6
+            with torch.no_grad():
+                got, gating = moe(_dev(t["x"]))
+            m = gating["m"][0].reshape(N, E).cpu() > 0
+            ex = O.experts_ffn_exact(t["x"].reshape(N, d), m, t["w1"], t["b1"], t["w2"]) + t["last_bias"].double()
+            ex = ex + (t["x"].reshape(N, d).double() if residual else 0.0)
+            assert O.rel_err(got.reshape(N, d).cpu().float(), ex) <= TOL["bf16"], (mode, k, residual)
+
+
+@pytest.mark.parametrize("mode,k", [("topk", 1), ("topk", 3), ("dynk", 0)])
+@pytest.mark.parametrize("N", [1025, 18944, 18945])
+def test_initial_rows_beside_given_scores_of_ranked_rules(N, mode, k):
+    """The same for top-k and dynk on given scores: more than one cluster, either side of 148 tiles."""
+    import d2dmoe_b200 as D
+    E, d, H = 24, 64, 16
+    c, t = _layer(N, d, H, E, 16, "bf16", N)
+    scores = torch.rand(1, N, E, generator=_gen(N)).bfloat16()
+    sd = _dev(scores)
+
+    class Given(torch.nn.Module):
+        def forward(self, x):
+            return sd
+
+    for residual in (False, True):
+        moe = D.MoeficationMoE("m", d, E, True, H, torch.nn.ReLU, add_residual_connection=residual).bfloat16()
+        moe.load_state_dict({"experts.w1": t["w1"], "experts.b1": t["b1"], "experts.w2": t["w2"], "last_bias": t["last_bias"]},
+                            strict=False)
+        moe = moe.cuda().eval()
+        moe.router = Given()
+        moe.forward_mode, moe.k, moe.tau = mode, k, 0.2
+        with torch.no_grad():
+            got, gating = moe(_dev(t["x"]))
+        m = gating["m"][0].reshape(N, E).cpu() > 0
+        if mode == "topk":
+            # (equal scores may be taken in either order: what was taken is no less than what was left)
+            s = scores.reshape(N, E).float()
+            assert (m.sum(1) == k).all()
+            assert (s.masked_fill(~m, 2.0).amin(1) >= s.masked_fill(m, -1.0).amax(1)).all()
+        ex = O.experts_ffn_exact(t["x"].reshape(N, d), m, t["w1"], t["b1"], t["w2"]) + t["last_bias"].double()
+        ex = ex + (t["x"].reshape(N, d).double() if residual else 0.0)
+        assert O.rel_err(got.reshape(N, d).cpu().float(), ex) <= TOL["bf16"], residual
