@@ -5,10 +5,11 @@
 // fusing architectures/moe/moe_impls.py:93-180 (gathered first layer) and :244-301 (second layer +
 // atomic add); h never leaves the SM's tensor memory.
 //
-// What bounds it: latency, not a unit.  A hand-over from the tensor pipe to a waiting thread
-// (commit, mbarrier, wake-up) takes about 300 cycles and one back to the issuing thread as much
-// again; an M = 128, K = 16 instruction takes 64 cycles at N = 128, a role's wait, four of them and a
-// commit 280; the tensor pipe and DRAM are busy below 30 % of the time.  Hence
+// What bounds it: two chains of nearly the same length, no unit at its rate (the tensor pipe and DRAM are busy below
+// 30 % of the time).  For 128 output columns of a tile the drain takes 1850 cycles (see role_drain) and the products
+// 1450: an M = 128, K = 16 instruction takes 64 cycles at N = 128, but a role's wait, four of them and a
+// commit 280, and a hand-over from the tensor pipe to a waiting thread (commit, mbarrier, wake-up) about 300, one
+// back to the issuing thread as much again.  Hence
 //   * the hidden tile replaces accumulator 1 in place: the second product reads its A operand
 //     from tensor memory, and no shared memory is spent on it (rings of 160 + 48 KB);
 //   * two tiles are in work at once: the first product of one runs while the second product of
@@ -811,11 +812,14 @@ __device__ __forceinline__ void put_rows(uint32_t (&w)[2][2][4], const int* rt, 
 // each); W2's columns are packed in the order (out_column) that gives a lane eight neighbouring
 // ones of each 32-column block, and the lanes of two rows trade a block, so that eight of them have
 // 128 bytes of one row: whole lines leave an SM at 25 bytes per clock where they are added, half lines at
-// 20 (stored: 32 and 29; 148 CTAs, rows of 1536 bytes).  A transposition through shared memory took
-// 1250 cycles a step with nothing written, this 730 (950 where rows are stored as well).
-// What bounds a tile of the two-layer form is this role: 1850 cycles a 128-column step, some 1350 of them the
-// write path's backlog (26 bytes a clock and SM, rows stored and added mixed), 1550 with nothing else
-// travelling.  A register that spills here waits behind the writes.
+// 20 (stored: 32 and 29; 148 CTAs, rows of 1536 bytes).  A transposition through shared memory took 1.7 times as
+// long, alone and with nothing written.
+// A tile of the two-layer form is bound by this role, and close behind it by the products (1450 cycles): a
+// 128-column step takes 1850 cycles, 1700 with no rows and weights coming in, 1530 with nothing written, whether
+// those come in or not (vit_256; BERT's 1850, 1750, 1530).  Of the 1530 a warp spends 1080 on its own instructions,
+// 780 of them the exchanges and selections of put_rows, and 450 on the loop and the wait for the next
+// accumulator; writes add 280 to put_rows.  Rows leave at 18 bytes a clock and SM: 26, mixed, is the way's rate.
+// A register that spills here waits behind the writes.
 // DIRECT: rows of tokens with one expert are stored, see DirectRows
 template <bool GLU, bool NORM, bool DIRECT>
 __device__ void role_drain(const Params& p, Ctl* c, uint32_t tmem, int j, int q4, int lane) {

@@ -569,8 +569,8 @@ def test_initial_rows_of_a_residual_layer(N, d, bias):
 @pytest.mark.parametrize("bias", [True, False])
 @pytest.mark.parametrize("N,d", [(1, 64), (127, 768), (130, 2048), (1024, 64), (1025, 320), (14208, 64), (14209, 64)])
 def test_initial_rows_by_other_blocks(N, d, bias):
-    """last_bias in every row, exactly, from the blocks that have no tile (one tile, one cluster of eight, more;
-    either side of the rule's line at 111 tiles), and the layer over them."""
+    """last_bias in every row, exactly, of the router's own call (by the blocks that have no tile up to 18 tiles: one
+    tile, one cluster of eight, more), and the layer on either side of its line at 111 tiles."""
     from d2dmoe_b200 import ops
     E, R = 3, 16
     c, t = _layer(N, d, 16, E, R, "bf16", N + d)
