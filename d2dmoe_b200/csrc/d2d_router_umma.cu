@@ -1067,16 +1067,17 @@ int launch_router_mask_umma(const void* x, const void* packed, float mult, uint3
   // tokens with several experts alone: the line follows the share of tokens that may be expected to have
   // them, 1 - E^(-2 (1 - mult)) for normal scores (the gap of the two largest of E is exponential).  Layer, us,
   // by the tiles' own CTAs / by others; 24 experts at mult 0.9 (share 0.47): 197 tokens 19.4 / 17.4, 1100 24.3 / 21.0,
-  // 6304 28.1 / 26.0, 12 608 36.8 / 36.7, 14 171 (111 tiles) 37.5 / 37.7; at 0.95 (0.27): 11 483 (90) 32.6 / 31.5, 12 635
-  // (99) 33.4 / 34.2; at 0.995 (0.03): 5723 (45) 25.9 / 25.9, 9435 (74) 27.0 / 27.7, 14 171 30.0 / 31.9; 96 experts at 0.9
-  // (0.60): 14 171 45.7 / 44.5; 16 of d = 1536 at 0.9 (0.43): 12 635 58.9 / 57.8, 14 171 60.5 / 63.9; with 123 tiles
-  // 38.7 / 44.0.  Half of the SMs if the rows of x are read for them: 788 21.9 / 19.3, 9456 26.6 / 24.5, 12 608 29.1 / 29.7.
+  // 6304 28.1 / 26.0, 12 608 36.8 / 36.7, 14 171 (111 tiles) 37.7 / 37.9; at 0.95 (0.27): 11 483 (90) 30.2 / 29.2, 12 635
+  // (99) 30.6 / 31.3; at 0.995 (0.03): 5723 (45) 25.8 / 25.8, 9435 (74) 27.6 / 28.3, 14 171 30.2 / 32.3; 96 experts at 0.9
+  // (0.60): 14 171 45.7 / 44.5; 16 of d = 1536 at 0.9 (0.43): 12 635 58.9 / 57.8, 14 171 60.5 / 63.9; 16 of d = 4096 there:
+  // 11 483 116.0 / 112.7, 12 635 140.6 / 144.3 (longer rows, written twice, no longer stay in L2); with 123 tiles 38.7 /
+  // 44.0.  Half of the SMs if the rows of x are read for them: 788 21.9 / 19.3, 9456 26.6 / 24.5, 12 608 29.1 / 29.7.
   // An eighth where every row starts from last_bias (ranked rules: the tile's own warps write those before its
   // gate).  Top-k: 591 23.3 / 20.7, 985 26.9 / 24.5, 2167 27.1 / 26.5, 5319 35.0 / 35.3, 12 608 47.3 / 48.4.
   // (Short calls, one cluster: up to six more clusters, which are all there at once.)
   const int64_t more = p.token_idx ? tiles * std::min<int64_t>((sms - tiles) / tiles, 6) : sms - ctas;
   const double share = 1.0 - std::pow((double)E, -2.0 * (1.0 - mult));
-  const double line = resid ? 0.5 : init_all ? 0.125 : std::min(0.75, 0.28 + share);
+  const double line = resid ? 0.5 : init_all ? 0.125 : std::min(0.75, 0.3 + share - d / 65536.0);
   const bool help = out_init && more > 0 && (double)tiles <= line * sms;
   if (help) {
     p.help_init = p.out_init;

@@ -676,7 +676,7 @@ def test_fp32_items_of_several_ragged_lists(mode, k, E, N):
     assert O.rel_err(out.reshape(N, d).cpu(), ex) <= TOL["fp32"]
 
 
-@pytest.mark.parametrize("tau,N", [(0.02, 47 * 128), (0.02, 47 * 128 + 1), (0.0, 41 * 128), (0.0, 41 * 128 + 1),
+@pytest.mark.parametrize("tau,N", [(0.02, 50 * 128), (0.02, 50 * 128 + 1), (0.0, 44 * 128), (0.0, 44 * 128 + 1),
                                    (1.0, 111 * 128), (1.0, 111 * 128 + 1)])
 def test_who_writes_initial_rows_by_the_threshold(tau, N):
     """The blocks without a tile write them up to a line that follows the threshold (no share of the tokens expected
