@@ -677,10 +677,11 @@ def test_fp32_items_of_several_ragged_lists(mode, k, E, N):
 
 
 @pytest.mark.parametrize("tau,N", [(0.02, 50 * 128), (0.02, 50 * 128 + 1), (0.0, 44 * 128), (0.0, 44 * 128 + 1),
-                                   (1.0, 111 * 128), (1.0, 111 * 128 + 1)])
+                                   (1.0, 111 * 128), (1.0, 111 * 128 + 1), (-1.0, 20), (-1.0, 1024), (-1.0, 1025)])
 def test_who_writes_initial_rows_by_the_threshold(tau, N):
     """The blocks without a tile write them up to a line that follows the threshold (no share of the tokens expected
-    to keep several experts, a small one, all): the layer on either side of it, on a device of 148 SMs."""
+    to keep several experts, a small one, all; a threshold above the maximum, where no blocks help): the layer on either
+    side of it, on a device of 148 SMs."""
     from d2dmoe_b200 import ops
     E, R, d = 3, 16, 64
     c, t = _layer(N, d, 16, E, R, "bf16", N)
@@ -692,7 +693,7 @@ def test_who_writes_initial_rows_by_the_threshold(tau, N):
                     experts_packed=ops.prepack_experts(w1, b1, w2))
     wsp.check_status()
     m = O.unpack_mask(wsp.mask_bits[:N].cpu().numpy().view(np.uint32), E)
-    assert (m.sum(1) == E).all() if tau == 1.0 else (m.sum(1) >= 1).all()
+    assert (m.sum(1) == E).all() if tau == 1.0 else tau < 0 or (m.sum(1) >= 1).all()
     ex = O.experts_ffn_exact(t["x"].reshape(N, d), m, t["w1"], t["b1"], t["w2"]) + t["last_bias"].double()
     assert O.rel_err(out.cpu().float(), ex) <= TOL["bf16"]
 
